@@ -43,6 +43,7 @@ struct mdg_handle {
   long long steps_host = 0;  // completed steps as last read from the device
   long long launches = 0;    // kernels enqueued (counting every node of a graph replay)
   long long pending = 0;     // steps enqueued by mdg_calculate and not yet confirmed
+  int evaluations = 0;       // observations and force evaluations (launch_observe, launch_forces)
   bool ev1_due = false;      // the timing end event is recorded when the steps are confirmed
 };
 
@@ -93,7 +94,7 @@ void dfree_all(mdg_handle *h) {
   mdg::Dev &d = h->d;
   void *ptrs[] = {d.q_end, d.q_mid[0], d.q_mid[1], d.p, d.q_build, d.t_q, d.t_p, d.qf, d.loc[0], d.loc[1], d.id,
                   d.inv, d.cell, d.t_id, d.t_cell, d.order, d.cell_count, d.cell_fill, d.cell_start, d.block_sums,
-                  d.nl, d.ncount, d.pl, d.pcount, d.loc_p, d.partials, d.vpart, d.cand, d.flags, d.io4, d.io4b,
+                  d.nl, d.ncount, d.pl, d.pcount, d.loc_p, d.xq[0], d.xq[1], d.xb, d.xp, d.partials, d.vpart, d.cand, d.flags, d.io4, d.io4b,
                   h->dobs};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -193,6 +194,31 @@ int setup_geometry(mdg_handle *h) {
     g.half_prune2_ref = (float)(hp > 0.0 ? hp * hp * (1.0 - 1e-4) : 0.0);
   } else {
     g.half_prune2_ref = 3.0e38f;
+  }
+  // The FP64 form's pair arithmetic in fixed point: positions modulo 8 sigma,
+  // so two particles of a listed pair, each within fx_guard of its place at
+  // the build, must stay below 4 sigma apart on every axis, and the guard must
+  // leave room for the half margin that brings a rebuild.  A cut-off below
+  // one sigma would leave most pairs to the double expression.
+  g.fixed = p.precision == MDG_FP64 && sl + p.margin < 3.9 && p.cutoff >= 1.0 ? 1 : 0;
+  if (g.fixed) {
+    const double r2_hi = std::ldexp(1.0, mdg::kFixR2Bits - 32);
+    g.fx_rc2 = (uint64_t)std::ldexp(g.rc2, mdg::kFixR2Bits);
+    g.fx_near = (uint32_t)(mdg::kFixNear * r2_hi) + 1;
+    g.fx_keep = g.prune_thr2 < 16.0f ? (uint32_t)((double)g.prune_thr2 * r2_hi) + 1 : 0xFFFFFFFFu;
+    g.fx_c8 = mdg::fix_c8(g.c2x8);
+    for (int k = 0; k < 3; k++) {
+      const int64_t L = mdg::fix_from_double(p.box[k]);
+      g.fx_L[k] = mdg::fix_shi(L);
+      g.fx_l[k] = mdg::fix_rest(L);
+    }
+    g.fx_guard = (float)(0.5 * (4.0 - sl) - 1.0 / 64.0);
+    g.fx_moved_lo = (float)std::fmax(0.0, g.half_margin2 * (1.0 - 4e-6) - 1e-7);
+    g.fx_moved_hi = (float)(g.half_margin2 * (1.0 + 4e-6) + 1e-7);
+    const double pmax = std::fmin(2.9 / p.dt, 1e300);
+    uint64_t bits;
+    memcpy(&bits, &pmax, sizeof bits);
+    g.fx_pmax = (int)(bits >> 32);
   }
   return MDG_OK;
 }
@@ -603,7 +629,9 @@ int mdg_create(const mdg_params *p, mdg_handle **out) {
   h->cap = p->capacity;
   mdg::Dev &d = h->d;
   const size_t ncell = (size_t)h->g.nrank;
-  const size_t nred = (cap + 127) / 128 + 1;
+  // one partial sum per block: 128 particles each, or up to 2,048 smaller blocks (mdg_fixed.cu)
+  const size_t nred = (cap + 127) / 128 + 1 > 2048 ? (cap + 127) / 128 + 1 : 2048;
+  const size_t cap_fx = h->g.fixed ? cap : 0, cap_loc = h->g.fixed ? 0 : cap;
   if (e == cudaSuccess) e = dalloc(&d.q_end, cap);
   if (e == cudaSuccess) e = dalloc(&d.q_mid[0], cap);
   if (e == cudaSuccess) e = dalloc(&d.q_mid[1], cap);
@@ -612,9 +640,13 @@ int mdg_create(const mdg_params *p, mdg_handle **out) {
   if (e == cudaSuccess) e = dalloc(&d.t_q, cap);
   if (e == cudaSuccess) e = dalloc(&d.t_p, cap);
   if (e == cudaSuccess) e = dalloc(&d.qf, cap);
-  if (e == cudaSuccess) e = dalloc(&d.loc[0], cap);
-  if (e == cudaSuccess) e = dalloc(&d.loc[1], cap);
-  if (e == cudaSuccess) e = dalloc(&d.loc_p, cap);
+  if (e == cudaSuccess) e = dalloc(&d.loc[0], cap_loc);
+  if (e == cudaSuccess) e = dalloc(&d.loc[1], cap_loc);
+  if (e == cudaSuccess) e = dalloc(&d.loc_p, cap_loc);
+  if (e == cudaSuccess) e = dalloc(&d.xq[0], cap_fx);
+  if (e == cudaSuccess) e = dalloc(&d.xq[1], cap_fx);
+  if (e == cudaSuccess) e = dalloc(&d.xb, cap_fx);
+  if (e == cudaSuccess) e = dalloc(&d.xp, cap_fx);
   if (e == cudaSuccess) e = dalloc(&d.pcount, cap);
   if (e == cudaSuccess) e = dalloc(&d.id, cap);
   if (e == cudaSuccess) e = dalloc(&d.inv, cap);
@@ -945,8 +977,9 @@ int mdg_observe(mdg_handle *h, double out[3]) {
   if (!out) return fail(h, MDG_ERR_INVALID, "null output");
   rc = ensure_list(h, false);
   if (rc) return rc;
-  mdg::launch_observe(h->g, h->d, h->dobs, h->stream, h->prm.precision != MDG_FP64, h->par);
-  h->launches += h->prm.precision != MDG_FP64 ? 3 : 2;
+  mdg::launch_observe(h->g, h->d, h->dobs, h->stream, h->prm.precision != MDG_FP64, h->par,
+                      ++h->evaluations);
+  h->launches += h->prm.precision != MDG_FP64 || h->g.fixed ? 3 : 2;
   MDG_CK(cudaMemcpyAsync(h->hobs, h->dobs, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   MDG_CK(cudaStreamSynchronize(h->stream));
   out[0] = h->hobs[0];
@@ -961,8 +994,8 @@ int mdg_forces(mdg_handle *h, double *f4) {
   if (!f4) return fail(h, MDG_ERR_INVALID, "null output");
   rc = ensure_list(h, false);
   if (rc) return rc;
-  mdg::launch_forces(h->g, h->d, h->prm.precision, h->par, h->stream);
-  h->launches += h->prm.precision != MDG_FP64 ? 2 : 1;
+  mdg::launch_forces(h->g, h->d, h->prm.precision, h->par, ++h->evaluations, h->stream);
+  h->launches += h->prm.precision != MDG_FP64 || h->g.fixed ? 2 : 1;
   MDG_CK(cudaMemcpyAsync(f4, h->d.io4, (size_t)h->g.n * sizeof(double4_32a), cudaMemcpyDeviceToHost, h->stream));
   MDG_CK(cudaStreamSynchronize(h->stream));
   return MDG_OK;

@@ -201,6 +201,7 @@ __global__ void k_cell_sort(Geom g, Dev d) {
 
 __global__ void k_reorder(Geom g, Dev d) {
   if (rebuild_off(d.flags)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) d.flags->fx_wide[0] = d.flags->fx_wide[1] = 0;  // k_finalize sets them anew
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.n; k += gridDim.x * blockDim.x) {
     const int o = d.order[k];
     d.t_q[k] = d.q_end[o];
@@ -261,7 +262,16 @@ __global__ void k_finalize(Geom g, Dev d, int q_mid_dst) {
       m.y = __dadd_rn(q.y, __dmul_rn(p.y, g.dt2));
       m.z = __dadd_rn(q.z, __dmul_rn(p.z, g.dt2));
       q_mid[k] = m;
-      d.loc[q_mid_dst][k] = make_float4((float)(m.x - ox), (float)(m.y - oy), (float)(m.z - oz), cw);
+      if (g.fixed) {
+        d.xq[q_mid_dst][k] = fix_position(m.x, m.y, m.z, c);
+        const FixPos b = fix_position(q.x, q.y, q.z, c);
+        d.xb[k] = make_int4(b.x, b.y, b.z, c);
+        // the first half-drift must stay inside the modulus's guard too
+        const double far = fmax(fmax(fabs(p.x), fabs(p.y)), fabs(p.z)) * g.dt2;
+        if (!(far <= (double)g.fx_guard)) d.flags->fx_wide[q_mid_dst] = 1;
+      } else {
+        d.loc[q_mid_dst][k] = make_float4((float)(m.x - ox), (float)(m.y - oy), (float)(m.z - oz), cw);
+      }
     }
   }
 }

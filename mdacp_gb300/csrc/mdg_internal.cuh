@@ -22,6 +22,7 @@
 #include <stdint.h>
 
 #include "../../include/mdg.h"
+#include "mdg_fixed.cuh"
 
 namespace mdg {
 
@@ -77,6 +78,8 @@ struct DevFlags {
   double c_d2;                  // candidate threshold of the displacement check
   unsigned long long lifetime;  // steps since the build
   unsigned long long checks;    // displacement checks run
+  int fx_wide[2];               // fixed-point form: q_mid[k] holds a particle outside the modulus's guard
+  int fx_wide_end;              // the same for q_end, as the number of the call that found it
   int need_check;               // this step runs the displacement check
   int cand_count;               // candidate entries (particles and their images) found by it
   int cand_slots;               // candidate particles recorded
@@ -125,6 +128,16 @@ struct Geom {
   // candidate limit min(CheckListLength, n)
   int rebuild_policy, check_list;
   double margin, sl;  // margin, search length rc + margin
+  // FP64 form on fixed-point pair arithmetic (mdg_fixed.cuh for the units)
+  int fixed;
+  int fx_pmax;          // high word of the |p| component that moves 2.9 sigma in a step
+  uint32_t fx_near, fx_keep;  // high words of R: kFixNear, the inner-list radius
+  uint64_t fx_rc2;
+  int64_t fx_c8;
+  int fx_L[3];          // box sides as fixed-point positions: high words and rests
+  float fx_l[3];
+  float fx_guard;       // displacement since the build that keeps two particles' separations below 4
+  float fx_moved_lo, fx_moved_hi;  // band of the displacement^2 around half_margin2 tested in double
 };
 
 // Home-cell-local position (|x| < w per axis) packed into the bits of a
@@ -162,6 +175,8 @@ struct Dev {
   uint32_t *pl;         // inner list, same layout and capacity as nl
   int *pcount;
   float4 *loc_p;        // home-cell-local position at the last prune
+  FixPos *xq[2];        // FP64 form: fixed-point positions at q_mid[0] / q_mid[1], w the home cell
+  int4 *xb, *xp;        // their high words at the last build (w the home cell) and the last prune
   double *partials;     // reduction scratch
   int nblocks_red;
   double *vpart;        // reference rebuild policy: per-block maxima
@@ -197,8 +212,14 @@ void launch_nh_init(const Geom &g, const Dev &d, cudaStream_t s);
 constexpr int kPolicyKernels = 2, kPolicyCheckKernels = 4;
 void launch_policy(const Geom &g, const Dev &d, cudaStream_t s, cudaGraphConditionalHandle check_cond, int use_cond);
 void launch_policy_check(const Geom &g, const Dev &d, int par, cudaStream_t s);
-void launch_observe(const Geom &g, const Dev &d, double *out_dev, cudaStream_t s, int mixed, int par);
-void launch_forces(const Geom &g, const Dev &d, int mixed, int par, cudaStream_t s);
+// call: a number of its own for every observation or force evaluation of a handle
+void launch_observe(const Geom &g, const Dev &d, double *out_dev, cudaStream_t s, int mixed, int par, int call);
+void launch_forces(const Geom &g, const Dev &d, int mixed, int par, int call, cudaStream_t s);
+// The FP64 form with g.fixed (mdg_fixed.cu); the step and the observers
+// return the blocks that wrote partial sums.
+int launch_step_fixed(const Geom &g, const Dev &d, int par, int thermostat, int compat, int pmode, cudaStream_t s);
+int launch_observe_fixed(const Geom &g, const Dev &d, int par, int call, cudaStream_t s);
+void launch_forces_fixed(const Geom &g, const Dev &d, int par, int call, cudaStream_t s);
 void launch_unsort(const Geom &g, const Dev &d, int par, double4_32a *qo, double4_32a *po, cudaStream_t s);
 void launch_sort_in(const Geom &g, const Dev &d, const double4_32a *qi, const double4_32a *pi, cudaStream_t s);
 void launch_pairs(const Geom &g, const Dev &d, const long long *row_off, int32_t *rec, cudaStream_t s);

@@ -1,0 +1,122 @@
+"""The FP64 form on fixed-point pair arithmetic: the calls and states where it changes path, against the oracle.
+
+Lanes per particle change with the particle count (12,288 and 65,536); a pair
+closer than r^2 = 0.8425 and a row whose sums may overflow take the double
+expression; a particle that leaves the modulus's guard sends the step there;
+a cut-off below one sigma or a search length near 4 keeps the double kernel.
+Forces: |dF_i| <= 1e-12 max(|F_i|, sum |f_ij|), as the parity tests.
+"""
+import numpy as np
+import pytest
+
+from oracle import port
+from tests.helpers import liquid_like, pair_force_abs_sum
+
+pytestmark = pytest.mark.gpu
+
+
+def _manager(L, n, **kw):
+    from mdacp_gb300.manager import MDManager
+    kw.setdefault("cutoff", 2.5)
+    kw.setdefault("margin", 0.5)
+    return MDManager(L, capacity=n, **kw)
+
+
+def _check(q, p, L, steps=20, **kw):
+    ref = port.System(q, p, L, rc=kw.get("cutoff", 2.5), margin=kw.get("margin", 0.5), dt=kw.get("dt", 0.001),
+                      rebuild_policy=port.REBUILD_HALFMARGIN)
+    ref.make_pairlist()
+    fr = ref.forces()
+    scale = np.maximum(np.linalg.norm(fr, axis=1), pair_force_abs_sum(q, L, ref.pairs(), kw.get("cutoff", 2.5)))
+    m = _manager(L, len(q), **kw)
+    m.set_state(q, p)
+    f = m.forces()
+    assert np.all(np.linalg.norm(f - fr, axis=1) <= 1e-12 * scale + 1e-14)
+    obs = m.observe_raw()
+    np.testing.assert_allclose(obs, ref.observe_raw(), rtol=1e-12)
+    if steps:
+        ref.calculate(steps)
+        m.calculate(steps)
+        np.testing.assert_allclose(m.observe_raw(), ref.observe_raw(), rtol=1e-10)
+    return m
+
+
+# particle counts on both sides of the lane thresholds and of block edges
+@pytest.mark.parametrize("n", [500, 1001, 12287, 12288, 65535, 65537])
+def test_lane_counts(n):
+    cells = int(np.ceil((n / 4) ** (1 / 3)))
+    q, p, L = liquid_like(0.7, cells, amp=0.08, seed=n)
+    q, p = q[:n].copy(), p[:n] - p[:n].mean(axis=0)
+    _check(q, p, L, steps=10 if n < 20000 else 2)
+
+
+# 3.4 + 0.3 fits the modulus, 3.5 + 0.3 does not; a cut-off of 1.12 does, 0.9 does not
+@pytest.mark.parametrize("cutoff,margin", [(3.0, 0.3), (3.2, 0.3), (3.5, 0.3), (1.12, 0.3), (0.9, 0.3)])
+def test_cutoffs_on_both_paths(cutoff, margin):
+    q, p, L = liquid_like(0.6, 7, amp=0.05, seed=3)
+    m = _manager(L, len(q), cutoff=cutoff, margin=margin)
+    m.set_state(q, p)
+    ref = port.System(q, p, L, rc=cutoff, margin=margin, rebuild_policy=port.REBUILD_HALFMARGIN)
+    ref.make_pairlist()
+    fr = ref.forces()
+    assert np.abs(m.forces() - fr).max() <= 1e-12 * max(np.abs(fr).max(), 1.0)
+    m.calculate(30)
+    ref.calculate(30)
+    np.testing.assert_allclose(m.observe_raw(), ref.observe_raw(), rtol=1e-10, atol=1e-10)
+
+
+@pytest.mark.parametrize("r", [0.7, 0.9, 0.9178, 0.918, 0.93, 1.0])
+def test_close_pairs(r):
+    # pairs at distance r along different directions, across a face of the box too
+    L = np.array([14.0, 13.0, 12.0])
+    d = np.array([[1, 0, 0], [0, 1, 0], [0, 0, 1], [1, 1, 1], [-1, 2, 0.5]], dtype=float)
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    base = np.array([[13.8, 3, 3], [3, 12.9, 3], [3, 3, 0.1], [7, 7, 7], [10, 3, 8]])
+    q = np.mod(np.concatenate([base, base + r * d]), L)
+    _check(q, np.zeros_like(q), L, steps=0)
+
+
+def test_row_sums_beyond_the_integer_range():
+    # 40 partners crowded at 0.93 on one side of a particle: the sum of their forces passes 2^11
+    rng = np.random.default_rng(5)
+    u = np.array([1.0, 0.0, 0.0]) + 0.02 * rng.normal(size=(40, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    q = np.concatenate([[[5.0, 5.0, 5.0]], np.array([5.0, 5.0, 5.0]) + 0.93 * u, rng.uniform(8, 10, (5, 3))])
+    L = np.array([12.0, 12.0, 12.0])
+    m = _manager(L, len(q), list_capacity=64)
+    m.set_state(q, np.zeros_like(q))
+    ref = port.System(q, np.zeros_like(q), L, rc=2.5, margin=0.5)
+    ref.make_pairlist()
+    fr = ref.forces()[0]
+    assert np.abs(fr).max() > 2.0 ** 11
+    np.testing.assert_allclose(m.forces()[0], fr, rtol=1e-12, atol=1e-9)
+
+
+@pytest.mark.parametrize("speed", [300.0, 900.0, 3200.0])
+def test_fast_particle_leaves_the_guard(speed):
+    # one particle that crosses 0.3, 0.9 or 3.2 sigma a step: guard, rebuild every step, modulus
+    q, p, L = liquid_like(0.3, 5, amp=0.05, seed=9)
+    p[7] = [speed, -0.6 * speed, 0.3 * speed]
+    m = _manager(L, len(q))
+    m.set_state(q, p)
+    ref = port.System(q, p, L, rc=2.5, margin=0.5, rebuild_policy=port.REBUILD_HALFMARGIN)
+    ref.make_pairlist()
+    m.make_pairlist()
+    for _ in range(2):
+        m.calculate(1)
+        ref.calculate(1)
+    qm, pm = m.state()
+    qr, pr = ref.state()[:2]
+    np.testing.assert_allclose(pm, pr[:, :3], rtol=1e-9, atol=1e-9 * speed)
+
+
+def test_lanes_and_graphs_do_not_change_the_trajectory():
+    # the same steps through graphs and plain launches: bit for bit
+    q, p, L = liquid_like(0.8, 12, seed=2)
+    out = []
+    for graphs in (True, False):
+        m = _manager(L, len(q), use_graphs=graphs)
+        m.set_state(q, p)
+        m.calculate(60)
+        out.append(np.concatenate(m.state()))
+    assert np.array_equal(out[0], out[1])
