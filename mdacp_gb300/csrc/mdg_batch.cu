@@ -43,6 +43,10 @@ namespace batch {
 
 constexpr int kMaxCellsPerBox = 4096;  // cell counters and starts live in shared memory
 constexpr int kErrOverflow = 1, kErrBadState = 2;
+// Template value of the step kernels beside mdg_precision: the FP64 form on
+// fixed-point pair arithmetic (mdg_fixed.cuh), its state the FP64 form's.
+constexpr int kFixedForm = 3;
+__host__ __device__ constexpr bool is_mixed(int form) { return form == MDG_MIXED || form == MDG_MIXED_PLAIN; }
 
 struct BoxDesc {
   double L[3];
@@ -55,6 +59,8 @@ struct BoxDesc {
   int atom_off;
   long long list_off;  // first entry of the box in the list pool (n * cap entries)
   int cell_off;        // first cell start of the box (ncell + 1 entries)
+  int fx_L[3];         // box sides as fixed-point positions: high words and rests
+  float fx_l[3];
   int pad;
 };
 
@@ -77,6 +83,13 @@ struct Params {
   // the largest cell width
   int local_pos;
   float half_margin2_ref, half_prune2_ref;
+  // fixed-point form, as the single box's (Geom)
+  int fixed, fx_pmax, fx_pmax_end;
+  uint32_t fx_near, fx_keep;
+  uint64_t fx_rc2;
+  int64_t fx_c8;
+  float fx_guard, fx_moved_lo, fx_moved_hi;
+  double c2, c0;
 };
 
 struct Dev {
@@ -96,6 +109,10 @@ struct Dev {
   // mixed forms: -1 when the box's q_end is current, else the q_mid slot
   // (0 or 1) its last step wrote, from which q_end is formed when needed
   int *box_mid;
+  FixPos *xq[2];     // fixed-point form: positions at q_mid[0] / q_mid[1]
+  int4 *xb, *xp;     // their high words at the last build and the last selection
+  int *box_wide;     // [2][nbox]: q_mid[k] of the box holds a particle outside the guard
+  int *box_wide_end; // the same for the positions an observation reads
   double *partials;  // per box: KE, PE, virial
   const int *box_of_slot;
   // this step's rebuilding boxes in box order and their first atom in the
@@ -215,6 +232,7 @@ __device__ __forceinline__ int rb_find(const Dev &d, int nb, int t) {
 // component) and home cell.  A particle outside [-L, 2L) fails its box.
 __device__ void bin_particle(const Params &P, const Dev &d, const BoxDesc &b, int bi, int a) {
   const int o = b.atom_off;
+  if (P.fixed && a == 0) d.box_wide[bi] = d.box_wide[P.nbox + bi] = 0;  // place_particle sets them anew
   const int mid = d.box_mid[bi];
   double4_32a q = mid >= 0 ? box_end_from_mid(P, d, b, o + a, mid) : d.q_end[o + a];
   double x[3] = {q.x, q.y, q.z};
@@ -309,7 +327,15 @@ __device__ void place_particle(const Params &P, const Dev &d, const BoxDesc &b, 
     m.y = __dadd_rn(q.y, __dmul_rn(p.y, P.dt2));
     m.z = __dadd_rn(q.z, __dmul_rn(p.z, P.dt2));
     d.q_mid[par][o + k] = m;
-    d.loc[par][o + k] = make_float4((float)(m.x - ox), (float)(m.y - oy), (float)(m.z - oz), 0.0f);
+    if (P.fixed) {
+      d.xq[par][o + k] = fix_position(m.x, m.y, m.z, 0);
+      const FixPos x = fix_position(q.x, q.y, q.z, 0);
+      d.xb[o + k] = make_int4(x.x, x.y, x.z, 0);
+      // the first half-drift must stay inside the modulus's guard too
+      if (!(fmax(fmax(fabs(p.x), fabs(p.y)), fabs(p.z)) * P.dt2 <= (double)P.fx_guard)) d.box_wide[par * P.nbox + bi] = 1;
+    } else {
+      d.loc[par][o + k] = make_float4((float)(m.x - ox), (float)(m.y - oy), (float)(m.z - oz), 0.0f);
+    }
   }
   d.p[o + k] = p;
 }
@@ -478,15 +504,22 @@ __global__ void __launch_bounds__(128) k_batch_list(Params P, Dev d) {
   }
 }
 
-// Force on local particle a of box b from its row, lanes l = 0..LPI-1 of a group
-// taking every LPI-th entry; returns the group sum on every lane.  MODE 0 walks
-// the outer row; MODE 1 (one lane per particle) walks the outer row and, when
-// `select` is set, copies the entries within the inner radius to the inner row
-// (*kept: their number); MODE 2 walks the inner row.
-template <int MIXED, int LPI, int MODE>
-__device__ __forceinline__ double3 box_force(const Params &P, const Dev &d, const BoxDesc &b, int a, int lane, int par,
-                                             bool select = false, int *kept = nullptr) {
-  static_assert(MODE == 0 || LPI == 1, "the inner list is kept for one lane per particle");
+// Lane sums of the LPI lanes that share a particle (every lane holds them).
+template <int LPI>
+__device__ __forceinline__ double3 lane_sums(double fx, double fy, double fz) {
+#pragma unroll
+  for (int off = LPI / 2; off > 0; off >>= 1) {
+    fx += __shfl_xor_sync(0xffffffffu, fx, off, LPI);
+    fy += __shfl_xor_sync(0xffffffffu, fy, off, LPI);
+    fz += __shfl_xor_sync(0xffffffffu, fz, off, LPI);
+  }
+  return make_double3(fx, fy, fz);
+}
+
+// box_force in double.
+template <int LPI, int MODE>
+__device__ __forceinline__ double3 box_force_double(const Params &P, const Dev &d, const BoxDesc &b, int a, int lane, int par,
+                                                    bool select, int *kept) {
   const int o = b.atom_off, n = b.n;
   int cx, cy, cz;
   cell_xyz(b, d.cell[o + a], cx, cy, cz);
@@ -495,7 +528,170 @@ __device__ __forceinline__ double3 box_force(const Params &P, const Dev &d, cons
   uint32_t *prow = d.pl + b.list_off + a;
   int m = 0;
   double fx = 0.0, fy = 0.0, fz = 0.0;
-  if (MIXED) {
+  const double4_32a qi = d.q_mid[par][o + a];
+  const bool edge = cx == 0 || cy == 0 || cz == 0 || cx == b.nc[0] - 1 || cy == b.nc[1] - 1 || cz == b.nc[2] - 1;
+  for (int k = lane; k < cnt; k += LPI) {
+    const uint32_t e = __ldg(row + (long long)k * n);
+    double4_32a qj = ldg4(d.q_mid[par] + o + entry_slot(e));
+    if (edge) {
+      const int ox = entry_sx(e), oy = entry_sy(e), oz = entry_sz(e);
+      if (ox == 0 && cx == 0) qj.x -= b.L[0]; else if (ox == 2 && cx == b.nc[0] - 1) qj.x += b.L[0];
+      if (oy == 0 && cy == 0) qj.y -= b.L[1]; else if (oy == 2 && cy == b.nc[1] - 1) qj.y += b.L[1];
+      if (oz == 0 && cz == 0) qj.z -= b.L[2]; else if (oz == 2 && cz == b.nc[2] - 1) qj.z += b.L[2];
+    }
+    const double dx = qj.x - qi.x, dy = qj.y - qi.y, dz = qj.z - qi.z;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    // bit-pattern comparisons of r2 >= +0: the integer pipe, not the FP64 one
+    const long long r2_bits = __double_as_longlong(r2);
+    if (MODE == 1 && select && r2_bits <= __double_as_longlong(P.prune_thr2d)) prow[(long long)(m++) * n] = e;
+    if (r2_bits <= __double_as_longlong(P.rc2)) {
+      const double inv = rcp_hh3(r2);
+      const double i6 = inv * inv * inv;
+      const double df = (i6 * inv) * fma(-48.0, i6, 24.0) + P.c2x8;
+      fx = fma(df, dx, fx);
+      fy = fma(df, dy, fy);
+      fz = fma(df, dz, fz);
+    }
+  }
+  if (MODE == 1 && kept) *kept = m;
+  return lane_sums<LPI>(fx, fy, fz);
+}
+
+// The double force on one entry's pair (pairs closer than kFixNear).
+__device__ __noinline__ double3 near_pair(const Params &P, const Dev &d, const BoxDesc &b, const double4_32a *pos, int a, uint32_t e) {
+  const int o = b.atom_off;
+  int cx, cy, cz;
+  cell_xyz(b, d.cell[o + a], cx, cy, cz);
+  const double4_32a qi = pos[o + a];
+  double4_32a qj = pos[o + entry_slot(e)];
+  const int ox = entry_sx(e), oy = entry_sy(e), oz = entry_sz(e);
+  if (ox == 0 && cx == 0) qj.x -= b.L[0]; else if (ox == 2 && cx == b.nc[0] - 1) qj.x += b.L[0];
+  if (oy == 0 && cy == 0) qj.y -= b.L[1]; else if (oy == 2 && cy == b.nc[1] - 1) qj.y += b.L[1];
+  if (oz == 0 && cz == 0) qj.z -= b.L[2]; else if (oz == 2 && cz == b.nc[2] - 1) qj.z += b.L[2];
+  return make_double3(qj.x - qi.x, qj.y - qi.y, qj.z - qi.z);
+}
+
+// Walks every LPI-th entry of the row of local particle a from `lane` on over
+// fixed-point positions xq of the box's slots: pair(e, sep, R), one position
+// and two entries in flight.  In boxes of a few cells a side almost every
+// warp has a particle at a face, so the image shifts are always applied.
+template <int LPI, class Pair>
+__device__ __forceinline__ void walk_box(const BoxDesc &b, const FixPos *__restrict__ xq, int a, int cell, const uint32_t *__restrict__ row,
+                                         int cnt, int lane, Pair &&pair) {
+  const int n = b.n;
+  int cx, cy, cz;
+  cell_xyz(b, cell, cx, cy, cz);
+  // per axis: the step code (entry ^ 0x15: 1 = step -1, 3 = step +1) that crosses a face, 2 = none, and the shift
+  const uint32_t kx = cx == 0 ? 1u : (cx == b.nc[0] - 1 ? 3u : 2u), ky = (cy == 0 ? 1u : (cy == b.nc[1] - 1 ? 3u : 2u)) << 2,
+                 kz = (cz == 0 ? 1u : (cz == b.nc[2] - 1 ? 3u : 2u)) << 4;
+  const int sx = cx == 0 ? -b.fx_L[0] : b.fx_L[0], sy = cy == 0 ? -b.fx_L[1] : b.fx_L[1], sz = cz == 0 ? -b.fx_L[2] : b.fx_L[2];
+  const float tx = cx == 0 ? -b.fx_l[0] : b.fx_l[0], ty = cy == 0 ? -b.fx_l[1] : b.fx_l[1], tz = cz == 0 ? -b.fx_l[2] : b.fx_l[2];
+  const FixPos own = ld_fix(xq + a);
+  const uint32_t none = entry_pack(a, 0, 0, 0);  // a valid address past the row's end
+  auto entry = [&](int k) { return k < cnt ? __ldg(row + (long long)k * n) : none; };
+  uint32_t e0 = entry(lane), e1 = entry(lane + LPI);
+  FixPos q0 = ld_fix(xq + entry_slot(e0));
+#pragma unroll 2
+  for (int k = lane; k < cnt; k += LPI) {
+    const FixPos q1 = ld_fix(xq + entry_slot(e1));
+    const uint32_t e2 = entry(k + 2 * LPI);
+    int dx = q0.x - own.x, dy = q0.y - own.y, dz = q0.z - own.z;
+    float lx = q0.lx - own.lx, ly = q0.ly - own.ly, lz = q0.lz - own.lz;
+    const uint32_t s = e0 ^ 0x15u;
+    if ((s & 0x03u) == kx) { dx += sx; lx += tx; }
+    if ((s & 0x0Cu) == ky) { dy += sy; ly += ty; }
+    if ((s & 0x30u) == kz) { dz += sz; lz += tz; }
+    const FixSep sep = fix_sep(dx, dy, dz, lx, ly, lz);
+    pair(e0, sep, fix_r2(sep));
+    e0 = e1;
+    q0 = q1;
+    e1 = e2;
+  }
+}
+
+// box_force on the fixed-point positions, in units of 2^-52 (mdg_fixed.cu's
+// force_fixed for a box of the batch).
+template <int LPI, int MODE>
+__device__ __forceinline__ double3 box_force_fixed(const Params &P, const Dev &d, const BoxDesc &b, int bi, int a, int lane, int par,
+                                                   bool select, int *kept) {
+  const int o = b.atom_off, n = b.n;
+  const double up = (double)(1ull << kFixSumBits);
+  if (d.box_wide[par * P.nbox + bi]) {  // the same for the lanes of a particle
+    const double3 F = box_force_double<1, MODE>(P, d, b, a, 0, par, select, kept);
+    return make_double3(F.x * up, F.y * up, F.z * up);
+  }
+  const int cnt = MODE == 2 ? d.pcount[o + a] : d.ncount[o + a];
+  const uint32_t *row = (MODE == 2 ? d.pl : d.nl) + b.list_off + a;
+  uint32_t *prow = d.pl + b.list_off + a;
+  int m = 0;
+  FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f};
+  double nx = 0.0, ny = 0.0, nz = 0.0;
+  bool near = false;
+  walk_box<LPI>(b, d.xq[par] + o, a, d.cell[o + a], row, cnt, lane, [&](uint32_t e, const FixSep &sep, uint64_t R) {
+    if (MODE == 1 && select && fix_hi(R) <= P.fx_keep) prow[(long long)(m++) * n] = e;
+    const bool in = R <= P.fx_rc2, close = in && fix_hi(R) < P.fx_near;
+    int64_t df = fix_force(R, P.fx_c8);
+    df = in && !close ? df : 0;
+    fix_add(f, df, sep);
+    if (close) {
+      const double3 t = near_pair(P, d, b, d.q_mid[par], a, e);
+      const double inv = rcp_hh3(t.x * t.x + t.y * t.y + t.z * t.z), i6 = inv * inv * inv;
+      const double g = (i6 * inv) * fma(-48.0, i6, 24.0) + P.c2x8;
+      nx += g * t.x;
+      ny += g * t.y;
+      nz += g * t.z;
+      near = true;
+    }
+  });
+  if (MODE == 1 && kept) *kept = m;
+  if (LPI > 1) {
+#pragma unroll
+    for (int off = LPI / 2; off > 0; off >>= 1) {
+      f.x += __shfl_xor_sync(0xffffffffu, f.x, off, LPI);
+      f.y += __shfl_xor_sync(0xffffffffu, f.y, off, LPI);
+      f.z += __shfl_xor_sync(0xffffffffu, f.z, off, LPI);
+      f.mx += __shfl_xor_sync(0xffffffffu, f.mx, off, LPI);
+      f.my += __shfl_xor_sync(0xffffffffu, f.my, off, LPI);
+      f.mz += __shfl_xor_sync(0xffffffffu, f.mz, off, LPI);
+      f.cx += __shfl_xor_sync(0xffffffffu, f.cx, off, LPI);
+      f.cy += __shfl_xor_sync(0xffffffffu, f.cy, off, LPI);
+      f.cz += __shfl_xor_sync(0xffffffffu, f.cz, off, LPI);
+      f.s += __shfl_xor_sync(0xffffffffu, f.s, off, LPI);
+    }
+    const double3 t = lane_sums<LPI>(nx, ny, nz);
+    nx = t.x;
+    ny = t.y;
+    nz = t.z;
+    near = true;
+  }
+  double3 F = make_double3(fix_sum(f.x, f.mx, f.cx), fix_sum(f.y, f.my, f.cy), fix_sum(f.z, f.mz, f.cz));
+  if (near) F = make_double3(F.x + nx * up, F.y + ny * up, F.z + nz * up);
+  if (!fix_sum_fits(f, cnt)) {  // the row again in double
+    F = box_force_double<1, MODE == 1 ? 0 : MODE>(P, d, b, a, 0, par, false, nullptr);
+    F = make_double3(F.x * up, F.y * up, F.z * up);
+  }
+  return F;
+}
+
+// Force on local particle a of box b from its row, lanes l = 0..LPI-1 of a group
+// taking every LPI-th entry; returns the group sum on every lane.  MODE 0 walks
+// the outer row; MODE 1 (one lane per particle) walks the outer row and, when
+// `select` is set, copies the entries within the inner radius to the inner row
+// (*kept: their number); MODE 2 walks the inner row.
+template <int MIXED, int LPI, int MODE>
+__device__ __forceinline__ double3 box_force(const Params &P, const Dev &d, const BoxDesc &b, int bi, int a, int lane, int par,
+                                             bool select = false, int *kept = nullptr) {
+  static_assert(MODE == 0 || LPI == 1, "the inner list is kept for one lane per particle");
+  if constexpr (MIXED == kFixedForm) return box_force_fixed<LPI, MODE>(P, d, b, bi, a, lane, par, select, kept);
+  const int o = b.atom_off, n = b.n;
+  int cx, cy, cz;
+  cell_xyz(b, d.cell[o + a], cx, cy, cz);
+  const int cnt = MODE == 2 ? d.pcount[o + a] : d.ncount[o + a];
+  const uint32_t *row = (MODE == 2 ? d.pl : d.nl) + b.list_off + a;
+  uint32_t *prow = d.pl + b.list_off + a;
+  int m = 0;
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  if constexpr (is_mixed(MIXED)) {
     const float4 li = d.loc[par][o + a];
     const AxisQuad qx = axis_quad(b.w32[0], b.dl32[0], cx == 0, cx == b.nc[0] - 1, li.x, 1.0f);
     const AxisQuad qy = axis_quad(b.w32[1], b.dl32[1], cy == 0, cy == b.nc[1] - 1, li.y, 0.25f);
@@ -566,31 +762,7 @@ __device__ __forceinline__ double3 box_force(const Params &P, const Dev &d, cons
     fy = (double)(sy - cy_);
     fz = (double)(sz - cz_);
   } else {
-    const double4_32a qi = d.q_mid[par][o + a];
-    const bool edge = cx == 0 || cy == 0 || cz == 0 || cx == b.nc[0] - 1 || cy == b.nc[1] - 1 || cz == b.nc[2] - 1;
-    for (int k = lane; k < cnt; k += LPI) {
-      const uint32_t e = __ldg(row + (long long)k * n);
-      double4_32a qj = ldg4(d.q_mid[par] + o + entry_slot(e));
-      if (edge) {
-        const int ox = entry_sx(e), oy = entry_sy(e), oz = entry_sz(e);
-        if (ox == 0 && cx == 0) qj.x -= b.L[0]; else if (ox == 2 && cx == b.nc[0] - 1) qj.x += b.L[0];
-        if (oy == 0 && cy == 0) qj.y -= b.L[1]; else if (oy == 2 && cy == b.nc[1] - 1) qj.y += b.L[1];
-        if (oz == 0 && cz == 0) qj.z -= b.L[2]; else if (oz == 2 && cz == b.nc[2] - 1) qj.z += b.L[2];
-      }
-      const double dx = qj.x - qi.x, dy = qj.y - qi.y, dz = qj.z - qi.z;
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      // bit-pattern comparisons of r2 >= +0: the integer pipe, not the FP64 one
-      const long long r2_bits = __double_as_longlong(r2);
-      if (MODE == 1 && select && r2_bits <= __double_as_longlong(P.prune_thr2d)) prow[(long long)(m++) * n] = e;
-      if (r2_bits <= __double_as_longlong(P.rc2)) {
-        const double inv = rcp_hh3(r2);
-        const double i6 = inv * inv * inv;
-        const double df = (i6 * inv) * fma(-48.0, i6, 24.0) + P.c2x8;
-        fx = fma(df, dx, fx);
-        fy = fma(df, dy, fy);
-        fz = fma(df, dz, fz);
-      }
-    }
+    return box_force_double<LPI, MODE>(P, d, b, a, lane, par, select, kept);
   }
   if (MODE == 1 && kept) *kept = m;
   if (LPI > 1) {
@@ -604,20 +776,76 @@ __device__ __forceinline__ double3 box_force(const Params &P, const Dev &d, cons
   return make_double3(fx, fy, fz);
 }
 
+// The rest of advance_particle in the fixed-point form: the FP64 form's
+// drifts, the displacements tested in float on the positions' high words (the
+// rebuild test within 1e-6 of its threshold in double).
+template <bool INNER>
+__device__ __forceinline__ void advance_fixed(const Params &P, const Dev &d, int s, int bi, const double4_32a &p,
+                                              const double4_32a &q0, int par, bool sel, int kept, bool &rebuild,
+                                              bool &reselect) {
+  const double hx = __dmul_rn(p.x, P.dt2), hy = __dmul_rn(p.y, P.dt2), hz = __dmul_rn(p.z, P.dt2);
+  double4_32a qe = q0, q1 = q0;
+  qe.x = __dadd_rn(q0.x, hx);
+  qe.y = __dadd_rn(q0.y, hy);
+  qe.z = __dadd_rn(q0.z, hz);
+  q1.x = __dadd_rn(qe.x, hx);
+  q1.y = __dadd_rn(qe.y, hy);
+  q1.z = __dadd_rn(qe.z, hz);
+  const FixPos xn = fix_position(q1.x, q1.y, q1.z, 0);
+  const int4 xb = d.xb[s];
+  const float u = 1.0f / (float)(1 << (kFixPosBits - 32));
+  const float bx = (float)(xn.x - xb.x) * u, by = (float)(xn.y - xb.y) * u, bz = (float)(xn.z - xb.z) * u;
+  const float b2 = bx * bx + by * by + bz * bz;
+  const int m = 0x7fffffff;
+  const bool far = (__double2hiint(p.x) & m) >= P.fx_pmax || (__double2hiint(p.y) & m) >= P.fx_pmax ||
+                   (__double2hiint(p.z) & m) >= P.fx_pmax;  // or not a number
+  if (far || b2 > P.fx_moved_hi) {
+    rebuild = true;
+  } else if (b2 >= P.fx_moved_lo) {
+    const double4_32a qb = d.q_build[s];
+    const double ux = q1.x - qb.x, uy = q1.y - qb.y, uz = q1.z - qb.z;
+    if (ux * ux + uy * uy + uz * uz > P.half_margin2) rebuild = true;
+  }
+  if (far || fmaxf(fabsf(bx), fmaxf(fabsf(by), fabsf(bz))) > P.fx_guard) d.box_wide[(par ^ 1) * P.nbox + bi] = 1;
+  if (INNER) {
+    int4 xp;
+    if (sel) {
+      const FixPos x0 = d.xq[par][s];
+      xp = make_int4(x0.x, x0.y, x0.z, 0);
+      d.xp[s] = xp;
+      d.pcount[s] = kept;
+    } else {
+      xp = d.xp[s];
+    }
+    const float vx = (float)(xn.x - xp.x) * u, vy = (float)(xn.y - xp.y) * u, vz = (float)(xn.z - xp.z) * u;
+    if (vx * vx + vy * vy + vz * vz > P.half_prune2) reselect = true;
+  }
+  d.xq[par ^ 1][s] = xn;
+  d.p[s] = p;
+  d.q_end[s] = qe;
+  d.q_mid[par ^ 1][s] = q1;
+}
+
 // Kick, both half-drifts, the displacement and inner-list tests and the
 // stores of slot s after its force F (one lane per particle does this).
 template <int MIXED, bool INNER>
-__device__ __forceinline__ void advance_particle(const Params &P, const Dev &d, const BoxDesc &b, int s,
+__device__ __forceinline__ void advance_particle(const Params &P, const Dev &d, const BoxDesc &b, int bi, int s,
                                                  const double3 &F, int par, bool sel, int kept, bool &rebuild,
                                                  bool &reselect) {
   const bool inner = INNER;
   double4_32a p = d.p[s];
-  p.x += F.x * P.dt;
-  p.y += F.y * P.dt;
-  p.z += F.z * P.dt;
+  // the fixed-point form's F is in units of 2^-52
+  const double dts = MIXED == kFixedForm ? P.dt * (1.0 / (double)(1ull << kFixSumBits)) : P.dt;
+  p.x += F.x * dts;
+  p.y += F.y * dts;
+  p.z += F.z * dts;
   const double4_32a q0 = d.q_mid[par][s];
   double4_32a qe = q0, q1 = q0;
   float4 ln;
+  if constexpr (MIXED == kFixedForm) {
+    advance_fixed<INNER>(P, d, s, bi, p, q0, par, sel, kept, rebuild, reselect);
+    return;
+  }
   if (MIXED) {
     // as the single-box mixed form: one rounding per half-drift (fused) on
     // home-cell-local positions, the new local position one conversion, the
@@ -682,7 +910,7 @@ __device__ __forceinline__ void advance_particle(const Params &P, const Dev &d, 
 #define MDG_BATCH_MIN_BLOCKS 2
 #endif
 template <int MIXED, int LPI, int INNER>
-__global__ void __launch_bounds__(512, MIXED ? MDG_BATCH_MIN_BLOCKS : 2) k_batch_step(Params P, Dev d, int par) {
+__global__ void __launch_bounds__(512, MIXED == kFixedForm ? 1 : (MIXED ? MDG_BATCH_MIN_BLOCKS : 2)) k_batch_step(Params P, Dev d, int par) {
   __shared__ int s_flag[3];
   const long long goal = *d.goal;
   static_assert(INNER == 0 || LPI == 1, "the inner list is kept for one lane per particle");
@@ -715,20 +943,20 @@ __global__ void __launch_bounds__(512, MIXED ? MDG_BATCH_MIN_BLOCKS : 2) k_batch
       double3 F;
       int kept = 0;
       if constexpr (INNER != 0) {
-        if (sel) F = box_force<MIXED, 1, 1>(P, d, b, a, lane, par, a0 < n, &kept);
-        else F = box_force<MIXED, 1, 2>(P, d, b, a, lane, par);
+        if (sel) F = box_force<MIXED, 1, 1>(P, d, b, bi, a, lane, par, a0 < n, &kept);
+        else F = box_force<MIXED, 1, 2>(P, d, b, bi, a, lane, par);
       } else {
-        F = box_force<MIXED, LPI, 0>(P, d, b, a, lane, par);
+        F = box_force<MIXED, LPI, 0>(P, d, b, bi, a, lane, par);
       }
       if (lane != 0 || a0 >= n) continue;
-      advance_particle<MIXED, inner>(P, d, b, o + a, F, par, sel, kept, rebuild, reselect);
+      advance_particle<MIXED, inner>(P, d, b, bi, o + a, F, par, sel, kept, rebuild, reselect);
     }
     const int any = __syncthreads_or(rebuild ? 1 : 0);
     const int anyp = __syncthreads_or(reselect ? 1 : 0);
     if (threadIdx.x == 0) {
       if (any) d.box_rebuild[bi] = 1;
       if (inner) d.box_prune[bi] = anyp;
-      if (MIXED) d.box_mid[bi] = par ^ 1;
+      if (is_mixed(MIXED)) d.box_mid[bi] = par ^ 1;
       d.box_steps[bi] += 1;
     }
     __syncthreads();
@@ -752,9 +980,12 @@ __global__ void __launch_bounds__(512, MIXED ? MDG_BATCH_MIN_BLOCKS : 2) k_batch
 #ifndef MDG_BATCH_FLAT_MIN_BLOCKS
 #define MDG_BATCH_FLAT_MIN_BLOCKS 4
 #endif
+// The fixed-point form's: 2 (128 registers, no spills) 0.255 ms per step of 48
+// boxes (205,044 atoms, observed every 100), 3 (80, 60 bytes spilled) 0.295.
+constexpr int kFlatFixedBlocks = 2;
 constexpr int kFlatMaxThreads = 256;
 template <int MIXED, int INNER>
-__global__ void __launch_bounds__(kFlatMaxThreads, MDG_BATCH_FLAT_MIN_BLOCKS) k_batch_step_flat(Params P, Dev d,
+__global__ void __launch_bounds__(kFlatMaxThreads, MIXED == kFixedForm ? kFlatFixedBlocks : MDG_BATCH_FLAT_MIN_BLOCKS) k_batch_step_flat(Params P, Dev d,
                                                                                             int par) {
   const long long goal = *d.goal;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < P.total; s += gridDim.x * blockDim.x) {
@@ -766,13 +997,13 @@ __global__ void __launch_bounds__(kFlatMaxThreads, MDG_BATCH_FLAT_MIN_BLOCKS) k_
     double3 F;
     int kept = 0;
     if constexpr (INNER != 0) {
-      if (sel) F = box_force<MIXED, 1, 1>(P, d, b, a, 0, par, true, &kept);
-      else F = box_force<MIXED, 1, 2>(P, d, b, a, 0, par);
+      if (sel) F = box_force<MIXED, 1, 1>(P, d, b, bi, a, 0, par, true, &kept);
+      else F = box_force<MIXED, 1, 2>(P, d, b, bi, a, 0, par);
     } else {
-      F = box_force<MIXED, 1, 0>(P, d, b, a, 0, par);
+      F = box_force<MIXED, 1, 0>(P, d, b, bi, a, 0, par);
     }
     bool rebuild = false, reselect = false;
-    advance_particle<MIXED, INNER != 0>(P, d, b, s, F, par, sel, kept, rebuild, reselect);
+    advance_particle<MIXED, INNER != 0>(P, d, b, bi, s, F, par, sel, kept, rebuild, reselect);
     if (rebuild) d.box_req[bi] = 1;
     if (INNER != 0 && reselect) d.box_preq[bi] = 1;
   }
@@ -802,53 +1033,99 @@ __global__ void k_batch_finish(Params P, Dev d, int par) {
   d.box_steps[bi] += 1;
 }
 
-// Per-box observer sums at q_end (observer.cc:5-79 expressions, pairs 1/2 each).
-__global__ void k_batch_observe(Params P, Dev d) {
-  __shared__ double sh[3][32];
-  const int bi = blockIdx.x;
-  const BoxDesc b = d.boxes[bi];
+// Observers (observer.cc:5-79) at q_end, pairs weighted 1/2 (each is listed
+// from both sides): block (c, box) sums the box's particles c kT .. c kT + kT - 1,
+// k_batch_observe_final adds a box's blocks in order.  With P.fixed the pair
+// sums are the integers of mdg_fixed.cu's observe_fixed over the fixed-point
+// positions in t_q (k_batch_fix_end), in the double expressions otherwise.
+constexpr int kObserveThreads = 256;
+constexpr int kObserveBoxes = 32768;  // boxes a launch (the grid's second dimension ends at 65,535)
+
+// Fixed-point positions of q_end into the reorder staging t_q (free outside
+// rebuilds).  A momentum that may have carried its particle too far from its
+// place at the build for the modulus marks the box: every particle was within
+// margin / 2 at the last mid-step, and moved p dt / 2 since.
+__global__ void k_batch_fix_end(Params P, Dev d) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= P.total) return;
+  const double4_32a q = d.q_end[s], p = d.p[s];
+  reinterpret_cast<FixPos *>(d.t_q)[s] = fix_position(q.x, q.y, q.z, 0);
+  const int m = 0x7fffffff;
+  if ((__double2hiint(p.x) & m) >= P.fx_pmax_end || (__double2hiint(p.y) & m) >= P.fx_pmax_end ||
+      (__double2hiint(p.z) & m) >= P.fx_pmax_end)
+    d.box_wide_end[d.box_of_slot[s]] = 1;
+}
+
+// A pair's energy and virial term in double at separation t, weighted 1/2.
+__device__ __forceinline__ void pair_observables(const Params &P, const double3 &t, double &pe, double &vir) {
+  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(t.x, t.x), __dmul_rn(t.y, t.y)), __dmul_rn(t.z, t.z));
+  if (r2 > P.rc2) return;
+  const double r4 = __dmul_rn(r2, r2), r6 = __dmul_rn(r4, r2), r8 = __dmul_rn(r6, r2), r10 = __dmul_rn(r8, r2),
+               r12 = __dmul_rn(r10, r2);
+  pe += 0.5 * (4.0 * (1.0 / r12 - 1.0 / r6 + __dmul_rn(P.c2, r2) + P.c0));
+  vir += 0.5 * ((__dsub_rn(__dmul_rn(24.0, r6), 48.0) / (__dmul_rn(__dmul_rn(r6, r6), r2)) + P.c2x8) * r2);
+}
+
+// Longest row whose integer sums fit (mdg_fixed.cu).
+constexpr int kFixObserveRow = 361;
+
+__global__ void __launch_bounds__(kObserveThreads) k_batch_observe(Params P, Dev d, double *part, int first) {
+  __shared__ double sh[3][kObserveThreads / 32];
+  const int bi = first + blockIdx.y;
+  const BoxDesc &b = d.boxes[bi];
   const int o = b.atom_off, n = b.n;
-  double ke = 0.0, pe = 0.0, vir = 0.0;
-  for (int a = threadIdx.x; a < n; a += blockDim.x) {
+  if (blockIdx.x * kObserveThreads >= n) return;
+  const int a = blockIdx.x * kObserveThreads + threadIdx.x;
+  double v[3] = {0.0, 0.0, 0.0};
+  if (a < n) {
     const double4_32a p = d.p[o + a];
-    ke += 0.5 * p.x * p.x + 0.5 * p.y * p.y + 0.5 * p.z * p.z;  // w is padding
-    const double4_32a qi = d.q_end[o + a];
-    int cx, cy, cz;
-    cell_xyz(b, d.cell[o + a], cx, cy, cz);
+    v[0] = 0.5 * p.x * p.x + 0.5 * p.y * p.y + 0.5 * p.z * p.z;  // w is padding
     const int cnt = d.ncount[o + a];
-    for (int k = 0; k < cnt; k++) {
-      const uint32_t e = d.nl[b.list_off + (long long)k * n + a];
-      double4_32a qj = d.q_end[o + entry_slot(e)];
-      const int ox = entry_sx(e), oy = entry_sy(e), oz = entry_sz(e);
-      if (ox == 0 && cx == 0) qj.x -= b.L[0]; else if (ox == 2 && cx == b.nc[0] - 1) qj.x += b.L[0];
-      if (oy == 0 && cy == 0) qj.y -= b.L[1]; else if (oy == 2 && cy == b.nc[1] - 1) qj.y += b.L[1];
-      if (oz == 0 && cz == 0) qj.z -= b.L[2]; else if (oz == 2 && cz == b.nc[2] - 1) qj.z += b.L[2];
-      const double dx = __dsub_rn(qi.x, qj.x), dy = __dsub_rn(qi.y, qj.y), dz = __dsub_rn(qi.z, qj.z);
-      const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-      if (r2 > P.rc2) continue;
-      const double r4 = __dmul_rn(r2, r2), r6 = __dmul_rn(r4, r2), r8 = __dmul_rn(r6, r2), r10 = __dmul_rn(r8, r2),
-                   r12 = __dmul_rn(r10, r2);
-      const double c2 = P.c2x8 / 8.0;
-      const double c0 = -1.0 / (P.rc2 * P.rc2 * P.rc2 * P.rc2 * P.rc2 * P.rc2) + 1.0 / (P.rc2 * P.rc2 * P.rc2) -
-                        c2 * P.rc2;
-      pe += 0.5 * (4.0 * (1.0 / r12 - 1.0 / r6 + __dmul_rn(c2, r2) + c0));
-      vir += 0.5 * ((__dsub_rn(__dmul_rn(24.0, r6), 48.0) / (__dmul_rn(__dmul_rn(r6, r6), r2)) + P.c2x8) * r2);
+    const uint32_t *row = d.nl + b.list_off + a;
+    if (P.fixed && cnt <= kFixObserveRow && d.box_wide_end[bi] == 0) {
+      uint64_t sz = 0, szz = 0, sr = 0;
+      int m = 0;
+      walk_box<1>(b, reinterpret_cast<const FixPos *>(d.t_q) + o, a, d.cell[o + a], row, cnt, 0,
+                  [&](uint32_t e, const FixSep &, uint64_t R) {
+                    const bool in = R <= P.fx_rc2, close = in && fix_hi(R) < P.fx_near, take = in && !close;
+                    uint64_t y2, z;
+                    fix_powers(fix_recip(R), y2, z);
+                    const uint64_t zz = fix_sqrhi(z);
+                    sz += take ? z >> 7 : 0;
+                    szz += take ? zz >> 4 : 0;
+                    sr += take ? R >> 7 : 0;
+                    m += take ? 1 : 0;
+                    if (close) pair_observables(P, near_pair(P, d, b, d.q_end, a, e), v[1], v[2]);
+                  });
+      const double u = 1.0 / (double)(1ull << 54), half = 0.5 * m;
+      const double z = ((double)sz + half) * u, zz = ((double)szz + half) * u;
+      const double r = P.c2 * (((double)sr + half) * (1.0 / (double)(1ull << 51)));
+      v[1] += 2.0 * ((zz - z) + (r + P.c0 * (double)m));
+      v[2] += 12.0 * (z - 2.0 * zz) + 4.0 * r;
+    } else {
+      for (int k = 0; k < cnt; k++) pair_observables(P, near_pair(P, d, b, d.q_end, a, row[(long long)k * n]), v[1], v[2]);
     }
   }
-  double v[3] = {ke, pe, vir};
   for (int k = 0; k < 3; k++)
     for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
   if ((threadIdx.x & 31) == 0)
     for (int k = 0; k < 3; k++) sh[k][threadIdx.x >> 5] = v[k];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t[3] = {0, 0, 0};
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++)
-      for (int k = 0; k < 3; k++) t[k] += sh[k][w];
-    d.partials[3 * bi + 0] = t[0];
-    d.partials[3 * bi + 1] = t[1];
-    d.partials[3 * bi + 2] = t[2] / 3.0;
+  if (threadIdx.x < 3) {
+    double t = 0.0;
+    for (int w = 0; w < kObserveThreads / 32; w++) t += sh[threadIdx.x][w];
+    part[3 * ((long long)bi * gridDim.x + blockIdx.x) + threadIdx.x] = t;
   }
+}
+
+__global__ void k_batch_observe_final(Params P, Dev d, const double *part, int chunks) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x, bi = k / 3, c = k % 3;
+  if (bi >= P.nbox) return;
+  const int used = (d.boxes[bi].n + kObserveThreads - 1) / kObserveThreads;
+  double t = 0.0;
+  for (int j = 0; j < used; j++) t += part[3 * ((long long)bi * chunks + j) + c];
+  d.partials[3 * bi + c] = c == 2 ? t / 3.0 : t;
+  if (c == 0) d.box_wide_end[bi] = 0;  // the next observation marks anew
 }
 
 // The caller's arrays in the caller's order; the fourth lane is padding and
@@ -915,6 +1192,8 @@ struct mdg_batch {
   double last_ms = 0.0;
   long long launches = 0;
   int grid = 0;
+  int chunks = 0;              // blocks of the largest box in an observation
+  double *obs_part = nullptr;  // their sums, [nbox][chunks][3]
 };
 
 namespace {
@@ -947,6 +1226,8 @@ cudaError_t balloc(T **p, size_t count) {
 // The persistent step kernel the shape selects (as launch_batch_step does).
 const void *step_kernel_fn(int prec, int lpi, bool inner, bool flat) {
   if (flat) {
+    if (prec == kFixedForm) return inner ? reinterpret_cast<const void *>(&k_batch_step_flat<kFixedForm, 1>)
+                                         : reinterpret_cast<const void *>(&k_batch_step_flat<kFixedForm, 0>);
     if (prec == MDG_MIXED) return inner ? reinterpret_cast<const void *>(&k_batch_step_flat<MDG_MIXED, 1>)
                                         : reinterpret_cast<const void *>(&k_batch_step_flat<MDG_MIXED, 0>);
     if (prec == MDG_MIXED_PLAIN)
@@ -956,6 +1237,9 @@ const void *step_kernel_fn(int prec, int lpi, bool inner, bool flat) {
                  : reinterpret_cast<const void *>(&k_batch_step_flat<MDG_FP64, 0>);
   }
 #define MDG_BFN(M, L, I) reinterpret_cast<const void *>(&k_batch_step<M, L, I>)
+  if (prec == kFixedForm)
+    return lpi == 4 ? MDG_BFN(kFixedForm, 4, 0) : lpi == 2 ? MDG_BFN(kFixedForm, 2, 0)
+           : inner  ? MDG_BFN(kFixedForm, 1, 1) : MDG_BFN(kFixedForm, 1, 0);
   if (prec == MDG_MIXED)
     return lpi == 4 ? MDG_BFN(MDG_MIXED, 4, 0) : lpi == 2 ? MDG_BFN(MDG_MIXED, 2, 0)
            : inner  ? MDG_BFN(MDG_MIXED, 1, 1) : MDG_BFN(MDG_MIXED, 1, 0);
@@ -967,13 +1251,16 @@ const void *step_kernel_fn(int prec, int lpi, bool inner, bool flat) {
 #undef MDG_BFN
 }
 
+// The step kernels' template value for this batch.
+int step_form(const mdg_batch *b) { return b->prm.precision == MDG_FP64 && b->P.fixed ? kFixedForm : b->prm.precision; }
+
 // CTAs of `threads` threads of the selected step kernel that fit on one SM
 // at once (registers, shared memory, thread slots): the persistent kernel's
 // grid must not exceed this, or its CTAs run in waves.
 int resident_ctas(const mdg_batch *b, int threads) {
   const bool inner = b->P.inner && b->lpi == 1 && b->use_inner;
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, step_kernel_fn(b->prm.precision, b->lpi, inner, b->flat != 0),
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, step_kernel_fn(step_form(b), b->lpi, inner, b->flat != 0),
                                                     threads,
                                                     0) != cudaSuccess)
     return 1;
@@ -988,6 +1275,7 @@ void set_prune_buffer(mdg_batch *b, double buffer) {
   P.prune_thr2d = rb * rb;
   P.prune_thr2f = (float)(rb * rb + 1e-4);  // float r2 of local positions is within ~1e-5
   P.half_prune2 = (float)(0.25 * buffer * buffer * (1.0 - 1e-4));
+  P.fx_keep = P.prune_thr2f < 16.0f ? (uint32_t)((double)P.prune_thr2f * (double)(1u << (mdg::kFixR2Bits - 32))) + 1 : 0xFFFFFFFFu;
   const double hp = 0.5 * buffer - 2.0 * b->ref_unit;
   P.half_prune2_ref = buffer > 0.0 ? (float)(hp > 0.0 ? hp * hp * (1.0 - 1e-4) : 0.0) : 3.0e38f;
   b->buffer = buffer;
@@ -1060,7 +1348,7 @@ int alloc_batch_list(mdg_batch *b, int cap) {
 
 void launch_batch_step(mdg_batch *b, int par) {
   const int T = b->threads;
-  const int prec = b->prm.precision;
+  const int prec = step_form(b);
   k_batch_rebuild_set<<<1, 1024, 0, b->stream>>>(b->P, b->d);
   k_batch_bin<<<b->num_sms * 16, 128, 0, b->stream>>>(b->P, b->d);
   k_batch_sort<<<b->nbox, kPrepThreads, 0, b->stream>>>(b->d);
@@ -1070,7 +1358,8 @@ void launch_batch_step(mdg_batch *b, int par) {
   const bool inner = b->P.inner && b->lpi == 1 && b->use_inner;
   if (b->flat) {
 #define MDG_FSTEP(M, I) k_batch_step_flat<M, I><<<b->grid, T, 0, b->stream>>>(b->P, b->d, par)
-    if (prec == MDG_MIXED) { if (inner) MDG_FSTEP(MDG_MIXED, 1); else MDG_FSTEP(MDG_MIXED, 0); }
+    if (prec == kFixedForm) { if (inner) MDG_FSTEP(kFixedForm, 1); else MDG_FSTEP(kFixedForm, 0); }
+    else if (prec == MDG_MIXED) { if (inner) MDG_FSTEP(MDG_MIXED, 1); else MDG_FSTEP(MDG_MIXED, 0); }
     else if (prec == MDG_MIXED_PLAIN) { if (inner) MDG_FSTEP(MDG_MIXED_PLAIN, 1); else MDG_FSTEP(MDG_MIXED_PLAIN, 0); }
     else { if (inner) MDG_FSTEP(MDG_FP64, 1); else MDG_FSTEP(MDG_FP64, 0); }
 #undef MDG_FSTEP
@@ -1080,7 +1369,10 @@ void launch_batch_step(mdg_batch *b, int par) {
     b->launches += kBatchKernelsPerStep + 1;
     return;
   }
-  if (prec == MDG_MIXED) {
+  if (prec == kFixedForm) {
+    if (b->lpi == 4) MDG_BSTEP(kFixedForm, 4, 0); else if (b->lpi == 2) MDG_BSTEP(kFixedForm, 2, 0);
+    else if (inner) MDG_BSTEP(kFixedForm, 1, 1); else MDG_BSTEP(kFixedForm, 1, 0);
+  } else if (prec == MDG_MIXED) {
     if (b->lpi == 4) MDG_BSTEP(MDG_MIXED, 4, 0); else if (b->lpi == 2) MDG_BSTEP(MDG_MIXED, 2, 0);
     else if (inner) MDG_BSTEP(MDG_MIXED, 1, 1); else MDG_BSTEP(MDG_MIXED, 1, 0);
   } else if (prec == MDG_MIXED_PLAIN) {
@@ -1207,7 +1499,6 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   P.rc2 = p->cutoff * p->cutoff;
   const double s2 = 1.0 / P.rc2, s6 = s2 * s2 * s2, s8 = s6 * s2, s12 = s6 * s6, s14 = s12 * s2;
   P.c2x8 = (6.0 * s14 - 3.0 * s8) * 8.0;
-  (void)s12;
   P.c2x8f = (float)P.c2x8;
   P.rc2f = (float)P.rc2;
   P.acc_lo = (float)(sl * sl - 1e-4);
@@ -1218,6 +1509,36 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   P.nbox = nbox;
   P.total = (int)total;
   P.local_pos = p->precision != MDG_FP64 ? 1 : 0;
+  P.c2 = P.c2x8 / 8.0;
+  P.c0 = -s12 + s6 - P.c2 * P.rc2;
+  // Pair arithmetic in fixed point where two particles of a listed pair, each
+  // within the guard of its place at the build, stay below 4 sigma apart (as
+  // the single box, setup_geometry in mdg_api.cu); the FP64 form's steps and
+  // every form's observers.
+  P.fixed = sl + p->margin < 3.9 && p->cutoff >= 1.0 ? 1 : 0;
+  if (P.fixed) {
+    const double r2_hi = (double)(1u << (mdg::kFixR2Bits - 32));
+    P.fx_rc2 = (uint64_t)std::ldexp(P.rc2, mdg::kFixR2Bits);
+    P.fx_near = (uint32_t)(mdg::kFixNear * r2_hi) + 1;
+    P.fx_c8 = mdg::fix_c8(P.c2x8);
+    P.fx_guard = (float)(0.5 * (4.0 - sl) - 1.0 / 64.0);
+    P.fx_moved_lo = (float)std::fmax(0.0, P.half_margin2 * (1.0 - 4e-6) - 1e-7);
+    P.fx_moved_hi = (float)(P.half_margin2 * (1.0 + 4e-6) + 1e-7);
+    auto high = [](double v) {
+      v = std::fmin(v, 1e300);
+      uint64_t bits;
+      memcpy(&bits, &v, sizeof bits);
+      return (int)(bits >> 32);
+    };
+    P.fx_pmax = high(2.9 / p->dt);
+    P.fx_pmax_end = high((0.5 * (4.0 - sl - p->margin) - 1.0 / 64.0) / (0.5 * p->dt));
+    for (auto &bx : b->boxes)
+      for (int a = 0; a < 3; a++) {
+        const int64_t L = mdg::fix_from_double(bx.L[a]);
+        bx.fx_L[a] = mdg::fix_shi(L);
+        bx.fx_l[a] = mdg::fix_rest(L);
+      }
+  }
   for (const auto &bx : b->boxes)
     for (int a = 0; a < 3; a++) b->ref_unit = std::fmax(b->ref_unit, (double)bx.w32[a] / 1048575.0);
   const double hm = 0.5 * p->margin - 2.0 * b->ref_unit;
@@ -1245,8 +1566,18 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   if (e == cudaSuccess) e = balloc(&d.t_q, n);
   if (e == cudaSuccess) e = balloc(&d.t_p, n);
   if (e == cudaSuccess) e = balloc(&d.qf, n);
-  if (e == cudaSuccess) e = balloc(&d.loc[0], n);
-  if (e == cudaSuccess) e = balloc(&d.loc[1], n);
+  const bool fixed = step_form(b) == kFixedForm;
+  const size_t n_fx = fixed ? n : 0, n_loc = fixed ? 0 : n;
+  if (e == cudaSuccess) e = balloc(&d.loc[0], n_loc);
+  if (e == cudaSuccess) e = balloc(&d.loc[1], n_loc);
+  if (e == cudaSuccess) e = balloc(&d.xq[0], n_fx);
+  if (e == cudaSuccess) e = balloc(&d.xq[1], n_fx);
+  if (e == cudaSuccess) e = balloc(&d.xb, n_fx);
+  if (e == cudaSuccess) e = balloc(&d.xp, n_fx);
+  if (e == cudaSuccess) e = balloc(&d.box_wide, 2 * (size_t)nbox);
+  if (e == cudaSuccess) e = cudaMemset(d.box_wide, 0, 2 * nbox * sizeof(int));
+  if (e == cudaSuccess) e = balloc(&d.box_wide_end, nbox);
+  if (e == cudaSuccess) e = cudaMemset(d.box_wide_end, 0, nbox * sizeof(int));
   if (e == cudaSuccess) e = balloc(&d.id, n);
   if (e == cudaSuccess) e = balloc(&d.cell, n);
   if (e == cudaSuccess) e = balloc(&d.t_id, n);
@@ -1254,7 +1585,7 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   if (e == cudaSuccess) e = balloc(&d.order, n);
   if (e == cudaSuccess) e = balloc(&d.ncount, n);
   if (e == cudaSuccess) e = balloc(&d.pcount, n);
-  if (e == cudaSuccess) e = balloc(&d.loc_p, n);
+  if (e == cudaSuccess) e = balloc(&d.loc_p, n_loc);
   if (e == cudaSuccess) e = balloc(&d.box_prune, nbox);
   if (e == cudaSuccess) e = balloc(&d.box_req, nbox);
   if (e == cudaSuccess) e = balloc(&d.box_preq, nbox);
@@ -1273,6 +1604,8 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   if (e == cudaSuccess) e = balloc(&d.box_rebuilds, nbox);
   if (e == cudaSuccess) e = balloc(&d.goal, 1);
   if (e == cudaSuccess) e = balloc(&d.partials, 3 * (size_t)nbox);
+  for (const auto &bx : b->boxes) b->chunks = std::max(b->chunks, (bx.n + kObserveThreads - 1) / kObserveThreads);
+  if (e == cudaSuccess) e = balloc(&b->obs_part, 3 * (size_t)nbox * b->chunks);
   if (e == cudaSuccess) e = balloc(&b->d_box_of_slot, n);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_box_of_slot, b->box_of_slot.data(), n * sizeof(int), cudaMemcpyHostToDevice);
   d.box_of_slot = b->d_box_of_slot;
@@ -1300,7 +1633,7 @@ int mdg_batch_destroy(mdg_batch *b) {
                   d.qf, d.loc[0], d.loc[1], d.id, d.cell, d.t_id, d.t_cell, d.order, d.cell_start, d.nl, d.ncount,
                   d.pl, d.pcount, d.loc_p, d.box_prune, d.box_req, d.box_preq, d.rb_boxes, d.rb_start, d.rb_count,
                   d.box_rebuild, d.box_err, d.box_need, d.box_steps, d.box_rebuilds, d.goal, d.partials,
-                  d.box_mid, b->d_box_of_slot};
+                  d.box_mid, d.xq[0], d.xq[1], d.xb, d.xp, d.box_wide, d.box_wide_end, b->obs_part, b->d_box_of_slot};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (b->ev0) cudaEventDestroy(b->ev0);
@@ -1408,7 +1741,12 @@ int mdg_batch_observe(mdg_batch *b, double *out) {
   if (!b || !out) return MDG_ERR_INVALID;
   cudaSetDevice(b->prm.device);
   make_end_current(b);
-  k_batch_observe<<<b->nbox, 256, 0, b->stream>>>(b->P, b->d);
+  if (b->P.fixed) k_batch_fix_end<<<(b->total + 255) / 256, 256, 0, b->stream>>>(b->P, b->d);
+  for (int first = 0; first < b->nbox; first += kObserveBoxes) {
+    const int boxes = std::min(kObserveBoxes, b->nbox - first);
+    k_batch_observe<<<dim3(b->chunks, boxes), kObserveThreads, 0, b->stream>>>(b->P, b->d, b->obs_part, first);
+  }
+  k_batch_observe_final<<<(3 * b->nbox + 255) / 256, 256, 0, b->stream>>>(b->P, b->d, b->obs_part, b->chunks);
   MDG_BCK(cudaMemcpyAsync(out, b->d.partials, 3 * (size_t)b->nbox * sizeof(double), cudaMemcpyDeviceToHost,
                           b->stream));
   MDG_BCK(cudaStreamSynchronize(b->stream));

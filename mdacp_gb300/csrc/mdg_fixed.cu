@@ -48,21 +48,6 @@ __host__ __device__ constexpr int fx_particles() { return fx_threads<LANES>() / 
 // the graph's hand-over).
 inline int fx_lanes(int n) { return n < 12288 ? 8 : (n < 65536 ? 2 : 1); }
 
-__device__ __forceinline__ FixPos ld_fix(const FixPos *p) {
-  long long a, b, c, d;
-  asm("ld.global.nc.v4.s64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
-  FixPos v;
-  v.x = (int)a;
-  v.y = (int)(a >> 32);
-  v.z = (int)b;
-  v.lx = __int_as_float((int)(b >> 32));
-  v.ly = __int_as_float((int)c);
-  v.lz = __int_as_float((int)(c >> 32));
-  v.w = (int)d;
-  v.pad = 0;
-  return v;
-}
-
 // Image shifts of a particle at the box faces: per axis the step code (after
 // entry ^ 0x15: 1 = step -1, 3 = step +1) that crosses the face, 2 = none,
 // and the shift of the partner, -L or +L.

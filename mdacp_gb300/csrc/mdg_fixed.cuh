@@ -200,4 +200,22 @@ MDG_HD double fix_sum(int64_t v, int64_t m, float c) {
   return (double)(v + (m >> 22)) + 2.0 * (double)rest;
 }
 
+#ifdef __CUDACC__
+// 32-byte read-only load of a position.
+__device__ __forceinline__ FixPos ld_fix(const FixPos *p) {
+  long long a, b, c, d;
+  asm("ld.global.nc.v4.s64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+  FixPos v;
+  v.x = (int)a;
+  v.y = (int)(a >> 32);
+  v.z = (int)b;
+  v.lx = __int_as_float((int)(b >> 32));
+  v.ly = __int_as_float((int)c);
+  v.lz = __int_as_float((int)(c >> 32));
+  v.w = (int)d;
+  v.pad = 0;
+  return v;
+}
+#endif
+
 }  // namespace mdg

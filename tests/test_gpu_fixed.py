@@ -120,3 +120,28 @@ def test_lanes_and_graphs_do_not_change_the_trajectory():
         m.calculate(60)
         out.append(np.concatenate(m.state()))
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("shape,flat", [((128, 1, 2), False), ((256, 2, 1), False), ((256, 1, 2), True)])
+def test_batch_paths_match_the_single_box(shape, flat):
+    # an ordinary box, one with a pair at 0.8 and one with a fast particle: each as MDManager runs it alone
+    from mdacp_gb300.batch import Batch
+    boxes = []
+    for k in range(3):
+        q, p, L = liquid_like(0.4, 5, amp=0.05, seed=20 + k)
+        if k == 1:
+            q[11] = np.mod(q[10] + [0.8, 0.0, 0.0], L)
+        if k == 2:
+            p[7] = [700.0, -200.0, 90.0]
+        boxes.append((q, p, L))
+    b = Batch(boxes, cutoff=2.5, margin=0.5, dt=0.001)
+    b.set_shape(*shape)
+    b.set_flat(flat)
+    b.calculate(2)
+    sums, states = b.observe_raw(), b.state()
+    for k, (q, p, L) in enumerate(boxes):
+        m = _manager(L, len(q))
+        m.set_state(q, p)
+        m.calculate(2)
+        np.testing.assert_allclose(states[k][1], m.state()[1], rtol=1e-9, atol=1e-9 * np.abs(p).max())
+        np.testing.assert_allclose(sums[k], m.observe_raw(), rtol=1e-9)
