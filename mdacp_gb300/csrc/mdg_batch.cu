@@ -36,7 +36,7 @@
 #include <string>
 #include <vector>
 
-#include "mdg_internal.cuh"
+#include "mdg_build.cuh"
 
 namespace mdg {
 namespace batch {
@@ -342,57 +342,101 @@ __device__ void place_particle(const Params &P, const Dev &d, const BoxDesc &b, 
 
 // Pair-list row of local particle a of box b (the box's cell starts and
 // build-time positions are in place): the 27 stencil cells with periodic
-// wrap, float-first exact acceptance.  Returns the row length (rows longer
-// than the capacity are truncated and flag the box).
-__device__ int build_row(const Params &P, const Dev &d, const BoxDesc &b, int bi, int a) {
+// wrap, float-first exact acceptance (mdg_build.cuh), by one thread (LANES = 1)
+// or by LANES = 9 neighbouring lanes of a warp, one for each (y, z) row of three
+// cells; `base` is the first of them.  Returns the row length to lane 0 (rows
+// longer than the capacity are truncated and flag the box); every lane of the
+// warp calls it, `active` or not.
+template <int LANES>
+__device__ __forceinline__ int build_row(const Params &P, const Dev &d, const BoxDesc &b, int a, bool active, int lane, int base) {
   const int n = b.n, o = b.atom_off;
   const int *cstart = d.cell_start + b.cell_off;
-  const float4 fi = d.qf[o + a];
-  int cx, cy, cz;
-  cell_xyz(b, d.cell[o + a], cx, cy, cz);
-  int cnt = 0;
-  for (int oz = -1; oz <= 1; oz++) {
-    int nz = cz + oz, sz = 0;
-    if (nz < 0) { nz += b.nc[2]; sz = -1; } else if (nz >= b.nc[2]) { nz -= b.nc[2]; sz = 1; }
-    const float offz = (float)oz * b.w32[2] + (float)sz * b.dl32[2];
-    for (int oy = -1; oy <= 1; oy++) {
-      int ny = cy + oy, sy = 0;
-      if (ny < 0) { ny += b.nc[1]; sy = -1; } else if (ny >= b.nc[1]) { ny -= b.nc[1]; sy = 1; }
-      const float offy = (float)oy * b.w32[1] + (float)sy * b.dl32[1];
+  const float4 *qf = d.qf + o;
+  uint32_t *row = d.nl + b.list_off + a;
+  float4 fi = make_float4(0.f, 0.f, 0.f, 0.f);
+  int cx = 0, cy = 0, cz = 0, cnt = 0;
+  if (active) {
+    fi = qf[a];
+    cell_xyz(b, d.cell[o + a], cx, cy, cz);
+  }
+  auto scan = [&](int ox, int oy, int oz, auto &&emit) {
+    int sx, sy, sz;
+    const int nx = wrap_cell(cx, ox, b.nc[0], sx), ny = wrap_cell(cy, oy, b.nc[1], sy), nz = wrap_cell(cz, oz, b.nc[2], sz);
+    const float fx = (float)ox * b.w32[0] + (float)sx * b.dl32[0] - fi.x;
+    const float fy = (float)oy * b.w32[1] + (float)sy * b.dl32[1] - fi.y;
+    const float fz = (float)oz * b.w32[2] + (float)sz * b.dl32[2] - fi.z;
+    const int cc = (nz * b.nc[1] + ny) * b.nc[0] + nx;
+    const int lo = cstart[cc], hi = cstart[cc + 1];
+    const uint32_t code = entry_pack(0, ox, oy, oz);
+    const bool own_image = (sx | sy | sz) == 0;
+    for (int j0 = lo; j0 < hi; j0 += 32) {
+      uint32_t in, sure;
+      chunk_masks(qf, j0, min(hi - j0, 32), fx, fy, fz, P.acc_lo, P.acc_hi, in, sure);
+      if (own_image && (unsigned)(a - j0) < 32u) in &= ~(1u << (a - j0));  // the particle itself
+      for (uint32_t band = in & ~sure; band; band &= band - 1u) {
+        const int u = __ffs(band) - 1;
+        const double4_32a qi = d.q_end[o + a], qj = d.q_end[o + j0 + u];
+        const double xj = sx ? __dadd_rn(qj.x, sx > 0 ? b.L[0] : -b.L[0]) : qj.x;
+        const double yj = sy ? __dadd_rn(qj.y, sy > 0 ? b.L[1] : -b.L[1]) : qj.y;
+        const double zj = sz ? __dadd_rn(qj.z, sz > 0 ? b.L[2] : -b.L[2]) : qj.z;
+        const double dx = __dsub_rn(qi.x, xj), dy = __dsub_rn(qi.y, yj), dz = __dsub_rn(qi.z, zj);
+        const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        if (!(r2 <= P.sl2)) in &= ~(1u << u);
+      }
+      emit(in, j0, code);
+    }
+  };
+  auto append = [&](uint32_t in, int j0, uint32_t code) {
+    for (; in; in &= in - 1u) {
+      const int j = j0 + __ffs(in) - 1;
+      if (cnt < P.list_cap) row[(long long)cnt * n] = ((uint32_t)j << kCodeBits) | code;
+      cnt++;
+    }
+  };
+  if (LANES == 1) {
+    if (active)
+      for (int oz = -1; oz <= 1; oz++)
+        for (int oy = -1; oy <= 1; oy++)
+          for (int ox = -1; ox <= 1; ox++) scan(ox, oy, oz, append);
+  } else {
+    // as k_build_list's lanes (mdg_list.cu)
+    const int oy = lane % 3 - 1, oz = lane / 3 - 1;
+    int own = 0;
+    uint32_t kept[3] = {0u, 0u, 0u};
+    int first[3] = {0, 0, 0};
+    bool again = false;
+    if (active)
+#pragma unroll
       for (int ox = -1; ox <= 1; ox++) {
-        int nx = cx + ox, sx = 0;
-        if (nx < 0) { nx += b.nc[0]; sx = -1; } else if (nx >= b.nc[0]) { nx -= b.nc[0]; sx = 1; }
-        const float offx = (float)ox * b.w32[0] + (float)sx * b.dl32[0];
-        const int cc = (nz * b.nc[1] + ny) * b.nc[0] + nx;
-        const int lo = cstart[cc], hi = cstart[cc + 1];
-        const uint32_t code = entry_pack(0, ox, oy, oz);
-        const bool self_cell = (sx | sy | sz) == 0;
-        const float fx = offx - fi.x, fy = offy - fi.y, fz = offz - fi.z;
-        for (int j = lo; j < hi; j++) {
-          const float4 fj = d.qf[o + j];
-          const float ex = fj.x + fx, ey = fj.y + fy, ez = fj.z + fz;
-          const float r2f = ex * ex + ey * ey + ez * ez;
-          if (r2f > P.acc_hi) continue;
-          if (self_cell && j == a) continue;
-          bool take = r2f < P.acc_lo;
-          if (!take) {
-            const double4_32a qi = d.q_end[o + a], qj = d.q_end[o + j];
-            const double xj = sx ? __dadd_rn(qj.x, sx > 0 ? b.L[0] : -b.L[0]) : qj.x;
-            const double yj = sy ? __dadd_rn(qj.y, sy > 0 ? b.L[1] : -b.L[1]) : qj.y;
-            const double zj = sz ? __dadd_rn(qj.z, sz > 0 ? b.L[2] : -b.L[2]) : qj.z;
-            const double dx = __dsub_rn(qi.x, xj), dy = __dsub_rn(qi.y, yj), dz = __dsub_rn(qi.z, zj);
-            const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-            take = r2 <= P.sl2;
+        int chunk = 0;
+        scan(ox, oy, oz, [&](uint32_t in, int j0, uint32_t) {
+          own += __popc(in);
+          if (chunk++ == 0) {
+            kept[ox + 1] = in;
+            first[ox + 1] = j0;
+          } else {
+            again = true;
           }
-          if (take) {
-            if (cnt < P.list_cap) d.nl[b.list_off + (long long)cnt * n + a] = ((uint32_t)j << kCodeBits) | code;
-            cnt++;
-          }
-        }
+        });
+      }
+    int before = 0, total = 0;
+#pragma unroll
+    for (int l = 0; l < LANES; l++) {
+      const int v = __shfl_sync(0xffffffffu, own, min(base + l, 31));
+      before += l < lane ? v : 0;
+      total += v;
+    }
+    cnt = before;
+    if (active) {
+#pragma unroll
+      for (int ox = -1; ox <= 1; ox++) {
+        if (again) scan(ox, oy, oz, append);
+        else append(kept[ox + 1], first[ox + 1], entry_pack(0, ox, oy, oz));
       }
     }
+    cnt = total;
   }
-  d.ncount[o + a] = cnt < P.list_cap ? cnt : P.list_cap;
+  if (active && lane == 0) d.ncount[o + a] = cnt < P.list_cap ? cnt : P.list_cap;
   return cnt;
 }
 
@@ -404,6 +448,12 @@ __device__ int build_row(const Params &P, const Dev &d, const BoxDesc &b, int bi
 #define MDG_BATCH_PREP_THREADS 1024
 #endif
 constexpr int kPrepThreads = MDG_BATCH_PREP_THREADS;
+// Lanes of a particle's row in the list build, and the number of rebuilding
+// particles below which they are used (100 steps of 256 boxes, about 50,000
+// rebuilding particles a step: 34.5 ms without, 33.3 below 30,000, 30.8 below
+// 60,000, 30.4 below 100,000, 30.5 below 200,000; 48 boxes FP64, about 10,000:
+// 24.2 without, 18.3).
+constexpr int kRowLanes = 9, kLanesBelow = 100000;
 constexpr int kBatchKernelsPerStep = 6;  // rebuild set, bin, sort, place, list, step (+ finish in the flat layout)
 
 __global__ void __launch_bounds__(128) k_batch_bin(Params P, Dev d) {
@@ -485,19 +535,28 @@ __global__ void __launch_bounds__(1024) k_batch_rebuild_set(Params P, Dev d) {
   }
 }
 
-// Rebuild part 2: one thread per particle slot of every rebuilding box, so a
-// box's list is built by the whole GPU rather than by the CTA that steps it.
+// Rebuild part 2: one thread, or nine lanes, per particle slot of every
+// rebuilding box, so a box's list is built by the whole GPU rather than by the
+// CTA that steps it.
 // A fixed grid walks the concatenated slots of this step's rebuilding boxes.
 __global__ void __launch_bounds__(128) k_batch_list(Params P, Dev d) {
   const int nb = *d.rb_count;
   if (nb == 0) return;
   const int total = d.rb_start[nb];
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int lo = rb_find(d, nb, t), bi = d.rb_boxes[lo];
-    if (d.box_err[bi] == kErrBadState) continue;
+  // few rebuilding particles: nine lanes each
+  const bool lanes = total < kLanesBelow;
+  const int wl = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+  const int per = lanes ? 32 / kRowLanes : 32;  // particles of a warp at a time
+  for (int t0 = warp * per; t0 < total; t0 += warps * per) {
+    const int k = lanes ? wl / kRowLanes : wl, lane = lanes ? wl % kRowLanes : 0;
+    const int t = t0 + k;
+    const bool in = k < per && t < total;
+    const int lo = rb_find(d, nb, in ? t : t0), bi = d.rb_boxes[lo];
+    const bool active = in && d.box_err[bi] != kErrBadState;
     const BoxDesc &b = d.boxes[bi];
-    const int cnt = build_row(P, d, b, bi, t - d.rb_start[lo]);
-    if (cnt > P.list_cap) {
+    const int a = in ? t - d.rb_start[lo] : 0;
+    const int cnt = lanes ? build_row<kRowLanes>(P, d, b, a, active, lane, wl - lane) : build_row<1>(P, d, b, a, active, 0, wl);
+    if (active && lane == 0 && cnt > P.list_cap) {
       atomicMax(&d.box_need[bi], cnt);
       atomicExch(&d.box_err[bi], kErrOverflow);
     }
