@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, "libmdg.so")
 # scatter index of the single-box path checked on the device
 OBJ_CHECK = os.path.join(HERE, "_build_check")
 LIB_CHECK = os.path.join(HERE, "libmdg_check.so")
-SOURCES = ["mdg_cells.cu", "mdg_list.cu", "mdg_step.cu", "mdg_fixed.cu", "mdg_batch.cu", "mdg_api.cu", "mdg_adjoint.cu", "mdg_noalloc.cu",
+SOURCES = ["mdg_cells.cu", "mdg_list.cu", "mdg_step.cu", "mdg_fixed.cu", "mdg_resident.cu", "mdg_batch.cu", "mdg_api.cu", "mdg_adjoint.cu", "mdg_noalloc.cu",
            "mdg_io.cu", "mdg_init.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -37,6 +37,8 @@ struct mdg_handle {
   int par = 0;
   cudaGraphExec_t gx_pair[2] = {nullptr, nullptr};
   cudaGraphExec_t gx_one[2] = {nullptr, nullptr};
+  void *ctl = nullptr;            // control words of the resident kernel
+  bool resident_off = false;      // its cooperative launch was refused
   int graph_n = -1;  // particle count the graphs were captured for
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0.0;
@@ -49,6 +51,8 @@ struct mdg_handle {
 
 // Steps mdg_calculate may leave enqueued before it waits for them.
 constexpr long long kMaxPending = 1024;
+// Steps of one launch of the resident kernel.
+constexpr int kResidentSteps = 1024;
 
 namespace {
 
@@ -284,6 +288,8 @@ int halt_error(mdg_handle *h) {
              2.0 * h->hflags->vmax * h->prm.dt, h->prm.margin);
     return fail(h, MDG_ERR_STATE, buf);
   }
+  if (h->hflags->halt == mdg::kHaltBarrier)
+    return fail(h, MDG_ERR_CUDA, "resident step kernel: a grid barrier was not reached in time");
   if (h->hflags->halt == mdg::kHaltCheck) {
     snprintf(buf, sizeof buf, "bounds check failed (site %d, index %d)", h->hflags->check_site,
              h->hflags->bad_slot);
@@ -475,8 +481,29 @@ int capture(mdg_handle *h, cudaGraphExec_t *out, int par, int nsteps, cudaEvent_
   return rc;
 }
 
+// Whether the handle's steps run in the resident kernel.
+bool resident(const mdg_handle *h) {
+  return h->prm.use_graphs && !h->resident_off && mdg::resident_box(h->g, h->prm.precision, h->num_sms);
+}
+
 int enqueue_steps(mdg_handle *h, int nsteps) {
   int par = h->par;
+  while (nsteps > 0 && resident(h)) {
+    const int m = nsteps < kResidentSteps ? nsteps : kResidentSteps;
+    const cudaError_t e = mdg::launch_resident(h->g, h->d, h->ctl, par, m, h->prm.thermostat, h->prm.langevin_half_drift_compat,
+                                               h->prm.precision, h->num_sms, h->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+      cudaGetLastError();  // fewer SMs than the device has (a partition): the graphs
+      h->resident_off = true;
+      break;
+    }
+    MDG_CK(e);
+    h->launches += 1;
+    nsteps -= m;
+    par ^= m & 1;
+    h->par = par;
+  }
+  if (nsteps == 0) return MDG_OK;
   if (!h->prm.use_graphs) {
     for (int k = 0; k < nsteps; k++) {
       enqueue_step(h, par);
@@ -528,7 +555,7 @@ int settle(mdg_handle *h) {
     int rc = read_flags(h);
     if (rc) return rc;
     long long completed = (long long)(h->hflags->steps - before);
-    if (h->prm.use_graphs)
+    if (h->prm.use_graphs && !resident(h))
       h->launches += graph_kernels(h, completed, (long long)(h->hflags->rebuilds - rebuilds0),
                                    (long long)(h->hflags->checks - checks0));
     if (h->hflags->halt == 0) {
@@ -667,6 +694,8 @@ int mdg_create(const mdg_params *p, mdg_handle **out) {
   if (e == cudaSuccess) e = dalloc(&d.io4, cap);
   if (e == cudaSuccess) e = dalloc(&d.io4b, cap);
   if (e == cudaSuccess) e = dalloc(&h->dobs, 4);
+  if (e == cudaSuccess) e = cudaMalloc(&h->ctl, mdg::resident_ctl_bytes());
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->ctl, 0, mdg::resident_ctl_bytes(), h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.cell_count, 0, ncell * sizeof(int), h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.cell_fill, 0, ncell * sizeof(int), h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.flags, 0, sizeof(DevFlags), h->stream);
@@ -688,6 +717,7 @@ int mdg_destroy(mdg_handle *h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   drop_graphs(h);
   dfree_all(h);
+  if (h->ctl) cudaFree(h->ctl);
   if (h->hflags) cudaFreeHost(h->hflags);
   if (h->hobs) cudaFreeHost(h->hobs);
   if (h->ev0) cudaEventDestroy(h->ev0);

@@ -645,14 +645,14 @@ __device__ __forceinline__ void walk_box(const BoxDesc &b, const FixPos *__restr
                  kz = (cz == 0 ? 1u : (cz == b.nc[2] - 1 ? 3u : 2u)) << 4;
   const int sx = cx == 0 ? -b.fx_L[0] : b.fx_L[0], sy = cy == 0 ? -b.fx_L[1] : b.fx_L[1], sz = cz == 0 ? -b.fx_L[2] : b.fx_L[2];
   const float tx = cx == 0 ? -b.fx_l[0] : b.fx_l[0], ty = cy == 0 ? -b.fx_l[1] : b.fx_l[1], tz = cz == 0 ? -b.fx_l[2] : b.fx_l[2];
-  const FixPos own = ld_fix(xq + a);
+  const FixPos own = ld_fix<false>(xq + a);
   const uint32_t none = entry_pack(a, 0, 0, 0);  // a valid address past the row's end
   auto entry = [&](int k) { return k < cnt ? __ldg(row + (long long)k * n) : none; };
   uint32_t e0 = entry(lane), e1 = entry(lane + LPI);
-  FixPos q0 = ld_fix(xq + entry_slot(e0));
+  FixPos q0 = ld_fix<false>(xq + entry_slot(e0));
 #pragma unroll 2
   for (int k = lane; k < cnt; k += LPI) {
-    const FixPos q1 = ld_fix(xq + entry_slot(e1));
+    const FixPos q1 = ld_fix<false>(xq + entry_slot(e1));
     const uint32_t e2 = entry(k + 2 * LPI);
     int dx = q0.x - own.x, dy = q0.y - own.y, dz = q0.z - own.z;
     float lx = q0.lx - own.lx, ly = q0.ly - own.ly, lz = q0.lz - own.lz;

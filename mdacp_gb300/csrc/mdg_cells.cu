@@ -12,7 +12,7 @@
 // Cells are stored in the order of cell_rank.  Order inside a cell is by
 // caller particle index, which makes the slot order (and with it every later
 // summation order) independent of the atomics used to fill the cells.
-#include "mdg_internal.cuh"
+#include "mdg_rebuild.cuh"
 
 namespace mdg {
 
@@ -67,20 +67,6 @@ __device__ __forceinline__ void start_step(DevFlags *f, int lang_step) {
   }
 }
 
-// Step-boundary position of slot i in the mixed form from the home-cell-local
-// mid-step position: the centre of the home cell plus (q_mid - p dt/2), the
-// inverse of the step's last half-drift.
-__device__ __forceinline__ double4_32a end_from_mid(const Geom &g, const Dev &d, int i, int mid) {
-  const double4_32a u = d.q_mid[mid][i], p = d.p[i];
-  int cx, cy, cz;
-  cell_unkey(d.cell[i], cx, cy, cz);
-  double4_32a q = u;
-  q.x = cell_centre(g, 0, cx) + fma(-p.x, g.dt2, u.x);
-  q.y = cell_centre(g, 1, cy) + fma(-p.y, g.dt2, u.y);
-  q.z = cell_centre(g, 2, cz) + fma(-p.z, g.dt2, u.z);
-  return q;
-}
-
 // Wraps q_end into the box with the reference rule (one +-L per component),
 // bins it and counts cell occupancy.  Thread 0 also advances the step and
 // Langevin counters of a step that is starting.  In the mixed form q_end is
@@ -90,31 +76,8 @@ __global__ void k_wrap_bin(Geom g, Dev d, int count_step, int lang_step, int mid
   if (count_step && blockIdx.x == 0 && threadIdx.x == 0 && f->halt == 0) start_step(f, lang_step);
   if (rebuild_off(f)) return;
   const bool from_mid = g.local_pos && f->end_stale;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x) {
-    double4_32a q = from_mid ? end_from_mid(g, d, i, mid) : d.q_end[i];
-    double x[3] = {q.x, q.y, q.z};
-    int c[3];
-    bool bad = false;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      double v = x[k];
-      if (v < 0.0) v += g.L[k];
-      else if (v > g.L[k]) v -= g.L[k];
-      if (!(v >= 0.0 && v <= g.L[k])) bad = true;  // also catches NaN
-      x[k] = v;
-      int ci = bad ? 0 : (int)(v * g.inv_w[k]);
-      c[k] = ci < 0 ? 0 : (ci >= g.nc[k] ? g.nc[k] - 1 : ci);
-    }
-    if (bad) {
-      halt_with(f, kHaltBadState);
-      atomicMin(&f->bad_slot, i);
-      continue;
-    }
-    q.x = x[0]; q.y = x[1]; q.z = x[2];
-    d.q_end[i] = q;
-    d.cell[i] = cell_key(c[0], c[1], c[2]);
-    atomicAdd(&d.cell_count[cell_rank(g, c[0], c[1], c[2])], 1);
-  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x)
+    wrap_bin_one(g, d, i, from_mid, mid);
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(Geom g, Dev d) {
@@ -217,7 +180,6 @@ __global__ void k_reorder(Geom g, Dev d) {
 // the mixed form q_mid is kept relative to the centre of the new home cell,
 // (q - centre) + p dt/2, and q_end is current again.
 __global__ void k_finalize(Geom g, Dev d, int q_mid_dst) {
-  double4_32a *q_mid = d.q_mid[q_mid_dst];
   if (rebuild_off(d.flags)) return;
   // k_wrap_bin, the only reader of end_stale in the rebuild, has finished;
   // a new list starts the reference policy's budget (PairList::Init,
@@ -228,52 +190,8 @@ __global__ void k_finalize(Geom g, Dev d, int q_mid_dst) {
     d.flags->lifetime = 0;
     d.flags->need_check = 0;
   }
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.n; k += gridDim.x * blockDim.x) {
-    const double4_32a q = d.t_q[k];
-    double4_32a p = d.t_p[k];
-    const int id = d.t_id[k], c = d.t_cell[k];
-    d.q_end[k] = q;
-    d.id[k] = id;
-    d.cell[k] = c;
-    d.inv[id] = k;
-    int cx, cy, cz;
-    cell_unkey(c, cx, cy, cz);
-    const float cw = __int_as_float(c);
-    const double ox = cell_centre(g, 0, cx), oy = cell_centre(g, 1, cy), oz = cell_centre(g, 2, cz);
-    const float4 lb = make_float4((float)(q.x - ox), (float)(q.y - oy), (float)(q.z - oz), cw);
-    d.qf[k] = lb;
-    double4_32a m = q;
-    if (g.local_pos) {
-      m.x = __dadd_rn(q.x - ox, __dmul_rn(p.x, g.dt2));
-      m.y = __dadd_rn(q.y - oy, __dmul_rn(p.y, g.dt2));
-      m.z = __dadd_rn(q.z - oz, __dmul_rn(p.z, g.dt2));
-      // the build reference (for the rebuild test) in q_mid's padding word, and
-      // the same position as the prune reference in p's until the step's
-      // re-selection records its own
-      m.w = pack_ref(g, lb.x, lb.y, lb.z);
-      p.w = m.w;
-      q_mid[k] = m;
-      d.p[k] = p;
-      d.loc[q_mid_dst][k] = make_float4((float)m.x, (float)m.y, (float)m.z, cw);
-    } else {
-      d.p[k] = p;
-      d.q_build[k] = q;
-      m.x = __dadd_rn(q.x, __dmul_rn(p.x, g.dt2));
-      m.y = __dadd_rn(q.y, __dmul_rn(p.y, g.dt2));
-      m.z = __dadd_rn(q.z, __dmul_rn(p.z, g.dt2));
-      q_mid[k] = m;
-      if (g.fixed) {
-        d.xq[q_mid_dst][k] = fix_position(m.x, m.y, m.z, c);
-        const FixPos b = fix_position(q.x, q.y, q.z, c);
-        d.xb[k] = make_int4(b.x, b.y, b.z, c);
-        // the first half-drift must stay inside the modulus's guard too
-        const double far = fmax(fmax(fabs(p.x), fabs(p.y)), fabs(p.z)) * g.dt2;
-        if (!(far <= (double)g.fx_guard)) d.flags->fx_wide[q_mid_dst] = 1;
-      } else {
-        d.loc[q_mid_dst][k] = make_float4((float)(m.x - ox), (float)(m.y - oy), (float)(m.z - oz), cw);
-      }
-    }
-  }
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.n; k += gridDim.x * blockDim.x)
+    finalize_one(g, d, k, d.t_q[k], d.t_p[k], d.t_id[k], d.t_cell[k], q_mid_dst);
 }
 
 // Mixed form: q_end from q_mid[mid] and p for every slot while the steps have

@@ -201,10 +201,13 @@ MDG_HD double fix_sum(int64_t v, int64_t m, float c) {
 }
 
 #ifdef __CUDACC__
-// 32-byte read-only load of a position.
+// 32-byte load of a position: read-only data, or (COH) data that the kernel
+// itself writes between grid barriers.
+template <bool COH>
 __device__ __forceinline__ FixPos ld_fix(const FixPos *p) {
   long long a, b, c, d;
-  asm("ld.global.nc.v4.s64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+  if (COH) asm volatile("ld.global.v4.s64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p) : "memory");
+  else asm("ld.global.nc.v4.s64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
   FixPos v;
   v.x = (int)a;
   v.y = (int)(a >> 32);

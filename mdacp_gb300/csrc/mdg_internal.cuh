@@ -51,6 +51,7 @@ __device__ __forceinline__ int entry_sz(uint32_t e) { return (int)((e >> 4) & 3u
 constexpr int kHaltOverflow = 1;
 constexpr int kHaltBadState = 2;
 constexpr int kHaltCheck = 3;  // checked builds: a bounds check failed
+constexpr int kHaltBarrier = 5;  // resident kernel: blocks did not arrive at a grid barrier
 constexpr int kHaltTooFast = 4;  // reference rebuild policy: 2 max|p| dt above the margin
 
 struct DevFlags {
@@ -220,6 +221,13 @@ void launch_forces(const Geom &g, const Dev &d, int mixed, int par, int call, cu
 int launch_step_fixed(const Geom &g, const Dev &d, int par, int thermostat, int compat, int pmode, cudaStream_t s);
 int launch_observe_fixed(const Geom &g, const Dev &d, int par, int call, cudaStream_t s);
 void launch_forces_fixed(const Geom &g, const Dev &d, int par, int call, cudaStream_t s);
+// The steps of a small box in one resident kernel (mdg_resident.cu): whether
+// this box takes it, and the launch of nsteps steps; ctl is zeroed device
+// memory of resident_ctl_bytes() that the launches keep to themselves.
+size_t resident_ctl_bytes();
+bool resident_box(const Geom &g, int precision, int num_sms);
+cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int nsteps, int thermostat, int compat, int precision,
+                            int num_sms, cudaStream_t s);
 void launch_unsort(const Geom &g, const Dev &d, int par, double4_32a *qo, double4_32a *po, cudaStream_t s);
 void launch_sort_in(const Geom &g, const Dev &d, const double4_32a *qi, const double4_32a *pi, cudaStream_t s);
 void launch_pairs(const Geom &g, const Dev &d, const long long *row_off, int32_t *rec, cudaStream_t s);

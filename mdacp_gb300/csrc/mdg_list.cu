@@ -16,7 +16,7 @@
 // of the exact value; only those within 1e-4 of SL^2 take the double test,
 // so the result is the exact set at float cost.  The order of the entries in
 // a row (stencil cell by cell, near side first) carries no meaning.
-#include "mdg_build.cuh"
+#include "mdg_rebuild.cuh"
 
 namespace mdg {
 
@@ -33,23 +33,7 @@ constexpr int kListThreads = 384, kListThreadsSmall = 128, kListLarge = 1000000;
 // (174 us with one thread per slot, 230 with nine lanes).
 constexpr int kLanesBelow = 49152;
 
-// Exact acceptance of a candidate in the float band: the reference's image
-// and rounding order (mdunit.cc:167, meshlist.cc:262-266).
-__device__ __forceinline__ bool exact_within(const Geom &g, const double4_32a &qi, const double4_32a &qj, int sx, int sy,
-                                             int sz) {
-  const double xj = sx ? __dadd_rn(qj.x, sx > 0 ? g.L[0] : -g.L[0]) : qj.x;
-  const double yj = sy ? __dadd_rn(qj.y, sy > 0 ? g.L[1] : -g.L[1]) : qj.y;
-  const double zj = sz ? __dadd_rn(qj.z, sz > 0 ? g.L[2] : -g.L[2]) : qj.z;
-  const double dx = __dsub_rn(qi.x, xj), dy = __dsub_rn(qi.y, yj), dz = __dsub_rn(qi.z, zj);
-  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-  return r2 <= g.sl2;
-}
-
-// One thread per slot (LANES = 1), or LANES = 9 lanes of a warp per slot, one for
-// each (y, z) row of three stencil cells: a row's candidates then take a
-// ninth of the time one after the other, which is what a small box waits for.
-// The rows' entries are in stencil order (z, y, x), candidates ascending, either way.
-constexpr int kRowLanes = 9;
+// One thread per slot (LANES = 1), or LANES = 9 lanes of a warp per slot.
 template <int LANES, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_build_list(Geom g, Dev d) {
   DevFlags *f = d.flags;
@@ -64,94 +48,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_build_list(Geom g, Dev d) {
   const int i = LANES == 1 ? blockIdx.x * blockDim.x + threadIdx.x
                            : (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * kPerWarp + wl / LANES;
   const bool active = i < g.n && wl < kPerWarp * LANES;
-  const float acc_lo = g.acc_lo, acc_hi = g.acc_hi;
   const int cap = g.list_cap;
-  const size_t stride = (size_t)g.stride;
-  uint32_t *row = d.nl + i;
-  int cnt = 0;
-  float4 fi = make_float4(0.f, 0.f, 0.f, 0.f);
-  int cx = 0, cy = 0, cz = 0;
-  if (active) {
-    fi = d.qf[i];
-    cell_unpack(fi.w, cx, cy, cz);
-  }
-  // candidates of stencil cell (ox, oy, oz): emit(mask, j0, code) for every 32
-  auto scan = [&](int ox, int oy, int oz, auto &&emit) {
-    int sx, sy, sz;
-    const int nx = wrap_cell(cx, ox, g.nc[0], sx), ny = wrap_cell(cy, oy, g.nc[1], sy), nz = wrap_cell(cz, oz, g.nc[2], sz);
-    // offset of the partner cell's centre: o*w + s*(L - nc*w)
-    const float fx = (float)ox * g.w32[0] + (float)sx * g.dl32[0] - fi.x;
-    const float fy = (float)oy * g.w32[1] + (float)sy * g.dl32[1] - fi.y;
-    const float fz = (float)oz * g.w32[2] + (float)sz * g.dl32[2] - fi.z;
-    const int cc = cell_rank(g, nx, ny, nz);
-    if (!MDG_IN_RANGE(f, kCheckBuildCell, cc, g.nrank)) return;
-    int a = d.cell_start[cc], b = d.cell_start[cc + 1];
-    if (!MDG_IN_RANGE(f, kCheckBuildRange, b, g.n + 1) || !MDG_IN_RANGE(f, kCheckBuildRange, a, b + 1)) a = b = 0;
-    const uint32_t code = entry_pack(0, ox, oy, oz);
-    for (int j0 = a; j0 < b; j0 += 32) {
-      uint32_t in, sure;
-      chunk_masks(d.qf, j0, min(b - j0, 32), fx, fy, fz, acc_lo, acc_hi, in, sure);
-      if ((unsigned)(i - j0) < 32u) in &= ~(1u << (i - j0));  // the particle itself (its images are a box away)
-      for (uint32_t band = in & ~sure; band; band &= band - 1u) {
-        const int u = __ffs(band) - 1;
-        if (!exact_within(g, d.q_end[i], d.q_end[j0 + u], sx, sy, sz)) in &= ~(1u << u);
-      }
-      emit(in, j0, code);
-    }
-  };
-  auto append = [&](uint32_t in, int j0, uint32_t code) {
-    for (; in; in &= in - 1u) {
-      const int j = j0 + __ffs(in) - 1;
-      if (cnt < cap) row[(size_t)cnt * stride] = ((uint32_t)j << kCodeBits) | code;
-      cnt++;
-    }
-  };
-  if (LANES == 1) {
-    if (active)
-      for (int oz = -1; oz <= 1; oz++)
-        for (int oy = -1; oy <= 1; oy++)
-          for (int ox = -1; ox <= 1; ox++) scan(ox, oy, oz, append);
-  } else {
-    // the first masks of each cell are kept between counting and writing;
-    // cells of more than 32 particles are scanned again
-    const int oy = lane % 3 - 1, oz = lane / 3 - 1;
-    int own = 0;
-    uint32_t kept[3] = {0u, 0u, 0u};
-    int first[3] = {0, 0, 0};
-    bool again = false;
-    if (active)
-#pragma unroll
-      for (int ox = -1; ox <= 1; ox++) {
-        int chunk = 0;
-        scan(ox, oy, oz, [&](uint32_t in, int j0, uint32_t) {
-          own += __popc(in);
-          if (chunk++ == 0) {
-            kept[ox + 1] = in;
-            first[ox + 1] = j0;
-          } else {
-            again = true;
-          }
-        });
-      }
-    // entries of the particle's lower lanes, and of all
-    const int base = wl - lane;
-    int before = 0, total = 0;
-#pragma unroll
-    for (int l = 0; l < LANES; l++) {
-      const int v = __shfl_sync(0xffffffffu, own, min(base + l, 31));
-      before += l < lane ? v : 0;
-      total += v;
-    }
-    cnt = before;
-    if (active) {
-#pragma unroll
-      for (int ox = -1; ox <= 1; ox++) {
-        if (again) scan(ox, oy, oz, append);
-        else append(kept[ox + 1], first[ox + 1], entry_pack(0, ox, oy, oz));
-      }
-    }
-    cnt = total;
-  }
+  const int cnt = build_slot_row<LANES>(g, d, i, active, lane, wl - lane);
   unsigned long long tot = 0;
   int mx = 0;
   if (active && lane == 0) {

@@ -79,173 +79,6 @@ __host__ __device__ constexpr int step_threads() {
 #ifndef MDG_PRUNE_MIN_BLOCKS
 #define MDG_PRUNE_MIN_BLOCKS 8
 #endif
-// Neighbour-list entries whose index and position loads are issued together
-// in the mixed-form force loop.
-#ifndef MDG_STEP_UNROLL
-#define MDG_STEP_UNROLL 4
-#endif
-constexpr int kUnroll = MDG_STEP_UNROLL;
-
-// List rows requested into L2 this many entries ahead of the pair loop (0:
-// none).  16 measured best at 4M atoms (step kernel 0.476 -> 0.440 ms; 8: 0.472,
-// 12: 0.472, 20: 0.442, 24: 0.445, 32: 0.452, 64: 0.458).
-#ifndef MDG_ENTRY_L2_AHEAD
-#define MDG_ENTRY_L2_AHEAD 16
-#endif
-constexpr int kEntryAhead = MDG_ENTRY_L2_AHEAD;
-
-// Walks the row of slot i on home-cell-local float positions and hands each
-// entry's partner offset q_j - q_i and its r^2 to pair(e, dx, dy, dz, r2).
-// The offset between the home cells of i and j is ox*w + s*(L - nc*w) per
-// axis, s the periodic wrap of the stencil step, evaluated as the quadratic
-// of axis_quad.  EDGE: the home cell touches the periodic boundary, so the
-// offset is the quadratic; otherwise it is linear with the cell width as
-// slope (b = 0, a = w: fmaf(fmaf(0, t, a), t, c) = fmaf(a, t, c) exactly), the
-// width coming from the kernel parameters instead of two registers per axis.
-// An entry whose slot a checked build rejects (code `site`) and the padding of
-// the last batch get a partner at 1e30, whose r^2 overflows to +inf.
-template <bool EDGE, int SITE, class Pair>
-__device__ __forceinline__ void walk_row(const Geom &g, const Dev &d, const float4 *__restrict__ loc, int i,
-                                         const float4 &li, const CellPos &cp, const uint32_t *__restrict__ list,
-                                         int cnt, Pair &&pair) {
-  AxisQuad qx, qy, qz;
-  if (EDGE) {
-    qx = axis_quad(g.w32[0], g.dl32[0], cp.cx == 0, cp.cx == g.nc[0] - 1, li.x, 1.0f);
-    qy = axis_quad(g.w32[1], g.dl32[1], cp.cy == 0, cp.cy == g.nc[1] - 1, li.y, 0.25f);
-    qz = axis_quad(g.w32[2], g.dl32[2], cp.cz == 0, cp.cz == g.nc[2] - 1, li.z, 0.0625f);
-  } else {
-    qx.a = g.w32[0];
-    qy.a = 0.25f * g.w32[1];
-    qz.a = 0.0625f * g.w32[2];
-    qx.b = qy.b = qz.b = 0.0f;
-    qx.c = -li.x;
-    qy.c = -li.y;
-    qz.c = -li.z;
-  }
-  const uint32_t *row = list + i;
-  const size_t stride = (size_t)g.stride;
-  auto gather = [&](uint32_t e) -> float4 {
-    const int j = entry_slot(e);
-    if (!MDG_IN_RANGE(d.flags, SITE, j, g.n)) return make_float4(1e30f, 1e30f, 1e30f, 0.f);
-    return __ldg(loc + j);
-  };
-  auto offset = [&](uint32_t e, const float4 &lj) {
-    const float tx = step_float(e, 0x03u, 8388609.0f);   // t
-    const float ty = step_float(e, 0x0Cu, 8388612.0f);   // 4 t
-    const float tz = step_float(e, 0x30u, 8388624.0f);   // 16 t
-    float dx, dy, dz;
-    if (EDGE) {
-      dx = lj.x + fmaf(fmaf(qx.b, tx, qx.a), tx, qx.c);
-      dy = lj.y + fmaf(fmaf(qy.b, ty, qy.a), ty, qy.c);
-      dz = lj.z + fmaf(fmaf(qz.b, tz, qz.a), tz, qz.c);
-    } else {
-      dx = lj.x + fmaf(qx.a, tx, qx.c);
-      dy = lj.y + fmaf(qy.a, ty, qy.c);
-      dz = lj.z + fmaf(qz.a, tz, qz.c);
-    }
-    pair(e, dx, dy, dz, dx * dx + dy * dy + dz * dz);
-  };
-  int k = 0;
-  // the next batch's list entries are requested before this batch's partner
-  // positions are used, so the entry load (from DRAM) overlaps the gathers;
-  // the last full batch requests the row's remaining (< kUnroll) entries
-  const int full = cnt - cnt % kUnroll;
-  uint32_t en[kUnroll];
-#pragma unroll
-  for (int u = 0; u < kUnroll; u++) en[u] = u < cnt ? __ldg(row + (size_t)u * stride) : 0u;
-#pragma unroll 1
-  for (; k < full; k += kUnroll) {
-    uint32_t e[kUnroll];
-    float4 l[kUnroll];
-#pragma unroll
-    for (int u = 0; u < kUnroll; u++) e[u] = en[u];
-#pragma unroll
-    for (int u = 0; u < kUnroll; u++) l[u] = gather(e[u]);
-#pragma unroll
-    for (int u = 0; u < kUnroll; u++) {
-      const int kn = k + kUnroll + u;
-      en[u] = kn < cnt ? __ldg(row + (size_t)kn * stride) : 0u;
-    }
-    if (kEntryAhead > 0) {
-      // rows kEntryAhead further on, into L2: lane l requests row
-      // k + kEntryAhead + (l mod 4) of its own column, so one instruction
-      // covers the warp's four next rows, one 128-byte line each
-      const int kp = k + kEntryAhead + (int)(threadIdx.x & 3);
-      if (kp < cnt) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (size_t)kp * stride));
-    }
-#pragma unroll
-    for (int u = 0; u < kUnroll; u++) offset(e[u], l[u]);
-  }
-  if (k < cnt) {
-    // the remainder as one batch
-    constexpr int kTail = kUnroll > 1 ? kUnroll - 1 : 1;
-    float4 l[kTail];
-#pragma unroll
-    for (int u = 0; u < kTail; u++)
-      l[u] = k + u < cnt ? gather(en[u]) : make_float4(1e30f, 1e30f, 1e30f, 0.f);
-#pragma unroll
-    for (int u = 0; u < kTail; u++) offset(en[u], l[u]);
-  }
-}
-
-// Mixed form of force_fp64: the sum over the row of slot i of f(r) (q_j - q_i)
-// in float.  KAHAN: the per-particle sums compensated (MDG_MIXED), else plain
-// float (MDG_MIXED_PLAIN).  With PRUNE every entry within the prune radius is
-// copied to the inner row of slot i, as in force_fp64.
-template <bool PRUNE, bool KAHAN, bool EDGE>
-__device__ __forceinline__ double3 pair_loop(const Geom &g, const Dev &d, const float4 *__restrict__ loc, int i,
-                                             const float4 &li, const CellPos &cp, const uint32_t *__restrict__ list,
-                                             const int *__restrict__ counts, int *kept) {
-  int cnt = counts[i];
-  if (!MDG_IN_RANGE(d.flags, kCheckStepRow, cnt, g.list_cap + 1)) cnt = 0;
-  const size_t stride = (size_t)g.stride;
-  float sx = 0.f, sy = 0.f, sz = 0.f;
-  float cx = 0.f, cy = 0.f, cz = 0.f;  // Kahan corrections
-  const float rc2 = g.rc2f, c2x8 = g.c2x8f, thr = g.prune_thr2;
-  int m = 0;
-  walk_row<EDGE, kCheckStepSlot>(g, d, loc, i, li, cp, list, cnt, [&](uint32_t e, float dx, float dy, float dz, float r2) {
-    if (PRUNE && r2 <= thr) d.pl[(size_t)(m++) * stride + i] = e;
-    // evaluated for every entry and masked: no divergent branch per pair
-    float inv;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r2));
-    const float i6 = inv * inv * inv;
-    float df = (i6 * inv) * fmaf(-48.0f, i6, 24.0f) + c2x8;
-    df = r2 <= rc2 ? df : 0.0f;
-    if (KAHAN) {
-      // a zero term (a pair beyond rc) leaves s - c unchanged as a real
-      // number (t - s is exact, and so is the new correction), but it moves
-      // the correction into s and the later additions round differently:
-      // lists that differ only by pairs beyond rc give forces that agree to
-      // about one float rounding, not bit for bit
-      kahan_fma(sx, cx, df, dx);
-      kahan_fma(sy, cy, df, dy);
-      kahan_fma(sz, cz, df, dz);
-    } else {
-      sx = fmaf(df, dx, sx);
-      sy = fmaf(df, dy, sy);
-      sz = fmaf(df, dz, sz);
-    }
-  });
-  if (PRUNE) *kept = m;
-  // the compensated sum rounded once to float (relative 6e-8 of the force),
-  // then one conversion per component: GB300 runs double at 1/64 of float
-  if (KAHAN) return make_double3((double)(sx - cx), (double)(sy - cy), (double)(sz - cz));
-  return make_double3((double)sx, (double)sy, (double)sz);
-}
-
-// The pair loop for the calling warp: the linear offset when no active lane's
-// home cell touches the periodic boundary (about four warps in five at 66
-// cells a side), the quadratic otherwise; both give the same forces bit for
-// bit.  Registers are allocated for the larger loop, but the interior one
-// needs six fewer and runs without the other's spills.
-template <bool PRUNE, bool KAHAN>
-__device__ __forceinline__ double3 force_mixed(const Geom &g, const Dev &d, const float4 *__restrict__ loc, int i,
-                                               const float4 &li, const CellPos &cp, const uint32_t *__restrict__ list,
-                                               const int *__restrict__ counts, int *kept) {
-  if (__all_sync(__activemask(), !cp.edge)) return pair_loop<PRUNE, KAHAN, false>(g, d, loc, i, li, cp, list, counts, kept);
-  return pair_loop<PRUNE, KAHAN, true>(g, d, loc, i, li, cp, list, counts, kept);
-}
-
 // PMODE: 0 = decide from flags->prune_now in the kernel (both paths compiled);
 // 1 = ordinary step only, 2 = re-selecting step only (each a no-op when the
 // flag says otherwise, so the graph path can run the lighter variant).
@@ -281,95 +114,9 @@ __global__ void __launch_bounds__(step_threads<THERMO, MIXED, PMODE>(), (PMODE !
     else
       F = MIXED ? force_mixed<false, MIXED == MDG_MIXED>(g, d, d.loc[par], i, lb, cp, d.pl, d.pcount, nullptr)
                 : force_fp64<false>(g, d, qm, i, cp, d.pl, d.pcount, nullptr);
-    // the w words are padding (zero in the FP64 form, packed reference
-    // positions in the mixed form): never scaled, never in the kinetic energy
-    double4_32a p = d.p[i];
-    if (THERMO == MDG_NOSEHOOVER) {
-      const double e1 = f->exp1;
-      p.x *= e1; p.y *= e1; p.z *= e1;
-      p.x += F.x * g.dt; p.y += F.y * g.dt; p.z += F.z * g.dt;
-      p.x *= e1; p.y *= e1; p.z *= e1;
-    } else {
-      p.x += F.x * g.dt; p.y += F.y * g.dt; p.z += F.z * g.dt;
-    }
-    if (THERMO == MDG_LANGEVIN) {
-      double z[3];
-      langevin_normals(g.seed, (uint32_t)d.id[i], f->lang - 1ull, z);
-      p.x += (-g.gamma * p.x + g.hb_d * z[0]) * g.dt;
-      p.y += (-g.gamma * p.y + g.hb_d * z[1]) * g.dt;
-      p.z += (-g.gamma * p.z + g.hb_d * z[2]) * g.dt;
-    }
-    const double4_32a q0 = qm[i];
-    double4_32a qe = q0, q1;
-    if (MIXED) {  // one rounding per half-drift (fused)
-      if (!(THERMO == MDG_LANGEVIN && COMPAT)) {
-        qe.x = fma(p.x, g.dt2, q0.x);
-        qe.y = fma(p.y, g.dt2, q0.y);
-        qe.z = fma(p.z, g.dt2, q0.z);
-      }
-      q1 = qe;
-      q1.x = fma(p.x, g.dt2, qe.x);
-      q1.y = fma(p.y, g.dt2, qe.y);
-      q1.z = fma(p.z, g.dt2, qe.z);
-    } else {  // the reference's separate product and sum
-      if (!(THERMO == MDG_LANGEVIN && COMPAT)) {
-        qe.x = __dadd_rn(q0.x, __dmul_rn(p.x, g.dt2));
-        qe.y = __dadd_rn(q0.y, __dmul_rn(p.y, g.dt2));
-        qe.z = __dadd_rn(q0.z, __dmul_rn(p.z, g.dt2));
-      }
-      q1 = qe;
-      q1.x = __dadd_rn(qe.x, __dmul_rn(p.x, g.dt2));
-      q1.y = __dadd_rn(qe.y, __dmul_rn(p.y, g.dt2));
-      q1.z = __dadd_rn(qe.z, __dmul_rn(p.z, g.dt2));
-    }
-    float4 ln;
-    if (MIXED) {
-      // positions relative to the home-cell centre: the new local position is
-      // one conversion, and the displacement since the build is measured in
-      // float against the build's local position, packed in q_mid.w
-      ln = make_float4((float)q1.x, (float)q1.y, (float)q1.z, lb.w);
-      float bx, by, bz;
-      unpack_ref(g, q0.w, bx, by, bz);
-      const float fx = ln.x - bx, fy = ln.y - by, fz = ln.z - bz;
-      // the half-margin rule, or a non-finite position (the rebuild's wrap
-      // reports it) under either policy
-      if ((g.rebuild_policy == MDG_REBUILD_HALFMARGIN && fx * fx + fy * fy + fz * fz > g.half_margin2_ref) ||
-          !(fx == fx && fy == fy && fz == fz))
-        d.flags->rebuild = 1;
-    } else {
-      const double4_32a qb = d.q_build[i];
-      const double ux = q1.x - qb.x, uy = q1.y - qb.y, uz = q1.z - qb.z;
-      // displacement since the build: in double for the rebuild test, in
-      // float for the new home-cell-local position (qf holds the local
-      // position at the build) and the inner-list test
-      ln = make_float4(lb.x + (float)ux, lb.y + (float)uy, lb.z + (float)uz, lb.w);
-      if ((g.rebuild_policy == MDG_REBUILD_HALFMARGIN && ux * ux + uy * uy + uz * uz > g.half_margin2) ||
-          !(q1.x == q1.x && q1.y == q1.y && q1.z == q1.z))
-        d.flags->rebuild = 1;
-    }
-    d.loc[par ^ 1][i] = ln;
-    // prune reference: the positions of this force evaluation when the
-    // inner list was re-selected now, else those of the last selection
-    // (mixed: packed in p.w)
-    float4 lp;
-    if (prune) {
-      lp = MIXED ? lb : d.loc[par][i];
-      if (MIXED) p.w = pack_ref(g, lp.x, lp.y, lp.z);
-      else d.loc_p[i] = lp;
-      d.pcount[i] = kept;
-    } else if (MIXED) {
-      unpack_ref(g, p.w, lp.x, lp.y, lp.z);
-    } else {
-      lp = d.loc_p[i];
-    }
-    const float vx = ln.x - lp.x, vy = ln.y - lp.y, vz = ln.z - lp.z;
-    if (vx * vx + vy * vy + vz * vz > (MIXED ? g.half_prune2_ref : g.half_prune2)) d.flags->prune_next = 1;
-    d.p[i] = p;
-    // the mixed form leaves q_end behind: q_mid - p dt/2 gives it back when a
-    // rebuild or a reader needs it (32 bytes a particle fewer per step)
-    if (!MIXED) d.q_end[i] = qe;
-    qn[i] = q1;
-    if (THERMO == MDG_NOSEHOOVER) ke = 0.5 * p.x * p.x + 0.5 * p.y * p.y + 0.5 * p.z * p.z;
+    ke = step_one<THERMO, COMPAT, MIXED>(g, d, par, i, prune, kept, F, lb, qm, qn, THERMO == MDG_NOSEHOOVER ? f->exp1 : 1.0,
+                                         THERMO == MDG_LANGEVIN ? f->lang - 1ull : 0ull, &d.flags->rebuild,
+                                         &d.flags->prune_next);
   }
   if (MIXED && i == 0) d.flags->end_stale = 1;
   if (THERMO == MDG_NOSEHOOVER) {
@@ -454,7 +201,7 @@ __device__ __forceinline__ void observe_row(const Geom &g, const Dev &d, const f
   // rounding of the sum, whatever the row length (GB300 runs double, and
   // conversions to 64-bit types, at 1/64 of the float rate)
   float se = 0.f, ce = 0.f, sv = 0.f, cv = 0.f;
-  walk_row<EDGE, kCheckObserve>(g, d, loc, i, li, cp, d.nl, cnt,
+  walk_row<EDGE, kCheckObserve, false, kUnroll>(g, d, loc, i, li, cp, d.nl, cnt,
                                 [&](uint32_t, float, float, float, float r2) {
     float inv;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r2));
