@@ -72,7 +72,14 @@ struct P {
   // coefficients of the pair terms in Horner form (pair_terms)
   double kf6, kf0, kfc, kp6, kp0, ke6, ke0, kec2, kec0, kd6, kd0, kdc, ks6, ks0, ksc;
   double kg6, kg0, kgc, kr6, kr0, krc, kq6, kq0, kqc;
-  int n, cap, objective, pad;
+  int n, cap, objective;
+  // Fixed-point pair arithmetic (mdg_fixed.cuh) in reduced units x = r / sigma:
+  // y = x^-2 is sigma^2 / r^2
+  int fixed, unit_sigma;
+  uint64_t fx_rc2, fx_near, fx_s2;  // (cutoff sigma)^2 and kFixNear sigma^2 in the unit of R; sigma^2, 2^-62
+  int64_t fx_c8;
+  int fx_L[3];
+  float fx_l[3];
 };
 
 // A list entry: partner index << kImageBits | per axis two bits r + 1, the
@@ -85,6 +92,8 @@ struct D {
   double4_32a *ckq, *ckp;    // checkpoints
   float4 *qf;                // float copy of the segment's first state (the list test)
   double4_32a *segq, *segp, *segqh;  // recomputed segment
+  // the same positions in fixed point (P.fixed): of q, q2, qh, qh2 and the segment's
+  FixPos *xq, *xq2, *xqh, *xqh2, *segxq, *segxqh;
   uint32_t *nbr;             // the current segment's list, row-major [n][cap]
   int *cnt;
   double *part;              // block partials
@@ -178,6 +187,172 @@ __device__ __forceinline__ void for_pairs(const P &c, const D &d, int i, int lan
   }
 }
 
+// Sum over the kLanes lanes that share a particle (all lanes hold the total).
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// ---------------------------------------------------------------------------
+// The pair kernels' sums in fixed point.  An FP64 pair of the step, of the
+// objective's gradient and of the Hessian-vector product took 21, 22 and 39
+// instructions of the FP64 pipe, which was busy 66-79 % of the time; here the
+// pair terms, force sums and objective sums are integers, and 13 of them are
+// left, all in the Hessian-vector product (its vectors have no fixed range).
+
+// Powers of y = (r / sigma)^-2: y 2^-62, y^3 2^-61, y^4 2^-62, y^7 2^-59.
+struct FixTerms {
+  uint64_t y, y3, y4, y7;
+};
+
+__device__ __forceinline__ uint64_t fix_y(const P &c, uint64_t R) {
+  const uint64_t y = fix_recip(R);
+  return c.unit_sigma ? y : fix_mulhi(y, c.fx_s2) << 2;
+}
+
+__device__ __forceinline__ FixTerms fix_terms(const P &c, uint64_t R) {
+  FixTerms t;
+  uint64_t y2;
+  t.y = fix_y(c, R);
+  fix_powers(t.y, y2, t.y3);
+  t.y4 = fix_sqrhi(y2);
+  t.y7 = fix_mulhi(t.y4, t.y3);
+  return t;
+}
+
+// psi = 24 y^4 - 48 y^7 + 8 C2, 2^-55 (fix_force).
+__device__ __forceinline__ int64_t fix_psi(const P &c, const FixTerms &t) {
+  const int64_t v = (int64_t)((t.y4 >> 4) - t.y7);
+  return v + (v << 1) + c.fx_c8;
+}
+
+// An eighth of 144 y^4 - 576 y^7 - 16 C2 = -(2 psi + x psi'), 2^-55: the sigma
+// derivative of the force, and minus the pressure objective's slope.
+__device__ __forceinline__ int64_t fix_dsigma(const P &c, const FixTerms &t) {
+  const int64_t q = (int64_t)((t.y4 >> 4) - (t.y7 << 1)) >> 2;
+  return (q << 3) + q - (c.fx_c8 >> 2);
+}
+
+// psi'(x) / x = 672 y^8 - 192 y^5, over 48, 2^-55.
+__device__ __forceinline__ int64_t fix_psi_slope(const FixTerms &t) {
+  const int64_t a = (int64_t)(14 * (t.y7 >> 2) - (t.y4 >> 3));  // 14 y^7 - 4 y^4, 2^-57
+  const int32_t ah = fix_shi(a), al = fix_slo(a), yh = fix_shi((int64_t)t.y), yl = fix_slo((int64_t)t.y);
+  const int64_t m = fix_mads(ah, yl, fix_mads(al, yh, 0));
+  return fix_mads((int32_t)fix_hi((uint64_t)m), 1, fix_mads(ah, yh, 0));
+}
+
+// v 2^-shift as a double, rounded, without the FP64 pipe's conversion.
+__device__ __forceinline__ double fix_double(int64_t v, int shift) {
+  const uint64_t a = v < 0 ? 0ull - (uint64_t)v : (uint64_t)v;
+  if (a == 0) return 0.0;
+  const int z = __clzll((long long)a);
+  const uint64_t m = ((a << z) >> 10) + 1 >> 1;  // 53 bits, rounded (2^53 carries into the exponent)
+  const uint64_t e = (uint64_t)(1023 + 63 - z - shift) << 52;
+  return __longlong_as_double((long long)((e + (m - 0x10000000000000ull)) | ((uint64_t)v & 0x8000000000000000ull)));
+}
+
+// Row i's entries k = lane, lane + kLanes, ... on the fixed-point positions x:
+// body(sep, R, j) for each pair beyond kFixNear and within the cut-off,
+// masked(take, ...) style: take is false for the others; close(e) follows for
+// the pairs nearer than that, which take the double terms.
+template <class Body, class Close>
+__device__ __forceinline__ void for_pairs_fixed(const P &c, const D &d, int i, int lane, const FixPos *x, Body &&body,
+                                                Close &&close) {
+  const int cnt = d.cnt[i];
+  const uint32_t *row = d.nbr + (size_t)i * c.cap;
+  const FixPos own = ld_fix<false>(x + i);
+  const uint32_t none = ((uint32_t)i << kImageBits) | 0x15u;
+  uint32_t e0 = lane < cnt ? row[lane] : none, e1 = lane + kLanes < cnt ? row[lane + kLanes] : none;
+  FixPos q0 = ld_fix<false>(x + (e0 >> kImageBits));
+  for (int k = lane; k < cnt; k += kLanes) {
+    const FixPos q1 = ld_fix<false>(x + (e1 >> kImageBits));
+    const uint32_t e2 = k + 2 * kLanes < cnt ? row[k + 2 * kLanes] : none;
+    int dx = q0.x - own.x, dy = q0.y - own.y, dz = q0.z - own.z;
+    float lx = q0.lx - own.lx, ly = q0.ly - own.ly, lz = q0.lz - own.lz;
+    const uint32_t ix = e0 & 3u, iy = (e0 >> 2) & 3u, iz = (e0 >> 4) & 3u;  // d = q_j - r L - q_i, r + 1 stored
+    if (ix != 1u) { dx += ix ? -c.fx_L[0] : c.fx_L[0]; lx += ix ? -c.fx_l[0] : c.fx_l[0]; }
+    if (iy != 1u) { dy += iy ? -c.fx_L[1] : c.fx_L[1]; ly += iy ? -c.fx_l[1] : c.fx_l[1]; }
+    if (iz != 1u) { dz += iz ? -c.fx_L[2] : c.fx_L[2]; lz += iz ? -c.fx_l[2] : c.fx_l[2]; }
+    const FixSep sep = fix_sep(dx, dy, dz, lx, ly, lz);
+    const uint64_t R = fix_r2(sep);
+    const bool in = R <= c.fx_rc2, near = in && R < c.fx_near;
+    body(in && !near, sep, R, (int)(e0 >> kImageBits));
+    if (near) close(e0);
+    e0 = e1;
+    q0 = q1;
+    e1 = e2;
+  }
+}
+
+// A double pair of the row of i (close pairs and rows whose integer sums do
+// not fit): body(t, dx, dy, dz, j) as for_pairs'.
+template <class Body>
+__device__ __forceinline__ void one_pair(const P &c, uint32_t e, const double4_32a *q, const Home &h, Body &&body) {
+  double dx, dy, dz;
+  const int j = pair_sep(e, q, h, dx, dy, dz);
+  PairTerms t;
+  if (pair_terms(c, dx * dx + dy * dy + dz * dz, t)) body(t, dx, dy, dz, j);
+}
+
+__device__ __forceinline__ void lane_sums(FixForce &f) {
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) {
+    f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
+    f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
+    f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
+    f.mx += __shfl_xor_sync(0xffffffffu, f.mx, o);
+    f.my += __shfl_xor_sync(0xffffffffu, f.my, o);
+    f.mz += __shfl_xor_sync(0xffffffffu, f.mz, o);
+    f.cx += __shfl_xor_sync(0xffffffffu, f.cx, o);
+    f.cy += __shfl_xor_sync(0xffffffffu, f.cy, o);
+    f.cz += __shfl_xor_sync(0xffffffffu, f.cz, o);
+    f.s += __shfl_xor_sync(0xffffffffu, f.s, o);
+  }
+}
+
+// Half the range of fix_sum_fits: the derivative sums are below twice the force's.
+__device__ __forceinline__ bool sums_fit(const FixForce &f, int n) { return f.s >= (float)(7 * n - 850) * 8388608.0f; }
+
+// scale times the vector sum; unit 2^-52.
+__device__ __forceinline__ double3 fix_vector(const FixForce &f, double scale) {
+  const double u = scale * (1.0 / (double)(1ull << kFixSumBits));
+  return make_double3(fix_sum(f.x, f.mx, f.cx) * u, fix_sum(f.y, f.my, f.cy) * u, fix_sum(f.z, f.mz, f.cz) * u);
+}
+
+// Sums of z = y^3, z^2 (2^-54) and r^2 (2^-51) over a row and its pair count,
+// as the single box's observers (mdg_fixed.cu).
+struct FixSums {
+  uint64_t z, zz, r;
+  int m;
+};
+constexpr int kFixSumsRow = 361;  // longest row whose sums fit
+
+__device__ __forceinline__ void fix_sums_add(FixSums &s, bool take, uint64_t y3, uint64_t R) {
+  const uint64_t zz = fix_sqrhi(y3);
+  s.z += take ? y3 >> 7 : 0;
+  s.zz += take ? zz >> 4 : 0;
+  s.r += take ? R >> 7 : 0;
+  s.m += take ? 1 : 0;
+}
+
+__device__ __forceinline__ void lane_sums(FixSums &s) {
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) {
+    s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+    s.zz += __shfl_xor_sync(0xffffffffu, s.zz, o);
+    s.r += __shfl_xor_sync(0xffffffffu, s.r, o);
+    s.m += __shfl_xor_sync(0xffffffffu, s.m, o);
+  }
+}
+
+// The row's sums of x^-6, x^-12, x^2 as doubles, and its pair count.
+__device__ __forceinline__ double3 fix_sums_double(const P &c, const FixSums &s) {
+  const double u = 1.0 / (double)(1ull << 54), half = 0.5 * s.m;
+  return make_double3(((double)s.z + half) * u, ((double)s.zz + half) * u,
+                      ((double)s.r + half) * (1.0 / (double)(1ull << 51)) * c.inv_s2);
+}
+
 // Block sums of three values at once (thread 0 holds them).
 __device__ __forceinline__ void block_sum3(double &a, double &b, double &e, double *sh) {
   for (int o = 16; o > 0; o >>= 1) {
@@ -231,13 +406,6 @@ __device__ void partials_accumulate(const D &d, double A, double B, double E, do
     d.acc[2] += w * e;
     *d.done = 0;
   }
-}
-
-// Sum over the kLanes lanes that share a particle (all lanes hold the total).
-__device__ __forceinline__ double lane_sum(double v) {
-#pragma unroll
-  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
 }
 
 // Pair list at positions q (wrapped into the box): every partner within the
@@ -308,122 +476,6 @@ __global__ void __launch_bounds__(kT) k_build(P c, D d, const double4_32a *q) {
   }
 }
 
-// One step from the half-step positions q: the forces F there (the lanes of
-// a particle), then, by its lane 0, p_out = p_in + F dt, q_out = q + p_out dt/2
-// and, when qh_next is given, the next step's first half-drift
-// qh_next = q_out + p_out dt/2 (the operations k_drift performs).  Out of
-// place: q_out and qh_next must not alias q, which other particles' lanes
-// still read; p_out may alias p_in.  Also the segment's displacement check
-// (a particle more than margin/2 from where the segment's list was built).
-// With VAL = 0 or 1 (the potential-energy or pressure objective) the kernel
-// also adds w times the objective's value at the previous whole-step state
-// (q_obj, p_in) to acc[0], as k_objective<VAL, 0> does (same row walk, lanes
-// and reductions, so the same bits); q_obj must be in this step's segment.
-template <int VAL>
-__global__ void k_step(P c, D d, const double4_32a *q, const double4_32a *p_in, double4_32a *q_out,
-                       double4_32a *p_out, double4_32a *qh_next, const double4_32a *q_obj, double w) {
-  __shared__ double sh[96];
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / kLanes, lane = tid % kLanes;
-  double fx = 0, fy = 0, fz = 0;
-  double u = 0, G = 0;
-  double4_32a qi = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-  if (i < c.n) {
-    qi = q[i];
-    if (lane == 0) {
-      const double4_32a z = d.q0[i];
-      const double ux = qi.x - z.x, uy = qi.y - z.y, uz = qi.z - z.z;
-      if (ux * ux + uy * uy + uz * uz > c.half_margin2) atomicMax(d.flag + 1, 1);
-    }
-    const Home h = make_home(c, qi);
-    for_pairs(c, d, i, lane, q, h, [&](const PairTerms &t, double dx, double dy, double dz, int) {
-      fx += t.f * dx;
-      fy += t.f * dy;
-      fz += t.f * dz;
-    });
-    if (VAL >= 0) {
-      const Home ho = make_home(c, q_obj[i]);
-      for_pairs(c, d, i, lane, q_obj, ho, [&](const PairTerms &t, double, double, double, int) {
-        if (VAL == 0) u += 0.5 * t.phi;
-        else G += 0.5 * t.g;
-      });
-    }
-  }
-  fx = lane_sum(fx);
-  fy = lane_sum(fy);
-  fz = lane_sum(fz);
-  double val = 0.0;
-  if (VAL == 0) u = lane_sum(u);
-  if (VAL == 1) G = lane_sum(G);
-  if (i < c.n && lane == 0) {
-    double4_32a b = p_in[i];
-    if (VAL == 0) val = u * (1.0 / (double)c.n);
-    if (VAL == 1) val = (2.0 * (0.5 * (b.x * b.x + b.y * b.y + b.z * b.z)) - G) * (1.0 / (3.0 * c.volume));
-    b.x += fx * c.dt;
-    b.y += fy * c.dt;
-    b.z += fz * c.dt;
-    p_out[i] = b;
-    double4_32a a = qi;
-    a.x += b.x * c.dt2;
-    a.y += b.y * c.dt2;
-    a.z += b.z * c.dt2;
-    q_out[i] = a;
-    if (qh_next) {
-      a.x += b.x * c.dt2;
-      a.y += b.y * c.dt2;
-      a.z += b.z * c.dt2;
-      qh_next[i] = a;
-    }
-  }
-  if (VAL >= 0) {
-    double none1 = 0.0, none2 = 0.0;
-    block_sum3(val, none1, none2, sh);
-    partials_accumulate(d, val, 0.0, 0.0, w);
-  }
-}
-
-// qh = q + p dt/2: the first half-drift of a trajectory or segment
-__global__ void k_drift(P c, const double4_32a *q, const double4_32a *p, double4_32a *out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n) return;
-  double4_32a a = q[i];
-  const double4_32a b = p[i];
-  a.x += b.x * c.dt2;
-  a.y += b.y * c.dt2;
-  a.z += b.z * c.dt2;
-  out[i] = a;
-}
-
-// A segment's first state: with wrap, positions into the box, q - k L per
-// axis with k = floor(q / L) (particles already inside keep their bits); then
-// the float copy for the list test.  The backward pass calls it without wrap
-// on the checkpoint the forward pass wrapped.
-__global__ void k_wrap(P c, double4_32a *q, float4 *qf, int wrap) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n) return;
-  double4_32a a = q[i];
-  if (wrap) {
-    const double kx = floor(a.x * c.inv_L[0]), ky = floor(a.y * c.inv_L[1]), kz = floor(a.z * c.inv_L[2]);
-    if (kx != 0.0) a.x = fma(-kx, c.L[0], a.x);
-    if (ky != 0.0) a.y = fma(-ky, c.L[1], a.y);
-    if (kz != 0.0) a.z = fma(-kz, c.L[2], a.z);
-    q[i] = a;
-  }
-  qf[i] = make_float4((float)a.x, (float)a.y, (float)a.z, 0.f);
-}
-
-// The reverse of a step's second half-drift q_n = qh + dt/2 p_n for particle
-// i, from the adjoints a, b of (q_n, p_n): a_p += dt/2 a_q.  tmp receives the
-// adjoint of p after the kick (the neighbours' H v reads it), aqh that of qh.
-__device__ __forceinline__ void reverse_drift(const P &c, const D &d, int i, const double4_32a &a, double4_32a b,
-                                              double4_32a *tmp) {
-  b.x += c.dt2 * a.x;
-  b.y += c.dt2 * a.y;
-  b.z += c.dt2 * a.z;
-  tmp[i] = b;
-  d.aqh[i] = a;
-}
-
 // Particle i's pair sums of the objective at positions q (every lane holds
 // them after the lane sums; all threads of the block call it).
 struct ObjSums {
@@ -470,6 +522,279 @@ __device__ __forceinline__ ObjSums objective_sums(const P &c, const D &d, int i,
   return r;
 }
 
+// The same in fixed point (every thread of the warp calls it).
+template <int OBJ, bool GRAD>
+__device__ __forceinline__ ObjSums objective_sums_fixed(const P &c, const D &d, int i, int lane, const double4_32a *q,
+                                                        const FixPos *x) {
+  ObjSums r{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  FixSums s{0, 0, 0, 0};
+  FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f};  // psi d (potential energy) or the slope of chi / 8 (pressure)
+  auto in_double = [&](const PairTerms &t, double dx, double dy, double dz, int) {
+    if (OBJ == 0) {
+      r.u += 0.5 * t.phi;
+      if (GRAD) {
+        r.us += 0.5 * t.dphis;
+        r.gx -= t.f * dx;
+        r.gy -= t.f * dy;
+        r.gz -= t.f * dz;
+      }
+    } else {
+      r.G += 0.5 * t.g;
+      if (GRAD) {
+        r.Gs += 0.5 * t.gs;
+        r.gx += t.gpr * dx;
+        r.gy += t.gpr * dy;
+        r.gz += t.gpr * dz;
+      }
+    }
+  };
+  bool near = false;
+  float psi = 0.f;
+  int cnt = 0;
+  if (i < c.n) {
+    cnt = d.cnt[i];
+    for_pairs_fixed(
+        c, d, i, lane, x,
+        [&](bool take, const FixSep &sep, uint64_t R, int) {
+          if (GRAD) {
+            const FixTerms t = fix_terms(c, R);
+            fix_sums_add(s, take, t.y3, R);
+            const int64_t v = OBJ == 0 ? fix_psi(c, t) : fix_dsigma(c, t);
+            fix_add(f, take ? v : 0, sep);
+            if (OBJ == 1) psi += (float)fix_shi(take ? fix_psi(c, t) : 0);
+          } else {
+            uint64_t y2, z;
+            fix_powers(fix_y(c, R), y2, z);
+            fix_sums_add(s, take, z, R);
+          }
+        },
+        [&](uint32_t e) {
+          near = true;
+          one_pair(c, e, q, make_home(c, q[i]), in_double);
+        });
+  }
+  __syncwarp();
+  lane_sums(s);
+  if (GRAD) lane_sums(f);
+  if (GRAD && OBJ == 1) {
+#pragma unroll
+    for (int o = 1; o < kLanes; o <<= 1) psi += __shfl_xor_sync(0xffffffffu, psi, o);
+    f.s = psi;
+  }
+  if (__any_sync(0xffffffffu, near)) {
+    if (GRAD) {
+      r.gx = lane_sum(r.gx);
+      r.gy = lane_sum(r.gy);
+      r.gz = lane_sum(r.gz);
+    }
+    if (OBJ == 0) {
+      r.u = lane_sum(r.u);
+      if (GRAD) r.us = lane_sum(r.us);
+    } else {
+      r.G = lane_sum(r.G);
+      if (GRAD) r.Gs = lane_sum(r.Gs);
+    }
+  }
+  if (lane != 0 || i >= c.n) return r;
+  if (cnt > kFixSumsRow || (GRAD && !sums_fit(f, cnt))) {  // the row again in double
+    r = ObjSums{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const Home h = make_home(c, q[i]);
+    for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], q, h, in_double);
+    return r;
+  }
+  const double3 t = fix_sums_double(c, s);  // x^-6, x^-12, x^2
+  if (OBJ == 0) {
+    r.u += 2.0 * c.eps * ((t.y - t.x) + (c.c2 * t.z + c.c0 * (double)s.m));
+    if (GRAD) {
+      const double3 g = fix_vector(f, c.e_s2);
+      r.us += c.e_s * (12.0 * (2.0 * t.y - t.x) - 4.0 * c.c2 * t.z);
+      r.gx -= g.x;
+      r.gy -= g.y;
+      r.gz -= g.z;
+    }
+  } else {
+    r.G += c.eps * (12.0 * (t.x - 2.0 * t.y) + 4.0 * c.c2 * t.z);
+    if (GRAD) {
+      const double3 g = fix_vector(f, -8.0 * c.e_s2);
+      r.Gs += c.e_s * (72.0 * (t.x - 4.0 * t.y) - 8.0 * c.c2 * t.z);
+      r.gx += g.x;
+      r.gy += g.y;
+      r.gz += g.z;
+    }
+  }
+  return r;
+}
+
+// The force on particle i in fixed point, to lane 0 (every thread of the warp
+// calls it).
+__device__ __forceinline__ double3 force_sums_fixed(const P &c, const D &d, int i, int lane, const double4_32a *q,
+                                                    const FixPos *x) {
+  FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f};
+  double3 n = make_double3(0.0, 0.0, 0.0);
+  auto in_double = [&](const PairTerms &t, double dx, double dy, double dz, int) {
+    n.x += t.f * dx;
+    n.y += t.f * dy;
+    n.z += t.f * dz;
+  };
+  bool near = false;
+  int cnt = 0;
+  if (i < c.n) {
+    cnt = d.cnt[i];
+    for_pairs_fixed(
+        c, d, i, lane, x,
+        [&](bool take, const FixSep &sep, uint64_t R, int) {
+          const int64_t v = fix_psi(c, fix_terms(c, R));
+          fix_add(f, take ? v : 0, sep);
+        },
+        [&](uint32_t e) {
+          near = true;
+          one_pair(c, e, q, make_home(c, q[i]), in_double);
+        });
+  }
+  __syncwarp();
+  lane_sums(f);
+  if (__any_sync(0xffffffffu, near)) n = make_double3(lane_sum(n.x), lane_sum(n.y), lane_sum(n.z));
+  if (lane != 0 || i >= c.n) return n;
+  if (!sums_fit(f, cnt)) {
+    n = make_double3(0.0, 0.0, 0.0);
+    const Home h = make_home(c, q[i]);
+    for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], q, h, in_double);
+    return n;
+  }
+  const double3 F = fix_vector(f, c.e_s2);
+  return make_double3(F.x + n.x, F.y + n.y, F.z + n.z);
+}
+
+// One step from the half-step positions q: the forces F there (the lanes of
+// a particle), then, by its lane 0, p_out = p_in + F dt, q_out = q + p_out dt/2
+// and, when qh_next is given, the next step's first half-drift
+// qh_next = q_out + p_out dt/2 (the operations k_drift performs).  Out of
+// place: q_out and qh_next must not alias q, which other particles' lanes
+// still read; p_out may alias p_in.  Also the segment's displacement check
+// (a particle more than margin/2 from where the segment's list was built).
+// With VAL = 0 or 1 (the potential-energy or pressure objective) the kernel
+// also adds w times the objective's value at the previous whole-step state
+// (q_obj, p_in) to acc[0], as k_objective<VAL, 0> does (same row walk, lanes
+// and reductions, so the same bits); q_obj must be in this step's segment.
+// FIXED: the pair sums in fixed point on xq, x_obj (the positions q, q_obj).
+template <int VAL, bool FIXED>
+__global__ void k_step(P c, D d, const double4_32a *q, const double4_32a *p_in, double4_32a *q_out,
+                       double4_32a *p_out, double4_32a *qh_next, const double4_32a *q_obj, double w, const FixPos *xq,
+                       FixPos *x_out, FixPos *xh_next, const FixPos *x_obj) {
+  __shared__ double sh[96];
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = tid / kLanes, lane = tid % kLanes;
+  double3 F = make_double3(0.0, 0.0, 0.0);
+  double u = 0, G = 0;
+  double4_32a qi = make_double4_32a(0.0, 0.0, 0.0, 0.0);
+  if (i < c.n) {
+    qi = q[i];
+    if (lane == 0) {
+      const double4_32a z = d.q0[i];
+      const double ux = qi.x - z.x, uy = qi.y - z.y, uz = qi.z - z.z;
+      if (ux * ux + uy * uy + uz * uz > c.half_margin2) atomicMax(d.flag + 1, 1);
+    }
+  }
+  if (FIXED) {
+    F = force_sums_fixed(c, d, i, lane, q, xq);
+    if (VAL >= 0) {
+      const ObjSums r = objective_sums_fixed<(VAL < 0 ? 0 : VAL), false>(c, d, i, lane, q_obj, x_obj);
+      u = r.u;
+      G = r.G;
+    }
+  } else {
+    if (i < c.n) {
+      const Home h = make_home(c, qi);
+      for_pairs(c, d, i, lane, q, h, [&](const PairTerms &t, double dx, double dy, double dz, int) {
+        F.x += t.f * dx;
+        F.y += t.f * dy;
+        F.z += t.f * dz;
+      });
+      if (VAL >= 0) {
+        const Home ho = make_home(c, q_obj[i]);
+        for_pairs(c, d, i, lane, q_obj, ho, [&](const PairTerms &t, double, double, double, int) {
+          if (VAL == 0) u += 0.5 * t.phi;
+          else G += 0.5 * t.g;
+        });
+      }
+    }
+    F = make_double3(lane_sum(F.x), lane_sum(F.y), lane_sum(F.z));
+    if (VAL == 0) u = lane_sum(u);
+    if (VAL == 1) G = lane_sum(G);
+  }
+  double val = 0.0;
+  if (i < c.n && lane == 0) {
+    double4_32a b = p_in[i];
+    if (VAL == 0) val = u * (1.0 / (double)c.n);
+    if (VAL == 1) val = (2.0 * (0.5 * (b.x * b.x + b.y * b.y + b.z * b.z)) - G) * (1.0 / (3.0 * c.volume));
+    b.x += F.x * c.dt;
+    b.y += F.y * c.dt;
+    b.z += F.z * c.dt;
+    p_out[i] = b;
+    double4_32a a = qi;
+    a.x += b.x * c.dt2;
+    a.y += b.y * c.dt2;
+    a.z += b.z * c.dt2;
+    q_out[i] = a;
+    if (FIXED) x_out[i] = fix_position(a.x, a.y, a.z, 0);
+    if (qh_next) {
+      a.x += b.x * c.dt2;
+      a.y += b.y * c.dt2;
+      a.z += b.z * c.dt2;
+      qh_next[i] = a;
+      if (FIXED) xh_next[i] = fix_position(a.x, a.y, a.z, 0);
+    }
+  }
+  if (VAL >= 0) {
+    double none1 = 0.0, none2 = 0.0;
+    block_sum3(val, none1, none2, sh);
+    partials_accumulate(d, val, 0.0, 0.0, w);
+  }
+}
+
+// qh = q + p dt/2: the first half-drift of a trajectory or segment
+__global__ void k_drift(P c, const double4_32a *q, const double4_32a *p, double4_32a *out, FixPos *xout) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c.n) return;
+  double4_32a a = q[i];
+  const double4_32a b = p[i];
+  a.x += b.x * c.dt2;
+  a.y += b.y * c.dt2;
+  a.z += b.z * c.dt2;
+  out[i] = a;
+  if (c.fixed) xout[i] = fix_position(a.x, a.y, a.z, 0);
+}
+
+// A segment's first state: with wrap, positions into the box, q - k L per
+// axis with k = floor(q / L) (particles already inside keep their bits); then
+// the float copy for the list test.  The backward pass calls it without wrap
+// on the checkpoint the forward pass wrapped.
+__global__ void k_wrap(P c, double4_32a *q, float4 *qf, int wrap) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c.n) return;
+  double4_32a a = q[i];
+  if (wrap) {
+    const double kx = floor(a.x * c.inv_L[0]), ky = floor(a.y * c.inv_L[1]), kz = floor(a.z * c.inv_L[2]);
+    if (kx != 0.0) a.x = fma(-kx, c.L[0], a.x);
+    if (ky != 0.0) a.y = fma(-ky, c.L[1], a.y);
+    if (kz != 0.0) a.z = fma(-kz, c.L[2], a.z);
+    q[i] = a;
+  }
+  qf[i] = make_float4((float)a.x, (float)a.y, (float)a.z, 0.f);
+}
+
+// The reverse of a step's second half-drift q_n = qh + dt/2 p_n for particle
+// i, from the adjoints a, b of (q_n, p_n): a_p += dt/2 a_q.  tmp receives the
+// adjoint of p after the kick (the neighbours' H v reads it), aqh that of qh.
+__device__ __forceinline__ void reverse_drift(const P &c, const D &d, int i, const double4_32a &a, double4_32a b,
+                                              double4_32a *tmp) {
+  b.x += c.dt2 * a.x;
+  b.y += c.dt2 * a.y;
+  b.z += c.dt2 * a.z;
+  tmp[i] = b;
+  d.aqh[i] = a;
+}
+
 // Particle i's objective terms from its sums (lane 0): the value and its
 // epsilon and sigma derivatives; with GRAD, w dj/dq added to a and w dj/dp
 // to b (the adjoints of the state's q and p).
@@ -512,14 +837,14 @@ __device__ __forceinline__ void objective_finish(const P &c, const ObjSums &r, c
 // the forward pass returns J alone (the parameter terms of the gradient are
 // summed in the backward pass), so without GRAD the sigma derivative is left
 // out and its partial is zero.
-template <int OBJ, int GRAD>
-__global__ void k_objective(P c, D d, const double4_32a *q, const double4_32a *p, double w, double4_32a *tmp) {
+template <int OBJ, int GRAD, bool FIXED>
+__global__ void k_objective(P c, D d, const double4_32a *q, const double4_32a *p, double w, double4_32a *tmp, const FixPos *x) {
   constexpr bool grad = GRAD != 0;
   __shared__ double sh[96];
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = tid / kLanes, lane = tid % kLanes;
   double val = 0, ge = 0, gs = 0;
-  const ObjSums r = objective_sums<OBJ, grad>(c, d, i, lane, q);
+  const ObjSums r = FIXED ? objective_sums_fixed<OBJ, grad>(c, d, i, lane, q, x) : objective_sums<OBJ, grad>(c, d, i, lane, q);
   if (i < c.n && lane == 0) {
     double4_32a a = make_double4_32a(0.0, 0.0, 0.0, 0.0), b = a;
     if (grad) {
@@ -542,38 +867,99 @@ __global__ void k_objective(P c, D d, const double4_32a *q, const double4_32a *p
 // computes them, and the reverse of step n - 1's second half-drift, into
 // tmp_out (not tmp: other particles' lanes still read it) and aqh instead of
 // aq, ap.
-template <int OBJ>
+template <int OBJ, bool FIXED>
 __global__ void k_reverse_hvp(P c, D d, const double4_32a *qh, const double4_32a *tmp, const double4_32a *q_obj,
-                              const double4_32a *p_obj, double w, double4_32a *tmp_out) {
+                              const double4_32a *p_obj, double w, double4_32a *tmp_out, const FixPos *xh, const FixPos *x_obj) {
   __shared__ double sh[96];
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = tid / kLanes, lane = tid % kLanes;
   double te = 0, ts = 0;
   double hx = 0, hy = 0, hz = 0, fx = 0, fy = 0, fz = 0, sx = 0, sy = 0, sz = 0;
-  if (i < c.n) {
-    const double4_32a qi = qh[i], vi = tmp[i];
-    const Home h = make_home(c, qi);
-    for_pairs(c, d, i, lane, qh, h, [&](const PairTerms &t, double dx, double dy, double dz, int j) {
-      const double4_32a vj = tmp[j];
-      const double wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
-      const double dw = dx * wx + dy * wy + dz * wz;
-      // (H v)_i = sum_j f (v_i - v_j) + (f'/r) d (d . (v_i - v_j))
-      hx += t.f * wx + t.fpr * dx * dw;
-      hy += t.f * wy + t.fpr * dy * dw;
-      hz += t.f * wz + t.fpr * dz * dw;
-      fx += t.f * dx;
-      fy += t.f * dy;
-      fz += t.f * dz;
-      sx += t.fs * dx;
-      sy += t.fs * dy;
-      sz += t.fs * dz;
-    });
-  }
-  hx = lane_sum(hx); hy = lane_sum(hy); hz = lane_sum(hz);
-  fx = lane_sum(fx); fy = lane_sum(fy); fz = lane_sum(fz);
-  sx = lane_sum(sx); sy = lane_sum(sy); sz = lane_sum(sz);
   ObjSums r{};
-  if (OBJ >= 0) r = objective_sums<(OBJ >= 0 ? OBJ : 0), true>(c, d, i, lane, q_obj);
+  auto in_double = [&](const PairTerms &t, double dx, double dy, double dz, int j) {
+    const double4_32a vi = tmp[i], vj = tmp[j];
+    const double wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
+    const double dw = dx * wx + dy * wy + dz * wz;
+    // (H v)_i = sum_j f (v_i - v_j) + (f'/r) d (d . (v_i - v_j))
+    hx += t.f * wx + t.fpr * dx * dw;
+    hy += t.f * wy + t.fpr * dy * dw;
+    hz += t.f * wz + t.fpr * dz * dw;
+    fx += t.f * dx;
+    fy += t.f * dy;
+    fz += t.f * dz;
+    sx += t.fs * dx;
+    sy += t.fs * dy;
+    sz += t.fs * dz;
+  };
+  if (FIXED) {
+    FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f}, g = f;  // psi d; the sigma derivative's eighth
+    // reduced sums psi w and (psi' / x) / 48 (d . w) d
+    double ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
+    bool near = false;
+    int cnt = 0;
+    if (i < c.n) {
+      cnt = d.cnt[i];
+      const double4_32a vi = tmp[i];
+      for_pairs_fixed(
+          c, d, i, lane, xh,
+          [&](bool take, const FixSep &sep, uint64_t R, int j) {
+            const double4_32a vj = tmp[j];
+            const FixTerms t = fix_terms(c, R);
+            const int64_t psi = take ? fix_psi(c, t) : 0, slope = take ? fix_psi_slope(t) : 0;
+            fix_add(f, psi, sep);
+            fix_add(g, take ? fix_dsigma(c, t) : 0, sep);
+            // the separation as doubles: high words and rests in units of 2^-59
+            auto whole = [](int h, float l) {
+              return fix_double(((int64_t)h << 30) + (int64_t)__float2int_rn(l * 2147483648.0f), 59);
+            };
+            const double dx = whole(sep.x, sep.lx), dy = whole(sep.y, sep.ly), dz = whole(sep.z, sep.lz);
+            const double wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
+            const double p = fix_double(psi, 55), k = fix_double(slope, 55) * fma(dz, wz, fma(dy, wy, dx * wx));
+            ax = fma(p, wx, ax);
+            ay = fma(p, wy, ay);
+            az = fma(p, wz, az);
+            bx = fma(k, dx, bx);
+            by = fma(k, dy, by);
+            bz = fma(k, dz, bz);
+          },
+          [&](uint32_t e) {
+            near = true;
+            one_pair(c, e, qh, make_home(c, qh[i]), in_double);
+          });
+    }
+    __syncwarp();
+    lane_sums(f);
+    lane_sums(g);
+    const double e4 = 48.0 * c.e_s4;
+    hx = lane_sum(fma(c.e_s2, ax, fma(e4, bx, hx)));
+    hy = lane_sum(fma(c.e_s2, ay, fma(e4, by, hy)));
+    hz = lane_sum(fma(c.e_s2, az, fma(e4, bz, hz)));
+    if (__any_sync(0xffffffffu, near)) {
+      fx = lane_sum(fx); fy = lane_sum(fy); fz = lane_sum(fz);
+      sx = lane_sum(sx); sy = lane_sum(sy); sz = lane_sum(sz);
+    }
+    if (lane == 0 && i < c.n) {
+      if (sums_fit(f, cnt)) {
+        const double3 F = fix_vector(f, c.e_s2), S = fix_vector(g, 8.0 * c.e_s3);
+        fx += F.x; fy += F.y; fz += F.z;
+        sx += S.x; sy += S.y; sz += S.z;
+      } else {  // the row again in double
+        hx = hy = hz = fx = fy = fz = sx = sy = sz = 0.0;
+        const Home h = make_home(c, qh[i]);
+        for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], qh, h, in_double);
+      }
+    }
+    if (OBJ >= 0) r = objective_sums_fixed<(OBJ >= 0 ? OBJ : 0), true>(c, d, i, lane, q_obj, x_obj);
+  } else {
+    if (i < c.n) {
+      const Home h = make_home(c, qh[i]);
+      for_pairs(c, d, i, lane, qh, h, in_double);
+    }
+    hx = lane_sum(hx); hy = lane_sum(hy); hz = lane_sum(hz);
+    fx = lane_sum(fx); fy = lane_sum(fy); fz = lane_sum(fz);
+    sx = lane_sum(sx); sy = lane_sum(sy); sz = lane_sum(sz);
+    if (OBJ >= 0) r = objective_sums<(OBJ >= 0 ? OBJ : 0), true>(c, d, i, lane, q_obj);
+  }
   double val = 0, ge = 0, gs = 0;
   if (i < c.n && lane == 0) {
     const double4_32a b = tmp[i];
@@ -607,6 +993,7 @@ __global__ void k_reverse_hvp(P c, D d, const double4_32a *qh, const double4_32a
 }  // namespace mdg
 
 using namespace mdg::adj;
+using mdg::FixPos;
 
 struct mdg_adjoint {
   mdg_adjoint_params prm;
@@ -643,37 +1030,52 @@ cudaError_t aalloc(T **p, size_t n) {
   return cudaMalloc((void **)p, (n ? n : 1) * sizeof(T));
 }
 
-void launch_objective(mdg_adjoint *a, const double4_32a *q, const double4_32a *p, bool grad, double w,
+// Launches kernel<.., true> or kernel<.., false> by the fixed-point flag.
+#define MDG_ADJ(KERNEL, TMPL, ...)                                               \
+  do {                                                                           \
+    if (a->c.fixed) KERNEL<TMPL, true><<<a->gridp, kT, 0, a->s>>>(__VA_ARGS__);  \
+    else KERNEL<TMPL, false><<<a->gridp, kT, 0, a->s>>>(__VA_ARGS__);            \
+  } while (0)
+#define MDG_TWO(A, B) A, B
+
+void launch_objective(mdg_adjoint *a, const double4_32a *q, const double4_32a *p, const FixPos *x, bool grad, double w,
                       double4_32a *tmp = nullptr) {
   const int obj = a->c.objective;
-  if (obj == 0 && !grad) k_objective<0, 0><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, q, p, w, tmp);
-  else if (obj == 0) k_objective<0, 1><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, q, p, w, tmp);
-  else if (!grad) k_objective<1, 0><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, q, p, w, tmp);
-  else k_objective<1, 1><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, q, p, w, tmp);
+  if (obj == 0 && !grad) MDG_ADJ(k_objective, MDG_TWO(0, 0), a->c, a->d, q, p, w, tmp, x);
+  else if (obj == 0) MDG_ADJ(k_objective, MDG_TWO(0, 1), a->c, a->d, q, p, w, tmp, x);
+  else if (!grad) MDG_ADJ(k_objective, MDG_TWO(1, 0), a->c, a->d, q, p, w, tmp, x);
+  else MDG_ADJ(k_objective, MDG_TWO(1, 1), a->c, a->d, q, p, w, tmp, x);
 }
 
-// The reverse of step n (half-step positions qh, tmp from its second
+// The reverse of step n (half-step positions qh, xh; tmp from its second
 // half-drift's reverse), with, when q_obj is given, the objective terms of
 // state n - 1 and the reverse of step n - 1's second half-drift into tmp_out.
-void launch_reverse(mdg_adjoint *a, const double4_32a *qh, const double4_32a *tmp, const double4_32a *q_obj,
-                    const double4_32a *p_obj, double w, double4_32a *tmp_out) {
+void launch_reverse(mdg_adjoint *a, const double4_32a *qh, const FixPos *xh, const double4_32a *tmp, const double4_32a *q_obj,
+                    const double4_32a *p_obj, const FixPos *x_obj, double w, double4_32a *tmp_out) {
   const int obj = a->c.objective;
-  if (!q_obj) k_reverse_hvp<-1><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, qh, tmp, nullptr, nullptr, 0.0, nullptr);
-  else if (obj == 0) k_reverse_hvp<0><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, qh, tmp, q_obj, p_obj, w, tmp_out);
-  else k_reverse_hvp<1><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, qh, tmp, q_obj, p_obj, w, tmp_out);
+  if (!q_obj) MDG_ADJ(k_reverse_hvp, -1, a->c, a->d, qh, tmp, nullptr, nullptr, 0.0, nullptr, xh, nullptr);
+  else if (obj == 0) MDG_ADJ(k_reverse_hvp, 0, a->c, a->d, qh, tmp, q_obj, p_obj, w, tmp_out, xh, x_obj);
+  else MDG_ADJ(k_reverse_hvp, 1, a->c, a->d, qh, tmp, q_obj, p_obj, w, tmp_out, xh, x_obj);
 }
 
-// One step from the half-step positions qh (already drifted from step k - 1)
-// and p_in: q_out, p_out and, when given, the next step's qh (not qh itself);
-// with q_obj, also w times the objective's value at (q_obj, p_in).
-void fwd_step(mdg_adjoint *a, const double4_32a *qh, const double4_32a *p_in, double4_32a *q_out,
-              double4_32a *p_out, double4_32a *qh_next, const double4_32a *q_obj = nullptr, double w = 0.0) {
-  if (!q_obj)
-    k_step<-1><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, qh, p_in, q_out, p_out, qh_next, nullptr, 0.0);
+// Positions with their fixed-point copy.
+struct Pos {
+  double4_32a *q;
+  FixPos *x;
+  Pos at(size_t k) const { return Pos{q + k, x + k}; }
+};
+
+// One step from the half-step positions h (already drifted from step k - 1)
+// and p_in: out, p_out and, when given, the next step's half-step positions
+// (not h itself); with obj, also w times the objective's value at (obj, p_in).
+void fwd_step(mdg_adjoint *a, const Pos &h, const double4_32a *p_in, const Pos &out, double4_32a *p_out, const Pos *next,
+              const Pos *obj = nullptr, double w = 0.0) {
+  double4_32a *nq = next ? next->q : nullptr;
+  FixPos *nx = next ? next->x : nullptr;
+  if (!obj) MDG_ADJ(k_step, -1, a->c, a->d, h.q, p_in, out.q, p_out, nq, nullptr, 0.0, h.x, out.x, nx, nullptr);
   else if (a->c.objective == 0)
-    k_step<0><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, qh, p_in, q_out, p_out, qh_next, q_obj, w);
-  else
-    k_step<1><<<a->gridp, kT, 0, a->s>>>(a->c, a->d, qh, p_in, q_out, p_out, qh_next, q_obj, w);
+    MDG_ADJ(k_step, 0, a->c, a->d, h.q, p_in, out.q, p_out, nq, obj->q, w, h.x, out.x, nx, obj->x);
+  else MDG_ADJ(k_step, 1, a->c, a->d, h.q, p_in, out.q, p_out, nq, obj->q, w, h.x, out.x, nx, obj->x);
 }
 
 // The horizon from the state in d.q, d.p: per segment its list, per step the
@@ -686,27 +1088,27 @@ int enqueue_forward(mdg_adjoint *a) {
   const int Ns = a->prm.steps, K = a->prm.checkpoint_every;
   const double w = 1.0 / Ns;
   // half-step and whole-step positions, both written out of place
-  double4_32a *qh = d.qh, *qh_alt = d.qh2, *q = d.q, *q_alt = d.q2;
+  Pos qh{d.qh, d.xqh}, qh_alt{d.qh2, d.xqh2}, q{d.q, d.xq}, q_alt{d.q2, d.xq2};
   for (int n = 1; n <= Ns; n++) {
     if ((n - 1) % K == 0) {  // a checkpoint segment starts: wrapped state, checkpoint, its own list
       const size_t ck = (size_t)((n - 1) / K);
-      k_wrap<<<a->grid, kT, 0, a->s>>>(a->c, q, d.qf, 1);
-      MDG_ACK(cudaMemcpyAsync(d.ckq + N * ck, q, bytes, cudaMemcpyDeviceToDevice, a->s));
+      k_wrap<<<a->grid, kT, 0, a->s>>>(a->c, q.q, d.qf, 1);
+      MDG_ACK(cudaMemcpyAsync(d.ckq + N * ck, q.q, bytes, cudaMemcpyDeviceToDevice, a->s));
       MDG_ACK(cudaMemcpyAsync(d.ckp + N * ck, d.p, bytes, cudaMemcpyDeviceToDevice, a->s));
-      MDG_ACK(cudaMemcpyAsync(d.q0, q, bytes, cudaMemcpyDeviceToDevice, a->s));
-      k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, q);
-      k_drift<<<a->grid, kT, 0, a->s>>>(a->c, q, d.p, qh);
+      MDG_ACK(cudaMemcpyAsync(d.q0, q.q, bytes, cudaMemcpyDeviceToDevice, a->s));
+      k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, q.q);
+      k_drift<<<a->grid, kT, 0, a->s>>>(a->c, q.q, d.p, qh.q, qh.x);
     }
     // the next step's half-drift here unless a segment starts there (as the
     // backward pass recomputes it: from the wrapped checkpoint); the
     // objective of state n - 1 rides along when that state is in this
     // step's segment (the states are summed in order either way)
-    double4_32a *next = n < Ns && n % K != 0 ? qh_alt : nullptr;
-    fwd_step(a, qh, d.p, q_alt, d.p, next, n > 1 && (n - 1) % K != 0 ? q : nullptr, w);
+    const Pos *next = n < Ns && n % K != 0 ? &qh_alt : nullptr;
+    fwd_step(a, qh, d.p, q_alt, d.p, next, n > 1 && (n - 1) % K != 0 ? &q : nullptr, w);
     std::swap(q, q_alt);
     if (next) std::swap(qh, qh_alt);
     // the last state of a segment (or of the horizon) with its own list
-    if (n % K == 0 || n == Ns) launch_objective(a, q, d.p, false, w);
+    if (n % K == 0 || n == Ns) launch_objective(a, q.q, d.p, q.x, false, w);
   }
   return cudaGetLastError() == cudaSuccess ? MDG_OK : afail(a, MDG_ERR_CUDA, "adjoint forward launch failed");
 }
@@ -731,22 +1133,26 @@ int enqueue_backward(mdg_adjoint *a) {
     MDG_ACK(cudaMemcpyAsync(d.q0, d.segq, bytes, cudaMemcpyDeviceToDevice, a->s));
     k_wrap<<<a->grid, kT, 0, a->s>>>(a->c, d.segq, d.qf, 0);
     k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, d.segq);
-    k_drift<<<a->grid, kT, 0, a->s>>>(a->c, d.segq, d.segp, d.segqh + N);
-    for (int k = 1; k <= len; k++)
-      fwd_step(a, d.segqh + N * k, d.segp + N * (k - 1), d.segq + N * k, d.segp + N * k,
-               k < len ? d.segqh + N * (k + 1) : nullptr);
+    k_drift<<<a->grid, kT, 0, a->s>>>(a->c, d.segq, d.segp, d.segqh + N, d.segxqh + N);
+    const Pos state{d.segq, d.segxq}, half{d.segqh, d.segxqh};
+    for (int k = 1; k <= len; k++) {
+      const Pos next = half.at(N * (k + 1));
+      fwd_step(a, half.at(N * k), d.segp + N * (k - 1), state.at(N * k), d.segp + N * k, k < len ? &next : nullptr);
+    }
     // objective terms of the segment's last state and the reverse of the
     // second half-drift of the step that produced it; then per step k the
     // rest of its reverse, going on (k > 1) with the objective terms of
     // state k - 1 and the reverse of step k - 1's second half-drift
     double4_32a *tmp = d.tmp, *tmp_alt = d.tmp2;
-    launch_objective(a, d.segq + N * len, d.segp + N * len, true, w, tmp);
+    launch_objective(a, d.segq + N * len, d.segp + N * len, d.segxq + N * len, true, w, tmp);
     for (int k = len; k >= 1; k--) {
+      const Pos h = half.at(N * k);
       if (k > 1) {
-        launch_reverse(a, d.segqh + N * k, tmp, d.segq + N * (k - 1), d.segp + N * (k - 1), w, tmp_alt);
+        const Pos o = state.at(N * (k - 1));
+        launch_reverse(a, h.q, h.x, tmp, o.q, d.segp + N * (k - 1), o.x, w, tmp_alt);
         std::swap(tmp, tmp_alt);
       } else {
-        launch_reverse(a, d.segqh + N * k, tmp, nullptr, nullptr, 0.0, nullptr);
+        launch_reverse(a, h.q, h.x, tmp, nullptr, nullptr, nullptr, 0.0, nullptr);
       }
     }
     seg_end = seg_start;
@@ -833,6 +1239,24 @@ int mdg_adjoint_create(const mdg_adjoint_params *p, int32_t n, mdg_adjoint **out
   c.sl2 = sl * sl;
   c.sl2f = (sl + 1e-3) * (sl + 1e-3);
   c.half_margin2 = 0.25 * p->margin * p->margin;
+  // Fixed-point pair arithmetic where every listed pair, each particle within
+  // margin / 2 of its place at the segment's start, stays below 4 sigma apart
+  // on every axis, sigma^2 / r^2 fits its format beyond kFixNear and the cut-off
+  // lies beyond it
+  c.fixed = sl + p->margin < 3.9 && p->sigma >= 0.8 && p->sigma <= 1.8 && p->cutoff >= 1.0 ? 1 : 0;
+  c.unit_sigma = p->sigma == 1.0 ? 1 : 0;
+  if (c.fixed) {
+    const double s2v = p->sigma * p->sigma, rcut = p->cutoff * p->sigma;
+    c.fx_rc2 = (uint64_t)std::ldexp(rcut * rcut, mdg::kFixR2Bits);
+    c.fx_near = (uint64_t)std::ldexp(mdg::kFixNear * s2v, mdg::kFixR2Bits);
+    c.fx_s2 = (uint64_t)std::ldexp(s2v, 62);
+    c.fx_c8 = mdg::fix_c8(8.0 * c.c2);
+    for (int k = 0; k < 3; k++) {
+      const int64_t L = mdg::fix_from_double(p->box[k]);
+      c.fx_L[k] = mdg::fix_shi(L);
+      c.fx_l[k] = mdg::fix_rest(L);
+    }
+  }
   c.volume = p->box[0] * p->box[1] * p->box[2];
   c.n = n;
   c.objective = p->objective;
@@ -854,6 +1278,13 @@ int mdg_adjoint_create(const mdg_adjoint_params *p, int32_t n, mdg_adjoint **out
   if (e == cudaSuccess) e = aalloc(&d.segq, N * (K + 1));
   if (e == cudaSuccess) e = aalloc(&d.segp, N * (K + 1));
   if (e == cudaSuccess) e = aalloc(&d.segqh, N * (K + 1));
+  const size_t X = c.fixed ? N : 0;
+  if (e == cudaSuccess) e = aalloc(&d.xq, X);
+  if (e == cudaSuccess) e = aalloc(&d.xq2, X);
+  if (e == cudaSuccess) e = aalloc(&d.xqh, X);
+  if (e == cudaSuccess) e = aalloc(&d.xqh2, X);
+  if (e == cudaSuccess) e = aalloc(&d.segxq, X * (K + 1));
+  if (e == cudaSuccess) e = aalloc(&d.segxqh, X * (K + 1));
   if (e == cudaSuccess) e = aalloc(&d.nbr, N * (size_t)c.cap);
   if (e == cudaSuccess) e = aalloc(&d.cnt, N);
   if (e == cudaSuccess) e = aalloc(&d.qf, N);
@@ -879,7 +1310,7 @@ int mdg_adjoint_destroy(mdg_adjoint *a) {
   if (a->gx_backward) cudaGraphExecDestroy(a->gx_backward);
   D &d = a->d;
   void *ptrs[] = {d.q, d.q2, d.p, d.qh, d.qh2, d.aq, d.ap, d.aqh, d.tmp, d.tmp2, d.q0, d.ckq, d.ckp, d.segq, d.segp, d.segqh,
-                  d.nbr, d.cnt, d.qf, d.part, d.acc, d.flag, d.done};
+                  d.nbr, d.cnt, d.qf, d.part, d.acc, d.flag, d.done, d.xq, d.xq2, d.xqh, d.xqh2, d.segxq, d.segxqh};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (a->s) cudaStreamDestroy(a->s);
