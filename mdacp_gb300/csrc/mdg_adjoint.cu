@@ -28,11 +28,21 @@
 // pair's image at the segment's first state, which stays the minimum image of
 // every pair within the cut-off for the whole segment (box > 2 (rc + margin)),
 // so the pair kernels form the separation with one subtraction per axis
-// (from q_i, q_i - L or q_i + L, held per lane) instead of a rounding.  The pair kernels give each particle kLanes lanes and evaluate
-// the pair terms in Horner form, without divisions (GB300's FP64 rate is 1/64
-// of FP32).
+// (from q_i, q_i - L or q_i + L) instead of a rounding.  The pair kernels give
+// each particle several lanes and take the pair terms in fixed point on the
+// integer units (P::fixed), else in Horner form in double without divisions
+// (GB300's FP64 rate is 1/64 of FP32).
+//
+// A segment is held whole: only the step itself and the Hessian-vector product
+// go state by state (400 and 200 launches per gradient of 200 steps); the
+// objective, its gradient and the force's sigma derivative take all states of
+// a segment in one launch.  A gradient of 4,000 atoms over 200 steps: 29.0 ms
+// with every term in double and state by state, 14.3 with the terms in fixed
+// point, 10.0 now (k_step 12.0 us x 400, k_reverse 25 x 200, k_build 50 x 20,
+// k_objective 94 x 10 with the gradient and 64 x 10 without, k_force_sigma 68 x 10).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -46,16 +56,24 @@ namespace mdg {
 namespace adj {
 
 constexpr int kT = 128;
-// Lanes sharing one particle's row in the pair kernels (FP64 runs at 1/64 of
-// the FP32 rate on GB300, so a few thousand particles need several lanes each
-// to occupy every SM's FP64 pipes).
-#ifndef MDG_ADJ_LANES
-#define MDG_ADJ_LANES 8
-#endif
-constexpr int kLanes = MDG_ADJ_LANES;
+// Lanes sharing one particle's row in the pair kernels of the double form (FP64
+// runs at 1/64 of the FP32 rate, so a few thousand particles need several lanes
+// each to occupy every SM's FP64 pipes).
+constexpr int kLanes = 8;
+// The same in fixed point, for the kernels of one step (8 / 16 / 32 lanes: 7.7 /
+// 5.8 / 5.3 ms per gradient of 864 atoms over 200 steps, 10.4 / 10.0 / 12.1 of
+// 4,000, 33.2 / 34.6 / 44.2 of 16,384: more lanes shorten a row's chain where
+// the rows don't fill the GPU).
+constexpr int kStepLanes = 16;
+// Lanes per particle of the fixed-point kernels that take all states of a
+// segment in one launch (1 / 2 / 4 lanes: 11.4 / 11.1 / 11.3 ms per gradient of
+// 4,000 atoms at 8 lanes a step): rows enough to fill the GPU, and the FP64
+// work that follows a row is done for more particles of a warp at once.
+constexpr int kBatchLanes = 2;
 // Lanes sharing one particle in the list build (a warp: the build's float
 // test is light, so it needs many warps per SM to hide its load latency).
 constexpr int kBuildLanes = 32;
+constexpr int kMaskWords = 8;  // a lane's candidates kept as bits: up to 8,192 particles
 
 struct P {
   double L[3];
@@ -87,16 +105,20 @@ struct P {
 constexpr int kImageBits = 6;
 constexpr int kMaxAdjointParticles = 1 << (32 - kImageBits);
 
+// A checkpoint segment is held whole: states 0 .. K, and the half steps 1 .. K
+// that lead to states 1 .. K, each array [K + 1][n] (with the forces at the half
+// steps, their sigma derivatives and the objective's gradients at the states
+// in the backward pass).
 struct D {
-  double4_32a *q, *q2, *p, *qh, *qh2, *aq, *ap, *aqh, *tmp, *tmp2, *q0;
+  double4_32a *q, *p;        // the initial state
+  double4_32a *aq, *ap, *aqh, *tmp, *tmp2;
   double4_32a *ckq, *ckp;    // checkpoints
   float4 *qf;                // float copy of the segment's first state (the list test)
-  double4_32a *segq, *segp, *segqh;  // recomputed segment
-  // the same positions in fixed point (P.fixed): of q, q2, qh, qh2 and the segment's
-  FixPos *xq, *xq2, *xqh, *xqh2, *segxq, *segxqh;
+  double4_32a *segq, *segp, *segqh, *segf, *segs, *segg;
+  FixPos *segxq, *segxqh;    // segq and segqh in fixed point (P.fixed)
   uint32_t *nbr;             // the current segment's list, row-major [n][cap]
   int *cnt;
-  double *part;              // block partials
+  double *part;              // block partials, [K + 1][gridp][3]
   double *acc;               // running sums: J, g_eps, g_sig
   int *flag;
   unsigned int *done;        // blocks of the current reduction that wrote their partials
@@ -187,10 +209,11 @@ __device__ __forceinline__ void for_pairs(const P &c, const D &d, int i, int lan
   }
 }
 
-// Sum over the kLanes lanes that share a particle (all lanes hold the total).
+// Sum over the LANES lanes that share a particle (all lanes hold the total).
+template <int LANES>
 __device__ __forceinline__ double lane_sum(double v) {
 #pragma unroll
-  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 1; o < LANES; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -252,36 +275,39 @@ __device__ __forceinline__ double fix_double(int64_t v, int shift) {
   return __longlong_as_double((long long)((e + (m - 0x10000000000000ull)) | ((uint64_t)v & 0x8000000000000000ull)));
 }
 
-// Row i's entries k = lane, lane + kLanes, ... on the fixed-point positions x:
-// body(sep, R, j) for each pair beyond kFixNear and within the cut-off,
-// masked(take, ...) style: take is false for the others; close(e) follows for
-// the pairs nearer than that, which take the double terms.
-template <class Body, class Close>
+// Row i's entries k = lane, lane + LANES, ... on the fixed-point positions x,
+// the next one's position in flight: body(take, sep, R, j), take where the pair
+// lies within the cut-off and beyond kFixNear; close(e) for a pair nearer than
+// that, which takes the double terms.  (Two pairs at a time took 84 registers
+// for 72 and 10.46 ms for 9.97 per gradient of 4,000 atoms, 39.0 for 34.6 of 16,384.)
+template <int LANES, class Body, class Close>
 __device__ __forceinline__ void for_pairs_fixed(const P &c, const D &d, int i, int lane, const FixPos *x, Body &&body,
                                                 Close &&close) {
   const int cnt = d.cnt[i];
   const uint32_t *row = d.nbr + (size_t)i * c.cap;
   const FixPos own = ld_fix<false>(x + i);
   const uint32_t none = ((uint32_t)i << kImageBits) | 0x15u;
-  uint32_t e0 = lane < cnt ? row[lane] : none, e1 = lane + kLanes < cnt ? row[lane + kLanes] : none;
-  FixPos q0 = ld_fix<false>(x + (e0 >> kImageBits));
-  for (int k = lane; k < cnt; k += kLanes) {
-    const FixPos q1 = ld_fix<false>(x + (e1 >> kImageBits));
-    const uint32_t e2 = k + 2 * kLanes < cnt ? row[k + 2 * kLanes] : none;
-    int dx = q0.x - own.x, dy = q0.y - own.y, dz = q0.z - own.z;
-    float lx = q0.lx - own.lx, ly = q0.ly - own.ly, lz = q0.lz - own.lz;
-    const uint32_t ix = e0 & 3u, iy = (e0 >> 2) & 3u, iz = (e0 >> 4) & 3u;  // d = q_j - r L - q_i, r + 1 stored
+  auto entry = [&](int k) { return k < cnt ? row[k] : none; };
+  uint32_t e = entry(lane);
+  FixPos q = ld_fix<false>(x + (e >> kImageBits));
+  uint32_t en = entry(lane + LANES);
+  for (int k = lane; k < cnt; k += LANES) {
+    const FixPos qn = ld_fix<false>(x + (en >> kImageBits));
+    const uint32_t ef = entry(k + 2 * LANES);
+    int dx = q.x - own.x, dy = q.y - own.y, dz = q.z - own.z;
+    float lx = q.lx - own.lx, ly = q.ly - own.ly, lz = q.lz - own.lz;
+    const uint32_t ix = e & 3u, iy = (e >> 2) & 3u, iz = (e >> 4) & 3u;  // d = q_j - r L - q_i, r + 1 stored
     if (ix != 1u) { dx += ix ? -c.fx_L[0] : c.fx_L[0]; lx += ix ? -c.fx_l[0] : c.fx_l[0]; }
     if (iy != 1u) { dy += iy ? -c.fx_L[1] : c.fx_L[1]; ly += iy ? -c.fx_l[1] : c.fx_l[1]; }
     if (iz != 1u) { dz += iz ? -c.fx_L[2] : c.fx_L[2]; lz += iz ? -c.fx_l[2] : c.fx_l[2]; }
     const FixSep sep = fix_sep(dx, dy, dz, lx, ly, lz);
     const uint64_t R = fix_r2(sep);
     const bool in = R <= c.fx_rc2, near = in && R < c.fx_near;
-    body(in && !near, sep, R, (int)(e0 >> kImageBits));
-    if (near) close(e0);
-    e0 = e1;
-    q0 = q1;
-    e1 = e2;
+    body(in && !near, sep, R, (int)(e >> kImageBits));
+    if (near) close(e);
+    e = en;
+    en = ef;
+    q = qn;
   }
 }
 
@@ -295,9 +321,10 @@ __device__ __forceinline__ void one_pair(const P &c, uint32_t e, const double4_3
   if (pair_terms(c, dx * dx + dy * dy + dz * dz, t)) body(t, dx, dy, dz, j);
 }
 
+template <int LANES>
 __device__ __forceinline__ void lane_sums(FixForce &f) {
 #pragma unroll
-  for (int o = 1; o < kLanes; o <<= 1) {
+  for (int o = 1; o < LANES; o <<= 1) {
     f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
     f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
     f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
@@ -336,9 +363,10 @@ __device__ __forceinline__ void fix_sums_add(FixSums &s, bool take, uint64_t y3,
   s.m += take ? 1 : 0;
 }
 
+template <int LANES>
 __device__ __forceinline__ void lane_sums(FixSums &s) {
 #pragma unroll
-  for (int o = 1; o < kLanes; o <<= 1) {
+  for (int o = 1; o < LANES; o <<= 1) {
     s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
     s.zz += __shfl_xor_sync(0xffffffffu, s.zz, o);
     s.r += __shfl_xor_sync(0xffffffffu, s.r, o);
@@ -385,16 +413,17 @@ __device__ void partials_accumulate(const D &d, double A, double B, double E, do
   __shared__ int last;
   __shared__ double sh2[96];
   if (threadIdx.x == 0) {
-    d.part[3 * blockIdx.x + 0] = A;
-    d.part[3 * blockIdx.x + 1] = B;
-    d.part[3 * blockIdx.x + 2] = E;
+    const size_t at = 3 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x);
+    d.part[at + 0] = A;
+    d.part[at + 1] = B;
+    d.part[at + 2] = E;
     __threadfence();
-    last = atomicAdd(d.done, 1u) == gridDim.x - 1 ? 1 : 0;
+    last = atomicAdd(d.done, 1u) == gridDim.x * gridDim.y - 1 ? 1 : 0;
   }
   __syncthreads();
   if (!last) return;
   double a = 0, b = 0, e = 0;
-  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+  for (size_t k = threadIdx.x; k < (size_t)gridDim.x * gridDim.y; k += blockDim.x) {
     a += __ldcg(d.part + 3 * k);
     b += __ldcg(d.part + 3 * k + 1);
     e += __ldcg(d.part + 3 * k + 2);
@@ -411,12 +440,13 @@ __device__ void partials_accumulate(const D &d, double A, double B, double E, do
 // Pair list at positions q (wrapped into the box): every partner within the
 // list radius, minimum image.  kBuildLanes lanes share a particle: lane l
 // tests partners j = l, l + kBuildLanes, ... (a particle's lanes read
-// neighbouring positions together), first counting, then writing at its
-// offset in the row (a prefix sum over the lanes), so the row order is fixed:
+// neighbouring positions together), keeps the hits as bits where they fit
+// kMaskWords words (4,000 particles: 49.9 us, 60 with the test made again) and
+// writes them at its offset in the row (a prefix sum over the lanes), so the row order is fixed:
 // lane 0's partners, then lane 1's, ...  The test runs in float against a radius widened by 1e-3
 // (float positions of a box of tens of sigma are within 1e-5), so every pair
 // within the exact radius is listed; a few more do no harm (the pair terms cut
-// at rc).  The float positions come from d.qf (k_wrap writes them), so a
+// at rc).  The float positions come from d.qf (k_begin writes them), so a
 // candidate costs one 16-byte load and no conversions.  The recorded image is
 // the double-precision minimum image, r = rint((q_j - q_i) / L) per axis, in
 // {-1, 0, 1} for wrapped positions.
@@ -443,9 +473,28 @@ __global__ void __launch_bounds__(kT) k_build(P c, D d, const double4_32a *q) {
     az = fminf(az, lz - az);
     return ax * ax + ay * ay + az * az <= sl2f && j != i;
   };
+  // one pass where the lane's candidates fit its mask words, else tested again
+  __shared__ uint32_t masks[kT][kMaskWords];
+  uint32_t *mask = masks[threadIdx.x];
+  const bool keep = c.n <= kBuildLanes * 32 * kMaskWords;
   int m = 0;
-  if (active)
-    for (int j = lane; j < c.n; j += kBuildLanes) m += within(j) ? 1 : 0;
+  if (active) {
+    if (keep) {
+      int word = 0;
+      for (int j0 = lane; j0 < c.n; j0 += 32 * kBuildLanes, word++) {
+        uint32_t bits = 0u;
+#pragma unroll 8
+        for (int u = 0; u < 32; u++) {
+          const int j = j0 + u * kBuildLanes;
+          if (within(min(j, c.n - 1)) && j < c.n) bits |= 1u << u;
+        }
+        mask[word] = bits;
+        m += __popc(bits);
+      }
+    } else {
+      for (int j = lane; j < c.n; j += kBuildLanes) m += within(j) ? 1 : 0;
+    }
+  }
   // offsets of the lanes' partners in the row
   int incl = m;
 #pragma unroll
@@ -458,17 +507,24 @@ __global__ void __launch_bounds__(kT) k_build(P c, D d, const double4_32a *q) {
     int w = incl - m;
     uint32_t *row = d.nbr + (size_t)i * c.cap;
     const double4_32a qi = q[i];
-    for (int j = lane; j < c.n; j += kBuildLanes)
-      if (within(j)) {
-        if (w < c.cap) {
-          const double4_32a v = q[j];
-          const int rx = (int)rint((v.x - qi.x) * c.inv_L[0]), ry = (int)rint((v.y - qi.y) * c.inv_L[1]),
-                    rz = (int)rint((v.z - qi.z) * c.inv_L[2]);
-          row[w] = ((uint32_t)j << kImageBits) | (uint32_t)(rx + 1) | ((uint32_t)(ry + 1) << 2) |
-                   ((uint32_t)(rz + 1) << 4);
-        }
-        w++;
+    auto append = [&](int j) {
+      if (w < c.cap) {
+        const double4_32a v = q[j];
+        const int rx = (int)rint((v.x - qi.x) * c.inv_L[0]), ry = (int)rint((v.y - qi.y) * c.inv_L[1]),
+                  rz = (int)rint((v.z - qi.z) * c.inv_L[2]);
+        row[w] = ((uint32_t)j << kImageBits) | (uint32_t)(rx + 1) | ((uint32_t)(ry + 1) << 2) |
+                 ((uint32_t)(rz + 1) << 4);
       }
+      w++;
+    };
+    if (keep) {
+      int word = 0;
+      for (int j0 = lane; j0 < c.n; j0 += 32 * kBuildLanes, word++)
+        for (uint32_t bits = mask[word]; bits; bits &= bits - 1u) append(j0 + (__ffs(bits) - 1) * kBuildLanes);
+    } else {
+      for (int j = lane; j < c.n; j += kBuildLanes)
+        if (within(j)) append(j);
+    }
     if (lane == 0) {
       d.cnt[i] = total < c.cap ? total : c.cap;
       if (total > c.cap) atomicMax(d.flag, total);
@@ -508,21 +564,22 @@ __device__ __forceinline__ ObjSums objective_sums(const P &c, const D &d, int i,
     });
   }
   if (GRAD) {
-    r.gx = lane_sum(r.gx);
-    r.gy = lane_sum(r.gy);
-    r.gz = lane_sum(r.gz);
+    r.gx = lane_sum<kLanes>(r.gx);
+    r.gy = lane_sum<kLanes>(r.gy);
+    r.gz = lane_sum<kLanes>(r.gz);
   }
   if (OBJ == 0) {
-    r.u = lane_sum(r.u);
-    if (GRAD) r.us = lane_sum(r.us);
+    r.u = lane_sum<kLanes>(r.u);
+    if (GRAD) r.us = lane_sum<kLanes>(r.us);
   } else {
-    r.G = lane_sum(r.G);
-    if (GRAD) r.Gs = lane_sum(r.Gs);
+    r.G = lane_sum<kLanes>(r.G);
+    if (GRAD) r.Gs = lane_sum<kLanes>(r.Gs);
   }
   return r;
 }
 
-// The same in fixed point (every thread of the warp calls it).
+// The same in fixed point by kBatchLanes lanes, to lane 0 (every thread of the
+// warp calls it).
 template <int OBJ, bool GRAD>
 __device__ __forceinline__ ObjSums objective_sums_fixed(const P &c, const D &d, int i, int lane, const double4_32a *q,
                                                         const FixPos *x) {
@@ -553,7 +610,7 @@ __device__ __forceinline__ ObjSums objective_sums_fixed(const P &c, const D &d, 
   int cnt = 0;
   if (i < c.n) {
     cnt = d.cnt[i];
-    for_pairs_fixed(
+    for_pairs_fixed<kBatchLanes>(
         c, d, i, lane, x,
         [&](bool take, const FixSep &sep, uint64_t R, int) {
           if (GRAD) {
@@ -574,25 +631,25 @@ __device__ __forceinline__ ObjSums objective_sums_fixed(const P &c, const D &d, 
         });
   }
   __syncwarp();
-  lane_sums(s);
-  if (GRAD) lane_sums(f);
+  lane_sums<kBatchLanes>(s);
+  if (GRAD) lane_sums<kBatchLanes>(f);
   if (GRAD && OBJ == 1) {
 #pragma unroll
-    for (int o = 1; o < kLanes; o <<= 1) psi += __shfl_xor_sync(0xffffffffu, psi, o);
+    for (int o = 1; o < kBatchLanes; o <<= 1) psi += __shfl_xor_sync(0xffffffffu, psi, o);
     f.s = psi;
   }
   if (__any_sync(0xffffffffu, near)) {
     if (GRAD) {
-      r.gx = lane_sum(r.gx);
-      r.gy = lane_sum(r.gy);
-      r.gz = lane_sum(r.gz);
+      r.gx = lane_sum<kBatchLanes>(r.gx);
+      r.gy = lane_sum<kBatchLanes>(r.gy);
+      r.gz = lane_sum<kBatchLanes>(r.gz);
     }
     if (OBJ == 0) {
-      r.u = lane_sum(r.u);
-      if (GRAD) r.us = lane_sum(r.us);
+      r.u = lane_sum<kBatchLanes>(r.u);
+      if (GRAD) r.us = lane_sum<kBatchLanes>(r.us);
     } else {
-      r.G = lane_sum(r.G);
-      if (GRAD) r.Gs = lane_sum(r.Gs);
+      r.G = lane_sum<kBatchLanes>(r.G);
+      if (GRAD) r.Gs = lane_sum<kBatchLanes>(r.Gs);
     }
   }
   if (lane != 0 || i >= c.n) return r;
@@ -640,7 +697,7 @@ __device__ __forceinline__ double3 force_sums_fixed(const P &c, const D &d, int 
   int cnt = 0;
   if (i < c.n) {
     cnt = d.cnt[i];
-    for_pairs_fixed(
+    for_pairs_fixed<kStepLanes>(
         c, d, i, lane, x,
         [&](bool take, const FixSep &sep, uint64_t R, int) {
           const int64_t v = fix_psi(c, fix_terms(c, R));
@@ -652,8 +709,8 @@ __device__ __forceinline__ double3 force_sums_fixed(const P &c, const D &d, int 
         });
   }
   __syncwarp();
-  lane_sums(f);
-  if (__any_sync(0xffffffffu, near)) n = make_double3(lane_sum(n.x), lane_sum(n.y), lane_sum(n.z));
+  lane_sums<kStepLanes>(f);
+  if (__any_sync(0xffffffffu, near)) n = make_double3(lane_sum<kStepLanes>(n.x), lane_sum<kStepLanes>(n.y), lane_sum<kStepLanes>(n.z));
   if (lane != 0 || i >= c.n) return n;
   if (!sums_fit(f, cnt)) {
     n = make_double3(0.0, 0.0, 0.0);
@@ -665,122 +722,96 @@ __device__ __forceinline__ double3 force_sums_fixed(const P &c, const D &d, int 
   return make_double3(F.x + n.x, F.y + n.y, F.z + n.z);
 }
 
-// One step from the half-step positions q: the forces F there (the lanes of
-// a particle), then, by its lane 0, p_out = p_in + F dt, q_out = q + p_out dt/2
-// and, when qh_next is given, the next step's first half-drift
-// qh_next = q_out + p_out dt/2 (the operations k_drift performs).  Out of
-// place: q_out and qh_next must not alias q, which other particles' lanes
-// still read; p_out may alias p_in.  Also the segment's displacement check
-// (a particle more than margin/2 from where the segment's list was built).
-// With VAL = 0 or 1 (the potential-energy or pressure objective) the kernel
-// also adds w times the objective's value at the previous whole-step state
-// (q_obj, p_in) to acc[0], as k_objective<VAL, 0> does (same row walk, lanes
-// and reductions, so the same bits); q_obj must be in this step's segment.
-// FIXED: the pair sums in fixed point on xq, x_obj (the positions q, q_obj).
-template <int VAL, bool FIXED>
-__global__ void k_step(P c, D d, const double4_32a *q, const double4_32a *p_in, double4_32a *q_out,
-                       double4_32a *p_out, double4_32a *qh_next, const double4_32a *q_obj, double w, const FixPos *xq,
-                       FixPos *x_out, FixPos *xh_next, const FixPos *x_obj) {
-  __shared__ double sh[96];
+// One step from the half-step positions q (x in fixed point): the forces F
+// there (the lanes of a particle), then, by one thread per particle, p_out =
+// p_in + F dt, q_out = q + p_out dt/2, the next step's first half-drift qh_next
+// = q_out + p_out dt/2, and F itself where f_out is given.  Also the segment's
+// displacement check (a particle more than margin/2 from q0, where the
+// segment's list was built).  12.0 us at 4,000 particles (18.9 with the terms in
+// double), a chain of launch, five or six entries a lane, the sum over the
+// lanes and the update: the update's FP64 by a lane in eight of every warp, not
+// by the block's first threads, cost 2 us of it.
+template <bool FIXED>
+__global__ void __launch_bounds__(kT) k_step(P c, D d, const double4_32a *q, const double4_32a *p_in, double4_32a *q_out,
+                                             double4_32a *p_out, double4_32a *qh_next, const double4_32a *q0,
+                                             double4_32a *f_out, const FixPos *x, FixPos *x_out, FixPos *xh_next) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / kLanes, lane = tid % kLanes;
+  constexpr int kL = FIXED ? kStepLanes : kLanes;
+  int i = tid / kL;
+  const int lane = tid % kL;
   double3 F = make_double3(0.0, 0.0, 0.0);
-  double u = 0, G = 0;
-  double4_32a qi = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-  if (i < c.n) {
-    qi = q[i];
-    if (lane == 0) {
-      const double4_32a z = d.q0[i];
-      const double ux = qi.x - z.x, uy = qi.y - z.y, uz = qi.z - z.z;
-      if (ux * ux + uy * uy + uz * uz > c.half_margin2) atomicMax(d.flag + 1, 1);
-    }
-  }
   if (FIXED) {
-    F = force_sums_fixed(c, d, i, lane, q, xq);
-    if (VAL >= 0) {
-      const ObjSums r = objective_sums_fixed<(VAL < 0 ? 0 : VAL), false>(c, d, i, lane, q_obj, x_obj);
-      u = r.u;
-      G = r.G;
-    }
+    F = force_sums_fixed(c, d, i, lane, q, x);
   } else {
     if (i < c.n) {
-      const Home h = make_home(c, qi);
+      const Home h = make_home(c, q[i]);
       for_pairs(c, d, i, lane, q, h, [&](const PairTerms &t, double dx, double dy, double dz, int) {
         F.x += t.f * dx;
         F.y += t.f * dy;
         F.z += t.f * dz;
       });
-      if (VAL >= 0) {
-        const Home ho = make_home(c, q_obj[i]);
-        for_pairs(c, d, i, lane, q_obj, ho, [&](const PairTerms &t, double, double, double, int) {
-          if (VAL == 0) u += 0.5 * t.phi;
-          else G += 0.5 * t.g;
-        });
-      }
     }
-    F = make_double3(lane_sum(F.x), lane_sum(F.y), lane_sum(F.z));
-    if (VAL == 0) u = lane_sum(u);
-    if (VAL == 1) G = lane_sum(G);
+    F = make_double3(lane_sum<kL>(F.x), lane_sum<kL>(F.y), lane_sum<kL>(F.z));
   }
-  double val = 0.0;
-  if (i < c.n && lane == 0) {
-    double4_32a b = p_in[i];
-    if (VAL == 0) val = u * (1.0 / (double)c.n);
-    if (VAL == 1) val = (2.0 * (0.5 * (b.x * b.x + b.y * b.y + b.z * b.z)) - G) * (1.0 / (3.0 * c.volume));
-    b.x += F.x * c.dt;
-    b.y += F.y * c.dt;
-    b.z += F.z * c.dt;
-    p_out[i] = b;
-    double4_32a a = qi;
-    a.x += b.x * c.dt2;
-    a.y += b.y * c.dt2;
-    a.z += b.z * c.dt2;
-    q_out[i] = a;
-    if (FIXED) x_out[i] = fix_position(a.x, a.y, a.z, 0);
-    if (qh_next) {
-      a.x += b.x * c.dt2;
-      a.y += b.y * c.dt2;
-      a.z += b.z * c.dt2;
-      qh_next[i] = a;
-      if (FIXED) xh_next[i] = fix_position(a.x, a.y, a.z, 0);
-    }
-  }
-  if (VAL >= 0) {
-    double none1 = 0.0, none2 = 0.0;
-    block_sum3(val, none1, none2, sh);
-    partials_accumulate(d, val, 0.0, 0.0, w);
-  }
+  // the block's particles move on to its first threads, one each: the FP64
+  // work below is then a warp's, not four
+  __shared__ double3 sF[kT / kL];
+  if (lane == 0) sF[threadIdx.x / kL] = F;
+  __syncthreads();
+  i = blockIdx.x * (kT / kL) + threadIdx.x;
+  if (threadIdx.x >= kT / kL || i >= c.n) return;
+  F = sF[threadIdx.x];
+  const double4_32a qi = q[i], z = q0[i];
+  const double ux = qi.x - z.x, uy = qi.y - z.y, uz = qi.z - z.z;
+  if (ux * ux + uy * uy + uz * uz > c.half_margin2) atomicMax(d.flag + 1, 1);
+  if (f_out) f_out[i] = make_double4_32a(F.x, F.y, F.z, 0.0);
+  double4_32a b = p_in[i];
+  b.x += F.x * c.dt;
+  b.y += F.y * c.dt;
+  b.z += F.z * c.dt;
+  p_out[i] = b;
+  double4_32a a = qi;
+  a.x += b.x * c.dt2;
+  a.y += b.y * c.dt2;
+  a.z += b.z * c.dt2;
+  q_out[i] = a;
+  if (FIXED) x_out[i] = fix_position(a.x, a.y, a.z, 0);
+  a.x += b.x * c.dt2;
+  a.y += b.y * c.dt2;
+  a.z += b.z * c.dt2;
+  qh_next[i] = a;
+  if (FIXED) xh_next[i] = fix_position(a.x, a.y, a.z, 0);
 }
 
-// qh = q + p dt/2: the first half-drift of a trajectory or segment
-__global__ void k_drift(P c, const double4_32a *q, const double4_32a *p, double4_32a *out, FixPos *xout) {
+// A segment's first state from (q, p): with wrap, positions into the box, q - k L
+// per axis with k = floor(q / L) (particles already inside keep their bits), and
+// the checkpoint; then state 0 of the segment, the float copy for the list
+// test and the first half-drift.  The backward pass calls it without wrap on the
+// checkpoint (ckq = ckp = null).
+__global__ void k_begin(P c, D d, const double4_32a *q, const double4_32a *p, double4_32a *ckq, double4_32a *ckp, int wrap) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.n) return;
   double4_32a a = q[i];
   const double4_32a b = p[i];
-  a.x += b.x * c.dt2;
-  a.y += b.y * c.dt2;
-  a.z += b.z * c.dt2;
-  out[i] = a;
-  if (c.fixed) xout[i] = fix_position(a.x, a.y, a.z, 0);
-}
-
-// A segment's first state: with wrap, positions into the box, q - k L per
-// axis with k = floor(q / L) (particles already inside keep their bits); then
-// the float copy for the list test.  The backward pass calls it without wrap
-// on the checkpoint the forward pass wrapped.
-__global__ void k_wrap(P c, double4_32a *q, float4 *qf, int wrap) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n) return;
-  double4_32a a = q[i];
   if (wrap) {
     const double kx = floor(a.x * c.inv_L[0]), ky = floor(a.y * c.inv_L[1]), kz = floor(a.z * c.inv_L[2]);
     if (kx != 0.0) a.x = fma(-kx, c.L[0], a.x);
     if (ky != 0.0) a.y = fma(-ky, c.L[1], a.y);
     if (kz != 0.0) a.z = fma(-kz, c.L[2], a.z);
-    q[i] = a;
   }
-  qf[i] = make_float4((float)a.x, (float)a.y, (float)a.z, 0.f);
+  if (ckq) {
+    ckq[i] = a;
+    ckp[i] = b;
+  }
+  d.segq[i] = a;
+  d.segp[i] = b;
+  d.qf[i] = make_float4((float)a.x, (float)a.y, (float)a.z, 0.f);
+  a.x += b.x * c.dt2;
+  a.y += b.y * c.dt2;
+  a.z += b.z * c.dt2;
+  const size_t at = (size_t)c.n + i;
+  d.segqh[at] = a;
+  if (c.fixed) d.segxqh[at] = fix_position(a.x, a.y, a.z, 0);
 }
 
 // The reverse of a step's second half-drift q_n = qh + dt/2 p_n for particle
@@ -795,198 +826,250 @@ __device__ __forceinline__ void reverse_drift(const P &c, const D &d, int i, con
   d.aqh[i] = a;
 }
 
-// Particle i's objective terms from its sums (lane 0): the value and its
-// epsilon and sigma derivatives; with GRAD, w dj/dq added to a and w dj/dp
-// to b (the adjoints of the state's q and p).
-template <int OBJ, bool GRAD>
-__device__ __forceinline__ void objective_finish(const P &c, const ObjSums &r, const double4_32a &pi, double w,
-                                                 double &val, double &ge, double &gs, double4_32a &a,
-                                                 double4_32a &b) {
-  if (OBJ == 0) {
-    const double inv_n = 1.0 / (double)c.n;
-    val = r.u * inv_n;
-    ge = r.u / c.eps * inv_n;
-    gs = r.us * inv_n;
-    if (GRAD) {
-      a.x += w * r.gx * inv_n;
-      a.y += w * r.gy * inv_n;
-      a.z += w * r.gz * inv_n;
-    }
-  } else {
-    const double ke = 0.5 * (pi.x * pi.x + pi.y * pi.y + pi.z * pi.z);
-    const double inv3v = 1.0 / (3.0 * c.volume);
-    val = (2.0 * ke - r.G) * inv3v;
-    ge = -r.G / c.eps * inv3v;
-    gs = -r.Gs * inv3v;
-    if (GRAD) {
-      a.x += w * r.gx * inv3v;
-      a.y += w * r.gy * inv3v;
-      a.z += w * r.gz * inv3v;
-      b.x += w * 2.0 * pi.x * inv3v;
-      b.y += w * 2.0 * pi.y * inv3v;
-      b.z += w * 2.0 * pi.z * inv3v;
-    }
-  }
-}
-
-// Objective j at (q, p) into partials (value, d/deps, d/dsigma); with GRAD,
-// also adds w * dj/dq and w * dj/dp (w = 1/Ns) to the adjoints aq, ap of
-// state n and applies the reverse of step n's second half-drift (into tmp
-// and aqh, which k_reverse_hvp takes up).  OBJ and GRAD are
-// template parameters so that each pass computes only the pair terms it uses:
-// the forward pass returns J alone (the parameter terms of the gradient are
-// summed in the backward pass), so without GRAD the sigma derivative is left
-// out and its partial is zero.
-template <int OBJ, int GRAD, bool FIXED>
-__global__ void k_objective(P c, D d, const double4_32a *q, const double4_32a *p, double w, double4_32a *tmp, const FixPos *x) {
-  constexpr bool grad = GRAD != 0;
+// The objective at states first .. first + gridDim.y - 1 of the segment,
+// weighted: values (and, with GRAD, the epsilon and sigma derivatives) into the
+// running sums, and with GRAD w dj/dq of state k into segg[k].  All states of a
+// segment share its list, so one launch takes them together: one state of 4,000
+// particles leaves the GPU mostly idle and cost 9 us forward and 10 backward, in
+// a launch of 20 it costs 3.2 and 4.7 (bound by the integer units).
+template <int OBJ, bool GRAD, bool FIXED>
+__global__ void __launch_bounds__(kT) k_objective(P c, D d, double w, int first) {
   __shared__ double sh[96];
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / kLanes, lane = tid % kLanes;
+  constexpr int kL = FIXED ? kBatchLanes : kLanes;
+  const int i = tid / kL, lane = tid % kL;
+  const size_t at = (size_t)c.n * (first + blockIdx.y);
+  const double4_32a *q = d.segq + at;
+  const ObjSums r = FIXED ? objective_sums_fixed<OBJ, GRAD>(c, d, i, lane, q, d.segxq + at) : objective_sums<OBJ, GRAD>(c, d, i, lane, q);
   double val = 0, ge = 0, gs = 0;
-  const ObjSums r = FIXED ? objective_sums_fixed<OBJ, grad>(c, d, i, lane, q, x) : objective_sums<OBJ, grad>(c, d, i, lane, q);
   if (i < c.n && lane == 0) {
-    double4_32a a = make_double4_32a(0.0, 0.0, 0.0, 0.0), b = a;
-    if (grad) {
-      a = d.aq[i];
-      b = d.ap[i];
+    const double scale = OBJ == 0 ? 1.0 / (double)c.n : 1.0 / (3.0 * c.volume);
+    if (OBJ == 0) {
+      val = r.u * scale;
+      ge = r.u / c.eps * scale;
+      gs = r.us * scale;
+    } else {
+      const double4_32a pi = d.segp[at + i];
+      const double ke = 0.5 * (pi.x * pi.x + pi.y * pi.y + pi.z * pi.z);
+      val = (2.0 * ke - r.G) * scale;
+      ge = -r.G / c.eps * scale;
+      gs = -r.Gs * scale;
     }
-    objective_finish<OBJ, grad>(c, r, p[i], w, val, ge, gs, a, b);
-    if (grad) reverse_drift(c, d, i, a, b, tmp);
+    if (GRAD) d.segg[at + i] = make_double4_32a(w * r.gx * scale, w * r.gy * scale, w * r.gz * scale, 0.0);
   }
   block_sum3(val, ge, gs, sh);
   partials_accumulate(d, val, ge, gs, w);
 }
 
-// The rest of the reverse of step n at half-step positions qh (kick and
-// first half-drift).  In: tmp (read by the neighbours too) and aqh from the
-// reverse of its second half-drift.  Out: aq, ap adjoints of (q_{n-1},
-// p_{n-1}); parameter terms dt * ap . dF/dtheta into partials (slots 1, 2).
-// With OBJ = 0 or 1 the kernel goes on with state n - 1 (in the same
-// segment): its objective terms at (q_obj, p_obj), as k_objective<OBJ, 1>
-// computes them, and the reverse of step n - 1's second half-drift, into
-// tmp_out (not tmp: other particles' lanes still read it) and aqh instead of
-// aq, ap.
-template <int OBJ, bool FIXED>
-__global__ void k_reverse_hvp(P c, D d, const double4_32a *qh, const double4_32a *tmp, const double4_32a *q_obj,
-                              const double4_32a *p_obj, double w, double4_32a *tmp_out, const FixPos *xh, const FixPos *x_obj) {
-  __shared__ double sh[96];
+// sum_j dF_ij/dsigma of the half steps first .. first + gridDim.y - 1 of the
+// segment, into segs.
+template <bool FIXED>
+__global__ void __launch_bounds__(kT) k_force_sigma(P c, D d, int first) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / kLanes, lane = tid % kLanes;
-  double te = 0, ts = 0;
-  double hx = 0, hy = 0, hz = 0, fx = 0, fy = 0, fz = 0, sx = 0, sy = 0, sz = 0;
-  ObjSums r{};
+  constexpr int kL = FIXED ? kBatchLanes : kLanes;
+  const int i = tid / kL, lane = tid % kL;
+  const size_t at = (size_t)c.n * (first + blockIdx.y);
+  const double4_32a *q = d.segqh + at;
+  double3 S = make_double3(0.0, 0.0, 0.0);
+  auto in_double = [&](const PairTerms &t, double dx, double dy, double dz, int) {
+    S.x += t.fs * dx;
+    S.y += t.fs * dy;
+    S.z += t.fs * dz;
+  };
+  if (FIXED) {
+    FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f};
+    float psi = 0.f;
+    bool near = false;
+    int cnt = 0;
+    if (i < c.n) {
+      cnt = d.cnt[i];
+      for_pairs_fixed<kL>(
+          c, d, i, lane, d.segxqh + at,
+          [&](bool take, const FixSep &sep, uint64_t R, int) {
+            const FixTerms t = fix_terms(c, R);
+            fix_add(f, take ? fix_dsigma(c, t) : 0, sep);
+            psi += (float)fix_shi(take ? fix_psi(c, t) : 0);
+          },
+          [&](uint32_t e) {
+            near = true;
+            one_pair(c, e, q, make_home(c, q[i]), in_double);
+          });
+    }
+    __syncwarp();
+    lane_sums<kL>(f);
+#pragma unroll
+    for (int o = 1; o < kL; o <<= 1) psi += __shfl_xor_sync(0xffffffffu, psi, o);
+    f.s = psi;
+    if (__any_sync(0xffffffffu, near)) S = make_double3(lane_sum<kL>(S.x), lane_sum<kL>(S.y), lane_sum<kL>(S.z));
+    if (i >= c.n || lane != 0) return;
+    if (sums_fit(f, cnt)) {
+      const double3 v = fix_vector(f, 8.0 * c.e_s3);
+      S = make_double3(S.x + v.x, S.y + v.y, S.z + v.z);
+    } else {  // the row again in double
+      S = make_double3(0.0, 0.0, 0.0);
+      const Home h = make_home(c, q[i]);
+      for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], q, h, in_double);
+    }
+  } else {
+    if (i < c.n) {
+      const Home h = make_home(c, q[i]);
+      for_pairs(c, d, i, lane, q, h, in_double);
+    }
+    S = make_double3(lane_sum<kL>(S.x), lane_sum<kL>(S.y), lane_sum<kL>(S.z));
+    if (i >= c.n || lane != 0) return;
+  }
+  d.segs[at + i] = make_double4_32a(S.x, S.y, S.z, 0.0);
+}
+
+// The objective's terms of state k added to its adjoints a, b (w dj/dq from
+// segg; dj/dp of the pressure here), then the reverse of step k's second half-drift.
+__device__ __forceinline__ void state_terms(const P &c, const D &d, int i, size_t at, double w, double4_32a a, double4_32a b,
+                                            double4_32a *tmp) {
+  const double4_32a g = d.segg[at + i];
+  a.x += g.x;
+  a.y += g.y;
+  a.z += g.z;
+  if (c.objective == 1) {
+    const double4_32a pi = d.segp[at + i];
+    const double k = 2.0 * w / (3.0 * c.volume);
+    b.x += k * pi.x;
+    b.y += k * pi.y;
+    b.z += k * pi.z;
+  }
+  reverse_drift(c, d, i, a, b, tmp);
+}
+
+// The segment's last state (number len): from the adjoints aq, ap of the state
+// that follows it.
+__global__ void k_seed(P c, D d, int len, double w, double4_32a *tmp) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < c.n) state_terms(c, d, i, (size_t)c.n * len, w, d.aq[i], d.ap[i], tmp);
+}
+
+// The rest of the reverse of step k at its half-step positions (kick and first
+// half-drift).  In: tmp (read by the neighbours too) and aqh from the reverse of
+// its second half-drift; the force and its sigma derivative there.  Parameter
+// terms dt * ap . dF/dtheta into part[k] (slots 1, 2).  For k > 1 it goes on
+// with the objective's terms of state k - 1 and the reverse of step k - 1's
+// second half-drift, into tmp_out (not tmp: other particles' lanes still read
+// it) and aqh; for k = 1 aq, ap receive the adjoints of the segment's first
+// state.  25 us at 4,000 particles (the FP64 pipe has 13 instructions a pair,
+// 8 us of it; 45 us with all terms in double and the objective in it).
+template <bool FIXED>
+__global__ void __launch_bounds__(kT) k_reverse(P c, D d, int k, const double4_32a *tmp, double w, double4_32a *tmp_out) {
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int kL = FIXED ? kStepLanes : kLanes;
+  int i = tid / kL;
+  const int lane = tid % kL;
+  const size_t at = (size_t)c.n * k;
+  const double4_32a *qh = d.segqh + at;
+  double hx = 0, hy = 0, hz = 0;
+  double4_32a vi = i < c.n ? tmp[i] : make_double4_32a(0.0, 0.0, 0.0, 0.0);
   auto in_double = [&](const PairTerms &t, double dx, double dy, double dz, int j) {
-    const double4_32a vi = tmp[i], vj = tmp[j];
+    const double4_32a vj = tmp[j];
     const double wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
     const double dw = dx * wx + dy * wy + dz * wz;
     // (H v)_i = sum_j f (v_i - v_j) + (f'/r) d (d . (v_i - v_j))
     hx += t.f * wx + t.fpr * dx * dw;
     hy += t.f * wy + t.fpr * dy * dw;
     hz += t.f * wz + t.fpr * dz * dw;
-    fx += t.f * dx;
-    fy += t.f * dy;
-    fz += t.f * dz;
-    sx += t.fs * dx;
-    sy += t.fs * dy;
-    sz += t.fs * dz;
   };
   if (FIXED) {
-    FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f}, g = f;  // psi d; the sigma derivative's eighth
     // reduced sums psi w and (psi' / x) / 48 (d . w) d
     double ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
-    bool near = false;
-    int cnt = 0;
-    if (i < c.n) {
-      cnt = d.cnt[i];
-      const double4_32a vi = tmp[i];
-      for_pairs_fixed(
-          c, d, i, lane, xh,
+    if (i < c.n)
+      for_pairs_fixed<kL>(
+          c, d, i, lane, d.segxqh + at,
           [&](bool take, const FixSep &sep, uint64_t R, int j) {
             const double4_32a vj = tmp[j];
             const FixTerms t = fix_terms(c, R);
             const int64_t psi = take ? fix_psi(c, t) : 0, slope = take ? fix_psi_slope(t) : 0;
-            fix_add(f, psi, sep);
-            fix_add(g, take ? fix_dsigma(c, t) : 0, sep);
             // the separation as doubles: high words and rests in units of 2^-59
             auto whole = [](int h, float l) {
               return fix_double(((int64_t)h << 30) + (int64_t)__float2int_rn(l * 2147483648.0f), 59);
             };
             const double dx = whole(sep.x, sep.lx), dy = whole(sep.y, sep.ly), dz = whole(sep.z, sep.lz);
             const double wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
-            const double p = fix_double(psi, 55), k = fix_double(slope, 55) * fma(dz, wz, fma(dy, wy, dx * wx));
+            const double p = fix_double(psi, 55), s = fix_double(slope, 55) * fma(dz, wz, fma(dy, wy, dx * wx));
             ax = fma(p, wx, ax);
             ay = fma(p, wy, ay);
             az = fma(p, wz, az);
-            bx = fma(k, dx, bx);
-            by = fma(k, dy, by);
-            bz = fma(k, dz, bz);
+            bx = fma(s, dx, bx);
+            by = fma(s, dy, by);
+            bz = fma(s, dz, bz);
           },
-          [&](uint32_t e) {
-            near = true;
-            one_pair(c, e, qh, make_home(c, qh[i]), in_double);
-          });
-    }
+          [&](uint32_t e) { one_pair(c, e, qh, make_home(c, qh[i]), in_double); });
     __syncwarp();
-    lane_sums(f);
-    lane_sums(g);
     const double e4 = 48.0 * c.e_s4;
-    hx = lane_sum(fma(c.e_s2, ax, fma(e4, bx, hx)));
-    hy = lane_sum(fma(c.e_s2, ay, fma(e4, by, hy)));
-    hz = lane_sum(fma(c.e_s2, az, fma(e4, bz, hz)));
-    if (__any_sync(0xffffffffu, near)) {
-      fx = lane_sum(fx); fy = lane_sum(fy); fz = lane_sum(fz);
-      sx = lane_sum(sx); sy = lane_sum(sy); sz = lane_sum(sz);
-    }
-    if (lane == 0 && i < c.n) {
-      if (sums_fit(f, cnt)) {
-        const double3 F = fix_vector(f, c.e_s2), S = fix_vector(g, 8.0 * c.e_s3);
-        fx += F.x; fy += F.y; fz += F.z;
-        sx += S.x; sy += S.y; sz += S.z;
-      } else {  // the row again in double
-        hx = hy = hz = fx = fy = fz = sx = sy = sz = 0.0;
-        const Home h = make_home(c, qh[i]);
-        for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], qh, h, in_double);
-      }
-    }
-    if (OBJ >= 0) r = objective_sums_fixed<(OBJ >= 0 ? OBJ : 0), true>(c, d, i, lane, q_obj, x_obj);
-  } else {
-    if (i < c.n) {
-      const Home h = make_home(c, qh[i]);
-      for_pairs(c, d, i, lane, qh, h, in_double);
-    }
-    hx = lane_sum(hx); hy = lane_sum(hy); hz = lane_sum(hz);
-    fx = lane_sum(fx); fy = lane_sum(fy); fz = lane_sum(fz);
-    sx = lane_sum(sx); sy = lane_sum(sy); sz = lane_sum(sz);
-    if (OBJ >= 0) r = objective_sums<(OBJ >= 0 ? OBJ : 0), true>(c, d, i, lane, q_obj);
+    hx = fma(c.e_s2, ax, fma(e4, bx, hx));
+    hy = fma(c.e_s2, ay, fma(e4, by, hy));
+    hz = fma(c.e_s2, az, fma(e4, bz, hz));
+  } else if (i < c.n) {
+    const Home h = make_home(c, qh[i]);
+    for_pairs(c, d, i, lane, qh, h, in_double);
   }
-  double val = 0, ge = 0, gs = 0;
-  if (i < c.n && lane == 0) {
-    const double4_32a b = tmp[i];
+  hx = lane_sum<kL>(hx);
+  hy = lane_sum<kL>(hy);
+  hz = lane_sum<kL>(hz);
+  // one thread per particle from here on, as in k_step
+  __shared__ double3 sH[kT / kL];
+  if (lane == 0) sH[threadIdx.x / kL] = make_double3(hx, hy, hz);
+  __syncthreads();
+  i = blockIdx.x * (kT / kL) + threadIdx.x;
+  double te = 0, ts = 0;
+  if (threadIdx.x < kT / kL && i < c.n) {
+    vi = tmp[i];
+    hx = sH[threadIdx.x].x;
+    hy = sH[threadIdx.x].y;
+    hz = sH[threadIdx.x].z;
     // parameter terms: dt * a_p . dF_i/deps (= F_i/eps), dt * a_p . dF_i/dsigma
-    te = c.dt * (b.x * fx + b.y * fy + b.z * fz) / c.eps;
-    ts = c.dt * (b.x * sx + b.y * sy + b.z * sz);
+    const double4_32a F = d.segf[at + i], S = d.segs[at + i];
+    te = c.dt * (vi.x * F.x + vi.y * F.y + vi.z * F.z) / c.eps;
+    ts = c.dt * (vi.x * S.x + vi.y * S.y + vi.z * S.z);
     // kick: a_qh = a_q - dt H a_p ; then drift qh = q + dt/2 p : a_p += dt/2 a_qh
-    double4_32a a = d.aqh[i];
+    double4_32a a = d.aqh[i], pb = vi;
     a.x -= c.dt * hx;
     a.y -= c.dt * hy;
     a.z -= c.dt * hz;
-    double4_32a pb = b;
     pb.x += c.dt2 * a.x;
     pb.y += c.dt2 * a.y;
     pb.z += c.dt2 * a.z;
-    if (OBJ >= 0) {
-      objective_finish<(OBJ >= 0 ? OBJ : 0), true>(c, r, p_obj[i], w, val, ge, gs, a, pb);
-      reverse_drift(c, d, i, a, pb, tmp_out);
+    if (k > 1) {
+      state_terms(c, d, i, (size_t)c.n * (k - 1), w, a, pb, tmp_out);
     } else {
       d.aq[i] = a;
       d.ap[i] = pb;
     }
   }
-  // the objective's partials carry the weight w, the kick terms 1
-  double A = w * val, B = te + w * ge, E = ts + w * gs;
-  block_sum3(A, B, E, sh);
-  partials_accumulate(d, A, B, E, 1.0);
+  static_assert(kT / kL <= 32, "one warp holds the block's particles");
+  if (threadIdx.x >= 32) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    te += __shfl_down_sync(0xffffffffu, te, o);
+    ts += __shfl_down_sync(0xffffffffu, ts, o);
+  }
+  if (threadIdx.x == 0) {
+    double *part = d.part + 3 * ((size_t)k * gridDim.x + blockIdx.x);
+    part[1] = te;
+    part[2] = ts;
+  }
+}
+
+// Adds the parameter terms of steps 1 .. len (k_reverse's partials) to the
+// running sums, in a fixed order.
+__global__ void __launch_bounds__(1024) k_reverse_sums(D d, int len, int blocks) {
+  __shared__ double sh[96];
+  double none = 0, te = 0, ts = 0;
+  const double *part = d.part + 3 * (size_t)blocks;
+  for (int k = threadIdx.x; k < len * blocks; k += blockDim.x) {
+    te += part[3 * (size_t)k + 1];
+    ts += part[3 * (size_t)k + 2];
+  }
+  block_sum3(none, te, ts, sh);
+  if (threadIdx.x == 0) {
+    d.acc[1] += te;
+    d.acc[2] += ts;
+  }
 }
 
 }  // namespace adj
@@ -1002,9 +1085,11 @@ struct mdg_adjoint {
   D d;
   cudaStream_t s = nullptr;
   int grid = 1;    // one thread per particle
-  int gridp = 1;   // kLanes threads per particle (pair kernels)
+  int gridp = 1;   // pair kernels of one step
+  int grids = 1;   // the kernels over all states of a segment
   int gridb = 1;   // kBuildLanes threads per particle (list build)
   int nck = 0;
+  char *slab = nullptr;  // every device array
   bool forward_done = false;
   // the device work of a forward and of a backward pass, captured once and
   // replayed (every pointer is fixed at creation)
@@ -1024,97 +1109,74 @@ int afail(mdg_adjoint *a, int code, const std::string &m) {
     if (e_ != cudaSuccess) return afail(a, MDG_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-template <class T>
-cudaError_t aalloc(T **p, size_t n) {
-  *p = nullptr;
-  return cudaMalloc((void **)p, (n ? n : 1) * sizeof(T));
+// Steps of a segment from its state 0 and first half-drift: states 1 .. len and
+// half steps 2 .. len (and the forces at the half steps).
+void run_segment(mdg_adjoint *a, int len, bool forces) {
+  const size_t N = (size_t)a->c.n;
+  D &d = a->d;
+  k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, d.segq);
+  for (int k = 1; k <= len; k++) {
+    const size_t at = N * k, before = N * (k - 1), after = N * (k + 1);
+    double4_32a *f = forces ? d.segf + at : nullptr;
+    // half step len + 1 is written too, and not used
+    if (a->c.fixed)
+      k_step<true><<<a->gridp, kT, 0, a->s>>>(a->c, d, d.segqh + at, d.segp + before, d.segq + at, d.segp + at, d.segqh + after,
+                                              d.segq, f, d.segxqh + at, d.segxq + at, d.segxqh + after);
+    else
+      k_step<false><<<a->gridp, kT, 0, a->s>>>(a->c, d, d.segqh + at, d.segp + before, d.segq + at, d.segp + at, d.segqh + after,
+                                               d.segq, f, nullptr, nullptr, nullptr);
+  }
 }
 
-// Launches kernel<.., true> or kernel<.., false> by the fixed-point flag.
-#define MDG_ADJ(KERNEL, TMPL, ...)                                               \
-  do {                                                                           \
-    if (a->c.fixed) KERNEL<TMPL, true><<<a->gridp, kT, 0, a->s>>>(__VA_ARGS__);  \
-    else KERNEL<TMPL, false><<<a->gridp, kT, 0, a->s>>>(__VA_ARGS__);            \
-  } while (0)
-#define MDG_TWO(A, B) A, B
+constexpr int kStates = 32768;  // states a launch (a grid's second dimension ends at 65,535)
 
-void launch_objective(mdg_adjoint *a, const double4_32a *q, const double4_32a *p, const FixPos *x, bool grad, double w,
-                      double4_32a *tmp = nullptr) {
-  const int obj = a->c.objective;
-  if (obj == 0 && !grad) MDG_ADJ(k_objective, MDG_TWO(0, 0), a->c, a->d, q, p, w, tmp, x);
-  else if (obj == 0) MDG_ADJ(k_objective, MDG_TWO(0, 1), a->c, a->d, q, p, w, tmp, x);
-  else if (!grad) MDG_ADJ(k_objective, MDG_TWO(1, 0), a->c, a->d, q, p, w, tmp, x);
-  else MDG_ADJ(k_objective, MDG_TWO(1, 1), a->c, a->d, q, p, w, tmp, x);
+template <bool GRAD>
+void launch_objective(mdg_adjoint *a, int len, double w) {
+  for (int first = 1; first <= len; first += kStates) {
+    const dim3 grid(a->grids, len - first + 1 < kStates ? len - first + 1 : kStates);
+    if (a->c.objective == 0) {
+      if (a->c.fixed) k_objective<0, GRAD, true><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
+      else k_objective<0, GRAD, false><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
+    } else {
+      if (a->c.fixed) k_objective<1, GRAD, true><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
+      else k_objective<1, GRAD, false><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
+    }
+  }
 }
 
-// The reverse of step n (half-step positions qh, xh; tmp from its second
-// half-drift's reverse), with, when q_obj is given, the objective terms of
-// state n - 1 and the reverse of step n - 1's second half-drift into tmp_out.
-void launch_reverse(mdg_adjoint *a, const double4_32a *qh, const FixPos *xh, const double4_32a *tmp, const double4_32a *q_obj,
-                    const double4_32a *p_obj, const FixPos *x_obj, double w, double4_32a *tmp_out) {
-  const int obj = a->c.objective;
-  if (!q_obj) MDG_ADJ(k_reverse_hvp, -1, a->c, a->d, qh, tmp, nullptr, nullptr, 0.0, nullptr, xh, nullptr);
-  else if (obj == 0) MDG_ADJ(k_reverse_hvp, 0, a->c, a->d, qh, tmp, q_obj, p_obj, w, tmp_out, xh, x_obj);
-  else MDG_ADJ(k_reverse_hvp, 1, a->c, a->d, qh, tmp, q_obj, p_obj, w, tmp_out, xh, x_obj);
+void launch_force_sigma(mdg_adjoint *a, int len) {
+  for (int first = 1; first <= len; first += kStates) {
+    const dim3 grid(a->grids, len - first + 1 < kStates ? len - first + 1 : kStates);
+    if (a->c.fixed) k_force_sigma<true><<<grid, kT, 0, a->s>>>(a->c, a->d, first);
+    else k_force_sigma<false><<<grid, kT, 0, a->s>>>(a->c, a->d, first);
+  }
 }
 
-// Positions with their fixed-point copy.
-struct Pos {
-  double4_32a *q;
-  FixPos *x;
-  Pos at(size_t k) const { return Pos{q + k, x + k}; }
-};
-
-// One step from the half-step positions h (already drifted from step k - 1)
-// and p_in: out, p_out and, when given, the next step's half-step positions
-// (not h itself); with obj, also w times the objective's value at (obj, p_in).
-void fwd_step(mdg_adjoint *a, const Pos &h, const double4_32a *p_in, const Pos &out, double4_32a *p_out, const Pos *next,
-              const Pos *obj = nullptr, double w = 0.0) {
-  double4_32a *nq = next ? next->q : nullptr;
-  FixPos *nx = next ? next->x : nullptr;
-  if (!obj) MDG_ADJ(k_step, -1, a->c, a->d, h.q, p_in, out.q, p_out, nq, nullptr, 0.0, h.x, out.x, nx, nullptr);
-  else if (a->c.objective == 0)
-    MDG_ADJ(k_step, 0, a->c, a->d, h.q, p_in, out.q, p_out, nq, obj->q, w, h.x, out.x, nx, obj->x);
-  else MDG_ADJ(k_step, 1, a->c, a->d, h.q, p_in, out.q, p_out, nq, obj->q, w, h.x, out.x, nx, obj->x);
-}
-
-// The horizon from the state in d.q, d.p: per segment its list, per step the
-// step and the objective terms, checkpoints every K steps.
+// The horizon from the state in d.q, d.p: per segment its checkpoint and list,
+// its steps, and the objective at its states.
 int enqueue_forward(mdg_adjoint *a) {
-  const size_t N = (size_t)a->c.n, bytes = N * 32;
+  const size_t N = (size_t)a->c.n;
   D &d = a->d;
   MDG_ACK(cudaMemsetAsync(d.flag, 0, 2 * sizeof(int), a->s));
   MDG_ACK(cudaMemsetAsync(d.acc, 0, 3 * sizeof(double), a->s));
   const int Ns = a->prm.steps, K = a->prm.checkpoint_every;
-  const double w = 1.0 / Ns;
-  // half-step and whole-step positions, both written out of place
-  Pos qh{d.qh, d.xqh}, qh_alt{d.qh2, d.xqh2}, q{d.q, d.xq}, q_alt{d.q2, d.xq2};
-  for (int n = 1; n <= Ns; n++) {
-    if ((n - 1) % K == 0) {  // a checkpoint segment starts: wrapped state, checkpoint, its own list
-      const size_t ck = (size_t)((n - 1) / K);
-      k_wrap<<<a->grid, kT, 0, a->s>>>(a->c, q.q, d.qf, 1);
-      MDG_ACK(cudaMemcpyAsync(d.ckq + N * ck, q.q, bytes, cudaMemcpyDeviceToDevice, a->s));
-      MDG_ACK(cudaMemcpyAsync(d.ckp + N * ck, d.p, bytes, cudaMemcpyDeviceToDevice, a->s));
-      MDG_ACK(cudaMemcpyAsync(d.q0, q.q, bytes, cudaMemcpyDeviceToDevice, a->s));
-      k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, q.q);
-      k_drift<<<a->grid, kT, 0, a->s>>>(a->c, q.q, d.p, qh.q, qh.x);
-    }
-    // the next step's half-drift here unless a segment starts there (as the
-    // backward pass recomputes it: from the wrapped checkpoint); the
-    // objective of state n - 1 rides along when that state is in this
-    // step's segment (the states are summed in order either way)
-    const Pos *next = n < Ns && n % K != 0 ? &qh_alt : nullptr;
-    fwd_step(a, qh, d.p, q_alt, d.p, next, n > 1 && (n - 1) % K != 0 ? &q : nullptr, w);
-    std::swap(q, q_alt);
-    if (next) std::swap(qh, qh_alt);
-    // the last state of a segment (or of the horizon) with its own list
-    if (n % K == 0 || n == Ns) launch_objective(a, q.q, d.p, q.x, false, w);
+  const double4_32a *q = d.q, *p = d.p;
+  for (int start = 0; start < Ns; start += K) {
+    const int len = Ns - start < K ? Ns - start : K;
+    const size_t ck = N * (size_t)(start / K);
+    k_begin<<<a->grid, kT, 0, a->s>>>(a->c, d, q, p, d.ckq + ck, d.ckp + ck, 1);
+    run_segment(a, len, false);
+    launch_objective<false>(a, len, 1.0 / Ns);
+    q = d.segq + N * len;
+    p = d.segp + N * len;
   }
   return cudaGetLastError() == cudaSuccess ? MDG_OK : afail(a, MDG_ERR_CUDA, "adjoint forward launch failed");
 }
 
 // Reverse of the horizon, segment by segment from the last: recompute the
-// segment from its checkpoint (with the same list), then reverse its steps.
+// segment from its checkpoint (with the same list), the objective's gradient at
+// all its states and the forces' sigma derivatives at all its half steps, then
+// reverse its steps.
 int enqueue_backward(mdg_adjoint *a) {
   const size_t N = (size_t)a->c.n, bytes = N * 32;
   D &d = a->d;
@@ -1126,35 +1188,19 @@ int enqueue_backward(mdg_adjoint *a) {
   for (int seg_end = Ns; seg_end > 0;) {
     const int seg_start = ((seg_end - 1) / K) * K;
     const int len = seg_end - seg_start;
-    // recompute the segment from its checkpoint: states 0..len, half steps 1..len
-    MDG_ACK(cudaMemcpyAsync(d.segq, d.ckq + N * (seg_start / K), bytes, cudaMemcpyDeviceToDevice, a->s));
-    MDG_ACK(cudaMemcpyAsync(d.segp, d.ckp + N * (seg_start / K), bytes, cudaMemcpyDeviceToDevice, a->s));
-    // the segment's list, built from the same state as in the forward pass
-    MDG_ACK(cudaMemcpyAsync(d.q0, d.segq, bytes, cudaMemcpyDeviceToDevice, a->s));
-    k_wrap<<<a->grid, kT, 0, a->s>>>(a->c, d.segq, d.qf, 0);
-    k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, d.segq);
-    k_drift<<<a->grid, kT, 0, a->s>>>(a->c, d.segq, d.segp, d.segqh + N, d.segxqh + N);
-    const Pos state{d.segq, d.segxq}, half{d.segqh, d.segxqh};
-    for (int k = 1; k <= len; k++) {
-      const Pos next = half.at(N * (k + 1));
-      fwd_step(a, half.at(N * k), d.segp + N * (k - 1), state.at(N * k), d.segp + N * k, k < len ? &next : nullptr);
-    }
-    // objective terms of the segment's last state and the reverse of the
-    // second half-drift of the step that produced it; then per step k the
-    // rest of its reverse, going on (k > 1) with the objective terms of
-    // state k - 1 and the reverse of step k - 1's second half-drift
+    const size_t ck = N * (size_t)(seg_start / K);
+    k_begin<<<a->grid, kT, 0, a->s>>>(a->c, d, d.ckq + ck, d.ckp + ck, nullptr, nullptr, 0);
+    run_segment(a, len, true);
+    launch_objective<true>(a, len, w);
+    launch_force_sigma(a, len);
     double4_32a *tmp = d.tmp, *tmp_alt = d.tmp2;
-    launch_objective(a, d.segq + N * len, d.segp + N * len, d.segxq + N * len, true, w, tmp);
+    k_seed<<<a->grid, kT, 0, a->s>>>(a->c, d, len, w, tmp);
     for (int k = len; k >= 1; k--) {
-      const Pos h = half.at(N * k);
-      if (k > 1) {
-        const Pos o = state.at(N * (k - 1));
-        launch_reverse(a, h.q, h.x, tmp, o.q, d.segp + N * (k - 1), o.x, w, tmp_alt);
-        std::swap(tmp, tmp_alt);
-      } else {
-        launch_reverse(a, h.q, h.x, tmp, nullptr, nullptr, nullptr, 0.0, nullptr);
-      }
+      if (a->c.fixed) k_reverse<true><<<a->gridp, kT, 0, a->s>>>(a->c, d, k, tmp, w, tmp_alt);
+      else k_reverse<false><<<a->gridp, kT, 0, a->s>>>(a->c, d, k, tmp, w, tmp_alt);
+      std::swap(tmp, tmp_alt);
     }
+    k_reverse_sums<<<1, 1024, 0, a->s>>>(d, len, a->gridp);
     seg_end = seg_start;
   }
   return cudaGetLastError() == cudaSuccess ? MDG_OK : afail(a, MDG_ERR_CUDA, "adjoint backward launch failed");
@@ -1263,35 +1309,34 @@ int mdg_adjoint_create(const mdg_adjoint_params *p, int32_t n, mdg_adjoint **out
   const double rho = n / c.volume;
   c.cap = ((int)(rho * 4.18879020478639 * sl * sl * sl * 1.5 + 32) + 7) & ~7;
   a->grid = (n + kT - 1) / kT;
-  a->gridp = (int)(((long long)n * kLanes + kT - 1) / kT);
+  a->gridp = (int)(((long long)n * (c.fixed ? kStepLanes : kLanes) + kT - 1) / kT);
+  a->grids = c.fixed ? (int)(((long long)n * kBatchLanes + kT - 1) / kT) : a->gridp;
   a->gridb = (int)(((long long)n * kBuildLanes + kT - 1) / kT);
   a->nck = p->steps / p->checkpoint_every + 1;
   const size_t N = (size_t)n, K = (size_t)p->checkpoint_every;
   D &d = a->d;
   cudaError_t e = cudaSetDevice(p->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&a->s, cudaStreamNonBlocking);
-  double4_32a **vecs[] = {&d.q, &d.q2, &d.p, &d.qh, &d.qh2, &d.aq, &d.ap, &d.aqh, &d.tmp, &d.tmp2, &d.q0};
-  for (auto v : vecs)
-    if (e == cudaSuccess) e = aalloc(v, N);
-  if (e == cudaSuccess) e = aalloc(&d.ckq, N * a->nck);
-  if (e == cudaSuccess) e = aalloc(&d.ckp, N * a->nck);
-  if (e == cudaSuccess) e = aalloc(&d.segq, N * (K + 1));
-  if (e == cudaSuccess) e = aalloc(&d.segp, N * (K + 1));
-  if (e == cudaSuccess) e = aalloc(&d.segqh, N * (K + 1));
   const size_t X = c.fixed ? N : 0;
-  if (e == cudaSuccess) e = aalloc(&d.xq, X);
-  if (e == cudaSuccess) e = aalloc(&d.xq2, X);
-  if (e == cudaSuccess) e = aalloc(&d.xqh, X);
-  if (e == cudaSuccess) e = aalloc(&d.xqh2, X);
-  if (e == cudaSuccess) e = aalloc(&d.segxq, X * (K + 1));
-  if (e == cudaSuccess) e = aalloc(&d.segxqh, X * (K + 1));
-  if (e == cudaSuccess) e = aalloc(&d.nbr, N * (size_t)c.cap);
-  if (e == cudaSuccess) e = aalloc(&d.cnt, N);
-  if (e == cudaSuccess) e = aalloc(&d.qf, N);
-  if (e == cudaSuccess) e = aalloc(&d.part, 3 * (size_t)a->gridp);
-  if (e == cudaSuccess) e = aalloc(&d.acc, 3);
-  if (e == cudaSuccess) e = aalloc(&d.flag, 2);
-  if (e == cudaSuccess) e = aalloc(&d.done, 1);
+  for (int pass = 0; pass < 2 && e == cudaSuccess; pass++) {
+    mdg::Slab s;
+    s.base = a->slab;
+    for (auto v : {&d.q, &d.p, &d.aq, &d.ap, &d.aqh, &d.tmp, &d.tmp2}) s.take(v, N);
+    s.take(&d.ckq, N * a->nck);
+    s.take(&d.ckp, N * a->nck);
+    for (auto v : {&d.segq, &d.segp, &d.segf, &d.segs, &d.segg}) s.take(v, N * (K + 1));
+    s.take(&d.segqh, N * (K + 2));
+    s.take(&d.segxq, X * (K + 1));
+    s.take(&d.segxqh, X * (K + 2));
+    s.take(&d.nbr, N * (size_t)c.cap);
+    s.take(&d.cnt, N);
+    s.take(&d.qf, N);
+    s.take(&d.part, 3 * (size_t)std::max(a->gridp, a->grids) * (K + 1));
+    s.take(&d.acc, 3);
+    s.take(&d.flag, 2);
+    s.take(&d.done, 1);
+    if (pass == 0) e = cudaMalloc((void **)&a->slab, s.used);
+  }
   if (e == cudaSuccess) e = cudaMemset(d.done, 0, sizeof(unsigned int));
   if (e != cudaSuccess) {
     fprintf(stderr, "mdg_adjoint_create: %s\n", cudaGetErrorString(e));
@@ -1308,11 +1353,7 @@ int mdg_adjoint_destroy(mdg_adjoint *a) {
   if (a->s) cudaStreamSynchronize(a->s);
   if (a->gx_forward) cudaGraphExecDestroy(a->gx_forward);
   if (a->gx_backward) cudaGraphExecDestroy(a->gx_backward);
-  D &d = a->d;
-  void *ptrs[] = {d.q, d.q2, d.p, d.qh, d.qh2, d.aq, d.ap, d.aqh, d.tmp, d.tmp2, d.q0, d.ckq, d.ckp, d.segq, d.segp, d.segqh,
-                  d.nbr, d.cnt, d.qf, d.part, d.acc, d.flag, d.done, d.xq, d.xq2, d.xqh, d.xqh2, d.segxq, d.segxqh};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
+  if (a->slab) cudaFree(a->slab);
   if (a->s) cudaStreamDestroy(a->s);
   delete a;
   return MDG_OK;

@@ -31,13 +31,14 @@ struct mdg_handle {
   mdg::Dev d;
   DevFlags *hflags = nullptr;  // pinned mirror
   double *hobs = nullptr, *dobs = nullptr;
+  char *slab = nullptr;  // the device arrays, all but the lists
   int cap = 0;
   bool has_state = false;
   bool nh_init = true;
   int par = 0;
   cudaGraphExec_t gx_pair[2] = {nullptr, nullptr};
   cudaGraphExec_t gx_one[2] = {nullptr, nullptr};
-  void *ctl = nullptr;            // control words of the resident kernel
+  char *ctl = nullptr;            // control words of the resident kernel
   bool resident_off = false;      // its cooperative launch was refused
   int graph_n = -1;  // particle count the graphs were captured for
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -96,12 +97,10 @@ cudaError_t dalloc(T **p, size_t count) {
 
 void dfree_all(mdg_handle *h) {
   mdg::Dev &d = h->d;
-  void *ptrs[] = {d.q_end, d.q_mid[0], d.q_mid[1], d.p, d.q_build, d.t_q, d.t_p, d.qf, d.loc[0], d.loc[1], d.id,
-                  d.inv, d.cell, d.t_id, d.t_cell, d.order, d.cell_count, d.cell_fill, d.cell_start, d.block_sums,
-                  d.nl, d.ncount, d.pl, d.pcount, d.loc_p, d.xq[0], d.xq[1], d.xb, d.xp, d.partials, d.vpart, d.cand, d.flags, d.io4, d.io4b,
-                  h->dobs};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
+  if (d.nl) cudaFree(d.nl);
+  if (d.pl) cudaFree(d.pl);
+  if (h->slab) cudaFree(h->slab);
+  h->slab = nullptr;
   memset(&h->d, 0, sizeof(h->d));
   h->dobs = nullptr;
 }
@@ -659,42 +658,46 @@ int mdg_create(const mdg_params *p, mdg_handle **out) {
   // one partial sum per block: 128 particles each, or up to 2,048 smaller blocks (mdg_fixed.cu)
   const size_t nred = (cap + 127) / 128 + 1 > 2048 ? (cap + 127) / 128 + 1 : 2048;
   const size_t cap_fx = h->g.fixed ? cap : 0, cap_loc = h->g.fixed ? 0 : cap;
-  if (e == cudaSuccess) e = dalloc(&d.q_end, cap);
-  if (e == cudaSuccess) e = dalloc(&d.q_mid[0], cap);
-  if (e == cudaSuccess) e = dalloc(&d.q_mid[1], cap);
-  if (e == cudaSuccess) e = dalloc(&d.p, cap);
-  if (e == cudaSuccess) e = dalloc(&d.q_build, cap);
-  if (e == cudaSuccess) e = dalloc(&d.t_q, cap);
-  if (e == cudaSuccess) e = dalloc(&d.t_p, cap);
-  if (e == cudaSuccess) e = dalloc(&d.qf, cap);
-  if (e == cudaSuccess) e = dalloc(&d.loc[0], cap_loc);
-  if (e == cudaSuccess) e = dalloc(&d.loc[1], cap_loc);
-  if (e == cudaSuccess) e = dalloc(&d.loc_p, cap_loc);
-  if (e == cudaSuccess) e = dalloc(&d.xq[0], cap_fx);
-  if (e == cudaSuccess) e = dalloc(&d.xq[1], cap_fx);
-  if (e == cudaSuccess) e = dalloc(&d.xb, cap_fx);
-  if (e == cudaSuccess) e = dalloc(&d.xp, cap_fx);
-  if (e == cudaSuccess) e = dalloc(&d.pcount, cap);
-  if (e == cudaSuccess) e = dalloc(&d.id, cap);
-  if (e == cudaSuccess) e = dalloc(&d.inv, cap);
-  if (e == cudaSuccess) e = dalloc(&d.cell, cap);
-  if (e == cudaSuccess) e = dalloc(&d.t_id, cap);
-  if (e == cudaSuccess) e = dalloc(&d.t_cell, cap);
-  if (e == cudaSuccess) e = dalloc(&d.order, cap);
-  if (e == cudaSuccess) e = dalloc(&d.cell_count, ncell);
-  if (e == cudaSuccess) e = dalloc(&d.cell_fill, ncell);
-  if (e == cudaSuccess) e = dalloc(&d.cell_start, ncell + 1);
-  if (e == cudaSuccess) e = dalloc(&d.block_sums, 4096);
-  if (e == cudaSuccess) e = dalloc(&d.ncount, cap);
-  if (e == cudaSuccess) e = dalloc(&d.partials, 3 * nred);
-  if (e == cudaSuccess) e = dalloc(&d.vpart, 2 * ((cap + 255) / 256 + 1));
-  if (e == cudaSuccess)
-    e = dalloc(&d.cand, p->rebuild_policy == MDG_REBUILD_REFERENCE ? 2 * (size_t)p->check_list_length : (size_t)2);
-  if (e == cudaSuccess) e = dalloc(&d.flags, 1);
-  if (e == cudaSuccess) e = dalloc(&d.io4, cap);
-  if (e == cudaSuccess) e = dalloc(&d.io4b, cap);
-  if (e == cudaSuccess) e = dalloc(&h->dobs, 4);
-  if (e == cudaSuccess) e = cudaMalloc(&h->ctl, mdg::resident_ctl_bytes());
+  for (int pass = 0; pass < 2 && e == cudaSuccess; pass++) {
+    mdg::Slab a;
+    a.base = h->slab;
+    a.take(&d.q_end, cap);
+    a.take(&d.q_mid[0], cap);
+    a.take(&d.q_mid[1], cap);
+    a.take(&d.p, cap);
+    a.take(&d.q_build, cap);
+    a.take(&d.t_q, cap);
+    a.take(&d.t_p, cap);
+    a.take(&d.qf, cap);
+    a.take(&d.loc[0], cap_loc);
+    a.take(&d.loc[1], cap_loc);
+    a.take(&d.loc_p, cap_loc);
+    a.take(&d.xq[0], cap_fx);
+    a.take(&d.xq[1], cap_fx);
+    a.take(&d.xb, cap_fx);
+    a.take(&d.xp, cap_fx);
+    a.take(&d.pcount, cap);
+    a.take(&d.id, cap);
+    a.take(&d.inv, cap);
+    a.take(&d.cell, cap);
+    a.take(&d.t_id, cap);
+    a.take(&d.t_cell, cap);
+    a.take(&d.order, cap);
+    a.take(&d.cell_count, ncell);
+    a.take(&d.cell_fill, ncell);
+    a.take(&d.cell_start, ncell + 1);
+    a.take(&d.block_sums, 4096);
+    a.take(&d.ncount, cap);
+    a.take(&d.partials, 3 * nred);
+    a.take(&d.vpart, 2 * ((cap + 255) / 256 + 1));
+    a.take(&d.cand, p->rebuild_policy == MDG_REBUILD_REFERENCE ? 2 * (size_t)p->check_list_length : (size_t)2);
+    a.take(&d.flags, 1);
+    a.take(&d.io4, cap);
+    a.take(&d.io4b, cap);
+    a.take(&h->dobs, 4);
+    a.take(&h->ctl, mdg::resident_ctl_bytes());
+    if (pass == 0) e = cudaMalloc((void **)&h->slab, a.used);
+  }
   if (e == cudaSuccess) e = cudaMemsetAsync(h->ctl, 0, mdg::resident_ctl_bytes(), h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.cell_count, 0, ncell * sizeof(int), h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.cell_fill, 0, ncell * sizeof(int), h->stream);
@@ -717,7 +720,6 @@ int mdg_destroy(mdg_handle *h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   drop_graphs(h);
   dfree_all(h);
-  if (h->ctl) cudaFree(h->ctl);
   if (h->hflags) cudaFreeHost(h->hflags);
   if (h->hobs) cudaFreeHost(h->hobs);
   if (h->ev0) cudaEventDestroy(h->ev0);

@@ -145,3 +145,38 @@ def test_batch_paths_match_the_single_box(shape, flat):
         m.calculate(2)
         np.testing.assert_allclose(states[k][1], m.state()[1], rtol=1e-9, atol=1e-9 * np.abs(p).max())
         np.testing.assert_allclose(sums[k], m.observe_raw(), rtol=1e-9)
+
+
+@pytest.mark.parametrize("objective,epsilon,sigma,seed", [("pe", 1.0, 1.0, 1), ("pressure", 1.0, 1.0, 2), ("pe", 1.3, 1.07, 3),
+                                                          ("pressure", 0.7, 0.93, 4)])
+def test_adjoint_in_fixed_point(objective, epsilon, sigma, seed):
+    # 500 atoms, one pair at 0.85 sigma, an uneven last segment: margin 0.4 takes the
+    # fixed-point sums, margin 1.2 (search length + margin above 3.9) the double ones
+    from mdacp_gb300.adjoint import Adjoint
+    q, p, L = liquid_like(0.7, 5, amp=0.08, temperature=0.7, seed=seed)
+    q[11] = np.mod(q[10] + [0.85 * sigma, 0.0, 0.0], L)
+    out = []
+    for margin in (0.4, 1.2):
+        a = Adjoint(L, len(q), steps=13, checkpoint_every=5, dt=0.001, cutoff=2.3, margin=margin, epsilon=epsilon, sigma=sigma,
+                    objective=objective)
+        J = a.forward(q, p)
+        out.append((J,) + a.backward())
+    (j0, dq0, dp0, de0, ds0), (j1, dq1, dp1, de1, ds1) = out
+    assert abs(j0 - j1) <= 1e-13 * abs(j1)
+    assert np.linalg.norm(dq0 - dq1) <= 1e-11 * np.linalg.norm(dq1)
+    assert np.linalg.norm(dp0 - dp1) <= 1e-11 * np.linalg.norm(dp1)
+    assert abs(de0 - de1) <= 1e-11 * abs(de1) and abs(ds0 - ds1) <= 1e-11 * abs(ds1)
+
+
+def test_adjoint_list_of_many_particles():
+    # 8,788 atoms: a lane's candidates no longer fit its mask words
+    from mdacp_gb300.adjoint import Adjoint
+    q, p, L = liquid_like(0.7, 13, amp=0.05, temperature=0.7, seed=5)
+    a = Adjoint(L, len(q), steps=3, checkpoint_every=2, dt=0.001, cutoff=2.5, margin=0.4)
+    m = _manager(L, len(q), margin=0.4)
+    m.set_state(q, p)
+    u = []
+    for _ in range(3):
+        m.calculate(1)
+        u.append(m.observe_raw()[1] / len(q))
+    assert abs(a.forward(q, p) - np.mean(u)) <= 1e-12 * abs(np.mean(u))
