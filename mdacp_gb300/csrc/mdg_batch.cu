@@ -1,5 +1,5 @@
 // Batched replicas: many independent periodic LJ boxes of uneven size,
-// density and temperature advanced together, one persistent kernel per step.
+// density and temperature advanced together.
 //
 // No reference counterpart (a new pattern on top of the drop-in): each box is
 // what one MDACP run does (NVE drift-kick-drift, cell list + Verlet list with a
@@ -10,15 +10,17 @@
 //   * a CTA advances each of its boxes by one step (the fused force/kick/
 //     drift over the box);
 //   * a box whose displacement test fired is rebuilt at the start of the next
-//     step by kernels ahead of the persistent one: k_batch_rebuild_set (the
-//     rebuilding boxes and their slot prefix), k_batch_bin (one thread per
-//     particle of every rebuilding box: wrap and home cell), k_batch_sort (one
-//     CTA per rebuilding box: counting sort with the cell counters in shared
-//     memory, each cell in id order), k_batch_place (one thread per particle:
-//     the reordered state and its float positions) and k_batch_list (one
-//     thread per particle, same float-first exact acceptance test as the
-//     single-box path), so a rebuild is spread over the whole GPU instead of
-//     stalling the CTA that steps the box;
+//     step by kernels over the particles of all rebuilding boxes, so a rebuild
+//     is spread over the whole GPU: k_batch_rebuild_set (the rebuilding boxes
+//     and their slot prefix), k_batch_bin (wrap, home cell, cell counts),
+//     k_batch_scan (cell starts, a CTA per box), k_batch_scatter (the cells'
+//     particles), k_batch_place (each cell in id order: the reordered state and
+//     its float positions) and k_batch_list (same float-first exact acceptance
+//     test as the single-box path);
+//   * in the flat layout (a thread per particle of all boxes) the boxes that
+//     need no rebuild are stepped while the others are rebuilt and then stepped
+//     by a second kernel, on a stream of higher priority, so that its small
+//     kernels get their turn beside the large one;
 //   * lanes-per-particle (1, 2 or 4 lanes share one particle's row and reduce
 //     with shuffles), threads per CTA and CTAs per SM are chosen by the
 //     autotuner (mdg_batch_tune);
@@ -41,7 +43,7 @@
 namespace mdg {
 namespace batch {
 
-constexpr int kMaxCellsPerBox = 4096;  // cell counters and starts live in shared memory
+constexpr int kMaxCellsPerBox = 4096;  // the largest box
 constexpr int kErrOverflow = 1, kErrBadState = 2;
 // Template value of the step kernels beside mdg_precision: the FP64 form on
 // fixed-point pair arithmetic (mdg_fixed.cuh), its state the FP64 form's.
@@ -97,7 +99,7 @@ struct Dev {
   int *cta_start, *cta_boxes;
   double4_32a *q_end, *q_mid[2], *p, *q_build, *t_q, *t_p;
   float4 *qf, *loc[2];
-  int *id, *cell, *t_id, *t_cell, *order, *cell_start;
+  int *id, *cell, *t_id, *t_cell, *order, *cell_start, *cell_count;
   uint32_t *nl, *pl;  // outer rows; inner rows in the same layout
   int *ncount, *pcount;
   float4 *loc_p;       // local positions at the last inner-list selection
@@ -176,9 +178,9 @@ __device__ __forceinline__ double4_32a box_end_from_mid(const Params &P, const D
   return q;
 }
 
-// Exclusive scan over cnt[0..m) in shared memory by the whole CTA; writes the
-// starts to out[0..m] (out[m] = total) and zeroes cnt.
-__device__ void cta_scan(int *cnt, int *out, int m) {
+// Exclusive scan over cnt[0..m) by the whole CTA; writes the starts to out[0..m]
+// (out[m] = total).
+__device__ void cta_scan(const int *cnt, int *out, int m) {
   __shared__ int warp_tot[32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -203,10 +205,7 @@ __device__ void cta_scan(int *cnt, int *out, int m) {
       if (lane < nw) warp_tot[lane] = t;
     }
     __syncthreads();
-    if (c < m) {
-      out[c] = carry + (wid ? warp_tot[wid - 1] : 0) + x - v;
-      cnt[c] = 0;
-    }
+    if (c < m) out[c] = carry + (wid ? warp_tot[wid - 1] : 0) + x - v;
     __syncthreads();
     if (threadIdx.x == 0) carry += warp_tot[nw - 1];
     __syncthreads();
@@ -229,7 +228,7 @@ __device__ __forceinline__ int rb_find(const Dev &d, int nb, int t) {
 // Rebuild part 1, one thread per particle of every rebuilding box (the FP64
 // work of a rebuild spread over the GPU: at 1/64 of the FP32 rate one SM
 // per box would take ~100 us for 8,000 particles): wrap (one +-L per
-// component) and home cell.  A particle outside [-L, 2L) fails its box.
+// component), home cell and its count.  A particle outside [-L, 2L) fails its box.
 __device__ void bin_particle(const Params &P, const Dev &d, const BoxDesc &b, int bi, int a) {
   const int o = b.atom_off;
   if (P.fixed && a == 0) d.box_wide[bi] = d.box_wide[P.nbox + bi] = 0;  // place_particle sets them anew
@@ -250,63 +249,31 @@ __device__ void bin_particle(const Params &P, const Dev &d, const BoxDesc &b, in
   if (bad) atomicExch(&d.box_err[bi], kErrBadState);
   q.x = x[0]; q.y = x[1]; q.z = x[2];
   d.q_end[o + a] = q;
-  d.cell[o + a] = (ci[2] * b.nc[1] + ci[1]) * b.nc[0] + ci[0];
+  const int c = (ci[2] * b.nc[1] + ci[1]) * b.nc[0] + ci[0];
+  d.cell[o + a] = c;
+  atomicAdd(&d.cell_count[b.cell_off + c], 1);
 }
 
-// Rebuild part 2, one CTA per rebuilding box: the integer reorder.  Cell
-// counts in shared memory, their scan, then each cell's particles in id order
-// (slots and ids scattered per cell, then one thread per particle counting
-// the cell's smaller ids: ids are distinct), cell starts, and the particles
-// gathered in the new order into the temporaries.
-__device__ void sort_box(const Dev &d, const BoxDesc &b, int *s_cnt, int *s_start) {
-  const int n = b.n, o = b.atom_off;
-  for (int c = threadIdx.x; c < b.ncell; c += blockDim.x) s_cnt[c] = 0;
-  __syncthreads();
-  for (int a = threadIdx.x; a < n; a += blockDim.x) atomicAdd(&s_cnt[d.cell[o + a]], 1);
-  __syncthreads();
-  cta_scan(s_cnt, s_start, b.ncell);
-  for (int a = threadIdx.x; a < n; a += blockDim.x) {
-    const int c = d.cell[o + a];
-    const int k = o + s_start[c] + atomicAdd(&s_cnt[c], 1);
-    d.t_cell[k] = a;
-    d.t_id[k] = d.id[o + a];
-  }
-  for (int c = threadIdx.x; c < b.ncell; c += blockDim.x) d.cell_start[b.cell_off + c] = s_start[c];
-  if (threadIdx.x == 0) d.cell_start[b.cell_off + b.ncell] = n;
-  __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    const int v = d.t_cell[o + k], key = d.t_id[o + k];
-    const int c = d.cell[o + v];
-    const int lo = s_start[c], hi = s_start[c + 1];
-    int r = 0;
-    for (int m = lo; m < hi; m++) r += d.t_id[o + m] < key ? 1 : 0;
-    d.order[o + lo + r] = v;
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    const int src = o + d.order[o + k];
-    d.t_q[o + k] = d.q_end[src];
-    d.t_p[o + k] = d.p[src];
-    d.t_id[o + k] = d.id[src];
-    d.t_cell[o + k] = d.cell[src];
-  }
-}
-
-// Rebuild part 3, one thread per particle of every rebuilding box: the
-// reordered state back in place, with the build-time and mid-step positions.
+// Rebuild part 4, one thread per particle of every rebuilding box: the place of
+// the particle at slot k of the cells' lists (d.order), its cell's particles
+// being in id order (distinct), and there its state in the temporaries (the
+// list kernel moves it back: other threads still read it here) and its
+// build-time and mid-step positions.
 // Mixed forms: q_mid relative to the home-cell centre, (q - c) + p dt/2,
 // with the build position packed in q_mid.w (the rebuild test's reference)
 // and in p.w (the prune reference until the step's re-selection records its
 // own); q_end is current until the box steps.
-__device__ void place_particle(const Params &P, const Dev &d, const BoxDesc &b, int bi, int k, int par) {
+__device__ void place_particle(const Params &P, const Dev &d, const BoxDesc &b, int bi, int slot, int par) {
   const int o = b.atom_off;
-  const double4_32a q = d.t_q[o + k];
-  double4_32a p = d.t_p[o + k];
-  const int c = d.t_cell[o + k];
-  d.q_end[o + k] = q;
-  d.id[o + k] = d.t_id[o + k];
-  d.cell[o + k] = c;
-  if (k == 0) d.box_mid[bi] = -1;
+  const int v = d.order[o + slot], id = d.id[o + v], c = d.cell[o + v];
+  const double4_32a q = d.q_end[o + v];
+  double4_32a p = d.p[o + v];
+  int k = d.cell_start[b.cell_off + c];
+  for (int m = k, hi = d.cell_start[b.cell_off + c + 1]; m < hi; m++) k += d.id[o + d.order[o + m]] < id ? 1 : 0;
+  d.t_q[o + k] = q;
+  d.t_id[o + k] = id;
+  d.t_cell[o + k] = c;
+  if (slot == 0) d.box_mid[bi] = -1;
   int cx, cy, cz;
   cell_xyz(b, c, cx, cy, cz);
   const double ox = box_cell_centre(b, 0, cx), oy = box_cell_centre(b, 1, cy), oz = box_cell_centre(b, 2, cz);
@@ -337,7 +304,7 @@ __device__ void place_particle(const Params &P, const Dev &d, const BoxDesc &b, 
       d.loc[par][o + k] = make_float4((float)(m.x - ox), (float)(m.y - oy), (float)(m.z - oz), 0.0f);
     }
   }
-  d.p[o + k] = p;
+  d.t_p[o + k] = p;
 }
 
 // Pair-list row of local particle a of box b (the box's cell starts and
@@ -357,7 +324,7 @@ __device__ __forceinline__ int build_row(const Params &P, const Dev &d, const Bo
   int cx = 0, cy = 0, cz = 0, cnt = 0;
   if (active) {
     fi = qf[a];
-    cell_xyz(b, d.cell[o + a], cx, cy, cz);
+    cell_xyz(b, d.t_cell[o + a], cx, cy, cz);
   }
   auto scan = [&](int ox, int oy, int oz, auto &&emit) {
     int sx, sy, sz;
@@ -375,7 +342,7 @@ __device__ __forceinline__ int build_row(const Params &P, const Dev &d, const Bo
       if (own_image && (unsigned)(a - j0) < 32u) in &= ~(1u << (a - j0));  // the particle itself
       for (uint32_t band = in & ~sure; band; band &= band - 1u) {
         const int u = __ffs(band) - 1;
-        const double4_32a qi = d.q_end[o + a], qj = d.q_end[o + j0 + u];
+        const double4_32a qi = d.t_q[o + a], qj = d.t_q[o + j0 + u];
         const double xj = sx ? __dadd_rn(qj.x, sx > 0 ? b.L[0] : -b.L[0]) : qj.x;
         const double yj = sy ? __dadd_rn(qj.y, sy > 0 ? b.L[1] : -b.L[1]) : qj.y;
         const double zj = sz ? __dadd_rn(qj.z, sz > 0 ? b.L[2] : -b.L[2]) : qj.z;
@@ -440,21 +407,16 @@ __device__ __forceinline__ int build_row(const Params &P, const Dev &d, const Bo
   return cnt;
 }
 
-// Rebuild part 1 for every box that rebuilds this step: one CTA per box.
-// One CTA per rebuilding box; the largest box's serial phases bound the
-// kernel, so the CTA is as wide as possible: 1,024 threads measured 1.04 ms per
-// step on 1,024 boxes against 1.09 (512) and 1.15 (256).
-#ifndef MDG_BATCH_PREP_THREADS
-#define MDG_BATCH_PREP_THREADS 1024
-#endif
-constexpr int kPrepThreads = MDG_BATCH_PREP_THREADS;
 // Lanes of a particle's row in the list build, and the number of rebuilding
 // particles below which they are used (100 steps of 256 boxes, about 50,000
 // rebuilding particles a step: 34.5 ms without, 33.3 below 30,000, 30.8 below
 // 60,000, 30.4 below 100,000, 30.5 below 200,000; 48 boxes FP64, about 10,000:
 // 24.2 without, 18.3).
 constexpr int kRowLanes = 9, kLanesBelow = 100000;
-constexpr int kBatchKernelsPerStep = 6;  // rebuild set, bin, sort, place, list, step (+ finish in the flat layout)
+// Kernels of a step: bin, scan, scatter, place, list and the step; one more
+// ahead of them (rebuild set), or in the flat layout two more after them (the
+// step of the rebuilt boxes, finish).
+constexpr int kBatchKernelsPerStep = 6;
 
 __global__ void __launch_bounds__(128) k_batch_bin(Params P, Dev d) {
   const int nb = *d.rb_count;
@@ -466,13 +428,32 @@ __global__ void __launch_bounds__(128) k_batch_bin(Params P, Dev d) {
   }
 }
 
-__global__ void __launch_bounds__(kPrepThreads) k_batch_sort(Dev d) {
-  __shared__ int s_cnt[kMaxCellsPerBox];
-  __shared__ int s_start[kMaxCellsPerBox + 1];
-  const int bi = blockIdx.x;
-  if (!rebuilding(d, bi, *d.goal)) return;  // uniform over the CTA; a box failed by k_batch_bin stops here
-  const BoxDesc b = d.boxes[bi];
-  sort_box(d, b, s_cnt, s_start);
+// Rebuild part 2: the cell starts of each rebuilding box from its counts, one
+// CTA per box in turn.  A box that k_batch_bin failed only drops its counts.
+__global__ void __launch_bounds__(256) k_batch_scan(Dev d) {
+  const int nb = *d.rb_count;
+  for (int k = blockIdx.x; k < nb; k += gridDim.x) {
+    const int bi = d.rb_boxes[k];
+    const BoxDesc &b = d.boxes[bi];
+    int *cnt = d.cell_count + b.cell_off;
+    if (d.box_err[bi] == 0) cta_scan(cnt, d.cell_start + b.cell_off, b.ncell);
+    else
+      for (int c = threadIdx.x; c < b.ncell; c += blockDim.x) cnt[c] = 0;
+  }
+}
+
+// Rebuild part 3: each cell's particles listed from its start, in any order;
+// the counts go down to 0.
+__global__ void __launch_bounds__(128) k_batch_scatter(Dev d) {
+  const int nb = *d.rb_count;
+  if (nb == 0) return;
+  const int total = d.rb_start[nb];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const int k = rb_find(d, nb, t), bi = d.rb_boxes[k], a = t - d.rb_start[k];
+    if (d.box_err[bi] != 0) continue;
+    const int o = d.boxes[bi].atom_off, c = d.boxes[bi].cell_off + d.cell[o + a];
+    d.order[o + d.cell_start[c] + atomicSub(&d.cell_count[c], 1) - 1] = a;
+  }
 }
 
 __global__ void __launch_bounds__(128) k_batch_place(Params P, Dev d, int par) {
@@ -488,7 +469,7 @@ __global__ void __launch_bounds__(128) k_batch_place(Params P, Dev d, int par) {
 // Ahead of the rebuild parts: the boxes that rebuild this step, in box order,
 // and the prefix of their particle counts (a box the rebuild then fails stays
 // in the set; the later parts skip it).  One CTA of 1,024 threads.
-__global__ void __launch_bounds__(1024) k_batch_rebuild_set(Params P, Dev d) {
+__device__ void rebuild_set(const Params &P, const Dev &d) {
   __shared__ int carry_n, carry_k;
   __shared__ long long wsum[32];
   const long long goal = *d.goal;
@@ -535,9 +516,11 @@ __global__ void __launch_bounds__(1024) k_batch_rebuild_set(Params P, Dev d) {
   }
 }
 
-// Rebuild part 2: one thread, or nine lanes, per particle slot of every
+__global__ void __launch_bounds__(1024) k_batch_rebuild_set(Params P, Dev d) { rebuild_set(P, d); }
+
+// Rebuild part 5: one thread, or nine lanes, per particle slot of every
 // rebuilding box, so a box's list is built by the whole GPU rather than by the
-// CTA that steps it.
+// CTA that steps it; and the particle's state back in place.
 // A fixed grid walks the concatenated slots of this step's rebuilding boxes.
 __global__ void __launch_bounds__(128) k_batch_list(Params P, Dev d) {
   const int nb = *d.rb_count;
@@ -556,6 +539,13 @@ __global__ void __launch_bounds__(128) k_batch_list(Params P, Dev d) {
     const BoxDesc &b = d.boxes[bi];
     const int a = in ? t - d.rb_start[lo] : 0;
     const int cnt = lanes ? build_row<kRowLanes>(P, d, b, a, active, lane, wl - lane) : build_row<1>(P, d, b, a, active, 0, wl);
+    if (active && lane == 0) {
+      const int s = b.atom_off + a;
+      d.q_end[s] = d.t_q[s];
+      d.p[s] = d.t_p[s];
+      d.id[s] = d.t_id[s];
+      d.cell[s] = d.t_cell[s];
+    }
     if (active && lane == 0 && cnt > P.list_cap) {
       atomicMax(&d.box_need[bi], cnt);
       atomicExch(&d.box_err[bi], kErrOverflow);
@@ -1022,15 +1012,18 @@ __global__ void __launch_bounds__(512, MIXED == kFixedForm ? 1 : (MIXED ? MDG_BA
   }
 }
 
-// The same step in the flat layout: the grid (only as many CTAs as are
-// resident at once) strides over the particles of all boxes, one thread per
-// particle, so no CTA waits for the slowest warp of a box before the next,
-// the work of a box spreads over the whole GPU and the kernel holds no box
-// description in registers (its fields are read where they are used, from
-// L1).  A particle whose displacement test fires raises its box's request
-// with a plain store of 1; k_batch_finish applies the requests and counts the
-// box's step after the kernel.  The box state the step reads (error, step
-// count, rebuild and re-selection flags) is not written during it.
+// The same step in the flat layout: one thread per particle of all boxes, so no
+// CTA waits for the slowest warp of a box before the next, the work of a box
+// spreads over the whole GPU and the kernel holds no box description in
+// registers (its fields are read where they are used, from L1).  A particle
+// whose displacement test fires raises its box's request with a plain store of
+// 1; k_batch_finish applies the requests and counts the box's step after the
+// kernel.  The box state the step reads (error, step count, rebuild and
+// re-selection flags) is not written during it, but for the error of a
+// rebuilding box, which this kernel leaves to k_batch_step_rebuilt.
+// 100 steps of 256 boxes, mixed, whose rebuilds (a dozen boxes a step) used to
+// run ahead of the step, 294 us a step: 240 with them beside it, 230 with the
+// sort spread over the GPU too (one CTA a box: 33 us); 48 boxes FP64 181, 146, 138.
 // Resident 256-thread CTAs per SM the flat kernel is compiled for: 4 gives
 // 64 registers, where the inner-list variant runs without spills and beats
 // the outer-list walk (1,024 boxes, mixed: 5.18e9 atom-steps/s at 128 x 8
@@ -1043,53 +1036,74 @@ __global__ void __launch_bounds__(512, MIXED == kFixedForm ? 1 : (MIXED ? MDG_BA
 // boxes (205,044 atoms, observed every 100), 3 (80, 60 bytes spilled) 0.295.
 constexpr int kFlatFixedBlocks = 2;
 constexpr int kFlatMaxThreads = 256;
+template <int MIXED, int INNER, bool REBUILT>
+__device__ __forceinline__ void flat_step(const Params &P, const Dev &d, int bi, int s, int par) {
+  const BoxDesc &b = d.boxes[bi];
+  const int a = s - b.atom_off;
+  double3 F;
+  bool sel = REBUILT;  // a rebuild is followed by a re-selection
+  int kept = 0;
+  if constexpr (INNER != 0) {
+    if (!REBUILT) sel = d.box_prune[bi] != 0;
+    if (sel) F = box_force<MIXED, 1, 1>(P, d, b, bi, a, 0, par, true, &kept);
+    else F = box_force<MIXED, 1, 2>(P, d, b, bi, a, 0, par);
+  } else {
+    F = box_force<MIXED, 1, 0>(P, d, b, bi, a, 0, par);
+  }
+  bool rebuild = false, reselect = false;
+  advance_particle<MIXED, INNER != 0>(P, d, b, bi, s, F, par, sel, kept, rebuild, reselect);
+  if (rebuild) d.box_req[bi] = 1;
+  if (INNER != 0 && reselect) d.box_preq[bi] = 1;
+}
+
 template <int MIXED, int INNER>
-__global__ void __launch_bounds__(kFlatMaxThreads, MIXED == kFixedForm ? kFlatFixedBlocks : MDG_BATCH_FLAT_MIN_BLOCKS) k_batch_step_flat(Params P, Dev d,
-                                                                                            int par) {
-  const long long goal = *d.goal;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < P.total; s += gridDim.x * blockDim.x) {
-    const int bi = d.box_of_slot[s];
-    if (d.box_err[bi] != 0 || d.box_steps[bi] >= goal) continue;
-    const BoxDesc &b = d.boxes[bi];
-    const int a = s - b.atom_off;
-    const bool sel = d.box_rebuild[bi] != 0 || d.box_prune[bi] != 0;
-    double3 F;
-    int kept = 0;
-    if constexpr (INNER != 0) {
-      if (sel) F = box_force<MIXED, 1, 1>(P, d, b, bi, a, 0, par, true, &kept);
-      else F = box_force<MIXED, 1, 2>(P, d, b, bi, a, 0, par);
-    } else {
-      F = box_force<MIXED, 1, 0>(P, d, b, bi, a, 0, par);
-    }
-    bool rebuild = false, reselect = false;
-    advance_particle<MIXED, INNER != 0>(P, d, b, bi, s, F, par, sel, kept, rebuild, reselect);
-    if (rebuild) d.box_req[bi] = 1;
-    if (INNER != 0 && reselect) d.box_preq[bi] = 1;
+__global__ void __launch_bounds__(kFlatMaxThreads, MIXED == kFixedForm ? kFlatFixedBlocks : MDG_BATCH_FLAT_MIN_BLOCKS)
+    k_batch_step_flat(Params P, Dev d, int par) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= P.total) return;
+  const int bi = d.box_of_slot[s];
+  if (d.box_rebuild[bi] != 0 || d.box_err[bi] != 0 || d.box_steps[bi] >= *d.goal) return;
+  flat_step<MIXED, INNER, false>(P, d, bi, s, par);
+}
+
+// The boxes that rebuild this step, once their lists are made.
+template <int MIXED, int INNER>
+__global__ void __launch_bounds__(kFlatMaxThreads, MIXED == kFixedForm ? kFlatFixedBlocks : MDG_BATCH_FLAT_MIN_BLOCKS)
+    k_batch_step_rebuilt(Params P, Dev d, int par) {
+  const int nb = *d.rb_count;
+  if (nb == 0) return;
+  const int total = d.rb_start[nb];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const int k = rb_find(d, nb, t), bi = d.rb_boxes[k];
+    if (d.box_err[bi] == 0) flat_step<MIXED, INNER, true>(P, d, bi, d.boxes[bi].atom_off + t - d.rb_start[k], par);
   }
 }
 
 // After the flat step, one thread per box (the same participation test as
 // the step): the rebuild this step consumed is counted, the requests become
-// the next step's flags, the box's step count advances.
+// the next step's flags, the box's step count advances; then the next step's
+// rebuild set.  One CTA of 1,024 threads.
 template <int INNER>
-__global__ void k_batch_finish(Params P, Dev d, int par) {
-  const int bi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (bi >= P.nbox) return;
-  if (d.box_err[bi] != 0 || d.box_steps[bi] >= *d.goal) return;
-  if (d.box_rebuild[bi]) {
-    d.box_rebuild[bi] = 0;
-    d.box_rebuilds[bi] += 1;
+__global__ void __launch_bounds__(1024) k_batch_finish(Params P, Dev d, int par) {
+  const long long goal = *d.goal;
+  for (int bi = threadIdx.x; bi < P.nbox; bi += blockDim.x) {
+    if (d.box_err[bi] != 0 || d.box_steps[bi] >= goal) continue;
+    if (d.box_rebuild[bi]) {
+      d.box_rebuild[bi] = 0;
+      d.box_rebuilds[bi] += 1;
+    }
+    if (d.box_req[bi]) {
+      d.box_rebuild[bi] = 1;
+      d.box_req[bi] = 0;
+    }
+    if (INNER != 0) {
+      d.box_prune[bi] = d.box_preq[bi];
+      d.box_preq[bi] = 0;
+    }
+    if (P.local_pos) d.box_mid[bi] = par ^ 1;
+    d.box_steps[bi] += 1;
   }
-  if (d.box_req[bi]) {
-    d.box_rebuild[bi] = 1;
-    d.box_req[bi] = 0;
-  }
-  if (INNER != 0) {
-    d.box_prune[bi] = d.box_preq[bi];
-    d.box_preq[bi] = 0;
-  }
-  if (P.local_pos) d.box_mid[bi] = par ^ 1;
-  d.box_steps[bi] += 1;
+  rebuild_set(P, d);  // each thread reads the boxes it wrote
 }
 
 // Observers (observer.cc:5-79) at q_end, pairs weighted 1/2 (each is listed
@@ -1239,6 +1253,9 @@ struct mdg_batch {
   double buffer = 0.0;  // inner-list buffer in use
   double ref_unit = 0.0;  // mixed forms: the largest packed-position unit, w / (2^20 - 1), over the boxes
   cudaStream_t stream = nullptr;
+  // flat layout: the rebuilding boxes' stream, of the highest priority, and its fork and join
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   Params P;
   Dev d;
   std::vector<BoxDesc> boxes;
@@ -1405,29 +1422,44 @@ int alloc_batch_list(mdg_batch *b, int cap) {
   return MDG_OK;
 }
 
+// The rebuild of the boxes that are due, on `stream`.
+void launch_batch_rebuild(mdg_batch *b, int par, cudaStream_t stream) {
+  k_batch_bin<<<b->num_sms * 16, 128, 0, stream>>>(b->P, b->d);
+  k_batch_scan<<<std::min(b->nbox, b->num_sms * 4), 256, 0, stream>>>(b->d);
+  k_batch_scatter<<<b->num_sms * 16, 128, 0, stream>>>(b->d);
+  k_batch_place<<<b->num_sms * 16, 128, 0, stream>>>(b->P, b->d, par);
+  k_batch_list<<<b->num_sms * 16, 128, 0, stream>>>(b->P, b->d);
+}
+
 void launch_batch_step(mdg_batch *b, int par) {
   const int T = b->threads;
   const int prec = step_form(b);
-  k_batch_rebuild_set<<<1, 1024, 0, b->stream>>>(b->P, b->d);
-  k_batch_bin<<<b->num_sms * 16, 128, 0, b->stream>>>(b->P, b->d);
-  k_batch_sort<<<b->nbox, kPrepThreads, 0, b->stream>>>(b->d);
-  k_batch_place<<<b->num_sms * 16, 128, 0, b->stream>>>(b->P, b->d, par);
-  k_batch_list<<<b->num_sms * 16, 128, 0, b->stream>>>(b->P, b->d);
-#define MDG_BSTEP(M, L, I) k_batch_step<M, L, I><<<b->grid, T, 0, b->stream>>>(b->P, b->d, par)
   const bool inner = b->P.inner && b->lpi == 1 && b->use_inner;
   if (b->flat) {
-#define MDG_FSTEP(M, I) k_batch_step_flat<M, I><<<b->grid, T, 0, b->stream>>>(b->P, b->d, par)
+    cudaEventRecord(b->ev_fork, b->stream);
+    cudaStreamWaitEvent(b->side, b->ev_fork, 0);
+    launch_batch_rebuild(b, par, b->side);
+    const int G = (b->total + T - 1) / T;
+#define MDG_FSTEP(M, I)                                                  \
+  do {                                                                   \
+    k_batch_step_rebuilt<M, I><<<b->grid, T, 0, b->side>>>(b->P, b->d, par); \
+    k_batch_step_flat<M, I><<<G, T, 0, b->stream>>>(b->P, b->d, par);    \
+  } while (0)
     if (prec == kFixedForm) { if (inner) MDG_FSTEP(kFixedForm, 1); else MDG_FSTEP(kFixedForm, 0); }
     else if (prec == MDG_MIXED) { if (inner) MDG_FSTEP(MDG_MIXED, 1); else MDG_FSTEP(MDG_MIXED, 0); }
     else if (prec == MDG_MIXED_PLAIN) { if (inner) MDG_FSTEP(MDG_MIXED_PLAIN, 1); else MDG_FSTEP(MDG_MIXED_PLAIN, 0); }
     else { if (inner) MDG_FSTEP(MDG_FP64, 1); else MDG_FSTEP(MDG_FP64, 0); }
 #undef MDG_FSTEP
-    const int fg = (b->nbox + 255) / 256;
-    if (inner) k_batch_finish<1><<<fg, 256, 0, b->stream>>>(b->P, b->d, par);
-    else k_batch_finish<0><<<fg, 256, 0, b->stream>>>(b->P, b->d, par);
-    b->launches += kBatchKernelsPerStep + 1;
+    cudaEventRecord(b->ev_join, b->side);
+    cudaStreamWaitEvent(b->stream, b->ev_join, 0);
+    if (inner) k_batch_finish<1><<<1, 1024, 0, b->stream>>>(b->P, b->d, par);
+    else k_batch_finish<0><<<1, 1024, 0, b->stream>>>(b->P, b->d, par);
+    b->launches += kBatchKernelsPerStep + 2;
     return;
   }
+  k_batch_rebuild_set<<<1, 1024, 0, b->stream>>>(b->P, b->d);
+  launch_batch_rebuild(b, par, b->stream);
+#define MDG_BSTEP(M, L, I) k_batch_step<M, L, I><<<b->grid, T, 0, b->stream>>>(b->P, b->d, par)
   if (prec == kFixedForm) {
     if (b->lpi == 4) MDG_BSTEP(kFixedForm, 4, 0); else if (b->lpi == 2) MDG_BSTEP(kFixedForm, 2, 0);
     else if (inner) MDG_BSTEP(kFixedForm, 1, 1); else MDG_BSTEP(kFixedForm, 1, 0);
@@ -1442,10 +1474,19 @@ void launch_batch_step(mdg_batch *b, int par) {
     else if (inner) MDG_BSTEP(0, 1, 1); else MDG_BSTEP(0, 1, 0);
   }
 #undef MDG_BSTEP
-  b->launches += kBatchKernelsPerStep;
+  b->launches += kBatchKernelsPerStep + 1;
+}
+
+// Ahead of the first of several steps in the flat layout: its rebuild set (the
+// others' is made by k_batch_finish).
+void begin_steps(mdg_batch *b) {
+  if (!b->flat) return;
+  k_batch_rebuild_set<<<1, 1024, 0, b->stream>>>(b->P, b->d);
+  b->launches++;
 }
 
 int run_steps(mdg_batch *b, int nsteps) {
+  begin_steps(b);
   if (!b->prm.use_graphs) {
     for (int k = 0; k < nsteps; k++) {
       launch_batch_step(b, b->par);
@@ -1465,12 +1506,12 @@ int run_steps(mdg_batch *b, int nsteps) {
         launch_batch_step(b, par ^ 1);
         b->launches = l0;
         MDG_BCK(cudaStreamEndCapture(b->stream, &g));
-        cudaError_t e = cudaGraphInstantiate(&b->gx[par], g, 0);
+        cudaError_t e = cudaGraphInstantiate(&b->gx[par], g, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return bfail(b, MDG_ERR_CUDA, cudaGetErrorString(e));
       }
       MDG_BCK(cudaGraphLaunch(b->gx[par], b->stream));
-      b->launches += 2 * (kBatchKernelsPerStep + (b->flat ? 1 : 0));
+      b->launches += 2 * (kBatchKernelsPerStep + (b->flat ? 2 : 1));
       left -= 2;
     } else {
       launch_batch_step(b, par);
@@ -1611,7 +1652,12 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   cap = (cap + 7) & ~7;
   cudaError_t e = cudaSetDevice(p->device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, p->device);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+  int low = 0, high = 0;
+  if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&low, &high);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, low);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->side, cudaStreamNonBlocking, high);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
   Dev &d = b->d;
@@ -1656,6 +1702,8 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   if (e == cudaSuccess) e = balloc(&d.rb_start, (size_t)nbox + 1);
   if (e == cudaSuccess) e = balloc(&d.rb_count, 1);
   if (e == cudaSuccess) e = balloc(&d.cell_start, (size_t)cells);
+  if (e == cudaSuccess) e = balloc(&d.cell_count, (size_t)cells);
+  if (e == cudaSuccess) e = cudaMemset(d.cell_count, 0, (size_t)cells * sizeof(int));
   if (e == cudaSuccess) e = balloc(&d.box_rebuild, nbox);
   if (e == cudaSuccess) e = balloc(&d.box_err, nbox);
   if (e == cudaSuccess) e = balloc(&d.box_need, nbox);
@@ -1689,7 +1737,7 @@ int mdg_batch_destroy(mdg_batch *b) {
   drop_batch_graphs(b);
   Dev &d = b->d;
   void *ptrs[] = {d.boxes, d.cta_start, d.cta_boxes, d.q_end, d.q_mid[0], d.q_mid[1], d.p, d.q_build, d.t_q, d.t_p,
-                  d.qf, d.loc[0], d.loc[1], d.id, d.cell, d.t_id, d.t_cell, d.order, d.cell_start, d.nl, d.ncount,
+                  d.qf, d.loc[0], d.loc[1], d.id, d.cell, d.t_id, d.t_cell, d.order, d.cell_start, d.cell_count, d.nl, d.ncount,
                   d.pl, d.pcount, d.loc_p, d.box_prune, d.box_req, d.box_preq, d.rb_boxes, d.rb_start, d.rb_count,
                   d.box_rebuild, d.box_err, d.box_need, d.box_steps, d.box_rebuilds, d.goal, d.partials,
                   d.box_mid, d.xq[0], d.xq[1], d.xb, d.xp, d.box_wide, d.box_wide_end, b->obs_part, b->d_box_of_slot};
@@ -1697,6 +1745,9 @@ int mdg_batch_destroy(mdg_batch *b) {
     if (p) cudaFree(p);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
+  if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+  if (b->ev_join) cudaEventDestroy(b->ev_join);
+  if (b->side) cudaStreamDestroy(b->side);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return MDG_OK;
@@ -1778,6 +1829,7 @@ int mdg_batch_calculate(mdg_batch *b, int32_t nsteps) {
       MDG_BCK(cudaMemcpyAsync(b->d.box_need, zeros.data(), b->nbox * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     }
     // catch-up: only boxes behind the goal advance
+    begin_steps(b);
     for (long long k = 0; k < behind; k++) {
       launch_batch_step(b, b->par);
       b->par ^= 1;
