@@ -117,9 +117,9 @@ struct Dev {
   int *box_wide_end; // the same for the positions an observation reads
   double *partials;  // per box: KE, PE, virial
   const int *box_of_slot;
-  // this step's rebuilding boxes in box order and their first atom in the
-  // concatenation of their slots (rb_start[rb_count] = atoms to list)
-  int *rb_boxes, *rb_start, *rb_count;
+  // this step's rebuilding boxes in box order, and their first atom and cell in
+  // the concatenation of their slots and cells (at rb_count the totals)
+  int *rb_boxes, *rb_start, *rb_cells, *rb_count;
 };
 
 // A box takes part in this step's rebuild: flagged, healthy, behind the goal.
@@ -214,13 +214,13 @@ __device__ void cta_scan(const int *cnt, int *out, int m) {
   __syncthreads();
 }
 
-// Slot t of this step's rebuilding boxes (their particles side by side):
-// the index k into rb_boxes / rb_start with rb_start[k] <= t < rb_start[k + 1].
-__device__ __forceinline__ int rb_find(const Dev &d, int nb, int t) {
+// Particle (or cell) t of this step's rebuilding boxes, laid side by side: the
+// index k into rb_boxes with start[k] <= t < start[k + 1].
+__device__ __forceinline__ int rb_find(const int *start, int nb, int t) {
   int lo = 0, hi = nb - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (d.rb_start[mid] <= t) lo = mid; else hi = mid - 1;
+    if (start[mid] <= t) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
@@ -307,112 +307,6 @@ __device__ void place_particle(const Params &P, const Dev &d, const BoxDesc &b, 
   d.t_p[o + k] = p;
 }
 
-// Pair-list row of local particle a of box b (the box's cell starts and
-// build-time positions are in place): the 27 stencil cells with periodic
-// wrap, float-first exact acceptance (mdg_build.cuh), by one thread (LANES = 1)
-// or by LANES = 9 neighbouring lanes of a warp, one for each (y, z) row of three
-// cells; `base` is the first of them.  Returns the row length to lane 0 (rows
-// longer than the capacity are truncated and flag the box); every lane of the
-// warp calls it, `active` or not.
-template <int LANES>
-__device__ __forceinline__ int build_row(const Params &P, const Dev &d, const BoxDesc &b, int a, bool active, int lane, int base) {
-  const int n = b.n, o = b.atom_off;
-  const int *cstart = d.cell_start + b.cell_off;
-  const float4 *qf = d.qf + o;
-  uint32_t *row = d.nl + b.list_off + a;
-  float4 fi = make_float4(0.f, 0.f, 0.f, 0.f);
-  int cx = 0, cy = 0, cz = 0, cnt = 0;
-  if (active) {
-    fi = qf[a];
-    cell_xyz(b, d.t_cell[o + a], cx, cy, cz);
-  }
-  auto scan = [&](int ox, int oy, int oz, auto &&emit) {
-    int sx, sy, sz;
-    const int nx = wrap_cell(cx, ox, b.nc[0], sx), ny = wrap_cell(cy, oy, b.nc[1], sy), nz = wrap_cell(cz, oz, b.nc[2], sz);
-    const float fx = (float)ox * b.w32[0] + (float)sx * b.dl32[0] - fi.x;
-    const float fy = (float)oy * b.w32[1] + (float)sy * b.dl32[1] - fi.y;
-    const float fz = (float)oz * b.w32[2] + (float)sz * b.dl32[2] - fi.z;
-    const int cc = (nz * b.nc[1] + ny) * b.nc[0] + nx;
-    const int lo = cstart[cc], hi = cstart[cc + 1];
-    const uint32_t code = entry_pack(0, ox, oy, oz);
-    const bool own_image = (sx | sy | sz) == 0;
-    for (int j0 = lo; j0 < hi; j0 += 32) {
-      uint32_t in, sure;
-      chunk_masks(qf, j0, min(hi - j0, 32), fx, fy, fz, P.acc_lo, P.acc_hi, in, sure);
-      if (own_image && (unsigned)(a - j0) < 32u) in &= ~(1u << (a - j0));  // the particle itself
-      for (uint32_t band = in & ~sure; band; band &= band - 1u) {
-        const int u = __ffs(band) - 1;
-        const double4_32a qi = d.t_q[o + a], qj = d.t_q[o + j0 + u];
-        const double xj = sx ? __dadd_rn(qj.x, sx > 0 ? b.L[0] : -b.L[0]) : qj.x;
-        const double yj = sy ? __dadd_rn(qj.y, sy > 0 ? b.L[1] : -b.L[1]) : qj.y;
-        const double zj = sz ? __dadd_rn(qj.z, sz > 0 ? b.L[2] : -b.L[2]) : qj.z;
-        const double dx = __dsub_rn(qi.x, xj), dy = __dsub_rn(qi.y, yj), dz = __dsub_rn(qi.z, zj);
-        const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-        if (!(r2 <= P.sl2)) in &= ~(1u << u);
-      }
-      emit(in, j0, code);
-    }
-  };
-  auto append = [&](uint32_t in, int j0, uint32_t code) {
-    for (; in; in &= in - 1u) {
-      const int j = j0 + __ffs(in) - 1;
-      if (cnt < P.list_cap) row[(long long)cnt * n] = ((uint32_t)j << kCodeBits) | code;
-      cnt++;
-    }
-  };
-  if (LANES == 1) {
-    if (active)
-      for (int oz = -1; oz <= 1; oz++)
-        for (int oy = -1; oy <= 1; oy++)
-          for (int ox = -1; ox <= 1; ox++) scan(ox, oy, oz, append);
-  } else {
-    // as k_build_list's lanes (mdg_list.cu)
-    const int oy = lane % 3 - 1, oz = lane / 3 - 1;
-    int own = 0;
-    uint32_t kept[3] = {0u, 0u, 0u};
-    int first[3] = {0, 0, 0};
-    bool again = false;
-    if (active)
-#pragma unroll
-      for (int ox = -1; ox <= 1; ox++) {
-        int chunk = 0;
-        scan(ox, oy, oz, [&](uint32_t in, int j0, uint32_t) {
-          own += __popc(in);
-          if (chunk++ == 0) {
-            kept[ox + 1] = in;
-            first[ox + 1] = j0;
-          } else {
-            again = true;
-          }
-        });
-      }
-    int before = 0, total = 0;
-#pragma unroll
-    for (int l = 0; l < LANES; l++) {
-      const int v = __shfl_sync(0xffffffffu, own, min(base + l, 31));
-      before += l < lane ? v : 0;
-      total += v;
-    }
-    cnt = before;
-    if (active) {
-#pragma unroll
-      for (int ox = -1; ox <= 1; ox++) {
-        if (again) scan(ox, oy, oz, append);
-        else append(kept[ox + 1], first[ox + 1], entry_pack(0, ox, oy, oz));
-      }
-    }
-    cnt = total;
-  }
-  if (active && lane == 0) d.ncount[o + a] = cnt < P.list_cap ? cnt : P.list_cap;
-  return cnt;
-}
-
-// Lanes of a particle's row in the list build, and the number of rebuilding
-// particles below which they are used (100 steps of 256 boxes, about 50,000
-// rebuilding particles a step: 34.5 ms without, 33.3 below 30,000, 30.8 below
-// 60,000, 30.4 below 100,000, 30.5 below 200,000; 48 boxes FP64, about 10,000:
-// 24.2 without, 18.3).
-constexpr int kRowLanes = 9, kLanesBelow = 100000;
 // Kernels of a step: bin, scan, scatter, place, list and the step; one more
 // ahead of them (rebuild set), or in the flat layout two more after them (the
 // step of the rebuilt boxes, finish).
@@ -423,7 +317,7 @@ __global__ void __launch_bounds__(128) k_batch_bin(Params P, Dev d) {
   if (nb == 0) return;
   const int total = d.rb_start[nb];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int k = rb_find(d, nb, t), bi = d.rb_boxes[k];
+    const int k = rb_find(d.rb_start, nb, t), bi = d.rb_boxes[k];
     bin_particle(P, d, d.boxes[bi], bi, t - d.rb_start[k]);
   }
 }
@@ -449,7 +343,7 @@ __global__ void __launch_bounds__(128) k_batch_scatter(Dev d) {
   if (nb == 0) return;
   const int total = d.rb_start[nb];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int k = rb_find(d, nb, t), bi = d.rb_boxes[k], a = t - d.rb_start[k];
+    const int k = rb_find(d.rb_start, nb, t), bi = d.rb_boxes[k], a = t - d.rb_start[k];
     if (d.box_err[bi] != 0) continue;
     const int o = d.boxes[bi].atom_off, c = d.boxes[bi].cell_off + d.cell[o + a];
     d.order[o + d.cell_start[c] + atomicSub(&d.cell_count[c], 1) - 1] = a;
@@ -461,7 +355,7 @@ __global__ void __launch_bounds__(128) k_batch_place(Params P, Dev d, int par) {
   if (nb == 0) return;
   const int total = d.rb_start[nb];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int k = rb_find(d, nb, t), bi = d.rb_boxes[k];
+    const int k = rb_find(d.rb_start, nb, t), bi = d.rb_boxes[k];
     if (d.box_err[bi] == 0) place_particle(P, d, d.boxes[bi], bi, t - d.rb_start[k], par);
   }
 }
@@ -470,86 +364,133 @@ __global__ void __launch_bounds__(128) k_batch_place(Params P, Dev d, int par) {
 // and the prefix of their particle counts (a box the rebuild then fails stays
 // in the set; the later parts skip it).  One CTA of 1,024 threads.
 __device__ void rebuild_set(const Params &P, const Dev &d) {
-  __shared__ int carry_n, carry_k;
+  __shared__ int carry_n, carry_k, carry_c;
   __shared__ long long wsum[32];
+  __shared__ int csum[32];
   const long long goal = *d.goal;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (threadIdx.x == 0) carry_n = carry_k = 0;
+  if (threadIdx.x == 0) carry_n = carry_k = carry_c = 0;
   __syncthreads();
   for (int base = 0; base < P.nbox; base += blockDim.x) {
     const int bi = base + threadIdx.x;
     const bool on = bi < P.nbox && rebuilding(d, bi, goal);
-    const int n = on ? d.boxes[bi].n : 0;
-    // inclusive scans of n and of the flag over the CTA, packed in one pass
+    const int n = on ? d.boxes[bi].n : 0, nc = on ? d.boxes[bi].ncell : 0;
+    // inclusive scans over the CTA: n and the flag packed, and the cells
     long long x = ((long long)n << 20) | (on ? 1 : 0);
+    int xc = nc;
     for (int o = 1; o < 32; o <<= 1) {
       const long long y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      const int z = __shfl_up_sync(0xffffffffu, xc, o);
+      if (lane >= o) {
+        x += y;
+        xc += z;
+      }
     }
-    if (lane == 31) wsum[wid] = x;
+    if (lane == 31) {
+      wsum[wid] = x;
+      csum[wid] = xc;
+    }
     __syncthreads();
     if (wid == 0) {
       long long t = lane < nw ? wsum[lane] : 0;
+      int tc = lane < nw ? csum[lane] : 0;
       for (int o = 1; o < 32; o <<= 1) {
         const long long y = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += y;
+        const int z = __shfl_up_sync(0xffffffffu, tc, o);
+        if (lane >= o) {
+          t += y;
+          tc += z;
+        }
       }
       wsum[lane] = t;
+      csum[lane] = tc;
     }
     __syncthreads();
     const long long incl = x + (wid ? wsum[wid - 1] : 0);
+    const int inclc = xc + (wid ? csum[wid - 1] : 0);
     const int k = carry_k + (int)(incl & 0xfffff) - 1, start = carry_n + (int)(incl >> 20) - n;
     if (on) {
       d.rb_boxes[k] = bi;
       d.rb_start[k] = start;
+      d.rb_cells[k] = carry_c + inclc - nc;
     }
     __syncthreads();
     if (threadIdx.x == blockDim.x - 1) {
       carry_k += (int)(incl & 0xfffff);
       carry_n += (int)(incl >> 20);
+      carry_c += inclc;
     }
     __syncthreads();
   }
   if (threadIdx.x == 0) {
     *d.rb_count = carry_k;
     d.rb_start[carry_k] = carry_n;
+    d.rb_cells[carry_k] = carry_c;
   }
 }
 
 __global__ void __launch_bounds__(1024) k_batch_rebuild_set(Params P, Dev d) { rebuild_set(P, d); }
 
-// Rebuild part 5: one thread, or nine lanes, per particle slot of every
-// rebuilding box, so a box's list is built by the whole GPU rather than by the
-// CTA that steps it; and the particle's state back in place.
-// A fixed grid walks the concatenated slots of this step's rebuilding boxes.
-__global__ void __launch_bounds__(128) k_batch_list(Params P, Dev d) {
+// Rebuild part 5: one warp per cell of every rebuilding box (cell_rows), so a
+// box's list is built by the whole GPU rather than by the CTA that steps it;
+// and the cell's particles back in place.
+// Few rebuilding cells: two or four warps each (100 steps of 256 boxes mixed,
+// about 3,700 cells a step: 23.3 ms with one warp, 22.0 with two, 23.3 with
+// four; of 48 boxes FP64, about 700: 16.0, 14.4, 14.1).
+constexpr int kListWarps = 4;
+constexpr int kSplitTwo = 12000, kSplitFour = 1500;
+__global__ void __launch_bounds__(32 * kListWarps) k_batch_list(Params P, Dev d) {
+  __shared__ CellRows s_rows[kListWarps];
   const int nb = *d.rb_count;
   if (nb == 0) return;
-  const int total = d.rb_start[nb];
-  // few rebuilding particles: nine lanes each
-  const bool lanes = total < kLanesBelow;
-  const int wl = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
-  const int per = lanes ? 32 / kRowLanes : 32;  // particles of a warp at a time
-  for (int t0 = warp * per; t0 < total; t0 += warps * per) {
-    const int k = lanes ? wl / kRowLanes : wl, lane = lanes ? wl % kRowLanes : 0;
-    const int t = t0 + k;
-    const bool in = k < per && t < total;
-    const int lo = rb_find(d, nb, in ? t : t0), bi = d.rb_boxes[lo];
-    const bool active = in && d.box_err[bi] != kErrBadState;
+  const int cells = d.rb_cells[nb], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int split = cells >= kSplitTwo ? 1 : (cells >= kSplitFour ? 2 : 4);
+  for (int item = blockIdx.x * kListWarps + warp; item < cells * split; item += gridDim.x * kListWarps) {
+    const int t = item / split, part = item % split;
+    const int k = rb_find(d.rb_cells, nb, t), bi = d.rb_boxes[k];
+    if (d.box_err[bi] == kErrBadState) continue;
     const BoxDesc &b = d.boxes[bi];
-    const int a = in ? t - d.rb_start[lo] : 0;
-    const int cnt = lanes ? build_row<kRowLanes>(P, d, b, a, active, lane, wl - lane) : build_row<1>(P, d, b, a, active, 0, wl);
-    if (active && lane == 0) {
-      const int s = b.atom_off + a;
+    const int c = t - d.rb_cells[k], o = b.atom_off;
+    const int *cstart = d.cell_start + b.cell_off;
+    const int lo = cstart[c], hi = cstart[c + 1];
+    const int from = lo + (hi - lo) * part / split, to = lo + (hi - lo) * (part + 1) / split;
+    if (from == to) continue;
+    for (int s = o + from + lane; s < o + to; s += 32) {
       d.q_end[s] = d.t_q[s];
       d.p[s] = d.t_p[s];
       d.id[s] = d.t_id[s];
-      d.cell[s] = d.t_cell[s];
+      d.cell[s] = c;
     }
-    if (active && lane == 0 && cnt > P.list_cap) {
-      atomicMax(&d.box_need[bi], cnt);
-      atomicExch(&d.box_err[bi], kErrOverflow);
-    }
+    int cx, cy, cz;
+    cell_xyz(b, c, cx, cy, cz);
+    cell_rows(
+        s_rows[warp], d.qf + o, lo, from, to, P.acc_lo, P.acc_hi, d.nl + b.list_off, (size_t)b.n, P.list_cap,
+        [&](int l, int &first, int &count, float3 &shift, uint32_t &code) {
+          const int ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = l / 9 - 1;
+          int sx, sy, sz;
+          const int nx = wrap_cell(cx, ox, b.nc[0], sx), ny = wrap_cell(cy, oy, b.nc[1], sy), nz = wrap_cell(cz, oz, b.nc[2], sz);
+          shift.x = (float)ox * b.w32[0] + (float)sx * b.dl32[0];
+          shift.y = (float)oy * b.w32[1] + (float)sy * b.dl32[1];
+          shift.z = (float)oz * b.w32[2] + (float)sz * b.dl32[2];
+          code = entry_pack(0, ox, oy, oz);
+          const int cc = (nz * b.nc[1] + ny) * b.nc[0] + nx;
+          first = cstart[cc];
+          count = cstart[cc + 1] - first;
+        },
+        [&](int i, int j, int l) {
+          int sx, sy, sz;
+          wrap_cell(cx, l % 3 - 1, b.nc[0], sx);
+          wrap_cell(cy, l / 3 % 3 - 1, b.nc[1], sy);
+          wrap_cell(cz, l / 9 - 1, b.nc[2], sz);
+          return image_within(d.t_q[o + i], d.t_q[o + j], b.L, sx, sy, sz, P.sl2);
+        },
+        [&](int i, int cnt) {
+          d.ncount[o + i] = cnt < P.list_cap ? cnt : P.list_cap;
+          if (cnt > P.list_cap) {
+            atomicMax(&d.box_need[bi], cnt);
+            atomicExch(&d.box_err[bi], kErrOverflow);
+          }
+        });
   }
 }
 
@@ -1074,7 +1015,7 @@ __global__ void __launch_bounds__(kFlatMaxThreads, MIXED == kFixedForm ? kFlatFi
   if (nb == 0) return;
   const int total = d.rb_start[nb];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int k = rb_find(d, nb, t), bi = d.rb_boxes[k];
+    const int k = rb_find(d.rb_start, nb, t), bi = d.rb_boxes[k];
     if (d.box_err[bi] == 0) flat_step<MIXED, INNER, true>(P, d, bi, d.boxes[bi].atom_off + t - d.rb_start[k], par);
   }
 }
@@ -1428,7 +1369,7 @@ void launch_batch_rebuild(mdg_batch *b, int par, cudaStream_t stream) {
   k_batch_scan<<<std::min(b->nbox, b->num_sms * 4), 256, 0, stream>>>(b->d);
   k_batch_scatter<<<b->num_sms * 16, 128, 0, stream>>>(b->d);
   k_batch_place<<<b->num_sms * 16, 128, 0, stream>>>(b->P, b->d, par);
-  k_batch_list<<<b->num_sms * 16, 128, 0, stream>>>(b->P, b->d);
+  k_batch_list<<<b->num_sms * 8, 32 * kListWarps, 0, stream>>>(b->P, b->d);
 }
 
 void launch_batch_step(mdg_batch *b, int par) {
@@ -1700,6 +1641,7 @@ int mdg_batch_create(const mdg_batch_params *p, int32_t nbox, const int32_t *n_p
   if (e == cudaSuccess) e = cudaMemset(d.box_mid, 0xFF, nbox * sizeof(int));  // -1: q_end current
   if (e == cudaSuccess) e = balloc(&d.rb_boxes, nbox);
   if (e == cudaSuccess) e = balloc(&d.rb_start, (size_t)nbox + 1);
+  if (e == cudaSuccess) e = balloc(&d.rb_cells, (size_t)nbox + 1);
   if (e == cudaSuccess) e = balloc(&d.rb_count, 1);
   if (e == cudaSuccess) e = balloc(&d.cell_start, (size_t)cells);
   if (e == cudaSuccess) e = balloc(&d.cell_count, (size_t)cells);
@@ -1738,7 +1680,7 @@ int mdg_batch_destroy(mdg_batch *b) {
   Dev &d = b->d;
   void *ptrs[] = {d.boxes, d.cta_start, d.cta_boxes, d.q_end, d.q_mid[0], d.q_mid[1], d.p, d.q_build, d.t_q, d.t_p,
                   d.qf, d.loc[0], d.loc[1], d.id, d.cell, d.t_id, d.t_cell, d.order, d.cell_start, d.cell_count, d.nl, d.ncount,
-                  d.pl, d.pcount, d.loc_p, d.box_prune, d.box_req, d.box_preq, d.rb_boxes, d.rb_start, d.rb_count,
+                  d.pl, d.pcount, d.loc_p, d.box_prune, d.box_req, d.box_preq, d.rb_boxes, d.rb_start, d.rb_cells, d.rb_count,
                   d.box_rebuild, d.box_err, d.box_need, d.box_steps, d.box_rebuilds, d.goal, d.partials,
                   d.box_mid, d.xq[0], d.xq[1], d.xb, d.xp, d.box_wide, d.box_wide_end, b->obs_part, b->d_box_of_slot};
   for (void *p : ptrs)

@@ -22,61 +22,79 @@ namespace mdg {
 
 namespace {
 
-// Threads per block of the list build.  A block's slots are consecutive in
-// cell order, so larger blocks keep more neighbouring cells on one SM and
-// their candidate loads hit L1 (forced rebuild of the 4M-atom liquid box: 128
-// threads 3.55 ms, 256 3.44, 384 3.21); below a million particles the grid
-// has too few of them for the SMs (256,000 atoms: 128 threads 0.366 ms, 384 0.404).
-constexpr int kListThreads = 384, kListThreadsSmall = 128, kListLarge = 1000000;
-// Below this many particles nine lanes share a slot: forced rebuild of 864
-// atoms 124 -> 95 us, of 32,000 143 -> 120; 108,000 atoms have warps enough
-// (174 us with one thread per slot, 230 with nine lanes).
-constexpr int kLanesBelow = 49152;
-
-// One thread per slot (LANES = 1), or LANES = 9 lanes of a warp per slot.
-template <int LANES, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1) k_build_list(Geom g, Dev d) {
+// One warp per home cell, or two below kSplitBelow cells an SM: forced rebuild of
+// 32,000 atoms 159 us with one, 149 with two, 158 with four; of 131,072 (about
+// 4,900 cells) 201, 213, 248.  The blocks' work is uneven (denser regions have
+// more candidates): many small blocks balance it, resident ones striding over
+// the cells did not (4M atoms, one wave: 25 % slower).
+constexpr int kListWarps = 8;
+constexpr long long kSplitBelow = 20;
+__global__ void __launch_bounds__(32 * kListWarps, 4) k_build_list(Geom g, Dev d, int split) {
   DevFlags *f = d.flags;
   // one read for the whole block: another block may set the halt meanwhile
   __shared__ int s_run;
+  __shared__ CellRows s_rows[kListWarps];
   if (threadIdx.x == 0) s_run = f->halt == 0 && f->rebuild != 0;
   __syncthreads();
   if (!s_run) return;
-  constexpr int kPerWarp = LANES == 1 ? 32 : 32 / LANES;  // slots of a warp
-  const int wl = threadIdx.x & 31;
-  const int lane = LANES == 1 ? 0 : wl % LANES;
-  const int i = LANES == 1 ? blockIdx.x * blockDim.x + threadIdx.x
-                           : (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * kPerWarp + wl / LANES;
-  const bool active = i < g.n && wl < kPerWarp * LANES;
+  const int warp = threadIdx.x >> 5, item = blockIdx.x * kListWarps + warp, home = item / split, part = item % split;
   const int cap = g.list_cap;
-  const int cnt = build_slot_row<LANES>(g, d, i, active, lane, wl - lane);
-  unsigned long long tot = 0;
-  int mx = 0;
-  if (active && lane == 0) {
-    d.ncount[i] = cnt < cap ? cnt : cap;
-    if (cnt > cap) {
-      atomicMax(&f->overflow_max, cnt);
-      halt_with(f, kHaltOverflow);
-    }
-    tot = (unsigned long long)(cnt < cap ? cnt : cap);
-    mx = cnt;
+  int a = 0, b = 0;
+  if (home < g.nrank) {
+    a = d.cell_start[home];
+    b = d.cell_start[home + 1];
+  }
+  if (!MDG_IN_RANGE(f, kCheckBuildRange, b, g.n + 1) || !MDG_IN_RANGE(f, kCheckBuildRange, a, b + 1)) a = b = 0;
+  int v = 0, mx = 0;
+  const int from = a + (b - a) * part / split, to = a + (b - a) * (part + 1) / split;
+  if (from < to) {
+    int cx, cy, cz;
+    cell_unpack(d.qf[a].w, cx, cy, cz);
+    cell_rows(
+        s_rows[warp], d.qf, a, from, to, g.acc_lo, g.acc_hi, d.nl, (size_t)g.stride, cap,
+        [&](int l, int &first, int &count, float3 &shift, uint32_t &code) {
+          const int ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = l / 9 - 1;
+          int sx, sy, sz;
+          const int nx = wrap_cell(cx, ox, g.nc[0], sx), ny = wrap_cell(cy, oy, g.nc[1], sy), nz = wrap_cell(cz, oz, g.nc[2], sz);
+          // offset of the partner cell's centre: o*w + s*(L - nc*w)
+          shift.x = (float)ox * g.w32[0] + (float)sx * g.dl32[0];
+          shift.y = (float)oy * g.w32[1] + (float)sy * g.dl32[1];
+          shift.z = (float)oz * g.w32[2] + (float)sz * g.dl32[2];
+          code = entry_pack(0, ox, oy, oz);
+          const int cc = cell_rank(g, nx, ny, nz);
+          if (!MDG_IN_RANGE(f, kCheckBuildCell, cc, g.nrank)) return;
+          int lo = d.cell_start[cc], hi = d.cell_start[cc + 1];
+          if (!MDG_IN_RANGE(f, kCheckBuildRange, hi, g.n + 1) || !MDG_IN_RANGE(f, kCheckBuildRange, lo, hi + 1)) return;
+          first = lo;
+          count = hi - lo;
+        },
+        [&](int i, int j, int l) {
+          int sx, sy, sz;
+          wrap_cell(cx, l % 3 - 1, g.nc[0], sx);
+          wrap_cell(cy, l / 3 % 3 - 1, g.nc[1], sy);
+          wrap_cell(cz, l / 9 - 1, g.nc[2], sz);
+          return image_within(d.q_end[i], d.q_end[j], g.L, sx, sy, sz, g.sl2);
+        },
+        [&](int i, int cnt) {
+          d.ncount[i] = cnt < cap ? cnt : cap;
+          if (cnt > cap) {
+            atomicMax(&f->overflow_max, cnt);
+            halt_with(f, kHaltOverflow);
+          }
+          v += cnt < cap ? cnt : cap;
+          mx = max(mx, cnt);
+        });
   }
   // block totals -> one atomic each
-  __shared__ unsigned long long s_sum[THREADS / 32];
-  __shared__ int s_max[THREADS / 32];
-  unsigned long long v = tot;
-  int m = mx;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v += __shfl_down_sync(0xffffffffu, v, o);
-    m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-  }
-  if ((threadIdx.x & 31) == 0) { s_sum[threadIdx.x >> 5] = v; s_max[threadIdx.x >> 5] = m; }
+  __shared__ int s_sum[kListWarps], s_max[kListWarps];
+  v = __reduce_add_sync(0xffffffffu, v);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) { s_sum[warp] = v; s_max[warp] = mx; }
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long tv = 0;
     int tm = 0;
-    for (int w = 0; w < THREADS / 32; w++) { tv += s_sum[w]; tm = max(tm, s_max[w]); }
+    for (int w = 0; w < kListWarps; w++) { tv += s_sum[w]; tm = max(tm, s_max[w]); }
     atomicAdd(&f->pairs, tv);
     atomicMax(&f->max_count, tm);
   }
@@ -109,17 +127,9 @@ __global__ void k_list_prepare(DevFlags *f) {
 
 void launch_build_list(const Geom &g, const Dev &d, int num_sms, cudaStream_t s, bool in_step) {
   k_list_prepare<<<1, 1, 0, s>>>(d.flags);
-  // one slot per thread, or per nine lanes: the blocks' work is uneven
-  // (denser regions have more candidates), and many blocks balance it where
-  // resident blocks striding over the slots did not (4M atoms, one wave: 25 % slower)
-  (void)num_sms;
-  auto grid = [&](int slots) { return g.n > 0 ? (g.n + slots - 1) / slots : 1; };
-  if (g.n < kLanesBelow)
-    k_build_list<kRowLanes, kListThreadsSmall><<<grid(kListThreadsSmall / 32 * (32 / kRowLanes)), kListThreadsSmall, 0, s>>>(g, d);
-  else if (g.n < kListLarge)
-    k_build_list<1, kListThreadsSmall><<<grid(kListThreadsSmall), kListThreadsSmall, 0, s>>>(g, d);
-  else
-    k_build_list<1, kListThreads><<<grid(kListThreads), kListThreads, 0, s>>>(g, d);
+  const long long cells = (long long)g.nc[0] * g.nc[1] * g.nc[2];
+  const int split = cells >= kSplitBelow * num_sms ? 1 : 2;
+  k_build_list<<<(g.nrank * split + kListWarps - 1) / kListWarps, 32 * kListWarps, 0, s>>>(g, d, split);
   k_rebuild_done<<<1, 1, 0, s>>>(d.flags, in_step ? 1 : 0);
 }
 

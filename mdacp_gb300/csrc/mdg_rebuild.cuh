@@ -94,18 +94,6 @@ __device__ __forceinline__ void finalize_one(const Geom &g, const Dev &d, int k,
   }
 }
 
-// Exact acceptance of a candidate in the float band: the reference's image
-// and rounding order (mdunit.cc:167, meshlist.cc:262-266).
-__device__ __forceinline__ bool exact_within(const Geom &g, const double4_32a &qi, const double4_32a &qj, int sx, int sy,
-                                             int sz) {
-  const double xj = sx ? __dadd_rn(qj.x, sx > 0 ? g.L[0] : -g.L[0]) : qj.x;
-  const double yj = sy ? __dadd_rn(qj.y, sy > 0 ? g.L[1] : -g.L[1]) : qj.y;
-  const double zj = sz ? __dadd_rn(qj.z, sz > 0 ? g.L[2] : -g.L[2]) : qj.z;
-  const double dx = __dsub_rn(qi.x, xj), dy = __dsub_rn(qi.y, yj), dz = __dsub_rn(qi.z, zj);
-  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-  return r2 <= g.sl2;
-}
-
 constexpr int kRowLanes = 9;
 
 // The row of slot i, by one thread (LANES = 1) or by LANES = 9 neighbouring
@@ -147,7 +135,7 @@ __device__ __forceinline__ int build_slot_row(const Geom &g, const Dev &d, int i
       if ((unsigned)(i - j0) < 32u) in &= ~(1u << (i - j0));  // the particle itself (its images are a box away)
       for (uint32_t band = in & ~sure; band; band &= band - 1u) {
         const int u = __ffs(band) - 1;
-        if (!exact_within(g, d.q_end[i], d.q_end[j0 + u], sx, sy, sz)) in &= ~(1u << u);
+        if (!image_within(d.q_end[i], d.q_end[j0 + u], g.L, sx, sy, sz, g.sl2)) in &= ~(1u << u);
       }
       emit(in, j0, code);
     }
