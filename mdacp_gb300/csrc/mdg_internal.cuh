@@ -188,7 +188,7 @@ struct Dev {
 };
 
 // kernels enqueued by one launch_rebuild and one launch_step call
-constexpr int kRebuildKernels = 11;
+constexpr int kRebuildKernels = 10;
 inline int step_kernels(int thermostat) { return thermostat == MDG_NOSEHOOVER ? 2 : 1; }
 
 // host-side launchers (stream-ordered; none synchronises)
