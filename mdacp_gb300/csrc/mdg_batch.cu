@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(32 * kListWarps) k_batch_list(Params P, Dev d)
     int cx, cy, cz;
     cell_xyz(b, c, cx, cy, cz);
     cell_rows(
-        s_rows[warp], d.qf + o, lo, from, to, P.acc_lo, P.acc_hi, d.nl + b.list_off, (size_t)b.n, P.list_cap,
+        s_rows[warp], d.qf + o, lo, from, to, P.acc_lo, P.acc_hi, P.list_cap,
         [&](int l, int &first, int &count, float3 &shift, uint32_t &code) {
           const int ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = l / 9 - 1;
           int sx, sy, sz;
@@ -484,6 +484,7 @@ __global__ void __launch_bounds__(32 * kListWarps) k_batch_list(Params P, Dev d)
           wrap_cell(cz, l / 9 - 1, b.nc[2], sz);
           return image_within(d.t_q[o + i], d.t_q[o + j], b.L, sx, sy, sz, P.sl2);
         },
+        RowSink{d.nl + b.list_off, (size_t)b.n, nullptr},
         [&](int i, int cnt) {
           d.ncount[o + i] = cnt < P.list_cap ? cnt : P.list_cap;
           if (cnt > P.list_cap) {

@@ -81,13 +81,25 @@ struct CellRows {
   uint32_t entry[kTileChunks][32];  // [chunk][candidate]
 };
 
+// Row entry k of slot i at row + i + k * stride.
+struct RowSink {
+  uint32_t *row;
+  size_t stride;
+  uint32_t *out;
+  __device__ __forceinline__ void start(int i, int k) { out = row + i + (size_t)k * stride; }
+  __device__ __forceinline__ void put(uint32_t e) {
+    *out = e;
+    out += stride;
+  }
+};
+
 // Home slots a .. b - 1 of qf, of the cell that starts at a0.  stencil(l, first, count, shift, code): stencil cell l = 0 .. 26 in
 // row order; exact(i, j, l): the exact test of a candidate in the float band;
-// rows at row + slot, entry k at k * stride, cap entries kept; done(slot, count).
-template <class Stencil, class Exact, class Done>
+// a lane's sink takes its entries: start(slot, k) ahead of entries k, k + 1, ...
+// of a slot, put(entry); cap entries a row are kept; done(slot, count).
+template <class Stencil, class Exact, class Sink, class Done>
 __device__ __forceinline__ void cell_rows(CellRows &m, const float4 *__restrict__ qf, int a0, int a, int b, float lo, float hi,
-                                          uint32_t *row, size_t stride, int cap, Stencil &&stencil, Exact &&exact,
-                                          Done &&done) {
+                                          int cap, Stencil &&stencil, Exact &&exact, Sink &&sink, Done &&done) {
   const int lane = threadIdx.x & 31;
   const uint32_t all = 0xffffffffu;
   const float mid = 0.5f * (lo + hi), half = 0.5f * (hi - lo);
@@ -169,7 +181,7 @@ __device__ __forceinline__ void cell_rows(CellRows &m, const float4 *__restrict_
         cnt += v;
       }
       mine = min(mine, cap - w);
-      uint32_t *out = row + h0 + h + (size_t)w * stride;
+      if (mine > 0) sink.start(h0 + h, w);
       const uint32_t *word = &m.mask[c0][h], *entry = m.entry[c0];
       uint32_t bits = mine > 0 ? *word : 0u;
       while (mine > 0) {
@@ -180,8 +192,7 @@ __device__ __forceinline__ void cell_rows(CellRows &m, const float4 *__restrict_
         }
         if (bits != 0u) {
           const int u = 31 - __clz(bits);
-          *out = entry[u];
-          out += stride;
+          sink.put(entry[u]);
           bits ^= 1u << u;
           mine--;
         }

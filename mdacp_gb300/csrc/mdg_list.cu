@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(32 * kListWarps, 4) k_build_list(Geom g, Dev d
     int cx, cy, cz;
     cell_unpack(d.qf[a].w, cx, cy, cz);
     cell_rows(
-        s_rows[warp], d.qf, a, from, to, g.acc_lo, g.acc_hi, d.nl, (size_t)g.stride, cap,
+        s_rows[warp], d.qf, a, from, to, g.acc_lo, g.acc_hi, cap,
         [&](int l, int &first, int &count, float3 &shift, uint32_t &code) {
           const int ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = l / 9 - 1;
           int sx, sy, sz;
@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(32 * kListWarps, 4) k_build_list(Geom g, Dev d
           wrap_cell(cz, l / 9 - 1, g.nc[2], sz);
           return image_within(d.q_end[i], d.q_end[j], g.L, sx, sy, sz, g.sl2);
         },
+        RowSink{d.nl, (size_t)g.stride, nullptr},
         [&](int i, int cnt) {
           d.ncount[i] = cnt < cap ? cnt : cap;
           if (cnt > cap) {
