@@ -297,7 +297,7 @@ int mdg_adjoint_backward(mdg_adjoint *a, double *dq0, double *dp0, double *depsi
  * smoothly truncated LJ potential.  Work is enqueued on `stream` (a
  * cudaStream_t; NULL = legacy default stream) and not synchronised.
  *
- * Working memory is one fixed static device array of about 11.3 MB per GPU,
+ * Working memory is one fixed static device array of about 62 MB per GPU,
  * held until the process exits: at most 1,048,576 particles and 262,144 cells
  * of width >= cutoff (box side / cutoff, rounded down, per axis); larger
  * inputs return MDG_ERR_CAPACITY with a message on stderr.  The first call on

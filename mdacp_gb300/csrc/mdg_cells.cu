@@ -263,7 +263,7 @@ __device__ __forceinline__ double block_sum_d(double v, double *sh) {
 // Largest of the block's values, none of them negative and NaN passed over as
 // fmax does, to thread 0: by the bit patterns, which are in the same order, with
 // the integer units' warp maximum (the FP64 pipe's comparisons and a last
-// loop over the warps by one thread took four of ten us of each of these
+// loop over the warps by one thread took over three of the eight us of these
 // kernels: k_policy_vmax 8.6 -> 5.1 at 256,000 atoms, k_policy_budget 8.2 -> 4.9).
 __device__ __forceinline__ unsigned long long warp_max(unsigned long long x) {
   const unsigned hi = (unsigned)(x >> 32), mh = __reduce_max_sync(0xffffffffu, hi);

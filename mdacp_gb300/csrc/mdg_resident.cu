@@ -3,7 +3,7 @@
 // A step graph costs a small box more than its steps: the prelude kernel, the
 // conditional node and the launch of its body take 11-13 us a step (864
 // atoms FP64: 24 us per single-step call, of which 11 are the step kernel;
-// 108,000 atoms mixed: 50 us for a 30 us kernel), and a rebuild is eleven
+// 108,000 atoms mixed: 50 us for a 30 us kernel), and a rebuild is ten
 // launches.  Here one cooperative launch runs all steps of an mdg_calculate
 // call: one block per SM, each with its share of the slots, a grid barrier
 // after every step, and the rebuild as phases between further barriers.  The
