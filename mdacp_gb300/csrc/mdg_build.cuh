@@ -159,6 +159,7 @@ __device__ __forceinline__ void cell_rows(CellRows &m, const float4 *__restrict_
           *reinterpret_cast<uint2 *>(&m.mask[c][g]) = make_uint2(in0, in1);
         }
         if (__any_sync(all, nearest <= half)) {
+          __syncwarp();  // the masks above are written
           for (int g = 0; g < H; g++) {
             const float t = test(g);
             const uint32_t in = __ballot_sync(all, t < -half || (t <= half && exact(h0 + g, j, k)));

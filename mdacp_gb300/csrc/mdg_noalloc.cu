@@ -443,7 +443,8 @@ extern "C" int mdg_observe_noalloc(const double *q4_dev, const double *p4_dev, i
   // few cells: two or four warps each, as the list build
   const int split = b.ncell < 1500 ? 4 : (b.ncell < 12000 ? 2 : 1);
   const int warps = (b.ncell * split + kWarps - 1) / kWarps;
-  const int blocks = warps < kMaxBlocks ? warps : kMaxBlocks;
+  const int most = warps > grid ? warps : grid;  // blocks of kThreads particles where the double sums run
+  const int blocks = most < kMaxBlocks ? most : kMaxBlocks;
   k_observe<<<blocks, kThreads, 0, st>>>(b, s, q, p, split);
   k_final<<<1, 1024, 0, st>>>(s, blocks, out3_dev);
   return cudaGetLastError() == cudaSuccess ? MDG_OK : MDG_ERR_CUDA;
