@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(1024) k_batch_rebuild_set(Params P, Dev d) { r
 constexpr int kListWarps = 4;
 constexpr int kSplitTwo = 12000, kSplitFour = 1500;
 __global__ void __launch_bounds__(32 * kListWarps) k_batch_list(Params P, Dev d) {
-  __shared__ CellRows s_rows[kListWarps];
+  __shared__ CellRows<kTileChunks> s_rows[kListWarps];
   const int nb = *d.rb_count;
   if (nb == 0) return;
   const int cells = d.rb_cells[nb], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -72,13 +72,15 @@ __device__ __forceinline__ bool image_within(const double4_32a &qi, const double
 // a particle, 64 with one warp a cell.  Tried: two home particles per packed
 // float instruction (moves ate the gain), the next candidates' loads in flight
 // during the tests (no faster: the other warps cover them).
-constexpr int kTileChunks = 16;  // candidates whose masks are held at a time, in 32s
+// TILE: candidates whose masks are held at a time, in 32s.
+constexpr int kTileChunks = 16;
+template <int TILE>
 struct CellRows {
   float4 home[32];  // positions relative to the home cell's centre
   float4 cell[32];  // a stencil cell's shift, and the offset from its candidates' places to their slots
   uint32_t code[32];
-  uint32_t mask[kTileChunks][32];   // [chunk][home particle]
-  uint32_t entry[kTileChunks][32];  // [chunk][candidate]
+  uint32_t mask[TILE][32];   // [chunk][home particle]
+  uint32_t entry[TILE][32];  // [chunk][candidate]
 };
 
 // Row entry k of slot i at row + i + k * stride.
@@ -97,8 +99,8 @@ struct RowSink {
 // row order; exact(i, j, l): the exact test of a candidate in the float band;
 // a lane's sink takes its entries: start(slot, k) ahead of entries k, k + 1, ...
 // of a slot, put(entry); cap entries a row are kept; done(slot, count).
-template <class Stencil, class Exact, class Sink, class Done>
-__device__ __forceinline__ void cell_rows(CellRows &m, const float4 *__restrict__ qf, int a0, int a, int b, float lo, float hi,
+template <int TILE, class Stencil, class Exact, class Sink, class Done>
+__device__ __forceinline__ void cell_rows(CellRows<TILE> &m, const float4 *__restrict__ qf, int a0, int a, int b, float lo, float hi,
                                           int cap, Stencil &&stencil, Exact &&exact, Sink &&sink, Done &&done) {
   const int lane = threadIdx.x & 31;
   const uint32_t all = 0xffffffffu;
@@ -126,8 +128,8 @@ __device__ __forceinline__ void cell_rows(CellRows &m, const float4 *__restrict_
     const int wide = H <= 8 ? 8 : (H <= 16 ? 16 : 32), parts = 32 / wide;
     const int h = lane & (wide - 1), part = lane / wide;
     int cnt = 0;
-    for (int t0 = 0; t0 < total; t0 += 32 * kTileChunks) {
-      const int chunks = min((total - t0 + 31) >> 5, kTileChunks);
+    for (int t0 = 0; t0 < total; t0 += 32 * TILE) {
+      const int chunks = min((total - t0 + 31) >> 5, TILE);
       for (int c = 0; c < chunks; c++) {
         const int f = t0 + 32 * c + 31 - lane;  // the first candidate at the top bit
         int k = 0;  // cells that end at or before f

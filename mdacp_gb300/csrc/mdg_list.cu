@@ -33,59 +33,13 @@ __global__ void __launch_bounds__(32 * kListWarps, 4) k_build_list(Geom g, Dev d
   DevFlags *f = d.flags;
   // one read for the whole block: another block may set the halt meanwhile
   __shared__ int s_run;
-  __shared__ CellRows s_rows[kListWarps];
+  __shared__ CellRows<kTileChunks> s_rows[kListWarps];
   if (threadIdx.x == 0) s_run = f->halt == 0 && f->rebuild != 0;
   __syncthreads();
   if (!s_run) return;
   const int warp = threadIdx.x >> 5, item = blockIdx.x * kListWarps + warp, home = item / split, part = item % split;
-  const int cap = g.list_cap;
-  int a = 0, b = 0;
-  if (home < g.nrank) {
-    a = d.cell_start[home];
-    b = d.cell_start[home + 1];
-  }
-  if (!MDG_IN_RANGE(f, kCheckBuildRange, b, g.n + 1) || !MDG_IN_RANGE(f, kCheckBuildRange, a, b + 1)) a = b = 0;
   int v = 0, mx = 0;
-  const int from = a + (b - a) * part / split, to = a + (b - a) * (part + 1) / split;
-  if (from < to) {
-    int cx, cy, cz;
-    cell_unpack(d.qf[a].w, cx, cy, cz);
-    cell_rows(
-        s_rows[warp], d.qf, a, from, to, g.acc_lo, g.acc_hi, cap,
-        [&](int l, int &first, int &count, float3 &shift, uint32_t &code) {
-          const int ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = l / 9 - 1;
-          int sx, sy, sz;
-          const int nx = wrap_cell(cx, ox, g.nc[0], sx), ny = wrap_cell(cy, oy, g.nc[1], sy), nz = wrap_cell(cz, oz, g.nc[2], sz);
-          // offset of the partner cell's centre: o*w + s*(L - nc*w)
-          shift.x = (float)ox * g.w32[0] + (float)sx * g.dl32[0];
-          shift.y = (float)oy * g.w32[1] + (float)sy * g.dl32[1];
-          shift.z = (float)oz * g.w32[2] + (float)sz * g.dl32[2];
-          code = entry_pack(0, ox, oy, oz);
-          const int cc = cell_rank(g, nx, ny, nz);
-          if (!MDG_IN_RANGE(f, kCheckBuildCell, cc, g.nrank)) return;
-          int lo = d.cell_start[cc], hi = d.cell_start[cc + 1];
-          if (!MDG_IN_RANGE(f, kCheckBuildRange, hi, g.n + 1) || !MDG_IN_RANGE(f, kCheckBuildRange, lo, hi + 1)) return;
-          first = lo;
-          count = hi - lo;
-        },
-        [&](int i, int j, int l) {
-          int sx, sy, sz;
-          wrap_cell(cx, l % 3 - 1, g.nc[0], sx);
-          wrap_cell(cy, l / 3 % 3 - 1, g.nc[1], sy);
-          wrap_cell(cz, l / 9 - 1, g.nc[2], sz);
-          return image_within(d.q_end[i], d.q_end[j], g.L, sx, sy, sz, g.sl2);
-        },
-        RowSink{d.nl, (size_t)g.stride, nullptr},
-        [&](int i, int cnt) {
-          d.ncount[i] = cnt < cap ? cnt : cap;
-          if (cnt > cap) {
-            atomicMax(&f->overflow_max, cnt);
-            halt_with(f, kHaltOverflow);
-          }
-          v += cnt < cap ? cnt : cap;
-          mx = max(mx, cnt);
-        });
-  }
+  if (home < g.nrank) build_cell_rows(g, d, s_rows[warp], home, part, split, v, mx);
   // block totals -> one atomic each
   __shared__ int s_sum[kListWarps], s_max[kListWarps];
   v = __reduce_add_sync(0xffffffffu, v);

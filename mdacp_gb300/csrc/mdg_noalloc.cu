@@ -282,7 +282,7 @@ struct PairSink {
 constexpr int kWarps = kThreads / 32;
 __global__ void __launch_bounds__(kThreads) k_observe(Box b, Scratch s, const double4_32a *q, const double4_32a *p, int split) {
   __shared__ double sh[kThreads / 32];
-  __shared__ CellRows s_rows[kWarps];
+  __shared__ CellRows<kTileChunks> s_rows[kWarps];
   double ke = 0.0;
   PairSink sink{b, s, q, 0.0, 0.0, {}, 0, 0, 0, 0, 0};
   const bool fixed = b.fixed && *s.flag == 0;

@@ -96,13 +96,12 @@ __device__ __forceinline__ void finalize_one(const Geom &g, const Dev &d, int k,
 
 constexpr int kRowLanes = 9;
 
-// The row of slot i, by one thread (LANES = 1) or by LANES = 9 neighbouring
-// lanes of a warp (`base` the first of them), one for each (y, z) row of three
-// stencil cells: a row's candidates then take a ninth of the time one after the
-// other, which is what a small box waits for.  The entries are in stencil
-// order (z, y, x), candidates ascending, either way.  Every lane of the warp calls
-// it; returns the row's length, which may exceed the capacity.
-template <int LANES>
+// The row of slot i by kRowLanes neighbouring lanes of a warp (`base` the first
+// of them), one for each (y, z) row of three stencil cells: a row's candidates
+// then take a ninth of the time one after the other, which is what a small box
+// waits for.  The entries are in stencil order (z, y, x), candidates ascending, as
+// cell_rows writes them.  Every lane of the warp calls it; returns the row's
+// length, which may exceed the capacity.
 __device__ __forceinline__ int build_slot_row(const Geom &g, const Dev &d, int i, bool active, int lane, int base) {
   DevFlags *f = d.flags;
   const float acc_lo = g.acc_lo, acc_hi = g.acc_hi;
@@ -147,52 +146,94 @@ __device__ __forceinline__ int build_slot_row(const Geom &g, const Dev &d, int i
       cnt++;
     }
   };
-  if (LANES == 1) {
-    if (active)
-      for (int oz = -1; oz <= 1; oz++)
-        for (int oy = -1; oy <= 1; oy++)
-          for (int ox = -1; ox <= 1; ox++) scan(ox, oy, oz, append);
-  } else {
-    // the first masks of each cell are kept between counting and writing;
-    // cells of more than 32 particles are scanned again
-    const int oy = lane % 3 - 1, oz = lane / 3 - 1;
-    int own = 0;
-    uint32_t kept[3] = {0u, 0u, 0u};
-    int first[3] = {0, 0, 0};
-    bool again = false;
-    if (active)
+  // the first masks of each cell are kept between counting and writing;
+  // cells of more than 32 particles are scanned again
+  const int oy = lane % 3 - 1, oz = lane / 3 - 1;
+  int own = 0;
+  uint32_t kept[3] = {0u, 0u, 0u};
+  int first[3] = {0, 0, 0};
+  bool again = false;
+  if (active)
 #pragma unroll
-      for (int ox = -1; ox <= 1; ox++) {
-        int chunk = 0;
-        scan(ox, oy, oz, [&](uint32_t in, int j0, uint32_t) {
-          own += __popc(in);
-          if (chunk++ == 0) {
-            kept[ox + 1] = in;
-            first[ox + 1] = j0;
-          } else {
-            again = true;
-          }
-        });
-      }
-    // entries of the particle's lower lanes, and of all
-    int before = 0, total = 0;
-#pragma unroll
-    for (int l = 0; l < LANES; l++) {
-      const int v = __shfl_sync(0xffffffffu, own, min(base + l, 31));
-      before += l < lane ? v : 0;
-      total += v;
+    for (int ox = -1; ox <= 1; ox++) {
+      int chunk = 0;
+      scan(ox, oy, oz, [&](uint32_t in, int j0, uint32_t) {
+        own += __popc(in);
+        if (chunk++ == 0) {
+          kept[ox + 1] = in;
+          first[ox + 1] = j0;
+        } else {
+          again = true;
+        }
+      });
     }
-    cnt = before;
-    if (active) {
+  // entries of the particle's lower lanes, and of all
+  int before = 0, total = 0;
 #pragma unroll
-      for (int ox = -1; ox <= 1; ox++) {
-        if (again) scan(ox, oy, oz, append);
-        else append(kept[ox + 1], first[ox + 1], entry_pack(0, ox, oy, oz));
-      }
-    }
-    cnt = total;
+  for (int l = 0; l < kRowLanes; l++) {
+    const int v = __shfl_sync(0xffffffffu, own, min(base + l, 31));
+    before += l < lane ? v : 0;
+    total += v;
   }
-  return cnt;
+  cnt = before;
+  if (active) {
+#pragma unroll
+    for (int ox = -1; ox <= 1; ox++) {
+      if (again) scan(ox, oy, oz, append);
+      else append(kept[ox + 1], first[ox + 1], entry_pack(0, ox, oy, oz));
+    }
+  }
+  return total;
+}
+
+// The rows of part `part` of `split` of cell `home`'s particles, by a warp: the kept
+// entries added to this lane's `pairs`, its longest row to `longest`.
+template <int TILE>
+__device__ __forceinline__ void build_cell_rows(const Geom &g, const Dev &d, CellRows<TILE> &rows, int home, int part, int split,
+                                                int &pairs, int &longest) {
+  DevFlags *f = d.flags;
+  const int cap = g.list_cap;
+  int a = d.cell_start[home], b = d.cell_start[home + 1];
+  if (!MDG_IN_RANGE(f, kCheckBuildRange, b, g.n + 1) || !MDG_IN_RANGE(f, kCheckBuildRange, a, b + 1)) a = b = 0;
+  const int from = a + (b - a) * part / split, to = a + (b - a) * (part + 1) / split;
+  if (from >= to) return;
+  int cx, cy, cz;
+  cell_unpack(d.qf[a].w, cx, cy, cz);
+  cell_rows(
+      rows, d.qf, a, from, to, g.acc_lo, g.acc_hi, cap,
+      [&](int l, int &first, int &count, float3 &shift, uint32_t &code) {
+        const int ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = l / 9 - 1;
+        int sx, sy, sz;
+        const int nx = wrap_cell(cx, ox, g.nc[0], sx), ny = wrap_cell(cy, oy, g.nc[1], sy), nz = wrap_cell(cz, oz, g.nc[2], sz);
+        // offset of the partner cell's centre: o*w + s*(L - nc*w)
+        shift.x = (float)ox * g.w32[0] + (float)sx * g.dl32[0];
+        shift.y = (float)oy * g.w32[1] + (float)sy * g.dl32[1];
+        shift.z = (float)oz * g.w32[2] + (float)sz * g.dl32[2];
+        code = entry_pack(0, ox, oy, oz);
+        const int cc = cell_rank(g, nx, ny, nz);
+        if (!MDG_IN_RANGE(f, kCheckBuildCell, cc, g.nrank)) return;
+        int lo = d.cell_start[cc], hi = d.cell_start[cc + 1];
+        if (!MDG_IN_RANGE(f, kCheckBuildRange, hi, g.n + 1) || !MDG_IN_RANGE(f, kCheckBuildRange, lo, hi + 1)) return;
+        first = lo;
+        count = hi - lo;
+      },
+      [&](int i, int j, int l) {
+        int sx, sy, sz;
+        wrap_cell(cx, l % 3 - 1, g.nc[0], sx);
+        wrap_cell(cy, l / 3 % 3 - 1, g.nc[1], sy);
+        wrap_cell(cz, l / 9 - 1, g.nc[2], sz);
+        return image_within(d.q_end[i], d.q_end[j], g.L, sx, sy, sz, g.sl2);
+      },
+      RowSink{d.nl, (size_t)g.stride, nullptr},
+      [&](int i, int cnt) {
+        d.ncount[i] = cnt < cap ? cnt : cap;
+        if (cnt > cap) {
+          atomicMax(&f->overflow_max, cnt);
+          halt_with(f, kHaltOverflow);
+        }
+        pairs += cnt < cap ? cnt : cap;
+        longest = max(longest, cnt);
+      });
 }
 
 }  // namespace mdg

@@ -8,7 +8,8 @@
 // call: one block per SM, each with its share of the slots, a grid barrier
 // after every step, and the rebuild as phases between further barriers.  The
 // particles' arithmetic is the step kernels' own (step_one, force_mixed,
-// step_one_fixed, force_fixed; finalize_one and build_slot_row for the list).
+// step_one_fixed, force_fixed; finalize_one, build_slot_row and build_cell_rows
+// for the list).
 //
 // All blocks are resident at once (the cooperative launch fails otherwise),
 // so every barrier is reached; its wait is bounded all the same, and a block
@@ -43,6 +44,16 @@ constexpr int kFixedForm = 3;  // template value beside MDG_MIXED and MDG_MIXED_
 // per step: 4 10.2 / 13.7 / 18.5, 8 9.2 / 12.7 / 19.2, 16 11.1 / 15.3 / 22.1;
 // 1024 threads 14.3 / 18.9 / 23.8).
 constexpr int kFewUnroll = 8;
+
+// The list build's shared memory: masks of 128 candidates a warp, 2.2 KB (the
+// rest of the SM's memory is the steps' L1 cache).
+constexpr int kResidentTile = 4;
+// Whether a rebuild's rows take nine lanes each (small boxes) rather than a warp
+// per cell (two or four where there are fewer cells than two a warp).  us per step at dt
+// 0.005 (a rebuild every 14 to 20 steps): 864 atoms 10.20 with nine lanes, 10.62
+// with the warps; 32,000 atoms FP64 34.7 with a thread per row, 32.7 with the
+// warps; 108,000 mixed 38.7 and 38.4 (39.0 with one warp a cell).
+__host__ __device__ __forceinline__ bool lanes_per_row(int n, long long threads) { return (long long)n * kRowLanes <= 2 * threads; }
 
 // About two seconds of polling; a barrier is reached within microseconds.
 constexpr int kPollLimit = 1 << 22;
@@ -192,34 +203,38 @@ __device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, Resid
   }
   if (!grid_barrier(c, ++r.barriers)) return false;
   r.stale = false;
-  // rows: nine lanes each while that fills fewer lanes than there are threads twice over
+  // rows: nine lanes each while that fills fewer lanes than there are threads
+  // twice over, else a warp per cell, or two or four of few cells
   const int wl = threadIdx.x & 31, warp = tid >> 5, warps = nt >> 5;
-  const bool lanes = (long long)g.n * kRowLanes <= 2ll * nt;
-  const int per = lanes ? 32 / kRowLanes : 32;
-  unsigned long long pairs = 0;
-  int longest = 0;
-  for (int i0 = warp * per; i0 < g.n; i0 += warps * per) {
-    const int k = lanes ? wl / kRowLanes : wl, lane = lanes ? wl % kRowLanes : 0, i = i0 + k;
-    const bool active = k < per && i < g.n;
-    const int cnt = lanes ? build_slot_row<kRowLanes>(g, d, i, active, lane, wl - lane) : build_slot_row<1>(g, d, i, active, 0, wl);
-    if (active && lane == 0) {
-      const int kept = min(cnt, g.list_cap);
-      d.ncount[i] = kept;
-      if (cnt > g.list_cap) {
-        atomicMax(&f->overflow_max, cnt);
-        halt_with(f, kHaltOverflow);
+  int pairs = 0, longest = 0;
+  if (lanes_per_row(g.n, nt)) {
+    const int per = 32 / kRowLanes, k = wl / kRowLanes, lane = wl % kRowLanes;
+    for (int i0 = warp * per; i0 < g.n; i0 += warps * per) {
+      const int i = i0 + k;
+      const bool active = k < per && i < g.n;
+      const int cnt = build_slot_row(g, d, i, active, lane, wl - lane);
+      if (active && lane == 0) {
+        const int kept = min(cnt, g.list_cap);
+        d.ncount[i] = kept;
+        if (cnt > g.list_cap) {
+          atomicMax(&f->overflow_max, cnt);
+          halt_with(f, kHaltOverflow);
+        }
+        pairs += kept;
+        longest = max(longest, cnt);
       }
-      pairs += (unsigned long long)kept;
-      longest = max(longest, cnt);
     }
+  } else {
+    extern __shared__ __align__(16) unsigned char s_dynamic[];
+    CellRows<kResidentTile> *rows = reinterpret_cast<CellRows<kResidentTile> *>(s_dynamic);
+    const int cells = g.nc[0] * g.nc[1] * g.nc[2], split = cells >= 2 * warps ? 1 : (cells >= warps ? 2 : 4);
+    for (int item = warp; item < g.nrank * split; item += warps)
+      build_cell_rows(g, d, rows[threadIdx.x >> 5], item / split, item % split, split, pairs, longest);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    pairs += __shfl_down_sync(0xffffffffu, pairs, o);
-    longest = max(longest, __shfl_down_sync(0xffffffffu, longest, o));
-  }
+  pairs = __reduce_add_sync(0xffffffffu, pairs);  // at most 2^20 particles of 2^10 entries
+  longest = __reduce_max_sync(0xffffffffu, longest);
   if (wl == 0 && longest) {
-    atomicAdd(&f->pairs, pairs);
+    atomicAdd(&f->pairs, (unsigned long long)pairs);
     atomicMax(&f->max_count, longest);
   }
   return grid_barrier(c, ++r.barriers) && *(volatile int *)&f->halt == 0;
@@ -471,7 +486,15 @@ cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int
   Dev dd = d;
   ResidentCtl *c = static_cast<ResidentCtl *>(ctl);
   void *args[] = {&gg, &dd, &c, &par, &nsteps, &share};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k), dim3(grid), dim3(threads), args, 0, s);
+  size_t shared = 0;
+  if (!lanes_per_row(g.n, (long long)grid * threads)) {
+    shared = threads / 32 * sizeof(CellRows<kResidentTile>);
+    if (shared > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k), dim3(grid), dim3(threads), args, shared, s);
 }
 
 }  // namespace mdg
