@@ -175,7 +175,7 @@ int mdg_get_state_device(mdg_handle *h, double *q4_dev, double *p4_dev);
  * Batched replicas (no reference counterpart; a pattern on top of the
  * drop-in): nbox independent periodic boxes of uneven size and density, each
  * an NVE drift-kick-drift run with its own cell list and Verlet list, all
- * advanced by one persistent kernel per step (replayed from a CUDA graph).
+ * advanced together, step by step (replayed from a CUDA graph).
  * Particles are concatenated box after box, [sum n][4] doubles; every box is
  * returned in the order it was given. */
 typedef struct mdg_batch_params {
@@ -197,7 +197,7 @@ typedef struct mdg_batch_stats {
   int64_t particles;
   int32_t boxes;
   int32_t list_capacity;
-  int32_t threads;            /* CTA size of the persistent kernel */
+  int32_t threads;            /* CTA size of the step kernel */
   int32_t lanes_per_particle; /* lanes sharing one particle's row */
   int32_t ctas_per_sm;
   int32_t inner_list;         /* 1: the step walks the inner list (chosen by mdg_batch_tune) */
@@ -230,16 +230,15 @@ int mdg_batch_tune(mdg_batch *b, int32_t trial_steps, int32_t *threads, int32_t 
                    int32_t *ctas_per_sm);
 /* Fixes the shape by hand; ctas_per_sm is capped at the CTAs of the step
  * kernel that fit on one SM at once (mdg_batch_get_stats reports the value
- * used), so the persistent kernel never runs in waves. */
+ * used), so the per-box step kernel never runs in waves. */
 int mdg_batch_set_shape(mdg_batch *b, int32_t threads, int32_t lanes_per_particle, int32_t ctas_per_sm);
 /* Whether one lane per particle walks the inner list (1, the default when the
  * buffer is > 0) or every listed pair (0); mdg_batch_tune chooses it too. */
 int mdg_batch_set_inner(mdg_batch *b, int32_t on);
-/* Layout of the persistent step kernel: 0 (default) = each CTA steps the
- * boxes assigned to it in turn; 1 = flat: the resident CTAs stride over the
- * particles of all boxes, one thread per particle, and a small per-box kernel
- * after the step applies the boxes' rebuild and re-selection requests.  The
- * flat layout takes one lane per particle and at most 256 threads per CTA;
+/* Layout of the step kernel: 0 (default) = each CTA steps the boxes assigned
+ * to it in turn; 1 = flat: one thread per particle of all boxes, the boxes that
+ * rebuild on a second stream beside the others, and a small kernel after the
+ * step that applies the boxes' rebuild and re-selection requests.  The flat layout takes one lane per particle and at most 256 threads per CTA;
  * mdg_batch_tune times both layouts. */
 int mdg_batch_set_flat(mdg_batch *b, int32_t on);
 int mdg_batch_get_stats(mdg_batch *b, mdg_batch_stats *s);

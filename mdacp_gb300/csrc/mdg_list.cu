@@ -25,8 +25,7 @@ namespace {
 // One warp per home cell, or two below kSplitBelow cells an SM: forced rebuild of
 // 32,000 atoms 159 us with one, 149 with two, 158 with four; of 131,072 (about
 // 4,900 cells) 201, 213, 248.  The blocks' work is uneven (denser regions have
-// more candidates): many small blocks balance it, resident ones striding over
-// the cells did not (4M atoms, one wave: 25 % slower).
+// more candidates): many small blocks balance it.
 constexpr int kListWarps = 8;
 constexpr long long kSplitBelow = 20;
 __global__ void __launch_bounds__(32 * kListWarps, 4) k_build_list(Geom g, Dev d, int split) {
