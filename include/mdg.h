@@ -220,7 +220,8 @@ const char *mdg_batch_last_error(const mdg_batch *b);
 int mdg_batch_set_state(mdg_batch *b, const double *q4, const double *p4);
 int mdg_batch_get_state(mdg_batch *b, double *q4, double *p4);
 int mdg_batch_calculate(mdg_batch *b, int32_t nsteps);
-/* out: nbox x 3 observer sums (as mdg_observe) at the current positions. */
+/* out: nbox x 3 observer sums (as mdg_observe) at the current positions; builds
+ * the pair lists where the state has none yet (ahead of the first step). */
 int mdg_batch_observe(mdg_batch *b, double *out);
 /* Autotuner: times trial_steps for every (threads per CTA, lanes per particle,
  * CTAs per SM) shape whose CTAs are all resident at once (occupancy of the

@@ -1204,6 +1204,8 @@ struct mdg_batch {
   std::vector<int> box_of_slot;
   int *d_box_of_slot = nullptr;
   int par = 0;
+  bool has_state = false;
+  bool lists_due = true;  // some box's rows are not its state's: a new or restored state, a pool that was regrown
   long long steps = 0;  // goal reached by every box
   cudaGraphExec_t gx[2] = {nullptr, nullptr};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1357,6 +1359,7 @@ int alloc_batch_list(mdg_batch *b, int cap) {
   MDG_BCK(balloc(&b->d.nl, (size_t)off));
   if (b->P.inner) MDG_BCK(balloc(&b->d.pl, (size_t)off));
   b->P.list_cap = cap;
+  b->lists_due = true;
   MDG_BCK(cudaMemcpy(b->d.boxes, b->boxes.data(), b->nbox * sizeof(BoxDesc), cudaMemcpyHostToDevice));
   std::vector<int> ones(b->nbox, 1);
   MDG_BCK(cudaMemcpy(b->d.box_rebuild, ones.data(), b->nbox * sizeof(int), cudaMemcpyHostToDevice));
@@ -1417,6 +1420,48 @@ void launch_batch_step(mdg_batch *b, int par) {
   }
 #undef MDG_BSTEP
   b->launches += kBatchKernelsPerStep + 1;
+}
+
+// The boxes' errors: MDG_ERR_STATE for a bad coordinate; rows that overflowed
+// are given a pool of the capacity they need, the boxes to be run again.
+int check_boxes(mdg_batch *b, bool *regrown) {
+  std::vector<int> err(b->nbox), need(b->nbox);
+  MDG_BCK(cudaMemcpyAsync(err.data(), b->d.box_err, b->nbox * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+  MDG_BCK(cudaMemcpyAsync(need.data(), b->d.box_need, b->nbox * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+  MDG_BCK(cudaStreamSynchronize(b->stream));
+  int maxneed = 0;
+  for (int k = 0; k < b->nbox; k++) {
+    if (err[k] == kErrBadState) return bfail(b, MDG_ERR_STATE, "box " + std::to_string(k) + ": bad coordinate");
+    if (err[k] == kErrOverflow) maxneed = std::max(maxneed, need[k]);
+  }
+  *regrown = maxneed > 0;
+  if (maxneed == 0) return MDG_OK;
+  const int cap = ((int)(maxneed * 1.25) + 15) & ~7;
+  int rc = alloc_batch_list(b, cap);  // every box rebuilds its list at the new capacity
+  if (rc) return rc;
+  MDG_BCK(cudaMemsetAsync(b->d.box_err, 0, b->nbox * sizeof(int), b->stream));
+  MDG_BCK(cudaMemsetAsync(b->d.box_need, 0, b->nbox * sizeof(int), b->stream));
+  return MDG_OK;
+}
+
+// Builds the rows of the state at hand where the pool holds none of it (readers
+// of the rows between steps).  Every box takes part, whatever its step count,
+// and keeps its request: the next step builds the same list again.
+int ensure_lists(mdg_batch *b) {
+  for (int attempt = 0; b->lists_due && attempt < 16; attempt++) {
+    const long long goal = LLONG_MAX;
+    const std::vector<int> ones(b->nbox, 1);
+    MDG_BCK(cudaMemcpyAsync(b->d.goal, &goal, sizeof goal, cudaMemcpyHostToDevice, b->stream));
+    MDG_BCK(cudaMemcpyAsync(b->d.box_rebuild, ones.data(), b->nbox * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    k_batch_rebuild_set<<<1, 1024, 0, b->stream>>>(b->P, b->d);
+    launch_batch_rebuild(b, b->par, b->stream);
+    b->launches += kBatchKernelsPerStep;  // the step's, less its last, and the rebuild set
+    bool regrown = false;
+    const int rc = check_boxes(b, &regrown);
+    if (rc) return rc;
+    b->lists_due = regrown;
+  }
+  return b->lists_due ? bfail(b, MDG_ERR_CAPACITY, "neighbour lists could not be sized") : MDG_OK;
 }
 
 // Ahead of the first of several steps in the flat layout: its rebuild set (the
@@ -1721,12 +1766,14 @@ int mdg_batch_set_state(mdg_batch *b, const double *q4, const double *p4) {
   MDG_BCK(cudaStreamSynchronize(b->stream));
   b->steps = 0;
   b->par = 0;
+  b->has_state = b->lists_due = true;
   drop_batch_graphs(b);
   return MDG_OK;
 }
 
 int mdg_batch_get_state(mdg_batch *b, double *q4, double *p4) {
   if (!b) return MDG_ERR_INVALID;
+  if (!b->has_state) return bfail(b, MDG_ERR_NOT_READY, "no particle state loaded");
   cudaSetDevice(b->prm.device);
   double4_32a *tq = b->d.t_q, *tp = b->d.t_p;  // staging (free outside rebuilds)
   make_end_current(b);
@@ -1743,34 +1790,23 @@ int mdg_batch_calculate(mdg_batch *b, int32_t nsteps) {
   if (!b || nsteps < 0) return MDG_ERR_INVALID;
   cudaSetDevice(b->prm.device);
   if (nsteps == 0) return MDG_OK;
+  if (!b->has_state) return bfail(b, MDG_ERR_NOT_READY, "no particle state loaded");
   const long long goal = b->steps + nsteps;
   MDG_BCK(cudaMemcpyAsync(b->d.goal, &goal, sizeof goal, cudaMemcpyHostToDevice, b->stream));
   MDG_BCK(cudaEventRecord(b->ev0, b->stream));
   int rc = run_steps(b, nsteps);
   if (rc) return rc;
+  bool any_regrown = false;
   for (int round = 0; round < 32; round++) {
-    std::vector<int> err(b->nbox), need(b->nbox);
     std::vector<long long> st(b->nbox);
-    MDG_BCK(cudaMemcpyAsync(err.data(), b->d.box_err, b->nbox * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
-    MDG_BCK(cudaMemcpyAsync(need.data(), b->d.box_need, b->nbox * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
     MDG_BCK(cudaMemcpyAsync(st.data(), b->d.box_steps, b->nbox * sizeof(long long), cudaMemcpyDeviceToHost, b->stream));
-    MDG_BCK(cudaStreamSynchronize(b->stream));
+    bool regrown = false;
+    rc = check_boxes(b, &regrown);
+    if (rc) return rc;
+    any_regrown |= regrown;
     long long behind = 0;
-    int maxneed = 0;
-    for (int k = 0; k < b->nbox; k++) {
-      if (err[k] == kErrBadState) return bfail(b, MDG_ERR_STATE, "box " + std::to_string(k) + ": bad coordinate");
-      behind = std::max(behind, goal - st[k]);
-      if (err[k] == kErrOverflow) maxneed = std::max(maxneed, need[k]);
-    }
+    for (int k = 0; k < b->nbox; k++) behind = std::max(behind, goal - st[k]);
     if (behind == 0) break;
-    if (maxneed > 0) {
-      int cap = ((int)(maxneed * 1.25) + 15) & ~7;
-      rc = alloc_batch_list(b, cap);  // every box rebuilds its list at the new capacity
-      if (rc) return rc;
-      std::vector<int> zeros(b->nbox, 0);
-      MDG_BCK(cudaMemcpyAsync(b->d.box_err, zeros.data(), b->nbox * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-      MDG_BCK(cudaMemcpyAsync(b->d.box_need, zeros.data(), b->nbox * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-    }
     // catch-up: only boxes behind the goal advance
     begin_steps(b);
     for (long long k = 0; k < behind; k++) {
@@ -1788,12 +1824,17 @@ int mdg_batch_calculate(mdg_batch *b, int32_t nsteps) {
   cudaEventElapsedTime(&ms, b->ev0, b->ev1);
   b->last_ms = ms;
   b->steps = goal;
+  // after a regrowth the boxes that were at the goal have no rows in the new pool
+  b->lists_due = any_regrown;
   return MDG_OK;
 }
 
 int mdg_batch_observe(mdg_batch *b, double *out) {
   if (!b || !out) return MDG_ERR_INVALID;
+  if (!b->has_state) return bfail(b, MDG_ERR_NOT_READY, "no particle state loaded");
   cudaSetDevice(b->prm.device);
+  const int rc = ensure_lists(b);
+  if (rc) return rc;
   make_end_current(b);
   if (b->P.fixed) k_batch_fix_end<<<(b->total + 255) / 256, 256, 0, b->stream>>>(b->P, b->d);
   for (int first = 0; first < b->nbox; first += kObserveBoxes) {
@@ -1810,6 +1851,7 @@ int mdg_batch_observe(mdg_batch *b, double *out) {
 int mdg_batch_tune(mdg_batch *b, int32_t trial_steps, int32_t *threads, int32_t *lanes_per_particle,
                    int32_t *ctas_per_sm) {
   if (!b || trial_steps <= 0) return MDG_ERR_INVALID;
+  if (!b->has_state) return bfail(b, MDG_ERR_NOT_READY, "no particle state loaded");
   cudaSetDevice(b->prm.device);
   // work on a copy of the state and restore it afterwards
   const size_t n = (size_t)b->total;
@@ -1934,6 +1976,7 @@ int mdg_batch_tune(mdg_batch *b, int32_t trial_steps, int32_t *threads, int32_t 
   MDG_BCK(cudaStreamSynchronize(b->stream));
   b->steps = steps0;
   b->par = 0;
+  b->lists_due = true;
   cudaFree(sq);
   cudaFree(sp);
   cudaFree(sid);
