@@ -53,8 +53,8 @@ __global__ void __launch_bounds__(fx_threads<LANES>(), LANES == 1 ? kOneBlocks :
   {
     const int ia = active ? i : g.n - 1;
     const FixPos own = xq[ia];
-    if (prune) F = force_fixed<true, LANES>(g, d, xq, qm, own, ia, wide, d.nl, d.ncount, active, lane, kept);
-    else F = force_fixed<false, LANES>(g, d, xq, qm, own, ia, wide, d.pl, d.pcount, active, lane, kept);
+    if (prune) F = force_fixed<true, LANES, false>(g, d, xq, qm, own, ia, wide, d.nl, d.ncount, active, lane, kept);
+    else F = force_fixed<false, LANES, false>(g, d, xq, qm, own, ia, wide, d.pl, d.pcount, active, lane, kept);
   }
   if (LANES > 1) {
     // the block's particles move on to its first threads, one each
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(fx_threads<LANES>()) k_forces_fixed(Geom g, De
   const bool active = i < g.n;
   const int ia = active ? i : g.n - 1;
   int kept = 0;
-  const double3 F = force_fixed<false, LANES>(g, d, d.xq[src], d.q_end, d.xq[src][ia], ia, d.flags->fx_wide_end == call,
+  const double3 F = force_fixed<false, LANES, false>(g, d, d.xq[src], d.q_end, d.xq[src][ia], ia, d.flags->fx_wide_end == call,
                                               d.nl, d.ncount, active, lane, kept);
   const double s = 1.0 / (double)(1ull << kFixSumBits);
   if (active && lane == 0) d.io4[d.id[i]] = make_double4_32a(F.x * s, F.y * s, F.z * s, 0.0);

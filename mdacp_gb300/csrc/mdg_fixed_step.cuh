@@ -124,9 +124,10 @@ __device__ __forceinline__ void walk_fixed(const Geom &g, const Dev &d, const Fi
 
 // The double expression for one entry of the row of i (pairs closer than
 // kFixNear), as force_fp64 evaluates it.
-__device__ __noinline__ inline double3 near_force(const Geom &g, const double4_32a *pos, int i, int key, uint32_t e) {
-  const double4_32a qi = pos[i];
-  double4_32a qj = pos[entry_slot(e)];
+template <bool COH>
+__device__ __noinline__ double3 near_force(const Geom &g, const double4_32a *pos, int i, int key, uint32_t e) {
+  const double4_32a qi = COH ? ld_ro<true>(pos + i) : pos[i];
+  double4_32a qj = COH ? ld_ro<true>(pos + entry_slot(e)) : pos[entry_slot(e)];
   apply_image(g, cell_pos(g, key), e, qj);
   const double dx = qj.x - qi.x, dy = qj.y - qi.y, dz = qj.z - qi.z;
   const double r2 = dx * dx + dy * dy + dz * dz;
@@ -173,7 +174,7 @@ __device__ __forceinline__ void row_fixed(const Geom &g, const Dev &d, const Fix
         return close;
       },
       [&](uint32_t e) {
-        const double3 f = near_force(g, pos, i, (int)own.w, e);
+        const double3 f = near_force<COH>(g, pos, i, (int)own.w, e);
         r.nx += f.x;
         r.ny += f.y;
         r.nz += f.z;
@@ -183,7 +184,7 @@ __device__ __forceinline__ void row_fixed(const Geom &g, const Dev &d, const Fix
 
 // The force on particle i in units of 2^-52 as doubles, from LANES lanes
 // (every lane of the group receives it); *kept the new inner row's length.
-template <bool PRUNE, int LANES, bool COH = false>
+template <bool PRUNE, int LANES, bool COH>
 __device__ __forceinline__ double3 force_fixed(const Geom &g, const Dev &d, const FixPos *__restrict__ xq,
                                                const double4_32a *__restrict__ pos, const FixPos &own, int i,
                                                bool wide, const uint32_t *__restrict__ list,
@@ -192,7 +193,7 @@ __device__ __forceinline__ double3 force_fixed(const Geom &g, const Dev &d, cons
   const CellPos cp = cell_pos(g, (int)own.w);
   if (wide) {  // uniform over the grid
     double3 F = make_double3(0.0, 0.0, 0.0);
-    if (active && lane == 0) F = force_fp64<PRUNE>(g, d, pos, i, cp, list, counts, &kept);
+    if (active && lane == 0) F = force_fp64<PRUNE, COH>(g, d, pos, i, cp, list, counts, &kept);
     return make_double3(F.x * up, F.y * up, F.z * up);
   }
   int cnt = active ? ld_ro<COH>(counts + i) : 0;
@@ -236,7 +237,7 @@ __device__ __forceinline__ double3 force_fixed(const Geom &g, const Dev &d, cons
   }
   // sums that may have left their range: the row again in double
   if (active && lane == 0 && !fix_sum_fits(r.f, cnt)) {
-    F = force_fp64<false>(g, d, pos, i, cp, list, counts, nullptr);
+    F = force_fp64<false, COH>(g, d, pos, i, cp, list, counts, nullptr);
     F = make_double3(F.x * up, F.y * up, F.z * up);
   }
   return F;

@@ -110,10 +110,10 @@ __global__ void __launch_bounds__(step_threads<THERMO, MIXED, PMODE>(), (PMODE !
     double3 F;
     if (prune)
       F = MIXED ? force_mixed<true, MIXED == MDG_MIXED>(g, d, d.loc[par], i, lb, cp, d.nl, d.ncount, &kept)
-                : force_fp64<true>(g, d, qm, i, cp, d.nl, d.ncount, &kept);
+                : force_fp64<true, false>(g, d, qm, i, cp, d.nl, d.ncount, &kept);
     else
       F = MIXED ? force_mixed<false, MIXED == MDG_MIXED>(g, d, d.loc[par], i, lb, cp, d.pl, d.pcount, nullptr)
-                : force_fp64<false>(g, d, qm, i, cp, d.pl, d.pcount, nullptr);
+                : force_fp64<false, false>(g, d, qm, i, cp, d.pl, d.pcount, nullptr);
     ke = step_one<THERMO, COMPAT, MIXED>(g, d, par, i, prune, kept, F, lb, qm, qn, THERMO == MDG_NOSEHOOVER ? f->exp1 : 1.0,
                                          THERMO == MDG_LANGEVIN ? f->lang - 1ull : 0ull, &d.flags->rebuild,
                                          &d.flags->prune_next);
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kStepThreads) k_forces(Geom g, Dev d, const fl
   if (i >= g.n) return;
   const CellPos cp = cell_pos(g, d.cell[i]);
   const double3 F = MIXED ? force_mixed<false, MIXED == MDG_MIXED>(g, d, loc, i, loc[i], cp, d.nl, d.ncount, nullptr)
-                          : force_fp64<false>(g, d, d.q_end, i, cp, d.nl, d.ncount, nullptr);
+                          : force_fp64<false, false>(g, d, d.q_end, i, cp, d.nl, d.ncount, nullptr);
   d.io4[d.id[i]] = make_double4_32a(F.x, F.y, F.z, 0.0);
 }
 

@@ -45,18 +45,47 @@ __device__ __forceinline__ void apply_image(const Geom &g, const CellPos &cp, ui
   else if (oz == 2 && cp.cz == g.nc[2] - 1) qj.z += g.L[2];
 }
 
+// A load of data that the kernel does not write (COH = false), or that it
+// does (COH: the resident kernel, whose grid barriers make it visible).
+template <bool COH>
+__device__ __forceinline__ uint32_t ld_ro(const uint32_t *p) {
+  if (!COH) return __ldg(p);
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+template <bool COH>
+__device__ __forceinline__ int ld_ro(const int *p) {
+  return COH ? (int)ld_ro<true>(reinterpret_cast<const uint32_t *>(p)) : *p;
+}
+template <bool COH>
+__device__ __forceinline__ float4 ld_ro(const float4 *p) {
+  if (!COH) return __ldg(p);
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+template <bool COH>
+__device__ __forceinline__ double4_32a ld_ro(const double4_32a *p) {
+  if (!COH) return ldg4(p);
+  double4_32a v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 // Sum over the row of slot i of f(r) (q_j - q_i), f(r) = 24 r^-8 - 48 r^-14 + 8 C2,
 // the force on i (fcalculator.cc:263-277 without the dt factor).
 // `list`/`counts` is the inner (pruned) list in an ordinary step and the outer
 // list for a stand-alone force evaluation.  With PRUNE the outer list is
 // walked and every entry within the prune radius is copied to the inner row
-// of slot i (d.pl); *kept receives the new row length.
-template <bool PRUNE>
+// of slot i (d.pl); *kept receives the new row length.  COH: rows and positions
+// that the calling kernel itself writes.
+template <bool PRUNE, bool COH>
 __device__ __forceinline__ double3 force_fp64(const Geom &g, const Dev &d, const double4_32a *__restrict__ pos, int i,
                                               const CellPos &cp, const uint32_t *__restrict__ list,
                                               const int *__restrict__ counts, int *kept) {
-  const double4_32a qi = pos[i];
-  int cnt = counts[i];
+  const double4_32a qi = COH ? ld_ro<true>(pos + i) : pos[i];
+  int cnt = ld_ro<COH>(counts + i);
   if (!MDG_IN_RANGE(d.flags, kCheckStepRow, cnt, g.list_cap + 1)) cnt = 0;
   const uint32_t *row = list + i;
   const double thr = (double)g.prune_thr2;
@@ -67,9 +96,9 @@ __device__ __forceinline__ double3 force_fp64(const Geom &g, const Dev &d, const
   int m = 0;
   double fx = 0.0, fy = 0.0, fz = 0.0;
   for (int k = 0; k < cnt; k++) {
-    const uint32_t e = __ldg(row + (size_t)k * g.stride);
+    const uint32_t e = ld_ro<COH>(row + (size_t)k * g.stride);
     if (!MDG_IN_RANGE(d.flags, kCheckStepSlot, entry_slot(e), g.n)) continue;
-    double4_32a qj = ldg4(pos + entry_slot(e));
+    double4_32a qj = ld_ro<COH>(pos + entry_slot(e));
     if (cp.edge) apply_image(g, cp, e, qj);
     const double dx = qj.x - qi.x, dy = qj.y - qi.y, dz = qj.z - qi.z;
     const double r2 = dx * dx + dy * dy + dz * dz;
@@ -151,27 +180,6 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[w];
   __syncthreads();
   return t;
-}
-
-// A load of data that the kernel does not write (COH = false), or that it
-// does (COH: the resident kernel, whose grid barriers make it visible).
-template <bool COH>
-__device__ __forceinline__ uint32_t ld_ro(const uint32_t *p) {
-  if (!COH) return __ldg(p);
-  uint32_t v;
-  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-template <bool COH>
-__device__ __forceinline__ int ld_ro(const int *p) {
-  return COH ? (int)ld_ro<true>(reinterpret_cast<const uint32_t *>(p)) : *p;
-}
-template <bool COH>
-__device__ __forceinline__ float4 ld_ro(const float4 *p) {
-  if (!COH) return __ldg(p);
-  float4 v;
-  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
-  return v;
 }
 
 // Neighbour-list entries whose index and position loads are issued together
