@@ -96,15 +96,21 @@ MDG_HD FixSep fix_sep(int32_t x, int32_t y, int32_t z, float lx, float ly, float
   return FixSep{x, y, z, (float)x, (float)y, (float)z, lx, ly, lz};
 }
 
+// The cross products of high words and rests, twice of which r^2 takes, are
+// rounded to 2^-55 (of the size 2^-51 that their float sum is good to where the
+// rests matter): across three faces the rests add up to 0.75 an axis, and a
+// sum in units of 2^-56 would leave 32 bits from 3.1 sigma on.  In this unit
+// it holds to 6.2 sigma; converted to 64 bits instead, 32,000 atoms took 2.5 %
+// longer a step.
 MDG_HD uint64_t fix_r2(const FixSep &d) {
   const int64_t h = fix_mads(d.z, d.z, fix_mads(d.y, d.y, fix_mads(d.x, d.x, 0)));
-  const float c = fmaf(d.fz, d.lz, fmaf(d.fy, d.ly, d.fx * d.lx));  // 2^-57
+  const float c = 0.5f * fmaf(d.fz, d.lz, fmaf(d.fy, d.ly, d.fx * d.lx));  // 2^-56
 #ifdef __CUDA_ARCH__
   const int32_t i = __float2int_rn(c);
 #else
   const int32_t i = (int32_t)lrintf(c);
 #endif
-  return (uint64_t)h + ((uint64_t)(int64_t)i << 2);  // twice the cross products
+  return (uint64_t)h + ((uint64_t)(int64_t)i << 3);  // twice the cross products
 }
 
 // High 64 bits of a * b, low by one or two: the product of the low words and
