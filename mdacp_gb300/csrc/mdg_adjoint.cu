@@ -98,6 +98,7 @@ struct P {
   int64_t fx_c8;
   int fx_L[3];
   float fx_l[3];
+  float fx_fit_n, fx_fit_0;  // derivative_sums_fit
 };
 
 // A list entry: partner index << kImageBits | per axis two bits r + 1, the
@@ -338,8 +339,35 @@ __device__ __forceinline__ void lane_sums(FixForce &f) {
   }
 }
 
-// Half the range of fix_sum_fits: the derivative sums are below twice the force's.
+// Whether the sum of psi d over n entries stays inside 2^11: as fix_sum_fits,
+// which bounds the sum of |psi| x by 7 n - 1.13 sum(psi), here at most 960, and
+// the separation is x sigma with sigma up to 1.8.
 __device__ __forceinline__ bool sums_fit(const FixForce &f, int n) { return f.s >= (float)(7 * n - 850) * 8388608.0f; }
+
+// The same for the sum of q d, q = fix_dsigma (the force's sigma derivative, the
+// pressure's slope), f.s the sum of psi: q does not vanish where psi does, so its
+// sum has a bound of its own (derivative_fit).
+__device__ __forceinline__ bool derivative_sums_fit(const P &c, const FixForce &f, int n) {
+  return f.s >= fmaf(c.fx_fit_n, (float)n, c.fx_fit_0);
+}
+
+// |q| x <= a - b psi for every pair that takes the fixed-point terms, so the sum
+// of q d is at most sigma (a n - b sum(psi)), and below 1,900 of 2^11 where
+// sum(psi) >= (a n - 1900 / sigma) / b.  a is found over the pairs' range of x for
+// b = 1.82, the ratio of |q| to -psi of the closest of them: a = 11 at a cut-off
+// of 2.5.
+void derivative_fit(P &c) {
+  const double b = 1.82, x0 = std::sqrt(kFixNear), x1 = std::sqrt(c.xc2);
+  double a = 0.0;
+  for (int k = 0; k <= 4096; k++) {
+    const double x = x0 + (x1 - x0) * k / 4096.0, y = 1.0 / (x * x), y4 = y * y * y * y, y7 = y4 * y * y * y;
+    const double psi = 24.0 * y4 - 48.0 * y7 + 8.0 * c.c2, q = 18.0 * y4 - 72.0 * y7 - 2.0 * c.c2;
+    a = std::fmax(a, std::fabs(q) * x + b * psi);
+  }
+  a += 0.5;  // between the samples
+  c.fx_fit_n = (float)(a / b * 8388608.0);
+  c.fx_fit_0 = (float)(-1900.0 / (c.sig * b) * 8388608.0);
+}
 
 // scale times the vector sum; unit 2^-52.
 __device__ __forceinline__ double3 fix_vector(const FixForce &f, double scale) {
@@ -653,7 +681,7 @@ __device__ __forceinline__ ObjSums objective_sums_fixed(const P &c, const D &d, 
     }
   }
   if (lane != 0 || i >= c.n) return r;
-  if (cnt > kFixSumsRow || (GRAD && !sums_fit(f, cnt))) {  // the row again in double
+  if (cnt > kFixSumsRow || (GRAD && !(OBJ == 0 ? sums_fit(f, cnt) : derivative_sums_fit(c, f, cnt)))) {  // the row again in double
     r = ObjSums{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const Home h = make_home(c, q[i]);
     for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], q, h, in_double);
@@ -902,7 +930,7 @@ __global__ void __launch_bounds__(kT) k_force_sigma(P c, D d, int first) {
     f.s = psi;
     if (__any_sync(0xffffffffu, near)) S = make_double3(lane_sum<kL>(S.x), lane_sum<kL>(S.y), lane_sum<kL>(S.z));
     if (i >= c.n || lane != 0) return;
-    if (sums_fit(f, cnt)) {
+    if (derivative_sums_fit(c, f, cnt)) {
       const double3 v = fix_vector(f, 8.0 * c.e_s3);
       S = make_double3(S.x + v.x, S.y + v.y, S.z + v.z);
     } else {  // the row again in double
@@ -1297,6 +1325,7 @@ int mdg_adjoint_create(const mdg_adjoint_params *p, int32_t n, mdg_adjoint **out
     c.fx_near = (uint64_t)std::ldexp(mdg::kFixNear * s2v, mdg::kFixR2Bits);
     c.fx_s2 = (uint64_t)std::ldexp(s2v, 62);
     c.fx_c8 = mdg::fix_c8(8.0 * c.c2);
+    derivative_fit(c);
     for (int k = 0; k < 3; k++) {
       const int64_t L = mdg::fix_from_double(p->box[k]);
       c.fx_L[k] = mdg::fix_shi(L);
