@@ -96,6 +96,19 @@ __device__ __forceinline__ void finalize_one(const Geom &g, const Dev &d, int k,
 
 constexpr int kRowLanes = 9;
 
+// The length `cnt` of slot i's row, which may exceed the capacity: kept, or the
+// run halted; the kept entries added to `pairs`, the longest row to `longest`.
+__device__ __forceinline__ void keep_row_length(const Geom &g, const Dev &d, int i, int cnt, int &pairs, int &longest) {
+  const int kept = min(cnt, g.list_cap);
+  d.ncount[i] = kept;
+  if (cnt > g.list_cap) {
+    atomicMax(&d.flags->overflow_max, cnt);
+    halt_with(d.flags, kHaltOverflow);
+  }
+  pairs += kept;
+  longest = max(longest, cnt);
+}
+
 // The row of slot i by kRowLanes neighbouring lanes of a warp (`base` the first
 // of them), one for each (y, z) row of three stencil cells: a row's candidates
 // then take a ninth of the time one after the other, which is what a small box
@@ -225,15 +238,7 @@ __device__ __forceinline__ void build_cell_rows(const Geom &g, const Dev &d, Cel
         return image_within(d.q_end[i], d.q_end[j], g.L, sx, sy, sz, g.sl2);
       },
       RowSink{d.nl, (size_t)g.stride, nullptr},
-      [&](int i, int cnt) {
-        d.ncount[i] = cnt < cap ? cnt : cap;
-        if (cnt > cap) {
-          atomicMax(&f->overflow_max, cnt);
-          halt_with(f, kHaltOverflow);
-        }
-        pairs += cnt < cap ? cnt : cap;
-        longest = max(longest, cnt);
-      });
+      [&](int i, int cnt) { keep_row_length(g, d, i, cnt, pairs, longest); });
 }
 
 }  // namespace mdg

@@ -213,16 +213,7 @@ __device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, Resid
       const int i = i0 + k;
       const bool active = k < per && i < g.n;
       const int cnt = build_slot_row(g, d, i, active, lane, wl - lane);
-      if (active && lane == 0) {
-        const int kept = min(cnt, g.list_cap);
-        d.ncount[i] = kept;
-        if (cnt > g.list_cap) {
-          atomicMax(&f->overflow_max, cnt);
-          halt_with(f, kHaltOverflow);
-        }
-        pairs += kept;
-        longest = max(longest, cnt);
-      }
+      if (active && lane == 0) keep_row_length(g, d, i, cnt, pairs, longest);
     }
   } else {
     extern __shared__ __align__(16) unsigned char s_dynamic[];
