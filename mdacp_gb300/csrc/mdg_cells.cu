@@ -172,6 +172,7 @@ __global__ void k_reorder(Geom g, Dev d) {
 // half-drift, fcalculator.cc:21-32, rounded as two separate operations).  In
 // the mixed form q_mid is kept relative to the centre of the new home cell,
 // (q - centre) + p dt/2, and q_end is current again.
+template <bool LOCAL, bool FIXED>
 __global__ void k_finalize(Geom g, Dev d, int q_mid_dst) {
   if (rebuild_off(d.flags)) return;
   // k_wrap_bin, the only reader of end_stale in the rebuild, has finished;
@@ -183,8 +184,11 @@ __global__ void k_finalize(Geom g, Dev d, int q_mid_dst) {
     d.flags->lifetime = 0;
     d.flags->need_check = 0;
   }
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.n; k += gridDim.x * blockDim.x)
-    finalize_one(g, d, k, d.t_q[k], d.t_p[k], d.t_id[k], d.t_cell[k], q_mid_dst);
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.n; k += gridDim.x * blockDim.x) {
+    const double4_32a q = d.t_q[k], p = d.t_p[k];
+    const int id = d.t_id[k], c = d.t_cell[k];
+    finalize_one<LOCAL, FIXED>(g, d, k, q, p, id, c, q_mid_dst);
+  }
 }
 
 // Mixed form: q_end from q_mid[mid] and p for every slot while the steps have
@@ -642,7 +646,9 @@ void launch_rebuild(const Geom &g, const Dev &d, int q_mid_dst, int num_sms, cud
   k_scan_apply<<<nb, kScanThreads, 0, s>>>(g, d);
   k_scatter<<<grid, threads, 0, s>>>(g, d);
   k_reorder<<<grid, threads, 0, s>>>(g, d);
-  k_finalize<<<grid, threads, 0, s>>>(g, d, q_mid_dst);
+  if (g.local_pos) k_finalize<true, false><<<grid, threads, 0, s>>>(g, d, q_mid_dst);
+  else if (g.fixed) k_finalize<false, true><<<grid, threads, 0, s>>>(g, d, q_mid_dst);
+  else k_finalize<false, false><<<grid, threads, 0, s>>>(g, d, q_mid_dst);
   launch_build_list(g, d, num_sms, s, in_step);
 }
 

@@ -199,7 +199,9 @@ __device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, Resid
     double4_32a q = d.t_q[k];
     const unsigned long long w = (unsigned long long)__double_as_longlong(q.w);
     q.w = 0.0;
-    finalize_one(g, d, k, q, d.t_p[k], (int)(unsigned)w, (int)(unsigned)(w >> 32), r.par);
+    const int id = (int)(unsigned)w, key = (int)(unsigned)(w >> 32);
+    if (g.local_pos) finalize_one<true, false>(g, d, k, q, d.t_p[k], id, key, r.par);
+    else finalize_one<false, true>(g, d, k, q, d.t_p[k], id, key, r.par);  // an FP64 box here is in fixed point
   }
   if (!grid_barrier(c, ++r.barriers)) return false;
   r.stale = false;
