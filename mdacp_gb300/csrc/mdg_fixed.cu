@@ -152,10 +152,7 @@ __device__ __forceinline__ void observe_fixed(const Geom &g, const Dev &d, const
           apply_image(g, cp, e, qj);
           const double dx = __dsub_rn(qi.x, qj.x), dy = __dsub_rn(qi.y, qj.y), dz = __dsub_rn(qi.z, qj.z);
           const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-          double a, b;
-          pair_observables(g, r2, a, b);
-          ne += a;
-          nv += b;
+          pair_observables(g, r2, ne, nv);
         }
       });
 }

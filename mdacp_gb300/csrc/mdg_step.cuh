@@ -116,15 +116,15 @@ __device__ __forceinline__ double3 force_fp64(const Geom &g, const Dev &d, const
   return make_double3(fx, fy, fz);
 }
 
-// A pair's energy and virial term at r2, weighted 1/2, in the reference's
-// expressions and rounding (observer.cc:17-79); zero beyond rc.
+// Adds a pair's energy and virial term at r2, weighted 1/2, in the reference's
+// expressions and rounding (observer.cc:17-79); nothing beyond rc (adding zeros
+// there took the FP64 pipe 4 % of the observers' time).
 __device__ __forceinline__ void pair_observables(const Geom &g, double r2, double &e, double &v) {
-  e = v = 0.0;
   if (r2 > g.rc2) return;
   const double r4 = __dmul_rn(r2, r2), r6 = __dmul_rn(r4, r2), r8 = __dmul_rn(r6, r2), r10 = __dmul_rn(r8, r2),
                r12 = __dmul_rn(r10, r2);
-  e = 0.5 * (4.0 * (1.0 / r12 - 1.0 / r6 + __dmul_rn(g.c2, r2) + g.c0));
-  v = 0.5 * ((__dsub_rn(__dmul_rn(24.0, r6), 48.0) / (__dmul_rn(__dmul_rn(r6, r6), r2)) + g.c2x8) * r2);
+  e += 0.5 * (4.0 * (1.0 / r12 - 1.0 / r6 + __dmul_rn(g.c2, r2) + g.c0));
+  v += 0.5 * ((__dsub_rn(__dmul_rn(24.0, r6), 48.0) / (__dmul_rn(__dmul_rn(r6, r6), r2)) + g.c2x8) * r2);
 }
 
 // Pair energy and virial sums of the outer row of slot i at q_end in double.
@@ -138,10 +138,7 @@ __device__ inline void observe_row_fp64(const Geom &g, const Dev &d, int i, cons
     if (cp.edge) apply_image(g, cp, e, qj);
     const double dx = __dsub_rn(qi.x, qj.x), dy = __dsub_rn(qi.y, qj.y), dz = __dsub_rn(qi.z, qj.z);
     const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    double a, b;
-    pair_observables(g, r2, a, b);
-    pe += a;
-    vir += b;
+    pair_observables(g, r2, pe, vir);
   }
 }
 
