@@ -890,11 +890,10 @@ __global__ void __launch_bounds__(kT) k_objective(P c, D d, double w, int first)
 }
 
 // sum_j dF_ij/dsigma of the half steps first .. first + gridDim.y - 1 of the
-// segment, into segs.
-template <bool FIXED>
+// segment, into segs (fixed-point form; the double form takes it in k_reverse).
 __global__ void __launch_bounds__(kT) k_force_sigma(P c, D d, int first) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  constexpr int kL = FIXED ? kBatchLanes : kLanes;
+  constexpr int kL = kBatchLanes;
   const int i = tid / kL, lane = tid % kL;
   const size_t at = (size_t)c.n * (first + blockIdx.y);
   const double4_32a *q = d.segqh + at;
@@ -904,47 +903,38 @@ __global__ void __launch_bounds__(kT) k_force_sigma(P c, D d, int first) {
     S.y += t.fs * dy;
     S.z += t.fs * dz;
   };
-  if (FIXED) {
-    FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f};
-    float psi = 0.f;
-    bool near = false;
-    int cnt = 0;
-    if (i < c.n) {
-      cnt = d.cnt[i];
-      for_pairs_fixed<kL>(
-          c, d, i, lane, d.segxqh + at,
-          [&](bool take, const FixSep &sep, uint64_t R, int) {
-            const FixTerms t = fix_terms(c, R);
-            fix_add(f, take ? fix_dsigma(c, t) : 0, sep);
-            psi += (float)fix_shi(take ? fix_psi(c, t) : 0);
-          },
-          [&](uint32_t e) {
-            near = true;
-            one_pair(c, e, q, make_home(c, q[i]), in_double);
-          });
-    }
-    __syncwarp();
-    lane_sums<kL>(f);
+  FixForce f{0, 0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0.f};
+  float psi = 0.f;
+  bool near = false;
+  int cnt = 0;
+  if (i < c.n) {
+    cnt = d.cnt[i];
+    for_pairs_fixed<kL>(
+        c, d, i, lane, d.segxqh + at,
+        [&](bool take, const FixSep &sep, uint64_t R, int) {
+          const FixTerms t = fix_terms(c, R);
+          fix_add(f, take ? fix_dsigma(c, t) : 0, sep);
+          psi += (float)fix_shi(take ? fix_psi(c, t) : 0);
+        },
+        [&](uint32_t e) {
+          near = true;
+          one_pair(c, e, q, make_home(c, q[i]), in_double);
+        });
+  }
+  __syncwarp();
+  lane_sums<kL>(f);
 #pragma unroll
-    for (int o = 1; o < kL; o <<= 1) psi += __shfl_xor_sync(0xffffffffu, psi, o);
-    f.s = psi;
-    if (__any_sync(0xffffffffu, near)) S = make_double3(lane_sum<kL>(S.x), lane_sum<kL>(S.y), lane_sum<kL>(S.z));
-    if (i >= c.n || lane != 0) return;
-    if (derivative_sums_fit(c, f, cnt)) {
-      const double3 v = fix_vector(f, 8.0 * c.e_s3);
-      S = make_double3(S.x + v.x, S.y + v.y, S.z + v.z);
-    } else {  // the row again in double
-      S = make_double3(0.0, 0.0, 0.0);
-      const Home h = make_home(c, q[i]);
-      for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], q, h, in_double);
-    }
-  } else {
-    if (i < c.n) {
-      const Home h = make_home(c, q[i]);
-      for_pairs(c, d, i, lane, q, h, in_double);
-    }
-    S = make_double3(lane_sum<kL>(S.x), lane_sum<kL>(S.y), lane_sum<kL>(S.z));
-    if (i >= c.n || lane != 0) return;
+  for (int o = 1; o < kL; o <<= 1) psi += __shfl_xor_sync(0xffffffffu, psi, o);
+  f.s = psi;
+  if (__any_sync(0xffffffffu, near)) S = make_double3(lane_sum<kL>(S.x), lane_sum<kL>(S.y), lane_sum<kL>(S.z));
+  if (i >= c.n || lane != 0) return;
+  if (derivative_sums_fit(c, f, cnt)) {
+    const double3 v = fix_vector(f, 8.0 * c.e_s3);
+    S = make_double3(S.x + v.x, S.y + v.y, S.z + v.z);
+  } else {  // the row again in double
+    S = make_double3(0.0, 0.0, 0.0);
+    const Home h = make_home(c, q[i]);
+    for (int k = 0; k < cnt; k++) one_pair(c, d.nbr[(size_t)i * c.cap + k], q, h, in_double);
   }
   d.segs[at + i] = make_double4_32a(S.x, S.y, S.z, 0.0);
 }
@@ -976,7 +966,9 @@ __global__ void k_seed(P c, D d, int len, double w, double4_32a *tmp) {
 
 // The rest of the reverse of step k at its half-step positions (kick and first
 // half-drift).  In: tmp (read by the neighbours too) and aqh from the reverse of
-// its second half-drift; the force and its sigma derivative there.  Parameter
+// its second half-drift; the force there and, in the fixed-point form, its sigma
+// derivative (the double form takes it along here: pair terms once more in a
+// launch of their own cost 16,384 particles 80 us a step of 873).  Parameter
 // terms dt * ap . dF/dtheta into part[k] (slots 1, 2).  For k > 1 it goes on
 // with the objective's terms of state k - 1 and the reverse of step k - 1's
 // second half-drift, into tmp_out (not tmp: other particles' lanes still read
@@ -992,6 +984,7 @@ __global__ void __launch_bounds__(kT) k_reverse(P c, D d, int k, const double4_3
   const size_t at = (size_t)c.n * k;
   const double4_32a *qh = d.segqh + at;
   double hx = 0, hy = 0, hz = 0;
+  double sx = 0, sy = 0, sz = 0;  // double form: the force's sigma derivative
   double4_32a vi = i < c.n ? tmp[i] : make_double4_32a(0.0, 0.0, 0.0, 0.0);
   auto in_double = [&](const PairTerms &t, double dx, double dy, double dz, int j) {
     const double4_32a vj = tmp[j];
@@ -1001,6 +994,11 @@ __global__ void __launch_bounds__(kT) k_reverse(P c, D d, int k, const double4_3
     hx += t.f * wx + t.fpr * dx * dw;
     hy += t.f * wy + t.fpr * dy * dw;
     hz += t.f * wz + t.fpr * dz * dw;
+    if (!FIXED) {
+      sx += t.fs * dx;
+      sy += t.fs * dy;
+      sz += t.fs * dz;
+    }
   };
   if (FIXED) {
     // reduced sums psi w and (psi' / x) / 48 (d . w) d
@@ -1040,8 +1038,14 @@ __global__ void __launch_bounds__(kT) k_reverse(P c, D d, int k, const double4_3
   hy = lane_sum<kL>(hy);
   hz = lane_sum<kL>(hz);
   // one thread per particle from here on, as in k_step
-  __shared__ double3 sH[kT / kL];
+  __shared__ double3 sH[kT / kL], sS[FIXED ? 1 : kT / kL];
   if (lane == 0) sH[threadIdx.x / kL] = make_double3(hx, hy, hz);
+  if (!FIXED) {
+    sx = lane_sum<kL>(sx);
+    sy = lane_sum<kL>(sy);
+    sz = lane_sum<kL>(sz);
+    if (lane == 0) sS[threadIdx.x / kL] = make_double3(sx, sy, sz);
+  }
   __syncthreads();
   i = blockIdx.x * (kT / kL) + threadIdx.x;
   double te = 0, ts = 0;
@@ -1051,7 +1055,8 @@ __global__ void __launch_bounds__(kT) k_reverse(P c, D d, int k, const double4_3
     hy = sH[threadIdx.x].y;
     hz = sH[threadIdx.x].z;
     // parameter terms: dt * a_p . dF_i/deps (= F_i/eps), dt * a_p . dF_i/dsigma
-    const double4_32a F = d.segf[at + i], S = d.segs[at + i];
+    const double4_32a F = d.segf[at + i];
+    const double3 S = FIXED ? make_double3(d.segs[at + i].x, d.segs[at + i].y, d.segs[at + i].z) : sS[threadIdx.x];
     te = c.dt * (vi.x * F.x + vi.y * F.y + vi.z * F.z) / c.eps;
     ts = c.dt * (vi.x * S.x + vi.y * S.y + vi.z * S.z);
     // kick: a_qh = a_q - dt H a_p ; then drift qh = q + dt/2 p : a_p += dt/2 a_qh
@@ -1175,8 +1180,7 @@ void launch_objective(mdg_adjoint *a, int len, double w) {
 void launch_force_sigma(mdg_adjoint *a, int len) {
   for (int first = 1; first <= len; first += kStates) {
     const dim3 grid(a->grids, len - first + 1 < kStates ? len - first + 1 : kStates);
-    if (a->c.fixed) k_force_sigma<true><<<grid, kT, 0, a->s>>>(a->c, a->d, first);
-    else k_force_sigma<false><<<grid, kT, 0, a->s>>>(a->c, a->d, first);
+    k_force_sigma<<<grid, kT, 0, a->s>>>(a->c, a->d, first);
   }
 }
 
@@ -1220,7 +1224,7 @@ int enqueue_backward(mdg_adjoint *a) {
     k_begin<<<a->grid, kT, 0, a->s>>>(a->c, d, d.ckq + ck, d.ckp + ck, nullptr, nullptr, 0);
     run_segment(a, len, true);
     launch_objective<true>(a, len, w);
-    launch_force_sigma(a, len);
+    if (a->c.fixed) launch_force_sigma(a, len);
     double4_32a *tmp = d.tmp, *tmp_alt = d.tmp2;
     k_seed<<<a->grid, kT, 0, a->s>>>(a->c, d, len, w, tmp);
     for (int k = len; k >= 1; k--) {
