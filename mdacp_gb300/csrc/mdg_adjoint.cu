@@ -106,20 +106,24 @@ struct P {
 constexpr int kImageBits = 6;
 constexpr int kMaxAdjointParticles = 1 << (32 - kImageBits);
 
-// A checkpoint segment is held whole: states 0 .. K, and the half steps 1 .. K
-// that lead to states 1 .. K, each array [K + 1][n] (with the forces at the half
-// steps, their sigma derivatives and the objective's gradients at the states
-// in the backward pass).
+// A checkpoint segment's states 0 .. K and the half steps 1 .. K that lead to
+// states 1 .. K are held whole, each array [K + 1][n].  The forces at the half
+// steps, their sigma derivatives, the objective's gradients at the states and
+// the fixed-point positions are held for a window of W <= K steps at a time
+// (kWindowBytes), [W + 1][n]; with them for all steps the longest segment that
+// fits the memory would be 2.7 times shorter.  The kernels take a window's D:
+// the whole arrays from its first state on, so that they count from 1 in both.
 struct D {
   double4_32a *q, *p;        // the initial state
   double4_32a *aq, *ap, *aqh, *tmp, *tmp2;
   double4_32a *ckq, *ckp;    // checkpoints
   float4 *qf;                // float copy of the segment's first state (the list test)
-  double4_32a *segq, *segp, *segqh, *segf, *segs, *segg;
-  FixPos *segxq, *segxqh;    // segq and segqh in fixed point (P.fixed)
+  double4_32a *segq, *segp, *segqh;   // of the segment
+  double4_32a *segf, *segs, *segg;    // of the window
+  FixPos *segxq, *segxqh;    // segq and segqh in fixed point (P.fixed), of the window
   uint32_t *nbr;             // the current segment's list, row-major [n][cap]
   int *cnt;
-  double *part;              // block partials, [K + 1][gridp][3]
+  double *part;              // block partials, [W + 1][gridp][3]
   double *acc;               // running sums: J, g_eps, g_sig
   int *flag;
   unsigned int *done;        // blocks of the current reduction that wrote their partials
@@ -842,6 +846,15 @@ __global__ void k_begin(P c, D d, const double4_32a *q, const double4_32a *p, do
   if (c.fixed) d.segxqh[at] = fix_position(a.x, a.y, a.z, 0);
 }
 
+// A window's first half step in fixed point, where the steps before it did not
+// leave it (k_begin and k_step write it within a window).
+__global__ void k_window(P c, D d) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c.n) return;
+  const double4_32a a = d.segqh[(size_t)c.n + i];
+  d.segxqh[(size_t)c.n + i] = fix_position(a.x, a.y, a.z, 0);
+}
+
 // The reverse of a step's second half-drift q_n = qh + dt/2 p_n for particle
 // i, from the adjoints a, b of (q_n, p_n): a_p += dt/2 a_q.  tmp receives the
 // adjoint of p after the kick (the neighbours' H v reads it), aqh that of qh.
@@ -1122,6 +1135,7 @@ struct mdg_adjoint {
   int grids = 1;   // the kernels over all states of a segment
   int gridb = 1;   // kBuildLanes threads per particle (list build)
   int nck = 0;
+  int window = 1;  // steps whose forces, derivatives and fixed-point positions are held
   char *slab = nullptr;  // every device array
   bool forward_done = false;
   // the device work of a forward and of a backward pass, captured once and
@@ -1142,45 +1156,61 @@ int afail(mdg_adjoint *a, int code, const std::string &m) {
     if (e_ != cudaSuccess) return afail(a, MDG_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-// Steps of a segment from its state 0 and first half-drift: states 1 .. len and
-// half steps 2 .. len (and the forces at the half steps).
-void run_segment(mdg_adjoint *a, int len, bool forces) {
+// The device's arrays as the window from state lo of the segment on sees them.
+D window(const mdg_adjoint *a, int lo) {
+  D d = a->d;
+  const size_t at = (size_t)a->c.n * lo;
+  d.segq += at;
+  d.segp += at;
+  d.segqh += at;
+  return d;
+}
+
+// Steps lo + 1 .. lo + m of a segment from its state lo and the half-drift that
+// follows it: states and half steps (and the forces at the half steps).  again:
+// the same steps once more, for what the window holds; they write the same
+// states.  The segment's list is built ahead of its first window.
+void run_steps(mdg_adjoint *a, int lo, int m, bool forces, bool again) {
   const size_t N = (size_t)a->c.n;
-  D &d = a->d;
-  k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, d.segq);
-  for (int k = 1; k <= len; k++) {
+  D d = window(a, lo);
+  if (lo == 0 && !again) k_build<<<a->gridb, kT, 0, a->s>>>(a->c, d, d.segq);
+  else if (a->c.fixed) k_window<<<a->grid, kT, 0, a->s>>>(a->c, d);
+  for (int k = 1; k <= m; k++) {
     const size_t at = N * k, before = N * (k - 1), after = N * (k + 1);
     double4_32a *f = forces ? d.segf + at : nullptr;
-    // half step len + 1 is written too, and not used
+    // the half step that follows the segment's last state is written too, and not used
     if (a->c.fixed)
       k_step<true><<<a->gridp, kT, 0, a->s>>>(a->c, d, d.segqh + at, d.segp + before, d.segq + at, d.segp + at, d.segqh + after,
-                                              d.segq, f, d.segxqh + at, d.segxq + at, d.segxqh + after);
+                                              a->d.segq, f, d.segxqh + at, d.segxq + at, d.segxqh + after);
     else
       k_step<false><<<a->gridp, kT, 0, a->s>>>(a->c, d, d.segqh + at, d.segp + before, d.segq + at, d.segp + at, d.segqh + after,
-                                               d.segq, f, nullptr, nullptr, nullptr);
+                                               a->d.segq, f, nullptr, nullptr, nullptr);
   }
 }
+
+// The longest window's arrays: 1 GB (4,000 particles 1,677 steps, 100,000 67).
+constexpr size_t kWindowBytes = (size_t)1 << 30;
 
 constexpr int kStates = 32768;  // states a launch (a grid's second dimension ends at 65,535)
 
 template <bool GRAD>
-void launch_objective(mdg_adjoint *a, int len, double w) {
+void launch_objective(mdg_adjoint *a, const D &d, int len, double w) {
   for (int first = 1; first <= len; first += kStates) {
     const dim3 grid(a->grids, len - first + 1 < kStates ? len - first + 1 : kStates);
     if (a->c.objective == 0) {
-      if (a->c.fixed) k_objective<0, GRAD, true><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
-      else k_objective<0, GRAD, false><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
+      if (a->c.fixed) k_objective<0, GRAD, true><<<grid, kT, 0, a->s>>>(a->c, d, w, first);
+      else k_objective<0, GRAD, false><<<grid, kT, 0, a->s>>>(a->c, d, w, first);
     } else {
-      if (a->c.fixed) k_objective<1, GRAD, true><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
-      else k_objective<1, GRAD, false><<<grid, kT, 0, a->s>>>(a->c, a->d, w, first);
+      if (a->c.fixed) k_objective<1, GRAD, true><<<grid, kT, 0, a->s>>>(a->c, d, w, first);
+      else k_objective<1, GRAD, false><<<grid, kT, 0, a->s>>>(a->c, d, w, first);
     }
   }
 }
 
-void launch_force_sigma(mdg_adjoint *a, int len) {
+void launch_force_sigma(mdg_adjoint *a, const D &d, int len) {
   for (int first = 1; first <= len; first += kStates) {
     const dim3 grid(a->grids, len - first + 1 < kStates ? len - first + 1 : kStates);
-    k_force_sigma<<<grid, kT, 0, a->s>>>(a->c, a->d, first);
+    k_force_sigma<<<grid, kT, 0, a->s>>>(a->c, d, first);
   }
 }
 
@@ -1197,8 +1227,11 @@ int enqueue_forward(mdg_adjoint *a) {
     const int len = Ns - start < K ? Ns - start : K;
     const size_t ck = N * (size_t)(start / K);
     k_begin<<<a->grid, kT, 0, a->s>>>(a->c, d, q, p, d.ckq + ck, d.ckp + ck, 1);
-    run_segment(a, len, false);
-    launch_objective<false>(a, len, 1.0 / Ns);
+    for (int lo = 0; lo < len; lo += a->window) {
+      const int m = std::min(a->window, len - lo);
+      run_steps(a, lo, m, false, false);
+      launch_objective<false>(a, window(a, lo), m, 1.0 / Ns);
+    }
     q = d.segq + N * len;
     p = d.segp + N * len;
   }
@@ -1206,9 +1239,10 @@ int enqueue_forward(mdg_adjoint *a) {
 }
 
 // Reverse of the horizon, segment by segment from the last: recompute the
-// segment from its checkpoint (with the same list), the objective's gradient at
-// all its states and the forces' sigma derivatives at all its half steps, then
-// reverse its steps.
+// segment from its checkpoint (with the same list), then window by window from
+// its last the objective's gradient at all states and the forces' sigma
+// derivatives at all half steps, and the reverse of the steps.  The windows
+// before the last run their steps once more for it.
 int enqueue_backward(mdg_adjoint *a) {
   const size_t N = (size_t)a->c.n, bytes = N * 32;
   D &d = a->d;
@@ -1222,17 +1256,23 @@ int enqueue_backward(mdg_adjoint *a) {
     const int len = seg_end - seg_start;
     const size_t ck = N * (size_t)(seg_start / K);
     k_begin<<<a->grid, kT, 0, a->s>>>(a->c, d, d.ckq + ck, d.ckp + ck, nullptr, nullptr, 0);
-    run_segment(a, len, true);
-    launch_objective<true>(a, len, w);
-    if (a->c.fixed) launch_force_sigma(a, len);
-    double4_32a *tmp = d.tmp, *tmp_alt = d.tmp2;
-    k_seed<<<a->grid, kT, 0, a->s>>>(a->c, d, len, w, tmp);
-    for (int k = len; k >= 1; k--) {
-      if (a->c.fixed) k_reverse<true><<<a->gridp, kT, 0, a->s>>>(a->c, d, k, tmp, w, tmp_alt);
-      else k_reverse<false><<<a->gridp, kT, 0, a->s>>>(a->c, d, k, tmp, w, tmp_alt);
-      std::swap(tmp, tmp_alt);
+    const int last = (len - 1) / a->window * a->window;
+    for (int lo = 0; lo < last; lo += a->window) run_steps(a, lo, a->window, false, false);
+    for (int lo = last; lo >= 0; lo -= a->window) {
+      const int m = std::min(a->window, len - lo);
+      const D dw = window(a, lo);
+      run_steps(a, lo, m, true, lo < last);
+      launch_objective<true>(a, dw, m, w);
+      if (a->c.fixed) launch_force_sigma(a, dw, m);
+      double4_32a *tmp = d.tmp, *tmp_alt = d.tmp2;
+      k_seed<<<a->grid, kT, 0, a->s>>>(a->c, dw, m, w, tmp);
+      for (int k = m; k >= 1; k--) {
+        if (a->c.fixed) k_reverse<true><<<a->gridp, kT, 0, a->s>>>(a->c, dw, k, tmp, w, tmp_alt);
+        else k_reverse<false><<<a->gridp, kT, 0, a->s>>>(a->c, dw, k, tmp, w, tmp_alt);
+        std::swap(tmp, tmp_alt);
+      }
+      k_reverse_sums<<<1, 1024, 0, a->s>>>(d, m, a->gridp);
     }
-    k_reverse_sums<<<1, 1024, 0, a->s>>>(d, len, a->gridp);
     seg_end = seg_start;
   }
   return cudaGetLastError() == cudaSuccess ? MDG_OK : afail(a, MDG_ERR_CUDA, "adjoint backward launch failed");
@@ -1351,25 +1391,39 @@ int mdg_adjoint_create(const mdg_adjoint_params *p, int32_t n, mdg_adjoint **out
   cudaError_t e = cudaSetDevice(p->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&a->s, cudaStreamNonBlocking);
   const size_t X = c.fixed ? N : 0;
+  const size_t step_bytes = N * (c.fixed ? 160 : 64);
+  size_t W = std::max<size_t>(1, std::min(K, kWindowBytes / step_bytes));
   for (int pass = 0; pass < 2 && e == cudaSuccess; pass++) {
     mdg::Slab s;
     s.base = a->slab;
     for (auto v : {&d.q, &d.p, &d.aq, &d.ap, &d.aqh, &d.tmp, &d.tmp2}) s.take(v, N);
     s.take(&d.ckq, N * a->nck);
     s.take(&d.ckp, N * a->nck);
-    for (auto v : {&d.segq, &d.segp, &d.segf, &d.segs, &d.segg}) s.take(v, N * (K + 1));
+    for (auto v : {&d.segq, &d.segp}) s.take(v, N * (K + 1));
     s.take(&d.segqh, N * (K + 2));
-    s.take(&d.segxq, X * (K + 1));
-    s.take(&d.segxqh, X * (K + 2));
+    for (auto v : {&d.segf, &d.segg}) s.take(v, N * (W + 1));
+    s.take(&d.segs, X * (W + 1));
+    s.take(&d.segxq, X * (W + 1));
+    s.take(&d.segxqh, X * (W + 2));
     s.take(&d.nbr, N * (size_t)c.cap);
     s.take(&d.cnt, N);
     s.take(&d.qf, N);
-    s.take(&d.part, 3 * (size_t)std::max(a->gridp, a->grids) * (K + 1));
+    s.take(&d.part, 3 * (size_t)std::max(a->gridp, a->grids) * (W + 1));
     s.take(&d.acc, 3);
     s.take(&d.flag, 2);
     s.take(&d.done, 1);
-    if (pass == 0) e = cudaMalloc((void **)&a->slab, s.used);
+    if (pass == 0) {
+      e = cudaMalloc((void **)&a->slab, s.used);
+      if (e == cudaErrorMemoryAllocation && W > 1) {  // what is left beside the segment itself
+        cudaGetLastError();
+        e = cudaSuccess;
+        a->slab = nullptr;
+        W = (W + 1) / 2;
+        pass = -1;
+      }
+    }
   }
+  a->window = (int)W;
   if (e == cudaSuccess) e = cudaMemset(d.done, 0, sizeof(unsigned int));
   if (e != cudaSuccess) {
     fprintf(stderr, "mdg_adjoint_create: %s\n", cudaGetErrorString(e));
