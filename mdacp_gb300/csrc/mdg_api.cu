@@ -482,7 +482,7 @@ int capture(mdg_handle *h, cudaGraphExec_t *out, int par, int nsteps, cudaEvent_
 
 // Whether the handle's steps run in the resident kernel.
 bool resident(const mdg_handle *h) {
-  return h->prm.use_graphs && !h->resident_off && mdg::resident_box(h->g, h->prm.precision, h->num_sms);
+  return h->prm.use_graphs && h->prm.use_graphs != 2 && !h->resident_off && mdg::resident_box(h->g, h->prm.precision, h->num_sms);
 }
 
 int enqueue_steps(mdg_handle *h, int nsteps) {

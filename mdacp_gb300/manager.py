@@ -49,7 +49,8 @@ class MDManager:
         prm.langevin_half_drift_compat = 1 if langevin_half_drift_compat else 0
         prm.list_capacity = int(list_capacity)
         prm.device = int(device)
-        prm.use_graphs = 1 if use_graphs else 0
+        # 2: step graphs also where a small box would run in one resident launch
+        prm.use_graphs = 2 if use_graphs == 2 else (1 if use_graphs else 0)
         if prune_buffer is not None:
             prm.prune_buffer = float(prune_buffer)
         prm.rebuild_policy = native.REBUILD_POLICIES[rebuild_policy]
