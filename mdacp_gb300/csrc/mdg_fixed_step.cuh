@@ -86,6 +86,7 @@ __device__ __forceinline__ void walk_fixed(const Geom &g, const Dev &d, const Fi
 #pragma unroll
       for (int u = 0; u < kInFlight; u++) {
         e[u] = en[u];
+        if (!MDG_IN_RANGE(d.flags, SITE, entry_slot(e[u]), g.n)) e[u] = none;
         q[u] = ld_fix<COH>(xq + entry_slot(e[u]));
       }
 #pragma unroll

@@ -180,6 +180,7 @@ __device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, Resid
   for (int i = tid; i < g.n; i += nt) {
     const int cell = rank_of(d.cell[i]);
     const int dst = d.cell_start[cell] + atomicAdd(&d.cell_fill[cell], 1);
+    if (!MDG_IN_RANGE(f, kCheckScatter, dst, g.n)) continue;
     d.order[dst] = i;
     d.t_id[dst] = d.id[i];
   }
@@ -189,6 +190,7 @@ __device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, Resid
     const int a = d.cell_start[cell], b = d.cell_start[cell + 1];
     int at = a;
     for (int m = a; m < b; m++) at += d.t_id[m] < id ? 1 : 0;
+    if (!MDG_IN_RANGE(f, kCheckScatter, at, g.n)) continue;
     double4_32a q = d.q_end[i];
     // index and home cell ride in the padding lane
     q.w = __longlong_as_double((long long)(((unsigned long long)(unsigned)key << 32) | (unsigned)id));
@@ -201,6 +203,7 @@ __device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, Resid
     const unsigned long long w = (unsigned long long)__double_as_longlong(q.w);
     q.w = 0.0;
     const int id = (int)(unsigned)w, key = (int)(unsigned)(w >> 32);
+    if (!MDG_IN_RANGE(f, kCheckScatter, id, g.n)) continue;
     if (g.local_pos) finalize_one<true, false>(g, d, k, q, d.t_p[k], id, key, r.par);
     else finalize_one<false, true>(g, d, k, q, d.t_p[k], id, key, r.par);  // an FP64 box here is in fixed point
   }
@@ -305,16 +308,17 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_resident(co
   constexpr int kThreads = THREADS;
   DevFlags *f = d.flags;
   // the flags of the state before this launch: nobody writes them until its end
-  // (a halt is set in the rebuild only, between barriers)
+  // (a halt is set in the rebuild only, between barriers; by a failed check
+  // anywhere, and read after the next rebuild's first barrier)
   if (*(volatile int *)&f->halt != 0) return;
   Run r{0u, f->end_stale != 0, par};
   bool rebuild = f->rebuild != 0, reselect = f->prune_next != 0;
   const unsigned long long lang0 = f->lang;
   double zeta = f->zeta, zeta_a = f->zeta_a, exp1 = f->exp1, T = f->t_cur;
   unsigned long long rebuilds = 0, prunes = 0;
-  // a rebuild of the first step may set the halt before its first barrier:
-  // not before every block has read it above
-  bool halted = false, lost = rebuild && !grid_barrier(c, ++r.barriers);
+  // a rebuild of the first step may set the halt before its first barrier (and a
+  // checked build any step): not before every block has read it above
+  bool halted = false, lost = (rebuild || kCheck) && !grid_barrier(c, ++r.barriers);
   const int lo = min((int)blockIdx.x * share, g.n), hi = min(lo + share, g.n);
   const bool first = blockIdx.x == 0 && threadIdx.x == 0;
   int s = 0, selected = -1;  // slot of the last selection's row total
@@ -468,7 +472,7 @@ int threads_of(const Geom &g, int precision, int num_sms) {
 size_t resident_ctl_bytes() { return sizeof(ResidentCtl); }
 
 bool resident_box(const Geom &g, int precision, int num_sms) {
-  return !kCheck && g.rebuild_policy == MDG_REBUILD_HALFMARGIN && (precision != MDG_FP64 || g.fixed) && num_sms <= 2048 &&
+  return g.rebuild_policy == MDG_REBUILD_HALFMARGIN && (precision != MDG_FP64 || g.fixed) && num_sms <= 2048 &&
          g.n <= (precision == MDG_FP64 ? kResidentFixed : kResidentMixed) * num_sms;
 }
 
