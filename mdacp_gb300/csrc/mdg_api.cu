@@ -235,14 +235,22 @@ int estimate_list_cap(const mdg_handle *h, int n) {
   return (cap + 7) & ~7;
 }
 
+// Rows of list_cap entries.  Where the memory is too short the handle is left
+// with rows of none: its next build overflows and comes here again, and nothing
+// reads or writes a row meanwhile.
 int alloc_list(mdg_handle *h, int list_cap) {
   if (h->d.nl) cudaFree(h->d.nl);
   if (h->d.pl) cudaFree(h->d.pl);
   h->d.nl = h->d.pl = nullptr;
-  MDG_CK(dalloc(&h->d.nl, (size_t)list_cap * (size_t)h->cap));
-  MDG_CK(dalloc(&h->d.pl, (size_t)list_cap * (size_t)h->cap));
-  h->g.list_cap = list_cap;
+  h->g.list_cap = 0;
   drop_graphs(h);
+  cudaError_t e = dalloc(&h->d.nl, (size_t)list_cap * (size_t)h->cap);
+  if (e == cudaSuccess) e = dalloc(&h->d.pl, (size_t)list_cap * (size_t)h->cap);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(h, MDG_ERR_CUDA, std::string("neighbour list: ") + cudaGetErrorString(e));
+  }
+  h->g.list_cap = list_cap;
   return MDG_OK;
 }
 
@@ -736,6 +744,7 @@ const char *mdg_last_error(const mdg_handle *h) {
 
 static int set_state_common(mdg_handle *h, int32_t n) {
   h->g.n = n;
+  h->has_state = false;  // until the list is there
   if (!h->d.nl || h->prm.list_capacity > 0 || h->g.list_cap < 8) {
     int lc = h->prm.list_capacity > 0 ? ((h->prm.list_capacity + 7) & ~7) : estimate_list_cap(h, n);
     if (!h->d.nl || lc != h->g.list_cap) {

@@ -1347,6 +1347,8 @@ int assign(mdg_batch *b) {
 }
 
 // (Re)allocates the list pool for capacity `cap` and uploads box descriptors.
+// Where the memory is too short the boxes are left with rows of no entries:
+// their next builds overflow and come here again.
 int alloc_batch_list(mdg_batch *b, int cap) {
   long long off = 0;
   for (auto &bx : b->boxes) {
@@ -1356,14 +1358,19 @@ int alloc_batch_list(mdg_batch *b, int cap) {
   if (b->d.nl) cudaFree(b->d.nl);
   if (b->d.pl) cudaFree(b->d.pl);
   b->d.nl = b->d.pl = nullptr;
-  MDG_BCK(balloc(&b->d.nl, (size_t)off));
-  if (b->P.inner) MDG_BCK(balloc(&b->d.pl, (size_t)off));
-  b->P.list_cap = cap;
+  b->P.list_cap = 0;
   b->lists_due = true;
+  drop_batch_graphs(b);
   MDG_BCK(cudaMemcpy(b->d.boxes, b->boxes.data(), b->nbox * sizeof(BoxDesc), cudaMemcpyHostToDevice));
   std::vector<int> ones(b->nbox, 1);
   MDG_BCK(cudaMemcpy(b->d.box_rebuild, ones.data(), b->nbox * sizeof(int), cudaMemcpyHostToDevice));
-  drop_batch_graphs(b);
+  cudaError_t e = balloc(&b->d.nl, (size_t)off);
+  if (e == cudaSuccess && b->P.inner) e = balloc(&b->d.pl, (size_t)off);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return bfail(b, MDG_ERR_CUDA, std::string("neighbour lists: ") + cudaGetErrorString(e));
+  }
+  b->P.list_cap = cap;
   return MDG_OK;
 }
 
