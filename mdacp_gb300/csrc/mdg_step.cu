@@ -168,7 +168,8 @@ __global__ void __launch_bounds__(kStepThreads) k_kinetic(Geom g, Dev d) {
 // Observers at the step-boundary positions q_end: kinetic energy
 // (observer.cc:5-15), pair energy (observer.cc:17-48) and virial
 // (observer.cc:50-79), each pair evaluated with the reference's expression
-// and rounding and weighted 1/2 (each pair is listed from both sides).
+// and rounding and weighted 1/2 (each pair is listed from both sides).  The FP64
+// form outside the fixed-point range (k_observe_fixed is the others').
 __global__ void __launch_bounds__(kStepThreads) k_observe(Geom g, Dev d) {
   __shared__ double sh[kStepThreads / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -191,8 +192,7 @@ __global__ void __launch_bounds__(kStepThreads) k_observe(Geom g, Dev d) {
 // Mixed-form observers: the same sums with each pair's energy and virial
 // term evaluated in float (from the home-cell-local float positions of q_end,
 // as the mixed force) and summed over the row in compensated float, walked
-// like the step kernel's row; the rows are added in double.  The FP64 form
-// keeps k_observe's reference rounding.
+// like the step kernel's row; the rows are added in double.
 template <bool EDGE>
 __device__ __forceinline__ void observe_row(const Geom &g, const Dev &d, const float4 *__restrict__ loc, int i,
                                             const float4 &li, const CellPos &cp, int cnt, double &pe, double &vir) {
