@@ -63,7 +63,8 @@ constexpr int kLanes = 8;
 // The same in fixed point, for the kernels of one step (8 / 16 / 32 lanes: 7.7 /
 // 5.8 / 5.3 ms per gradient of 864 atoms over 200 steps, 10.4 / 10.0 / 12.1 of
 // 4,000, 33.2 / 34.6 / 44.2 of 16,384: more lanes shorten a row's chain where
-// the rows don't fill the GPU).
+// the rows don't fill the GPU; one value for all, the middle one's best, within
+// 9 % of each size's own).
 constexpr int kStepLanes = 16;
 // Lanes per particle of the fixed-point kernels that take all states of a
 // segment in one launch (1 / 2 / 4 lanes: 11.4 / 11.1 / 11.3 ms per gradient of

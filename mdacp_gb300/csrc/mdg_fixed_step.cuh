@@ -16,12 +16,15 @@ constexpr int kPairsPerTrip = 2;
 // 70,304 atoms, us per step: 2 8.1 / 17.8 / 35.9, 3 8.4 / 18.7 / 36.4, 4 8.9 / 19.3 / 37.3).
 constexpr int kInFlight = 2;
 
-// Lanes per particle for n particles outside the resident kernel.  A row's pairs take about half a
-// microsecond one after the other, so a GPU that one thread per particle does
-// not fill (152 SMs x 24 warps) is better used by several: step kernel of 864
-// atoms 34.0, 26.2, 21.7, 19.1 us with 1, 2, 4, 8 lanes; 32,000 atoms 32.3,
-// 28.3, 30.8, 36.1; 256,000 atoms 141, 187, 229, 304 (of which about 8 us are
-// the graph's hand-over).
+// Lanes per particle for n particles outside the resident kernel.  A row's
+// pairs take about half a microsecond one after the other, so a GPU that one
+// thread per particle does not fill (152 SMs x 24 warps) is better used by
+// several.  Step kernel with 1 / 2 / 8 / 32 lanes, us (density 0.6): 864 atoms 29.9 /
+// 23.9 / 19.0 / 17.5, 2,400 31.3 / 24.7 / 18.9 / 18.8, 5,000 31.4 / 24.7 / 19.9 / 25.7, 9,700
+// 31.8 / 24.9 / 20.4 / 32.0, 16,000 31.8 / 25.3 / 25.9, 38,900 34.4 / 29.9 / 38.5, 64,000
+// 45.5 / 43.5, 110,000 57.8 / 57.8 (two lanes still gain a little where the line puts
+// one; by 256,000 they cost 187 for 141).  The lines are 16, 64 and 256 particles
+// per SM of 152.
 inline int fx_lanes(int n) { return n < 2432 ? 32 : (n < 9728 ? 8 : (n < 38912 ? 2 : 1)); }
 
 // Image shifts of a particle at the box faces: per axis the step code (after
