@@ -5,7 +5,7 @@
 // atoms FP64: 24 us per single-step call, of which 11 are the step kernel;
 // 108,000 atoms mixed: 50 us for a 30 us kernel), and a rebuild is ten
 // launches.  Here one cooperative launch runs all steps of an mdg_calculate
-// call: at most one block per SM, each with its share of the slots, a grid barrier
+// call: one block per SM, each with its share of the slots, a grid barrier
 // after every step, and the rebuild as phases between further barriers.  The
 // particles' arithmetic is the step kernels' own (step_one, force_mixed,
 // step_one_fixed, force_fixed; finalize_one, build_slot_row and build_cell_rows
@@ -38,9 +38,8 @@ namespace {
 
 constexpr int kFixedForm = 3;  // template value beside MDG_MIXED and MDG_MIXED_PLAIN
 
-// Threads of a block: 512 (128 registers), or for the mixed forms 256 of as many
-// registers where a row each is enough (threads_of), and of boxes with more
-// particles than 512 per SM 1024 (64).  With 512 or fewer the mixed
+// Threads of the one block per SM: 512 (128 registers), or for the mixed forms
+// of boxes with more particles than 512 per SM 1024 (64).  With 512 the mixed
 // row walk has kFewUnroll gathers in flight (864 / 16,384 / 70,304 atoms, us
 // per step: 4 10.2 / 13.7 / 18.5, 8 9.2 / 12.7 / 19.2, 16 11.1 / 15.3 / 22.1;
 // 1024 threads 14.3 / 18.9 / 23.8).
@@ -285,7 +284,7 @@ __device__ __forceinline__ double resident_step(const Geom &g, const Dev &d, int
     for (int i = lo + threadIdx.x; i < hi; i += kThreads) {
       int kept = 0;
       const float4 lb = ld_ro<true>(d.loc[par] + i);
-      const double3 F = force_mixed<PRUNE, FORM == MDG_MIXED, true, THREADS <= 512 ? kFewUnroll : kUnroll>(g, d, d.loc[par], i, lb, cell_pos_packed(g, lb.w), list,
+      const double3 F = force_mixed<PRUNE, FORM == MDG_MIXED, true, THREADS == 512 ? kFewUnroll : kUnroll>(g, d, d.loc[par], i, lb, cell_pos_packed(g, lb.w), list,
                                                                     counts, &kept);
       ke += step_one<THERMO, COMPAT, FORM>(g, d, par, i, PRUNE, kept, F, lb, d.q_mid[par], d.q_mid[par ^ 1], exp1, lang, rebuild,
                                            reselect);
@@ -302,7 +301,7 @@ __device__ __forceinline__ double resident_step(const Geom &g, const Dev &d, int
 }
 
 template <int FORM, int THERMO, int COMPAT, int LANES, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_resident(const __grid_constant__ Geom g,
+__global__ void __launch_bounds__(THREADS, 1) k_resident(const __grid_constant__ Geom g,
                                                                       const __grid_constant__ Dev d, ResidentCtl *c, int par,
                                                                       int nsteps, int share) {
   constexpr int kThreads = THREADS;
@@ -446,29 +445,6 @@ Kernel kernel_of(int thermostat, int compat) {
 // 108,000 27.1 / 39.3, 157,216 47.1 / 48.1, 256,000 54.9 / 66.7, 389,344 84.9 / 89.7.
 constexpr int kResidentFixed = 512, kResidentMixed = 2048;
 
-// A block of 512 threads takes an SM's registers and the launch all its blocks'
-// SMs at once, so boxes whose launches fill the GPU step one after the other
-// where a program has several handles.  In the mixed forms, whose steps by graphs
-// overlap well, a launch leaves room instead: at least kRowsPerBlock particles a
-// block (a warp on each sub-partition; 128 alone take as long as 32), which
-// lets boxes of up to 9,728 particles share the SMs out, and above that 256
-// threads a block, two of which fit an SM.  us per step of all handles, density
-// 0.6, dt 0.002, one handle / four / eight, now (before: 32 particles a block, 512
-// threads; step graphs): 864 9.7 / 9.9 / 10.0 (9.4 / 9.8 / 16.7; 30 / 40 / 80), 4,000 10.3 /
-// 10.5 / 20.8 (10.2 / 40.7 / 81.8; 32 / 39 / 78), 8,000 10.9 / 21.9 / 44.0 (11.0 / 43.5 / 86.7; 34 /
-// 42 / 83), 16,384 11.5 / 27.8 / 56.1 (11.4 / 43.9 / 90.4; 34 / 42 / 85), 32,000 14.2 / 37.9 / 74.9
-// (14.3 / 57.2 / 114; 35 / 47 / 93).  The rebuild has fewer threads for it: at dt
-// 0.005 one handle of 16,384 17.5 (16.4), of 32,000 22.2 (21.7).  Larger boxes keep a
-// thread a row: four handles of 108,000 111 us (graphs 79), one 27.7 (39.5); the
-// step graphs alone are the caller's choice (use_graphs).  FP64 handles side by
-// side are faster than their graphs at every size (four of 32,000 95 us, 272).
-constexpr int kRowsPerBlock = 128;
-int threads_of(const Geom &g, int precision, int num_sms) {
-  if (precision == MDG_FP64) return 512;
-  if (2 * g.n <= kRowsPerBlock * num_sms) return 512;
-  return g.n <= 256 * num_sms ? 256 : g.n <= 512 * num_sms ? 512 : 1024;
-}
-
 size_t resident_ctl_bytes() { return sizeof(ResidentCtl); }
 
 bool resident_box(const Geom &g, int precision, int num_sms) {
@@ -479,10 +455,10 @@ bool resident_box(const Geom &g, int precision, int num_sms) {
 cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int nsteps, int thermostat, int compat, int precision,
                             int num_sms, cudaStream_t s) {
   Kernel k;
-  const int threads = threads_of(g, precision, num_sms);
-  int lanes = 1, share = (g.n + num_sms - 1) / num_sms;
+  int threads = 512, lanes = 1;
   if (precision == MDG_FP64) {
     // as many lanes as the block has threads for
+    const int share = (g.n + num_sms - 1) / num_sms;
     while (lanes < 32 && 2 * lanes * share <= threads) lanes *= 2;
     k = lanes == 32   ? kernel_of<kFixedForm, 32, 512>(thermostat, compat)
         : lanes == 16 ? kernel_of<kFixedForm, 16, 512>(thermostat, compat)
@@ -490,19 +466,17 @@ cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int
         : lanes == 4  ? kernel_of<kFixedForm, 4, 512>(thermostat, compat)
         : lanes == 2  ? kernel_of<kFixedForm, 2, 512>(thermostat, compat)
                       : kernel_of<kFixedForm, 1, 512>(thermostat, compat);
+  } else if (g.n <= 512 * num_sms) {
+    k = precision == MDG_MIXED ? kernel_of<MDG_MIXED, 1, 512>(thermostat, compat)
+                               : kernel_of<MDG_MIXED_PLAIN, 1, 512>(thermostat, compat);
   } else {
-    share = share < kRowsPerBlock ? kRowsPerBlock : share;
-    if (precision == MDG_MIXED)
-      k = threads == 256   ? kernel_of<MDG_MIXED, 1, 256>(thermostat, compat)
-          : threads == 512 ? kernel_of<MDG_MIXED, 1, 512>(thermostat, compat)
-                           : kernel_of<MDG_MIXED, 1, 1024>(thermostat, compat);
-    else
-      k = threads == 256   ? kernel_of<MDG_MIXED_PLAIN, 1, 256>(thermostat, compat)
-          : threads == 512 ? kernel_of<MDG_MIXED_PLAIN, 1, 512>(thermostat, compat)
-                           : kernel_of<MDG_MIXED_PLAIN, 1, 1024>(thermostat, compat);
+    threads = 1024;
+    k = precision == MDG_MIXED ? kernel_of<MDG_MIXED, 1, 1024>(thermostat, compat)
+                               : kernel_of<MDG_MIXED_PLAIN, 1, 1024>(thermostat, compat);
   }
   // whole warps of particles per block
   const int unit = 32 / lanes;
+  int share = (g.n + num_sms - 1) / num_sms;
   share = (share + unit - 1) / unit * unit;
   int grid = (g.n + share - 1) / share;
   Geom gg = g;
