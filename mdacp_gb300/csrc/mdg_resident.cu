@@ -53,7 +53,7 @@ constexpr int kResidentTile = 4;
 // 0.005 (a rebuild every 14 to 20 steps): 864 atoms 10.20 with nine lanes, 10.62
 // with the warps; 32,000 atoms FP64 34.7 with a thread per row, 32.7 with the
 // warps; 108,000 mixed 38.7 and 38.4 (39.0 with one warp a cell).
-__host__ __device__ __forceinline__ bool lanes_per_row(int n, long long threads) { return (long long)n * kRowLanes <= 2 * threads; }
+bool lanes_per_row(int n, long long threads) { return (long long)n * kRowLanes <= 2 * threads; }
 
 // About two seconds of polling; a barrier is reached within microseconds.
 constexpr int kPollLimit = 1 << 22;
@@ -111,7 +111,7 @@ struct Run {
 // halted (or a barrier failed).  Slots are sorted by cell and, in a cell, by
 // caller index, as there: here each particle counts the smaller indices in its
 // cell instead of sorting the cell.
-__device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, ResidentCtl *c, Run &r) {
+__device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, ResidentCtl *c, Run &r, int row_lanes) {
   DevFlags *f = d.flags;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
   __shared__ int sh[32];
@@ -212,7 +212,7 @@ __device__ __noinline__ bool resident_rebuild(const Geom &g, const Dev &d, Resid
   // twice over, else a warp per cell, or two or four of few cells
   const int wl = threadIdx.x & 31, warp = tid >> 5, warps = nt >> 5;
   int pairs = 0, longest = 0;
-  if (lanes_per_row(g.n, nt)) {
+  if (row_lanes) {
     const int per = 32 / kRowLanes, k = wl / kRowLanes, lane = wl % kRowLanes;
     for (int i0 = warp * per; i0 < g.n; i0 += warps * per) {
       const int i = i0 + k;
@@ -303,7 +303,7 @@ __device__ __forceinline__ double resident_step(const Geom &g, const Dev &d, int
 template <int FORM, int THERMO, int COMPAT, int LANES, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_resident(const __grid_constant__ Geom g,
                                                                       const __grid_constant__ Dev d, ResidentCtl *c, int par,
-                                                                      int nsteps, int share) {
+                                                                      int nsteps, int share, int row_lanes) {
   constexpr int kThreads = THREADS;
   DevFlags *f = d.flags;
   // the flags of the state before this launch: nobody writes them until its end
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_resident(const __grid_constant__
       selected = -1;
     }
     if (rebuild) {
-      if (!resident_rebuild(g, d, c, r)) {
+      if (!resident_rebuild(g, d, c, r, row_lanes)) {
         halted = true;
         break;
       }
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_resident(const __grid_constant__
   c->arrived = 0;
 }
 
-using Kernel = void (*)(const Geom, const Dev, ResidentCtl *, int, int, int);
+using Kernel = void (*)(const Geom, const Dev, ResidentCtl *, int, int, int, int);
 
 template <int FORM, int LANES, int THREADS>
 Kernel kernel_of(int thermostat, int compat) {
@@ -444,6 +444,28 @@ Kernel kernel_of(int thermostat, int compat) {
 // over the block's 512 threads); mixed 864 9.2 / 28.6, 32,000 14.6 / 33.9,
 // 108,000 27.1 / 39.3, 157,216 47.1 / 48.1, 256,000 54.9 / 66.7, 389,344 84.9 / 89.7.
 constexpr int kResidentFixed = 512, kResidentMixed = 2048;
+
+// Particles per block at least.  A block of 512 threads has an SM's registers to
+// itself, so launches of several handles run side by side only where they leave
+// SMs over.  In the mixed forms, whose step graphs overlap well, boxes of 16 to 32
+// particles per SM take 64 a block (their lists then by a warp per cell), of more than 40
+// 96: that costs one handle nothing (5,000, between them, would take 1-3 % longer).  us
+// per step of all handles, density 0.6, dt 0.002, one / four / eight, now (with 32 a
+// block; step graphs): 864 9.6 / 9.7 / 16.7 (the same; 30 / 40 / 79), 4,000 9.9 / 19.8 / 39.6
+// (10.2 / 40.7 / 81; 32 / 39 / 78), 7,200 10.3 / 20.8 / 42 (10.9 / 42.5 / 86; 34 / 41 / 82); one
+// handle of 4,000 at dt 0.005 13.8 (14.2).
+// From about 7,300 particles on a launch fills the GPU and handles take turns: 8,000
+// 43.9 / 87 (four, eight; graphs 41 / 83), 32,000 57 / 115 (47 / 93), 108,000 111 / 221 (79 /
+// 158), one handle 10.8, 14.4 and 27.7 (34, 35 and 40): several of those at once step
+// faster by graphs, which is the caller's choice (use_graphs = 2).  Blocks of 256
+// threads, two an SM, made four of 32,000 38, but one handle 2-6 % slower where lists are
+// rebuilt every 15 steps.  FP64 handles side by side are faster than their graphs at
+// every size (four of 32,000 95, 272).
+int rows_per_block(const Geom &g, int precision, int num_sms) {
+  if (precision == MDG_FP64) return 1;
+  if (g.n > 40 * num_sms) return 96;
+  return g.n > 16 * num_sms && g.n <= 32 * num_sms ? 64 : 32;
+}
 
 size_t resident_ctl_bytes() { return sizeof(ResidentCtl); }
 
@@ -476,15 +498,18 @@ cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int
   }
   // whole warps of particles per block
   const int unit = 32 / lanes;
+  const int least = rows_per_block(g, precision, num_sms);
   int share = (g.n + num_sms - 1) / num_sms;
+  if (share < least) share = least;
   share = (share + unit - 1) / unit * unit;
   int grid = (g.n + share - 1) / share;
   Geom gg = g;
   Dev dd = d;
   ResidentCtl *c = static_cast<ResidentCtl *>(ctl);
-  void *args[] = {&gg, &dd, &c, &par, &nsteps, &share};
+  int row_lanes = least != 64 && lanes_per_row(g.n, (long long)grid * threads) ? 1 : 0;
+  void *args[] = {&gg, &dd, &c, &par, &nsteps, &share, &row_lanes};
   size_t shared = 0;
-  if (!lanes_per_row(g.n, (long long)grid * threads)) {
+  if (!row_lanes) {
     shared = threads / 32 * sizeof(CellRows<kResidentTile>);
     if (shared > 48 * 1024) {
       const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
