@@ -73,9 +73,10 @@ typedef struct mdg_params {
   int32_t list_capacity;   /* neighbour slots per particle; 0 = sized from the first build */
   int32_t device;          /* CUDA device ordinal */
   int32_t use_graphs;      /* 1 (default) = replay steps as CUDA graphs, those of a small box in
-                              one resident launch per call; 2 = by graphs whatever the size
-                              (for programs that run several boxes of more than 7,000
-                              particles in mixed precision side by side); 0 = plain launches */
+                              one resident launch per call (beside other handles with steps
+                              outstanding a narrower one or, in mixed precision from 256
+                              particles per SM on, by graphs: the same trajectory);
+                              2 = by graphs whatever the size; 0 = plain launches */
   int32_t rebuild_policy;  /* mdg_rebuild_policy (.cfg RebuildPolicy), default HALFMARGIN */
   double prune_buffer;     /* inner-list buffer: the force kernels walk the pairs within
                               cutoff + prune_buffer, re-selected from the list whenever a

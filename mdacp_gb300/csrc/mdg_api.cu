@@ -10,6 +10,8 @@
 // list is regrown and the run continues from that step.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -46,9 +48,17 @@ struct mdg_handle {
   long long steps_host = 0;  // completed steps as last read from the device
   long long launches = 0;    // kernels enqueued (counting every node of a graph replay)
   long long pending = 0;     // steps enqueued by mdg_calculate and not yet confirmed
+  long long by_graph = 0;    // of them by step graphs
+  bool outstanding = false;  // counted in g_outstanding
   int evaluations = 0;       // observations and force evaluations (launch_observe, launch_forces)
   bool ev1_due = false;      // the timing end event is recorded when the steps are confirmed
 };
+
+// Handles of each device with steps that mdg_calculate left outstanding: what a
+// small box's launch may find beside it.  Which of two equal ways a call takes is
+// all that it decides.
+constexpr int kCountedDevices = 64;
+static std::atomic<int> g_outstanding[kCountedDevices];
 
 // Steps mdg_calculate may leave enqueued before it waits for them.
 constexpr long long kMaxPending = 1024;
@@ -493,12 +503,36 @@ bool resident(const mdg_handle *h) {
   return h->prm.use_graphs && h->prm.use_graphs != 2 && !h->resident_off && mdg::resident_box(h->g, h->prm.precision, h->num_sms);
 }
 
+void mark_outstanding(mdg_handle *h, bool on) {
+  if (on == h->outstanding || h->prm.device < 0 || h->prm.device >= kCountedDevices) return;
+  g_outstanding[h->prm.device].fetch_add(on ? 1 : -1);
+  h->outstanding = on;
+}
+
+// Other handles of the device with steps outstanding.
+int others_outstanding(const mdg_handle *h) {
+  if (h->prm.device < 0 || h->prm.device >= kCountedDevices) return 0;
+  return g_outstanding[h->prm.device].load() - (h->outstanding ? 1 : 0);
+}
+
+// Whether a box that would take the resident kernel steps faster by graphs beside
+// `others` handles like it: mixed forms of more than 256 particles per SM, whose launch
+// has no narrow form (mdg_resident.cu).  us per step of two / three / four handles in
+// turn and by graphs: 70,000 particles 40 / 60 / 79 and 50 / 56 / 62, 108,000 55 / 83 / 111
+// and 57 / 68 / 79, 160,000 92 / 137 / 183 and 75 / 92 / 108.
+bool crowded(const mdg_handle *h, int others) {
+  if (h->prm.precision == MDG_FP64 || h->prm.thermostat == MDG_NOSEHOOVER || h->g.n <= 256 * h->num_sms) return false;
+  return others >= (h->g.n <= 1000 * h->num_sms ? 2 : 1);
+}
+
 int enqueue_steps(mdg_handle *h, int nsteps) {
   int par = h->par;
-  while (nsteps > 0 && resident(h)) {
+  const int others = others_outstanding(h);
+  const bool in_kernel = resident(h) && !crowded(h, others);
+  while (nsteps > 0 && in_kernel && !h->resident_off) {
     const int m = nsteps < kResidentSteps ? nsteps : kResidentSteps;
     const cudaError_t e = mdg::launch_resident(h->g, h->d, h->ctl, par, m, h->prm.thermostat, h->prm.langevin_half_drift_compat,
-                                               h->prm.precision, h->num_sms, h->stream);
+                                               h->prm.precision, h->num_sms, others > 0, h->stream);
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
       cudaGetLastError();  // fewer SMs than the device has (a partition): the graphs
       h->resident_off = true;
@@ -521,6 +555,7 @@ int enqueue_steps(mdg_handle *h, int nsteps) {
     return cudaGetLastError() == cudaSuccess ? MDG_OK : fail(h, MDG_ERR_CUDA, "kernel launch failed");
   }
   int left = nsteps;
+  h->by_graph += nsteps;
   if (left >= 2) {
     if (!h->gx_pair[par]) {
       int rc = capture(h, &h->gx_pair[par], par, 2);
@@ -550,6 +585,13 @@ int settle(mdg_handle *h) {
   if (h->pending == 0) return MDG_OK;
   const long long want = h->pending;
   h->pending = 0;
+  struct Confirmed {
+    mdg_handle *h;
+    ~Confirmed() {
+      h->by_graph = 0;
+      mark_outstanding(h, false);
+    }
+  } confirmed{h};
   long long done = 0;
   for (int attempt = 0; attempt < 64 && done < want; attempt++) {
     const unsigned long long before = (unsigned long long)h->steps_host;
@@ -562,9 +604,12 @@ int settle(mdg_handle *h) {
     int rc = read_flags(h);
     if (rc) return rc;
     long long completed = (long long)(h->hflags->steps - before);
-    if (h->prm.use_graphs && !resident(h))
-      h->launches += graph_kernels(h, completed, (long long)(h->hflags->rebuilds - rebuilds0),
+    if (h->by_graph) {  // of steps in both ways, the graphs' share of the rebuilds by their steps
+      const long long rebuilds = (long long)(h->hflags->rebuilds - rebuilds0), graph = std::min(completed, h->by_graph);
+      h->launches += graph_kernels(h, graph, completed > graph ? rebuilds * graph / completed : rebuilds,
                                    (long long)(h->hflags->checks - checks0));
+      h->by_graph -= graph;
+    }
     if (h->hflags->halt == 0) {
       done += completed;
       h->steps_host = (long long)h->hflags->steps;
@@ -597,7 +642,10 @@ int check_handle(mdg_handle *h, bool need_state, Pending pending = kSettle) {
   cudaError_t e = cudaSetDevice(h->prm.device);
   if (e != cudaSuccess) return fail(h, MDG_ERR_CUDA, cudaGetErrorString(e));
   if (pending == kSettle) return settle(h);
-  if (pending == kDrop) h->pending = 0;
+  if (pending == kDrop) {
+    h->pending = h->by_graph = 0;
+    mark_outstanding(h, false);
+  }
   return MDG_OK;
 }
 
@@ -726,6 +774,7 @@ int mdg_destroy(mdg_handle *h) {
   if (!h) return MDG_OK;
   cudaSetDevice(h->prm.device);
   if (h->stream) cudaStreamSynchronize(h->stream);
+  mark_outstanding(h, false);
   drop_graphs(h);
   dfree_all(h);
   if (h->hflags) cudaFreeHost(h->hflags);
@@ -864,6 +913,7 @@ int mdg_calculate(mdg_handle *h, int32_t nsteps) {
   h->ev1_due = nsteps == 1;
   if (!h->ev1_due) MDG_CK(cudaEventRecord(h->ev1, h->stream));
   h->pending += nsteps;
+  mark_outstanding(h, true);
   if (h->pending >= kMaxPending) return settle(h);
   return MDG_OK;
 }

@@ -223,11 +223,12 @@ int launch_observe_fixed(const Geom &g, const Dev &d, int par, int call, cudaStr
 void launch_forces_fixed(const Geom &g, const Dev &d, int par, int call, cudaStream_t s);
 // The steps of a small box in one resident kernel (mdg_resident.cu): whether
 // this box takes it, and the launch of nsteps steps; ctl is zeroed device
-// memory of resident_ctl_bytes() that the launches keep to themselves.
+// memory of resident_ctl_bytes() that the launches keep to themselves; beside:
+// other handles have steps outstanding.
 size_t resident_ctl_bytes();
 bool resident_box(const Geom &g, int precision, int num_sms);
 cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int nsteps, int thermostat, int compat, int precision,
-                            int num_sms, cudaStream_t s);
+                            int num_sms, bool beside, cudaStream_t s);
 void launch_unsort(const Geom &g, const Dev &d, int par, double4_32a *qo, double4_32a *po, cudaStream_t s);
 void launch_sort_in(const Geom &g, const Dev &d, const double4_32a *qi, const double4_32a *pi, cudaStream_t s);
 void launch_pairs(const Geom &g, const Dev &d, const long long *row_off, int32_t *rec, cudaStream_t s);

@@ -38,8 +38,9 @@ namespace {
 
 constexpr int kFixedForm = 3;  // template value beside MDG_MIXED and MDG_MIXED_PLAIN
 
-// Threads of the one block per SM: 512 (128 registers), or for the mixed forms
-// of boxes with more particles than 512 per SM 1024 (64).  With 512 the mixed
+// Threads of a block: 512 (128 registers), or for the mixed forms
+// of boxes with more particles than 512 per SM 1024 (64), and beside other handles'
+// launches 256 (narrow_block).  With 512 or fewer the mixed
 // row walk has kFewUnroll gathers in flight (864 / 16,384 / 70,304 atoms, us
 // per step: 4 10.2 / 13.7 / 18.5, 8 9.2 / 12.7 / 19.2, 16 11.1 / 15.3 / 22.1;
 // 1024 threads 14.3 / 18.9 / 23.8).
@@ -284,7 +285,7 @@ __device__ __forceinline__ double resident_step(const Geom &g, const Dev &d, int
     for (int i = lo + threadIdx.x; i < hi; i += kThreads) {
       int kept = 0;
       const float4 lb = ld_ro<true>(d.loc[par] + i);
-      const double3 F = force_mixed<PRUNE, FORM == MDG_MIXED, true, THREADS == 512 ? kFewUnroll : kUnroll>(g, d, d.loc[par], i, lb, cell_pos_packed(g, lb.w), list,
+      const double3 F = force_mixed<PRUNE, FORM == MDG_MIXED, true, THREADS <= 512 ? kFewUnroll : kUnroll>(g, d, d.loc[par], i, lb, cell_pos_packed(g, lb.w), list,
                                                                     counts, &kept);
       ke += step_one<THERMO, COMPAT, FORM>(g, d, par, i, PRUNE, kept, F, lb, d.q_mid[par], d.q_mid[par ^ 1], exp1, lang, rebuild,
                                            reselect);
@@ -301,7 +302,7 @@ __device__ __forceinline__ double resident_step(const Geom &g, const Dev &d, int
 }
 
 template <int FORM, int THERMO, int COMPAT, int LANES, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1) k_resident(const __grid_constant__ Geom g,
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_resident(const __grid_constant__ Geom g,
                                                                       const __grid_constant__ Dev d, ResidentCtl *c, int par,
                                                                       int nsteps, int share, int row_lanes) {
   constexpr int kThreads = THREADS;
@@ -445,26 +446,26 @@ Kernel kernel_of(int thermostat, int compat) {
 // 108,000 27.1 / 39.3, 157,216 47.1 / 48.1, 256,000 54.9 / 66.7, 389,344 84.9 / 89.7.
 constexpr int kResidentFixed = 512, kResidentMixed = 2048;
 
-// Particles per block at least.  A block of 512 threads has an SM's registers to
-// itself, so launches of several handles run side by side only where they leave
-// SMs over.  In the mixed forms, whose step graphs overlap well, boxes of 16 to 32
-// particles per SM take 64 a block (their lists then by a warp per cell), of more than 40
-// 96: that costs one handle nothing (5,000, between them, would take 1-3 % longer).  us
-// per step of all handles, density 0.6, dt 0.002, one / four / eight, now (with 32 a
-// block; step graphs): 864 9.6 / 9.7 / 16.7 (the same; 30 / 40 / 79), 4,000 9.9 / 19.8 / 39.6
-// (10.2 / 40.7 / 81; 32 / 39 / 78), 7,200 10.3 / 20.8 / 42 (10.9 / 42.5 / 86; 34 / 41 / 82); one
-// handle of 4,000 at dt 0.005 13.8 (14.2).
-// From about 7,300 particles on a launch fills the GPU and handles take turns: 8,000
-// 43.9 / 87 (four, eight; graphs 41 / 83), 32,000 57 / 115 (47 / 93), 108,000 111 / 221 (79 /
-// 158), one handle 10.8, 14.4 and 27.7 (34, 35 and 40): several of those at once step
-// faster by graphs, which is the caller's choice (use_graphs = 2).  Blocks of 256
-// threads, two an SM, made four of 32,000 38, but one handle 2-6 % slower where lists are
-// rebuilt every 15 steps.  FP64 handles side by side are faster than their graphs at
-// every size (four of 32,000 95, 272).
-int rows_per_block(const Geom &g, int precision, int num_sms) {
-  if (precision == MDG_FP64) return 1;
-  if (g.n > 40 * num_sms) return 96;
-  return g.n > 16 * num_sms && g.n <= 32 * num_sms ? 64 : 32;
+// Beside other handles.  A block of 512 threads has an SM's registers to itself
+// and a launch takes nearly every SM, so the launches of several handles run one
+// after the other, where step graphs overlap.  In the mixed forms a call made while
+// other handles have steps outstanding therefore takes, up to 256 particles per SM,
+// a narrow launch: kNarrowRows particles a block (a warp on each sub-partition),
+// which shares the SMs out up to 64 per SM, and above that blocks of 256 threads, two
+// of which fit an SM.  Larger boxes step by graphs where those are faster (crowded in
+// mdg_api.cu).  us per step of all handles, density 0.6, dt 0.002, one / four / eight, now
+// (wide launches only; graphs only): 864 9.5 / 9.9 / 10.1 (9.4 / 9.8 / 16.7; 30 / 40 / 79),
+// 4,000 10.3 / 13.2 / 23.3 (10.2 / 40.7 / 82; 32 / 39 / 78), 16,384 11.4 / 30.5 / 58.7 (11.4 /
+// 43.9 / 90; 34 / 42 / 84), 32,000 14.4 / 40 / 77 (14.3 / 57 / 114; 35 / 47 / 93), 108,000
+// 27.8 / 82 / 155 (27.7 / 111 / 221; 40 / 79 / 158), 300,000 60.8 / 189 / 372 (60.5 / 242 / 482;
+// 78 / 189 / 376).  Not narrow always: fewer threads make the rebuild longer, and one
+// handle 5-14 % slower at dt 0.005 (1,500 13.2 -> 15.2, 16,384 16.4 -> 17.4).  The
+// particles' arithmetic is the same, bit for bit; Nose-Hoover, whose kinetic sum
+// goes by blocks, stays with the wide launch, and FP64 handles side by side are
+// faster than their graphs at every size (four of 32,000 95, 272).
+constexpr int kNarrowRows = 128;
+bool narrow_box(const Geom &g, int thermostat, int precision, int num_sms) {
+  return precision != MDG_FP64 && thermostat != MDG_NOSEHOOVER && g.n <= 256 * num_sms;
 }
 
 size_t resident_ctl_bytes() { return sizeof(ResidentCtl); }
@@ -475,8 +476,9 @@ bool resident_box(const Geom &g, int precision, int num_sms) {
 }
 
 cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int nsteps, int thermostat, int compat, int precision,
-                            int num_sms, cudaStream_t s) {
+                            int num_sms, bool beside, cudaStream_t s) {
   Kernel k;
+  const bool narrow = beside && narrow_box(g, thermostat, precision, num_sms);
   int threads = 512, lanes = 1;
   if (precision == MDG_FP64) {
     // as many lanes as the block has threads for
@@ -488,6 +490,10 @@ cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int
         : lanes == 4  ? kernel_of<kFixedForm, 4, 512>(thermostat, compat)
         : lanes == 2  ? kernel_of<kFixedForm, 2, 512>(thermostat, compat)
                       : kernel_of<kFixedForm, 1, 512>(thermostat, compat);
+  } else if (narrow && 2 * g.n > kNarrowRows * num_sms) {
+    threads = 256;
+    k = precision == MDG_MIXED ? kernel_of<MDG_MIXED, 1, 256>(thermostat, compat)
+                               : kernel_of<MDG_MIXED_PLAIN, 1, 256>(thermostat, compat);
   } else if (g.n <= 512 * num_sms) {
     k = precision == MDG_MIXED ? kernel_of<MDG_MIXED, 1, 512>(thermostat, compat)
                                : kernel_of<MDG_MIXED_PLAIN, 1, 512>(thermostat, compat);
@@ -498,15 +504,14 @@ cudaError_t launch_resident(const Geom &g, const Dev &d, void *ctl, int par, int
   }
   // whole warps of particles per block
   const int unit = 32 / lanes;
-  const int least = rows_per_block(g, precision, num_sms);
   int share = (g.n + num_sms - 1) / num_sms;
-  if (share < least) share = least;
+  if (narrow && share < kNarrowRows) share = kNarrowRows;
   share = (share + unit - 1) / unit * unit;
   int grid = (g.n + share - 1) / share;
   Geom gg = g;
   Dev dd = d;
   ResidentCtl *c = static_cast<ResidentCtl *>(ctl);
-  int row_lanes = least != 64 && lanes_per_row(g.n, (long long)grid * threads) ? 1 : 0;
+  int row_lanes = lanes_per_row(g.n, (long long)grid * threads) ? 1 : 0;
   void *args[] = {&gg, &dd, &c, &par, &nsteps, &share, &row_lanes};
   size_t shared = 0;
   if (!row_lanes) {
