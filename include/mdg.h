@@ -76,7 +76,9 @@ typedef struct mdg_params {
                               one resident launch per call (beside other handles with steps
                               outstanding a narrower one or, in mixed precision from 256
                               particles per SM on, by graphs: the same trajectory);
-                              2 = by graphs whatever the size; 0 = plain launches */
+                              2 = by graphs whatever the size (beside kernels that hold SMs for
+                              long: the resident launch needs all of its own at once); 0 = plain
+                              launches */
   int32_t rebuild_policy;  /* mdg_rebuild_policy (.cfg RebuildPolicy), default HALFMARGIN */
   double prune_buffer;     /* inner-list buffer: the force kernels walk the pairs within
                               cutoff + prune_buffer, re-selected from the list whenever a
