@@ -73,9 +73,9 @@ typedef struct mdg_params {
   int32_t list_capacity;   /* neighbour slots per particle; 0 = sized from the first build */
   int32_t device;          /* CUDA device ordinal */
   int32_t use_graphs;      /* 1 (default) = replay steps as CUDA graphs, those of a small box in
-                              one resident launch per call (beside other handles with steps
-                              outstanding a narrower one or, in mixed precision from 256
-                              particles per SM on, by graphs: the same trajectory);
+                              one resident launch per call (mixed precision beside other handles
+                              with steps outstanding: a narrower launch or, from 256 particles
+                              per SM on, graphs; the same trajectory);
                               2 = by graphs whatever the size (beside kernels that hold SMs for
                               long: the resident launch needs all of its own at once); 0 = plain
                               launches */
